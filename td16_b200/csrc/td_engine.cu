@@ -394,6 +394,10 @@ __device__ __forceinline__ int td_finish_unit(const td_dfs_out &r, td_inst_state
         if (found == 1) td_write_result(out, TD_FOUND, 0, 0, path, exp, 7, 8);
         else td_write_result(out, found == 2 || !err ? TD_NOT_FOUND : err, 0, 0, path, exp, 0, 8);
         __syncwarp();
+        // the caller stamps the record as done: the host must see the record
+        // (written by lanes 0..7) before the stamp, or it reads the ring
+        // slot's record of an earlier request
+        if (HOST_OUT && lane == 0) __threadfence_system();
     }
     return last;
 }

@@ -182,3 +182,18 @@ def test_idle_server_exits_and_restarts(slots):
         time.sleep(0.01)
         moves = td.search(i % SLOTS, beta[i].tobytes(), omega[i].tobytes(), int(init[i]), 0.0, 9)
         assert 1 <= len(moves) <= 9
+
+
+def test_per_call_verdicts_after_the_ring_wraps(slots, oracle):
+    """80,000 calls through the per-call server's ring of 65,536 requests,
+    some without a witness: once a ring slot is used again, a "not
+    found" must not be read as the slot's earlier record."""
+    td = slots
+    perms, n = td.synth_perms(21, 8000, 5, 9, 50, 1, 3)
+    beta, omega, init, N = _pairs(oracle, perms, n)
+    maxd = np.maximum(1, (N - init + 1) // 2).astype(np.int32)  # the cycle-graph lower bound
+    st, _, _, _ = _oracle(oracle, beta, omega, N, init, maxd)
+    assert (st == 0).sum() > 1000
+    for _ in range(10):
+        r = _run(td, "td_search", beta, omega, N, init, maxd)
+        assert (r["status"] == st).all(), np.nonzero(r["status"] != st)[0][:10]
