@@ -53,25 +53,8 @@ static_assert(sizeof(td_result) == 32, "td_result layout");
 // kernels
 // ============================================================================
 
-#define TD_LUT_BYTES 4096
 #define TD_TT_BITS 12  // default: 4096 explored-state entries (32 KiB) per warp of a free-order launch
 #define TD_RESTART_BASE 16  // default base of the free order's restart budgets (expansions)
-
-// Class table (td_class_of_index for every 12-bit index), filled by the host.
-__device__ __align__(16) uint8_t td_lut_global[TD_LUT_BYTES];
-
-// Copies the class table into shared memory (kernels of the reference order;
-// `lut` is null in the free-order batch kernel, which does not use it).
-__device__ __forceinline__ void td_block_init(uint8_t *lut, td_warp_smem *ws, int warps) {
-    if (lut) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(td_lut_global);
-        uint4 *dst = reinterpret_cast<uint4 *>(lut);
-        for (int i = threadIdx.x; i < TD_LUT_BYTES / 16; i += blockDim.x) dst[i] = src[i];
-    }
-    for (int w = 0; w < warps; ++w)
-        for (int b = threadIdx.x; b < TD_PT_STRIDE; b += blockDim.x) ws[w].pt[TD_PT_DUMMY + b] = 0;
-    __syncthreads();
-}
 
 __device__ __forceinline__ td_search_limits td_make_limits(uint64_t max_exp, uint64_t time_limit_ns,
                                                            const int *abort_flag) {
@@ -94,32 +77,28 @@ __global__ void __launch_bounds__(256) td_plain_kernel(const td_instance *__rest
                                                       uint64_t max_exp, uint64_t time_limit_ns) {
     extern __shared__ __align__(16) uint8_t td_smem[];
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5;
-    uint8_t *lut = td_smem;
-    td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem + TD_LUT_BYTES);
-    td_block_init(lut, ws, warps);
+    td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
     const int idx = blockIdx.x * warps + warp;
     if (idx >= count) return;
     const td_search_limits lim = td_make_limits(max_exp, time_limit_ns, nullptr);
-    uint32_t code[TD_MAX_STEPS];
+    td_codes code;
     int codeN = -1;
     const td_instance x = in[idx];
-    td_warp_search<ORDERED>(x, &out[idx], ws[warp], lut, code, codeN, lim);
+    td_warp_search<ORDERED>(x, &out[idx], ws[warp], code, codeN, lim);
 }
 
 // hard_count / hard_list (or null): instances that end with TD_ERR_BUDGET are
 // listed there, for the split pass of the reference order (td_split_*).
 template <bool ORDERED>
-__global__ void __launch_bounds__(256) td_persistent_kernel(const td_instance *__restrict__ in,
+__global__ void __launch_bounds__(256, 4) td_persistent_kernel(const td_instance *__restrict__ in,
                                                            td_result *__restrict__ out, int count,
                                                            int *ticket, int grain, uint64_t max_exp,
                                                            uint64_t time_limit_ns, int *hard_count = nullptr,
                                                            int *hard_list = nullptr) {
     extern __shared__ __align__(16) uint8_t td_smem[];
-    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint8_t *lut = td_smem;
-    td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem + TD_LUT_BYTES);
-    td_block_init(lut, ws, warps);
-    uint32_t code[TD_MAX_STEPS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
+    td_codes code;
     int codeN = -1;
     const td_search_limits lim = td_make_limits(max_exp, time_limit_ns, nullptr);
     for (;;) {
@@ -130,7 +109,7 @@ __global__ void __launch_bounds__(256) td_persistent_kernel(const td_instance *_
         const int last = min(count, first + grain);
         for (int idx = first; idx < last; ++idx) {
             const td_instance x = in[idx];
-            const int st = td_warp_search<ORDERED>(x, &out[idx], ws[warp], lut, code, codeN, lim);
+            const int st = td_warp_search<ORDERED>(x, &out[idx], ws[warp], code, codeN, lim);
             if (hard_list && st == TD_ERR_BUDGET && lane == 0) hard_list[atomicAdd(hard_count, 1)] = idx;
         }
     }
@@ -180,40 +159,42 @@ __global__ void __launch_bounds__(256) td_split_roots_kernel(const td_instance *
                                                             int records) {
     extern __shared__ __align__(16) uint8_t td_smem[];
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint8_t *lut = td_smem;
-    td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem + TD_LUT_BYTES);
-    td_block_init(lut, ws, warps);
+    td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
     td_warp_smem &s = ws[warp];
     const int H = *(volatile int *)&ctl->hard;
-    uint32_t code[TD_MAX_STEPS];
+    td_codes code;
     int codeN = -1;
     for (int h = blockIdx.x * warps + warp; h < H; h += gridDim.x * warps) {
         const td_instance x = in[hard_list[h]];
-        td_setup_root<true>(s, x, code, codeN);
-        const int N = x.n_symbols, T = td_triple_count(N), tb = td_tri_base(N);
-        // count the children, reserve their records, then list them (the
-        // walk consumes the root's outcome words, so the root is evaluated twice)
-        int c = 0, at = -1;
-        for (int pass = 0; pass < 2; ++pass) {
-            if (pass == 1 && at < 0) break;
-            const int odd = td_prepare_node(s, s.L[0], s.off[0], N);
-            td_evaluate(s, lut, code, (T + 31) >> 5, 0, odd, x.max_moves);
-            int k = 0;
-            for (;;) {
-                int accepted;
-                const int u = td_next_child(s, 0, &accepted);
-                if (u < 0) break;
-                if (pass == 1 && lane == 0)
-                    kids[at + k] = (uint16_t)(td_tri_table[tb + T - 1 - u] | (accepted ? 0x8000u : 0u));
-                ++k;
-            }
-            if (pass == 0) {
-                c = k;
-                if (lane == 0) {
-                    at = atomicAdd(&ctl->items_used, c);
-                    if (at > records - c) at = -1;
-                }
-                at = __shfl_sync(TD_FULL, at, 0);
+        td_setup_root(s, x, code, codeN);
+        const int N = x.n_symbols, last_tri = td_tri_base(N) + td_triple_count(N) - 1;
+        td_unpack_state(s, 0, x.perm, x.offset, N);
+        uint32_t O, F;
+        const int odd = td_prepare_rows(s, 0, N, O, F);
+        td_evaluate(s, code, N, 0, odd, O, F);
+        // count the children, reserve their records, then list them from the
+        // last one (the root's visiting order is descending u)
+        const uint32_t w = lane < TD_MAX_STEPS ? s.cw[0][lane] : 0u;
+        const uint32_t fw = lane < TD_MAX_STEPS ? s.root_found[lane] : 0u;
+        int from = __popc(w);  // children in this lane's word and those after it
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_down_sync(TD_FULL, from, o);
+            if (lane + o < 32) from += v;
+        }
+        const int c = __shfl_sync(TD_FULL, from, 0);
+        int at = -1;
+        if (lane == 0) {
+            at = atomicAdd(&ctl->items_used, c);
+            if (at > records - c) at = -1;
+        }
+        at = __shfl_sync(TD_FULL, at, 0);
+        if (at >= 0) {
+            int k = at + from - __popc(w);
+            for (uint32_t rest = w; rest; ++k) {
+                const int bit = 31 - __clz(rest);
+                rest &= ~(1u << bit);
+                kids[k] = (uint16_t)(td_tri_table[last_tri - 32 * lane - bit] | (((fw >> bit) & 1u) << 15));
             }
         }
         if (lane == 0) {
@@ -230,23 +211,21 @@ __global__ void __launch_bounds__(256) td_split_roots_kernel(const td_instance *
 // r = u / H of listed instance h = u % H, i.e. subtree r of its root, or for
 // an instance without records (nkids[h] < 0) the whole search at r = 0 (so
 // the longest units start first).
-__global__ void __launch_bounds__(256) td_split_kernel(const td_instance *__restrict__ in,
+__global__ void __launch_bounds__(256, 4) td_split_kernel(const td_instance *__restrict__ in,
                                                       td_result *__restrict__ out, const int *__restrict__ hard_list,
                                                       td_split_ctl *ctl, const uint16_t *__restrict__ kids,
                                                       const int *__restrict__ base, const int *__restrict__ nkids,
                                                       int *cutoff, td_result *__restrict__ items,
                                                       uint64_t time_limit_ns) {
     extern __shared__ __align__(16) uint8_t td_smem[];
-    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint8_t *lut = td_smem;
-    td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem + TD_LUT_BYTES);
-    td_block_init(lut, ws, warps);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
     td_warp_smem &s = ws[warp];
     const int H = *(volatile int *)&ctl->hard;
     const int R = max(1, *(volatile int *)&ctl->max_rank);
     const unsigned long long units = (unsigned long long)H * (unsigned long long)R;
     td_search_limits lim = td_make_limits(0, time_limit_ns, nullptr);
-    uint32_t code[TD_MAX_STEPS];
+    td_codes code;
     int codeN = -1;
     for (;;) {
         unsigned long long u = 0;
@@ -259,7 +238,7 @@ __global__ void __launch_bounds__(256) td_split_kernel(const td_instance *__rest
             if (r == 0) {
                 const int idx = hard_list[h];
                 lim.cutoff = nullptr;
-                td_warp_search<true>(in[idx], &out[idx], s, lut, code, codeN, lim);
+                td_warp_search<true>(in[idx], &out[idx], s, code, codeN, lim);
             }
             continue;
         }
@@ -272,7 +251,7 @@ __global__ void __launch_bounds__(256) td_split_kernel(const td_instance *__rest
         const uint32_t kid = kids[base[h] + r];
         const uint32_t t = kid & 0x7fffu;
         const td_instance x = in[hard_list[h]];
-        td_setup_root<true>(s, x, code, codeN);
+        td_setup_root(s, x, code, codeN);
         const int N = x.n_symbols;
         if (lane == 0) s.path[0] = (uint16_t)t;
         __syncwarp();
@@ -291,7 +270,7 @@ __global__ void __launch_bounds__(256) td_split_kernel(const td_instance *__rest
         __syncwarp();
         lim.cutoff = &cutoff[h];
         lim.rank = r;
-        const td_dfs_out d = td_dfs<true>(s, lut, code, N, x.max_moves, 1, lim, nullptr);
+        const td_dfs_out d = td_dfs<true>(s, code, N, 1, lim, nullptr);
         int status = TD_NOT_FOUND;
         if (d.status == TD_DFS_FOUND) status = TD_FOUND;
         else if (d.status == TD_DFS_ABORTED) status = TD_SPLIT_SKIPPED;
@@ -415,12 +394,9 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                                                       unsigned max_backoff_ns, int race, int spawn_base) {
     extern __shared__ __align__(16) uint8_t td_smem[];
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // free order only: no class table, the warp frames start the block's shared memory
-    const uint8_t *lut = nullptr;
     td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
-    td_block_init(nullptr, ws, warps);
     td_warp_smem &s = ws[warp];
-    uint32_t code[TD_MAX_STEPS];
+    td_codes code;
     int codeN = -1;
     // the expansion budget bounds each unit (the root search and each donated
     // subtree); an instance without a witness whose unit ran out reports
@@ -541,12 +517,12 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                 td_write_result(&out[unit], td_instance_ok(x) ? TD_NOT_FOUND : TD_ERR_ARG, 0, 0, s.path, 0, 0, 8);
             } else {
                 if (lane == 0) atomicAdd(&st->pending, 1);
-                td_setup_root<false>(s, x, code, codeN);
+                td_setup_root(s, x, code, codeN);
                 dc.inst = (uint32_t)unit;
                 dc.state = st;
                 dc.side = 0;
                 dc.race = td_inst_full(x) ? race : 0;
-                const td_dfs_out r = td_dfs<false>(s, lut, code, x.n_symbols, x.max_moves, 0, lim, &dc);
+                const td_dfs_out r = td_dfs<false>(s, code, x.n_symbols, 0, lim, &dc);
                 dc.race = 0;
                 td_finish_unit<false>(r, st, &out[unit], s.path);
             }
@@ -587,7 +563,7 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                 }
                 const td_instance x = in[idx];
                 td_inst_state *st = &state[idx];
-                td_setup_root<false>(s, x, code, codeN);
+                td_setup_root(s, x, code, codeN);
                 if (lane == 0) {
                     s.L[d0] = it.L;
                     s.off[d0] = it.off;
@@ -612,7 +588,7 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                     dc.inst = idx;
                     dc.state = st;
                     dc.side = side;
-                    r = td_dfs<false>(s, lut, code, x.n_symbols, x.max_moves, d0, ilim, &dc);
+                    r = td_dfs<false>(s, code, x.n_symbols, d0, ilim, &dc);
                     dc.side = 0;
                     // a witness of the inverse becomes one of the instance; one that
                     // does not convert is reported as a failed replay, and one that
@@ -842,9 +818,7 @@ std::string cuda_msg(cudaError_t e, const char *file, int line) {
         }                                                                \
     } while (0)
 
-size_t smem_bytes(int warps) { return TD_LUT_BYTES + (size_t)warps * sizeof(td_warp_smem); }
-// td_steal_kernel keeps no class table
-size_t steal_smem_bytes(int warps) { return (size_t)warps * sizeof(td_warp_smem); }
+size_t smem_bytes(int warps) { return (size_t)warps * sizeof(td_warp_smem); }
 
 std::atomic<uint64_t> g_time_limit_ns{0};
 
@@ -899,7 +873,7 @@ int launch_cfg(int device, LaunchCfg *c, char *err, size_t errlen) {
     if (d.steal_blocks_per_sm == 0) {
         int b = 0;
         TD_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, td_steal_kernel, threads,
-                                                               steal_smem_bytes(c->warps)));
+                                                               smem_bytes(c->warps)));
         d.steal_blocks_per_sm = std::max(1, b);
     }
     if (d.blocks_per_sm == 0) {
@@ -927,9 +901,6 @@ int ensure_device(int device, char *err, size_t errlen) {
                 for (int k = j + 1; k < N; ++k) tri[base + t++] = td_pack_move(i, j, k);
     }
     TD_CHECK(cudaMemcpyToSymbol(td_tri_table, tri.data(), tri.size() * sizeof(uint16_t)));
-    std::vector<uint8_t> lut(TD_LUT_BYTES);
-    for (int i = 0; i < TD_LUT_BYTES; ++i) lut[i] = (uint8_t)td_class_of_index(i);
-    TD_CHECK(cudaMemcpyToSymbol(td_lut_global, lut.data(), lut.size()));
     TD_CHECK(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device));
     const int max_warps = 8;
     const size_t max_smem = smem_bytes(max_warps);
@@ -1060,7 +1031,7 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
         // at the top of the item space, which keeps at least half for donation
         const int race = cfg.restart_base > 0 && max_exp == 0 && count <= s.item_capacity / 2 ? cfg.race : 0;
         const int spawn_base = race ? s.item_capacity - count : s.item_capacity;
-        td_steal_kernel<<<grid, threads, steal_smem_bytes(warps), stream>>>(
+        td_steal_kernel<<<grid, threads, smem_bytes(warps), stream>>>(
             d_in, d_out, count, s.d_pool, s.d_items, s.d_ready, s.d_epoch, s.item_capacity, s.d_state,
             cfg.steal_grain, cfg.split_level, cfg.check_every, time_limit_ns(), cfg.tt_bits > 0 ? s.d_tt : nullptr,
             s.d_tt_gen, cfg.tt_bits, cfg.restart_base, max_exp, count == 1 ? 4096u : 32768u, race, spawn_base);
@@ -1842,11 +1813,10 @@ struct NoAllocDevice {
 
 std::mutex g_noalloc_mu;
 NoAllocDevice g_noalloc[kNoAllocDevices];
-uint16_t g_noalloc_tri[TD_TRI_TABLE];  // host copies of the device tables, no heap
-uint8_t g_noalloc_lut[TD_LUT_BYTES];
+uint16_t g_noalloc_tri[TD_TRI_TABLE];  // host copy of the device table, no heap
 
-// Once per device, with that device current: uploads the triple and class
-// tables and takes the scratch array's device address.  In host code the
+// Once per device, with that device current: uploads the triple
+// table and takes the scratch array's device address.  In host code the
 // name td_noalloc_scratch is only a host-side stand-in, never a device address.
 int noalloc_setup(int device, char *err, size_t errlen) {
     NoAllocDevice &d = g_noalloc[device];
@@ -1858,9 +1828,7 @@ int noalloc_setup(int device, char *err, size_t errlen) {
             for (int j = i + 1; j < N - 1; ++j)
                 for (int k = j + 1; k < N; ++k) g_noalloc_tri[base + t++] = td_pack_move(i, j, k);
     }
-    for (int i = 0; i < TD_LUT_BYTES; ++i) g_noalloc_lut[i] = (uint8_t)td_class_of_index(i);
     TD_CHECK_NA(cudaMemcpyToSymbol(td_tri_table, g_noalloc_tri, sizeof g_noalloc_tri));
-    TD_CHECK_NA(cudaMemcpyToSymbol(td_lut_global, g_noalloc_lut, sizeof g_noalloc_lut));
     void *ptr = nullptr;
     TD_CHECK_NA(cudaGetSymbolAddress(&ptr, td_noalloc_scratch));
     TD_CHECK_NA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device));
@@ -1870,9 +1838,9 @@ int noalloc_setup(int device, char *err, size_t errlen) {
     TD_CHECK_NA(cudaFuncSetAttribute(td_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
     TD_CHECK_NA(cudaFuncSetAttribute(td_steal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)steal_smem_bytes(4)));
+                                     (int)smem_bytes(4)));
     TD_CHECK_NA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.steal_blocks, td_steal_kernel, 128,
-                                                              steal_smem_bytes(4)));
+                                                              smem_bytes(4)));
     TD_CHECK_NA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.persistent_blocks, td_persistent_kernel<true>,
                                                               128, smem));
     d.scratch = static_cast<uint8_t *>(ptr);
@@ -1951,7 +1919,7 @@ TD_API int td_search_batch_noalloc(int count, const td_instance *d_instances, td
         // small batch is spread over the GPU; a single search wakes its
         // waiting warps sooner (backoff cap 4 us instead of 32 us)
         const int grid = d.sms * std::max(1, d.steal_blocks);
-        td_steal_kernel<<<grid, threads, steal_smem_bytes(warps), st>>>(
+        td_steal_kernel<<<grid, threads, smem_bytes(warps), st>>>(
             d_instances, d_results, count, pool, items, ready, epoch, TD_NOALLOC_ITEMS, state, grain, split_level,
             check_every, limit, nullptr, nullptr, 0, restart_base, max_exp, count == 1 ? 4096u : 32768u,
             /*race=*/0, /*spawn_base=*/TD_NOALLOC_ITEMS);

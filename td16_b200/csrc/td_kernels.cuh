@@ -1,23 +1,21 @@
 // td_kernels.cuh -- the sm_100a witness-search warp engine.
 //
 // One warp owns one search (a DFS over move sequences), or one donated
-// subtree of it.  Two node evaluations share the DFS:
+// subtree of it.  The state of a level is the caller's array, one byte per
+// position.  Per node the warp labels the omega cycles by pointer jumping
+// (lane c = caller position c) and builds cycle row masks, and each lane then
+// classifies the children (i, j, k) of its pair slots for every k at once with
+// LOP3 logic (td_prepare_rows, td_row_classes).  The two move orders differ in
+// how the children are kept and picked:
 //
-// Reference order (td_prepare_node, td_evaluate, td_next_child): per node the
-// warp labels the omega cycles of the pinned state by pointer jumping (lane p
-// = pinned position p), writes the pair table (4 bits per ordered pair of
-// caller positions), and evaluates every triple: lane l takes u = 32*s + l in
-// step s, reads three pair entries and one class-table byte, and keeps one bit
-// per step in per-lane masks.  The next child comes from a warp max-reduction
-// in the reference's single-queue order.
+// Reference order (td_evaluate, td_next_child): one bit per child at its
+// position u in the reference's single-queue order, 22 words of 32 per level.
+// The next child comes from one ballot over the words.
 //
-// Free order (td_prepare_rows, td_evaluate_rows, td_next_child_rows): the
-// state is the caller's array, one byte per position; per node the warp builds
-// cycle row masks (one per caller position), and each lane classifies all the
-// children (i, j, k) of its pair slots at once with LOP3 logic
-// (td_row_classes).  The next child, +2 moves first, comes from per-level lane
-// summaries.  A table of explored states skips children reached before by
-// another move order, and busy warps donate subtrees to idle ones.
+// Free order (td_evaluate_rows, td_next_child_rows): each lane keeps the
+// children of its pair slots.  The next child, +2 moves first, comes from
+// per-level lane summaries.  A table of explored states skips children reached
+// before by another move order, and busy warps donate subtrees to idle ones.
 //
 // Reference: emitter/src/native/backtracking/sorting_search.cu:478-712.
 #pragma once
@@ -25,48 +23,36 @@
 #include "td_core.cuh"
 
 #define TD_FULL 0xffffffffu
-#define TD_PT_ROWS 18          // 17 position rows + one zero row for idle lanes
-#define TD_PT_DUMMY (17 * TD_PT_STRIDE)
 #define TD_TRI_TABLE 3060      // sum over N <= 17 of C(N,3) = C(18,4)
-#define TD_G0 0x09249249u      // bit 0 of each 3-bit group
-#define TD_G1 0x12492492u      // bit 1 of each group
-
-// floor(b / 3) for 0 <= b <= 29: the step of a bit inside a packed word
-__device__ __forceinline__ int td_group_of(int b) { return (b * 11) >> 5; }
 
 // Per-warp shared state.
 struct td_warp_smem {
+    // per caller position c: the row masks S, G, P and H (positions after c),
+    // and the odd-cycle / fixed-point flags as full masks
+    uint4 rows[TD_MAX_N];
+    uint2 flg[TD_MAX_N];
     union {
-        struct {  // reference move order (one triple per lane and step)
-            uint8_t pt[TD_PT_ROWS * TD_PT_STRIDE];     // pair table of the current node
-            // per level, per lane: the outcome of every step in 3-bit groups, ten
-            // steps per word (step st in word st/10 at bit 3*(st%10)): bit 0 found
-            // (or, at the root level, accepted when visited), bit 1 a child to visit
-            uint32_t pm[TD_MAX_DEPTH][3][32];
+        struct {  // reference move order
+            // per level: bit u % 32 of word u / 32 is child u still to visit
+            uint32_t cw[TD_MAX_DEPTH][TD_MAX_STEPS];
+            uint32_t root_found[TD_MAX_STEPS];  // the root's children accepted when visited
         };
-        struct {  // free move order (bit-sliced: one pair and all its k per lane and round)
-            // per caller position c: the row masks S, G, P and H (positions
-            // after c), and the odd-cycle / fixed-point flags as full masks
-            uint4 rows[TD_MAX_N];
-            uint2 flg[TD_MAX_N];
+        struct {  // free move order
             // per level and lane: the expandable children of the lane's four
             // pair slots (word r = slot R*lane + r), +2 class at bits k-1
             // (1..15), 0 class at bits k+15 (17..31)
             uint4 pw[TD_MAX_DEPTH][32];
             uint32_t m2[TD_MAX_DEPTH];                 // per level: lanes that hold +2 children
             uint32_t m0[TD_MAX_DEPTH];                 // per level: lanes that hold 0 children
-            // per level: the caller's array, one pinned label per caller position
-            uint8_t A[TD_MAX_DEPTH + 1][32];
-            uint8_t inv[32];                           // caller position of each label
         };
     };
-    uint64_t L[TD_MAX_DEPTH + 1];              // pinned state per level
+    uint64_t L[TD_MAX_DEPTH + 1];              // pinned state where a search or subtree starts
     uint32_t acc[TD_MAX_DEPTH + 2];            // accept mask over odd counts, per depth
     uint32_t reach[TD_MAX_DEPTH + 2];          // prune mask over odd counts, per depth
     uint16_t path[TD_MAX_DEPTH];               // caller-position move per level
     uint8_t off[TD_MAX_DEPTH + 1];
-    alignas(16) uint8_t lead[32];              // cycle leader by caller position
-    alignas(16) uint8_t dist[32];              // omega steps to the leader
+    uint8_t A[TD_MAX_DEPTH + 1][32];           // per level: the caller's array, one pinned label per position
+    uint8_t inv[32];                           // caller position of each label
 };
 
 // Lexicographic position triples i|j<<5|k<<10 for every N, at offset C(N,4).
@@ -74,108 +60,6 @@ __device__ uint16_t td_tri_table[TD_TRI_TABLE];
 
 TD_HD int td_tri_base(int N) {
     return N < 4 ? 0 : N * (N - 1) * (N - 2) * (N - 3) / 24;
-}
-
-// Load this lane's per-step pair-table offsets for triples of size N.
-__device__ __forceinline__ void td_load_codes(int N, uint32_t (&code)[TD_MAX_STEPS]) {
-    const int lane = threadIdx.x & 31;
-    const int T = td_triple_count(N);
-    const int base = td_tri_base(N);
-#pragma unroll
-    for (int s = 0; s < TD_MAX_STEPS; ++s) {
-        const int u = 32 * s + lane;
-        uint32_t c = TD_PT_DUMMY | (TD_PT_DUMMY << 10) | (TD_PT_DUMMY << 20);
-        if (u < T) {
-            const uint32_t t = td_tri_table[base + T - 1 - u];
-            const uint32_t i = t & 31, j = (t >> 5) & 31, k = (t >> 10) & 31;
-            c = (i * TD_PT_STRIDE + j) | ((j * TD_PT_STRIDE + k) << 10) | ((k * TD_PT_STRIDE + i) << 20);
-        }
-        code[s] = c;
-    }
-}
-
-// Cycle labels and pair table for the state (L, off); returns the number of
-// odd-length omega cycles.
-__device__ __forceinline__ int td_prepare_node(td_warp_smem &s, uint64_t L, int off, int N) {
-    const int p = threadIdx.x & 31;
-    const bool act = p < N;
-    const uint32_t Bp = (p == 0 || !act) ? 0u : td_nib(L, p - 1) + 1u;
-    // inverse of L by a warp OR of one nibble per lane
-    uint32_t lo = 0, hi = 0;
-    if (p < N - 1) {
-        const uint64_t c = (uint64_t)p << (4 * td_nib(L, p));
-        lo = (uint32_t)c;
-        hi = (uint32_t)(c >> 32);
-    }
-    lo = __reduce_or_sync(TD_FULL, lo);
-    hi = __reduce_or_sync(TD_FULL, hi);
-    const uint64_t inv = ((uint64_t)hi << 32) | lo;
-    // omega(B[p]) = B[p-1] + 1 (mod N): next position along omega
-    const uint32_t Bq = __shfl_sync(TD_FULL, Bp, p == 0 ? N - 1 : p - 1);
-    uint32_t y = Bq + 1;
-    if (y == (uint32_t)N) y = 0;
-    const int nx = act ? (y ? (int)td_nib(inv, (int)y - 1) + 1 : 0) : p;
-    // leader = smallest position on the cycle and dist = omega steps to it,
-    // in one pointer-jumping pass: each lane keeps the minimum of the window
-    // p, next(p), ..., next^(w-1)(p) and its distance; windows double per round
-    // and 32 >= any cycle length, so the first occurrence of the minimum wins.
-    int m = p, d = 0, j = nx;
-#pragma unroll
-    for (int r = 0; r < 5; ++r) {
-        const int mB = __shfl_sync(TD_FULL, m, j);
-        const int dB = __shfl_sync(TD_FULL, d, j);
-        const int jB = __shfl_sync(TD_FULL, j, j);
-        if (mB < m) {
-            m = mB;
-            d = (1 << r) + dB;
-        }
-        j = jB;
-    }
-    const bool leader = m == p;
-    const int after_leader = __shfl_sync(TD_FULL, nx, m);
-    const int len = __shfl_sync(TD_FULL, d, after_leader) + 1;
-    const int odd = __popc(__ballot_sync(TD_FULL, act && leader && (len & 1)));
-    // descriptors by caller position, one byte each
-    int rp = p - off;
-    rp += rp < 0 ? N : 0;
-    if (act) {
-        s.lead[rp] = (uint8_t)m;
-        s.dist[rp] = (uint8_t)d;
-    }
-    __syncwarp();
-    // pair table row of this lane's caller position, four entries per word
-    // (byte-SIMD: every byte stays below 0x80, so no borrow crosses a byte)
-    const uint32_t H = 0x80808080u, ONE = 0x01010101u;
-    const uint32_t Mp = (uint32_t)m * ONE, Dp = (uint32_t)d * ONE;
-    const uint32_t O8 = (len & 1) ? 0x08080808u : 0u;
-    const uint32_t F4 = len == 1 ? 0x04040404u : 0u;
-    const uint32_t Lodd = (len & 1) ? ONE : 0u;
-    const uint4 ml = *reinterpret_cast<const uint4 *>(s.lead);
-    const uint4 dl = *reinterpret_cast<const uint4 *>(s.dist);
-    const uint32_t m4 = *reinterpret_cast<const uint32_t *>(s.lead + 16);
-    const uint32_t d4 = *reinterpret_cast<const uint32_t *>(s.dist + 16);
-    const uint32_t Mw[5] = {ml.x, ml.y, ml.z, ml.w, m4};
-    const uint32_t Dw[5] = {dl.x, dl.y, dl.z, dl.w, d4};
-    uint32_t row[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        const uint32_t xm = (Mw[k] ^ Mp) | H;
-        const uint32_t same = ~(xm - ONE) & H;                          // 0x80 where leaders match
-        const uint32_t gt = ((Dp | H) - Dw[k] - ONE) & H;               // 0x80 where dist_p > dist_q
-        const uint32_t G = gt >> 7;
-        uint32_t P = (Dp ^ Dw[k]) & ONE;                                // parity of the dist difference
-        P ^= (G ^ ONE) & Lodd;                                          // wrap of an odd cycle flips it
-        const uint32_t sel = (same << 1) - (same >> 7);                 // 0xff in bytes with the same leader
-        const uint32_t in_cycle = ONE | (P << 1) | (G << 2) | O8;
-        const uint32_t apart = F4 | O8;
-        row[k] = (in_cycle & sel) | (apart & ~sel);
-    }
-    if (act) {
-        uint32_t *dst = reinterpret_cast<uint32_t *>(&s.pt[rp * TD_PT_STRIDE]);
-        *reinterpret_cast<uint4 *>(dst) = make_uint4(row[0], row[1], row[2], row[3]);
-        dst[4] = row[4];
-    }
-    return odd;
 }
 
 // Accept / prune masks of one instance: lane D computes the masks of depth D
@@ -226,85 +110,7 @@ __device__ __forceinline__ uint64_t td_globaltimer() {
     return t;
 }
 
-// Reference order: evaluate all children of the node at `level`.  Fills the
-// level's packed outcome words and returns the found child's u, or -1.
-__device__ __forceinline__ int td_evaluate(td_warp_smem &s, const uint8_t *lut,
-                                           const uint32_t (&code)[TD_MAX_STEPS], int steps,
-                                           int level, int odd, int maxd) {
-    const int lane = threadIdx.x & 31;
-    const int D = level + 1;
-    const uint32_t accD = s.acc[D], reachD = s.reach[D];
-    const uint32_t f0 = (accD >> odd) & 1u, f2 = (accD >> (odd + 2)) & 1u;
-    const uint32_t x0 = ((reachD >> odd) & 1u) & (f0 ^ 1u);
-    const uint32_t x2 = ((reachD >> (odd + 2)) & 1u) & (f2 ^ 1u);
-    // byte c of nt holds the flags of class c; byte 0 (filtered out) is zero
-    const uint32_t flags0 = f0 | (x0 << 1);
-    const uint32_t flags2 = f2 | (x2 << 1);
-    const uint32_t nt = (flags0 << (8 * TD_CLASS_ZERO)) | (flags2 << (8 * TD_CLASS_PLUS2));
-    (void)maxd;
-    __syncwarp();
-    uint32_t P0 = 0, P1 = 0, P2 = 0;
-#pragma unroll
-    for (int st = 0; st < TD_MAX_STEPS; ++st) {
-        if (st < steps) {
-            const uint32_t c = code[st];
-            const uint32_t A = s.pt[c & 1023u];
-            const uint32_t B = s.pt[(c >> 10) & 1023u];
-            const uint32_t C = s.pt[c >> 20];
-            const uint32_t cls = lut[A | (B << 4) | (C << 8)];
-            const uint32_t tb = __byte_perm(nt, 0, cls);  // flags of this child's class
-            const uint32_t mul = 1u << (3 * (st % 10));
-            if (st < 10) P0 += tb * mul;
-            else if (st < 20) P1 += tb * mul;
-            else P2 += tb * mul;
-        }
-    }
-    s.pm[level][0][lane] = P0;
-    s.pm[level][1][lane] = P1;
-    s.pm[level][2][lane] = P2;
-    if (level == 0) return -1;  // roots are accepted on visit, not on seeding
-    const uint32_t q0 = P0 & TD_G0, q1 = P1 & TD_G0, q2 = P2 & TD_G0;
-    if (__any_sync(TD_FULL, (q0 | q1 | q2) != 0)) {
-        int st = -1;
-        if (q0) st = td_group_of(__ffs(q0) - 1);
-        else if (q1) st = 10 + td_group_of(__ffs(q1) - 1);
-        else if (q2) st = 20 + td_group_of(__ffs(q2) - 1);
-        const uint32_t key = st >= 0 ? ((uint32_t)st << 5) | (uint32_t)lane : 0xffffffffu;
-        return (int)__reduce_min_sync(TD_FULL, key);
-    }
-    return -1;
-}
-
-// Reference order: next child of `level`; returns u or -1.  *accepted is set
-// for a root that is accepted when visited.
-__device__ __forceinline__ int td_next_child(td_warp_smem &s, int level, int *accepted) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t P0 = s.pm[level][0][lane], P1 = s.pm[level][1][lane], P2 = s.pm[level][2][lane];
-    const bool desc_lanes = level > 0;
-    const uint32_t cm = level == 0 ? (TD_G0 | TD_G1) : TD_G1;
-    const uint32_t w0 = P0 & cm, w1 = P1 & cm, w2 = P2 & cm;
-    int st = -1;
-    if (w2) st = 20 + td_group_of(31 - __clz(w2));
-    else if (w1) st = 10 + td_group_of(31 - __clz(w1));
-    else if (w0) st = td_group_of(31 - __clz(w0));
-    uint32_t key = 0;
-    if (st >= 0) key = ((uint32_t)st << 5) + (uint32_t)(desc_lanes ? 31 - lane : lane) + 1u;
-    key = __reduce_max_sync(TD_FULL, key);
-    *accepted = 0;
-    if (key == 0) return -1;
-    key -= 1;
-    st = (int)(key >> 5);
-    const int win = desc_lanes ? 31 - (int)(key & 31) : (int)(key & 31);
-    const int k = st < 10 ? 0 : (st < 20 ? 1 : 2);
-    const int j = st - 10 * k;
-    const uint32_t Pk = k == 0 ? P0 : (k == 1 ? P1 : P2);
-    if (level == 0) *accepted = __shfl_sync(TD_FULL, (int)((Pk >> (3 * j)) & 1u), win);
-    if (lane == win) s.pm[level][k][lane] = Pk & ~(7u << (3 * j));
-    __syncwarp();
-    return st * 32 + win;
-}
-
-// ---- free move order: bit-sliced evaluation ---------------------------------
+// ---- node evaluation, bit-sliced ---------------------------------------------
 //
 // The state of a level is the caller's array, one byte per caller position
 // holding the pinned label (A[c] = B[(c + off) mod N]).  In these terms omega
@@ -320,14 +126,20 @@ __device__ __forceinline__ int td_pair_rounds(int N) {
     return (NP + 31) >> 5;
 }
 
-// Lane l owns slots R l + r, r < R = td_pair_rounds(N); code[r] for r >= R
-// (and code[TD_MAX_ROUNDS]) holds R.
-__device__ __forceinline__ void td_load_pairs(int N, uint32_t (&code)[TD_MAX_STEPS]) {
+// A lane's pair slots and, in the last word, R | u0 << 8 (see td_load_pairs).
+typedef uint32_t td_codes[TD_MAX_ROUNDS + 1];
+
+// Lane l owns slots R l + r, r < R = td_pair_rounds(N).  Child (i, j, k) is
+// number u = C(N-1-i, 3) + C(N-1-j, 2) + (N-1-k) in the reference's reversed
+// triple order (T-1-t, sorting_search.cu:588-590), so the children of a lane's
+// slots r = 0, 1, ... are one run of consecutive u, from u0.
+__device__ __forceinline__ void td_load_pairs(int N, td_codes &code) {
     const int lane = threadIdx.x & 31;
     const int R = td_pair_rounds(N);
 #pragma unroll
     for (int r = 0; r < TD_MAX_ROUNDS; ++r) code[r] = td_pair_code(N, r < R ? R * lane + r : -1);
-    code[TD_MAX_ROUNDS] = (uint32_t)R;
+    const int a = N - 1 - (int)(code[0] & 31u), b = N - 1 - (int)((code[0] >> 5) & 31u);
+    code[TD_MAX_ROUNDS] = (uint32_t)R | (uint32_t)(a * (a - 1) * (a - 2) / 6 + b * (b - 1) / 2) << 8;
 }
 
 // Pinned state (L, off) -> the caller's array of `level`.
@@ -436,7 +248,7 @@ __device__ __forceinline__ int td_prepare_rows(td_warp_smem &s, int level, int N
 
 // Classifies every child of the node at `level`; fills the level's outcome
 // words and lane summaries and returns a found move (i | j<<5 | k<<10) or -1.
-__device__ __forceinline__ int td_evaluate_rows(td_warp_smem &s, const uint32_t (&code)[TD_MAX_STEPS], int N,
+__device__ __forceinline__ int td_evaluate_rows(td_warp_smem &s, const td_codes &code, int N,
                                                 int level, int odd, uint32_t O, uint32_t F) {
     const int lane = threadIdx.x & 31;
     const int D = level + 1;
@@ -445,7 +257,7 @@ __device__ __forceinline__ int td_evaluate_rows(td_warp_smem &s, const uint32_t 
     const uint32_t x0 = (0u - ((reachD >> odd) & 1u)) & ~f0;
     const uint32_t x2 = (0u - ((reachD >> (odd + 2)) & 1u)) & ~f2;
     const bool accepting = (f0 | f2) != 0;  // warp-uniform
-    const int R = (int)code[TD_MAX_ROUNDS];  // warp-uniform
+    const int R = (int)(code[TD_MAX_ROUNDS] & 255u);  // warp-uniform
     uint32_t key = 0xffffffffu;
     uint32_t W[TD_MAX_ROUNDS] = {0u, 0u, 0u, 0u};
 #pragma unroll
@@ -493,7 +305,7 @@ __device__ __forceinline__ int td_evaluate_rows(td_warp_smem &s, const uint32_t 
 // smallest pair) and its smallest k.  `ord` (td_order_variant) rotates the
 // lane priority, reverses the round order and takes the largest k first.
 // Returns the move or -1.
-__device__ __forceinline__ int td_next_child_rows(td_warp_smem &s, const uint32_t (&code)[TD_MAX_STEPS],
+__device__ __forceinline__ int td_next_child_rows(td_warp_smem &s, const td_codes &code,
                                                   int level, uint32_t ord) {
     const int lane = threadIdx.x & 31;
     const uint32_t m2 = s.m2[level], m0 = s.m0[level];
@@ -534,6 +346,99 @@ __device__ __forceinline__ int td_next_child_rows(td_warp_smem &s, const uint32_
     __syncwarp();
     const int k = c2 ? b + 1 : b - 15;
     return (int)((pc & 1023u) | ((uint32_t)k << 10));
+}
+
+// Reference order: classifies every child of the node at `level`; fills the
+// level's child words and returns the found child's u, or -1.  A node's found
+// child is the one of lowest u (the lowest lane of the first 32-chunk,
+// sorting_search.cu:585-641); the root's children are accepted when visited.
+// Integer issue bounds it.  A lane's pair slots hold one run of consecutive u,
+// so at most three shared-memory ORs per lane put 680 children in order.  The
+// earlier form read three pair-table entries and a class-table byte per triple
+// (22 steps per lane): 16,384 S_12 instances at bound 6 took 12.2 ms, and take
+// 7.6 ms with this one.
+__device__ __forceinline__ int td_evaluate(td_warp_smem &s, const td_codes &code, int N, int level, int odd,
+                                           uint32_t O, uint32_t F) {
+    const int lane = threadIdx.x & 31;
+    const int D = level + 1;
+    const uint32_t accD = s.acc[D], reachD = s.reach[D];
+    const uint32_t f0 = 0u - ((accD >> odd) & 1u), f2 = 0u - ((accD >> (odd + 2)) & 1u);
+    const uint32_t x0 = (0u - ((reachD >> odd) & 1u)) & ~f0;
+    const uint32_t x2 = (0u - ((reachD >> (odd + 2)) & 1u)) & ~f2;
+    const bool accepting = (f0 | f2) != 0;  // warp-uniform
+    const int R = (int)(code[TD_MAX_ROUNDS] & 255u);
+    if (lane < TD_MAX_STEPS) {
+        s.cw[level][lane] = 0;
+        if (level == 0) s.root_found[lane] = 0;
+    }
+    __syncwarp();
+    // the lane's children and found children, in order of u from u0
+    uint64_t ch = 0, fd = 0;
+    int at = 0;
+#pragma unroll
+    for (int r = 0; r < TD_MAX_ROUNDS; ++r) {
+        if (r >= R) break;
+        const uint32_t pc = code[r];
+        const int i = pc & 31, j = (pc >> 5) & 31;
+        const uint4 ri = s.rows[i], rj = s.rows[j];
+        const uint2 fi = s.flg[i], fj = s.flg[j];
+        uint32_t plus, zero;
+        td_row_classes_x(ri.x, ri.y, ri.z, rj.x, rj.y, rj.z, O, F, fi.x, fj.x, fi.y, fj.y, (int)(pc >> 15), &plus,
+                         &zero);
+        const uint32_t km = rj.w;  // k > j
+        // k = N-1 comes first: reverse the bits
+        ch |= (uint64_t)(__brev(km & ((x2 & plus) | (x0 & zero))) >> (32 - N)) << at;
+        if (accepting) fd |= (uint64_t)(__brev(km & ((f2 & plus) | (f0 & zero))) >> (32 - N)) << at;
+        at += N - 1 - j;
+    }
+    const int u0 = (int)(code[TD_MAX_ROUNDS] >> 8), w = u0 >> 5, sh = u0 & 31;
+    if (level == 0) ch |= fd;
+    if (ch) {
+        const uint64_t lo = ch << sh;
+        const uint32_t hi = sh ? (uint32_t)(ch >> (64 - sh)) : 0u;
+        if ((uint32_t)lo) atomicOr(&s.cw[level][w], (uint32_t)lo);
+        if (lo >> 32) atomicOr(&s.cw[level][w + 1], (uint32_t)(lo >> 32));
+        if (hi) atomicOr(&s.cw[level][w + 2], hi);
+    }
+    if (accepting) {
+        if (level == 0) {
+            if (fd) {
+                const uint64_t lo = fd << sh;
+                const uint32_t hi = sh ? (uint32_t)(fd >> (64 - sh)) : 0u;
+                if ((uint32_t)lo) atomicOr(&s.root_found[w], (uint32_t)lo);
+                if (lo >> 32) atomicOr(&s.root_found[w + 1], (uint32_t)(lo >> 32));
+                if (hi) atomicOr(&s.root_found[w + 2], hi);
+            }
+        } else {
+            const uint32_t key = __reduce_min_sync(TD_FULL, fd ? (uint32_t)(u0 + __ffsll((long long)fd) - 1) : ~0u);
+            if (key != ~0u) {
+                __syncwarp();
+                return (int)key;
+            }
+        }
+    }
+    __syncwarp();
+    return -1;
+}
+
+// Reference order: takes the next child of `level`; returns u or -1.  Chunks
+// of 32 are visited from the last one, lanes of a chunk in ascending order (the
+// owner's LIFO pop, sorting_search.cu:165-174, 677-686), and the root's
+// children in descending order of u.  *accepted is set for a root's child
+// that is accepted when visited.
+__device__ __forceinline__ int td_next_child(td_warp_smem &s, int level, int *accepted) {
+    const int lane = threadIdx.x & 31;
+    uint32_t w = lane < TD_MAX_STEPS ? s.cw[level][lane] : 0u;
+    const uint32_t some = __ballot_sync(TD_FULL, w != 0);
+    *accepted = 0;
+    if (!some) return -1;
+    const int st = 31 - __clz(some);
+    w = __shfl_sync(TD_FULL, w, st);
+    const int b = level == 0 ? 31 - __clz(w) : __ffs(w) - 1;
+    if (level == 0) *accepted = (int)((s.root_found[st] >> b) & 1u);
+    if (lane == 0) s.cw[level][st] = w & ~(1u << b);
+    __syncwarp();
+    return 32 * st + b;
 }
 
 // ---- work items (subtree roots handed between warps) ----------------------
@@ -618,7 +523,7 @@ struct td_dfs_out {
 // pool as items (free move order).  Returns the number donated (uniform
 // across the warp).
 __device__ __forceinline__ int td_donate(td_warp_smem &s, const td_donate_ctx &dc,
-                                         const uint32_t (&code)[TD_MAX_STEPS], int d0, int level, int N,
+                                         const td_codes &code, int d0, int level, int N,
                                          int want) {
     const int lane = threadIdx.x & 31;
     int lv = -1;
@@ -992,17 +897,13 @@ __device__ __forceinline__ bool td_tt_visit(const td_warp_smem &s, const td_sear
 }
 
 // Depth-first search from the node held at level d0 of `s` (state, path and
-// rate masks already set).  Leaves the frames intact on TD_DFS_BUDGET.  The
-// reference order evaluates one triple per lane and step (`code` holds the
-// lane's triple codes); the free order is bit-sliced (`code` holds the lane's
-// pair slots) and may donate subtrees through `dc`.
+// rate masks already set; `code` holds the lane's pair slots).  Leaves the
+// frames intact on TD_DFS_BUDGET.  The free order may donate subtrees through
+// `dc`.
 template <bool ORDERED>
-__device__ td_dfs_out td_dfs(td_warp_smem &s, const uint8_t *lut, const uint32_t (&code)[TD_MAX_STEPS],
-                             int N, int maxd, int d0, const td_search_limits &lim, const td_donate_ctx *dc) {
+__device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d0, const td_search_limits &lim, const td_donate_ctx *dc) {
     const int lane = threadIdx.x & 31;
-    const int T = td_triple_count(N);
-    const int steps = (T + 31) >> 5;
-    const int tri_base = td_tri_base(N);
+    const int last_tri = td_tri_base(N) + td_triple_count(N) - 1;  // child u is triple last_tri - u
     td_dfs_out r;
     r.status = TD_DFS_EXHAUSTED;
     r.depth = 0;
@@ -1011,15 +912,18 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const uint8_t *lut, const uint32_t
     int level = d0;
     uint32_t O = 0, F = 0;
     int found;
-    if constexpr (ORDERED) {
-        const int odd = td_prepare_node(s, s.L[d0], s.off[d0], N);
-        found = td_evaluate(s, lut, code, steps, d0, odd, maxd);
-        if (found >= 0) found = td_tri_table[tri_base + T - 1 - found];
-    } else {
-        td_unpack_state(s, d0, s.L[d0], s.off[d0], N);
-        const int odd = td_prepare_rows(s, d0, N, O, F);
-        found = td_evaluate_rows(s, code, N, d0, odd, O, F);
-    }
+    // prepares and evaluates the node at `level`
+    auto expand = [&]() {
+        const int odd = td_prepare_rows(s, level, N, O, F);
+        if constexpr (ORDERED) {
+            found = td_evaluate(s, code, N, level, odd, O, F);
+            if (found >= 0) found = td_tri_table[last_tri - found];
+        } else {
+            found = td_evaluate_rows(s, code, N, level, odd, O, F);
+        }
+    };
+    td_unpack_state(s, d0, s.L[d0], s.off[d0], N);
+    expand();
     r.expansions = 1;
     int since_check = 0;
     bool tt_on = false;  // the table is in use (free order, after TD_TT_AFTER expansions)
@@ -1057,8 +961,7 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const uint8_t *lut, const uint32_t
                 attempt_exp = 1;
                 if (tt_on) tt_gen = td_tt_next_gen(lim);  // the abandoned attempt's entries no longer match
                 level = d0;
-                const int odd = td_prepare_rows(s, d0, N, O, F);
-                found = td_evaluate_rows(s, code, N, d0, odd, O, F);
+                expand();
                 ++r.expansions;
                 continue;
             }
@@ -1132,8 +1035,13 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const uint8_t *lut, const uint32_t
                     --level;
                     continue;
                 }
-                t = td_tri_table[tri_base + T - 1 - u];
-                if (accepted) walk = 2;
+                t = td_tri_table[last_tri - u];
+                if (accepted) {
+                    walk = 2;
+                    break;
+                }
+                if (lane == 0) s.path[level] = (uint16_t)t;
+                td_apply_bytes(s, level, t, N);
                 break;
             } else {
                 const int m = td_next_child_rows(s, code, level, td_level_order(ord, attempt, level));
@@ -1162,26 +1070,9 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const uint8_t *lut, const uint32_t
             r.status = TD_DFS_FOUND;
             break;
         }
-        if constexpr (ORDERED) {
-            uint64_t nL;
-            int noff;
-            td_apply_move(s.L[level], s.off[level], N, t & 31, (t >> 5) & 31, (t >> 10) & 31, &nL, &noff);
-            __syncwarp();
-            if (lane == 0) {
-                s.path[level] = (uint16_t)t;
-                s.L[level + 1] = nL;
-                s.off[level + 1] = (uint8_t)noff;
-            }
-            ++level;
-            const int odd = td_prepare_node(s, nL, noff, N);
-            found = td_evaluate(s, lut, code, steps, level, odd, maxd);
-            if (found >= 0) found = td_tri_table[tri_base + T - 1 - found];
-        } else {
-            ++level;
-            const int odd = td_prepare_rows(s, level, N, O, F);
-            found = td_evaluate_rows(s, code, N, level, odd, O, F);
-            ++attempt_exp;
-        }
+        ++level;
+        expand();
+        if constexpr (!ORDERED) ++attempt_exp;
         ++r.expansions;
     }
     __syncwarp();
@@ -1193,19 +1084,13 @@ __device__ __forceinline__ bool td_instance_ok(const td_instance &x) {
            td_inst_init(x) <= TD_MAX_N;
 }
 
-// Loads the lane's codes for N (triple codes in the reference order, pair
-// slots in the free order) and the instance's rate masks; places its root at
-// level 0.  `codeN` caches the N the codes were loaded for (negative for the
-// other order's codes).
-template <bool ORDERED>
-__device__ __forceinline__ void td_setup_root(td_warp_smem &s, const td_instance &x, uint32_t (&code)[TD_MAX_STEPS],
-                                              int &codeN) {
+// Loads the lane's pair slots for N (`codeN` caches the N they were loaded
+// for) and the instance's rate masks; places its root at level 0.
+__device__ __forceinline__ void td_setup_root(td_warp_smem &s, const td_instance &x, td_codes &code, int &codeN) {
     const int lane = threadIdx.x & 31;
-    const int want = ORDERED ? x.n_symbols : -1 - x.n_symbols;
-    if (codeN != want) {
-        if constexpr (ORDERED) td_load_codes(x.n_symbols, code);
-        else td_load_pairs(x.n_symbols, code);
-        codeN = want;
+    if (codeN != x.n_symbols) {
+        td_load_pairs(x.n_symbols, code);
+        codeN = x.n_symbols;
     }
     td_rate_masks(s, x);
     if (lane == 0) {
@@ -1240,16 +1125,15 @@ __device__ __forceinline__ void td_write_result(td_result *out, int status, int 
 // the status it wrote (uniform across the warp).
 template <bool ORDERED>
 __device__ int td_warp_search(const td_instance &x, td_result *out, td_warp_smem &s,
-                               const uint8_t *lut, uint32_t (&code)[TD_MAX_STEPS], int &codeN,
-                               const td_search_limits &lim) {
+                               td_codes &code, int &codeN, const td_search_limits &lim) {
     int status = TD_NOT_FOUND, depth = 0;
     uint32_t expansions = 0;
     uint16_t found_move = 0;
     if (!td_instance_ok(x)) {
         status = TD_ERR_ARG;
     } else if (td_triple_count(x.n_symbols) > 0) {
-        td_setup_root<ORDERED>(s, x, code, codeN);
-        const td_dfs_out r = td_dfs<ORDERED>(s, lut, code, x.n_symbols, x.max_moves, 0, lim, nullptr);
+        td_setup_root(s, x, code, codeN);
+        const td_dfs_out r = td_dfs<ORDERED>(s, code, x.n_symbols, 0, lim, nullptr);
         expansions = r.expansions;
         if (r.status == TD_DFS_FOUND) {
             status = TD_FOUND;

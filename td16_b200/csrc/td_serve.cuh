@@ -86,9 +86,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
     constexpr bool ALL_ORDERED = MODE == TD_SERVE_ORDERED;
     extern __shared__ __align__(16) uint8_t td_smem[];
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint8_t *lut = td_smem;
-    td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem + TD_LUT_BYTES);
-    td_block_init(lut, ws, warps);
+    td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
     const uint64_t deadline = td_globaltimer() + time_limit_ns;
     if (blockIdx.x == 0 && warp == 0) {
         // dispatcher: host ring -> device queue, from the launch's first
@@ -147,7 +145,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
         return;
     }
     td_warp_smem &s = ws[warp];
-    uint32_t code[TD_MAX_STEPS];
+    td_codes code;
     int codeN = -1;
     td_search_limits lim;
     lim.max_expansions = max_exp ? max_exp : ~0ull;
@@ -260,8 +258,8 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 }
             } else {
                 if (MODE == TD_SERVE_PER_REQUEST) ord = (x.packed & TD_PACKED_ORDERED) != 0;
-                if (ord) td_setup_root<true>(s, x, code, codeN);
-                else td_setup_root<false>(s, x, code, codeN);
+                if (ord) td_setup_root(s, x, code, codeN);
+                else td_setup_root(s, x, code, codeN);
                 run = true;
             }
         } else {
@@ -296,7 +294,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 const unsigned slot = (unsigned)(req % ring_size);
                 const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(&queue[slot]));
                 const td_instance x = *reinterpret_cast<const td_instance *>(&v);
-                td_setup_root<false>(s, x, code, codeN);
+                td_setup_root(s, x, code, codeN);
                 d0 = it.depth & 0x7f;
                 side = it.depth >> 7;
                 if (lane == 0) {
@@ -331,8 +329,8 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
             ulim.restart_base = kind == 1 || d0 == 0 ? restart_base : 0;
             dc.side = side;
             dc.race = MODE == TD_SERVE_PER_REQUEST && kind == 1 && !ord && restart_base && td_inst_full(x) ? race : 0;
-            if (ord) r = td_dfs<true>(s, lut, code, x.n_symbols, x.max_moves, d0, ulim, nullptr);
-            else r = td_dfs<false>(s, lut, code, x.n_symbols, x.max_moves, d0, ulim, &dc);
+            if (ord) r = td_dfs<true>(s, code, x.n_symbols, d0, ulim, nullptr);
+            else r = td_dfs<false>(s, code, x.n_symbols, d0, ulim, &dc);
             dc.side = 0;
             dc.race = 0;
             // a witness of the inverse becomes one of the request; one that does
