@@ -1833,12 +1833,13 @@ int noalloc_setup(int device, char *err, size_t errlen) {
     TD_CHECK_NA(cudaGetSymbolAddress(&ptr, td_noalloc_scratch));
     TD_CHECK_NA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device));
     const size_t smem = smem_bytes(4);
-    TD_CHECK_NA(cudaFuncSetAttribute(td_plain_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    TD_CHECK_NA(cudaFuncSetAttribute(td_plain_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    TD_CHECK_NA(cudaFuncSetAttribute(td_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
-    TD_CHECK_NA(cudaFuncSetAttribute(td_steal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_bytes(4)));
+    // the limit holds for every launch of a kernel, so it must fit the 8-warp
+    // blocks that td_configure allows too
+    const int limit = (int)smem_bytes(8);
+    TD_CHECK_NA(cudaFuncSetAttribute(td_plain_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+    TD_CHECK_NA(cudaFuncSetAttribute(td_plain_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+    TD_CHECK_NA(cudaFuncSetAttribute(td_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+    TD_CHECK_NA(cudaFuncSetAttribute(td_steal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
     TD_CHECK_NA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.steal_blocks, td_steal_kernel, 128,
                                                               smem_bytes(4)));
     TD_CHECK_NA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.persistent_blocks, td_persistent_kernel<true>,

@@ -120,3 +120,25 @@ def test_noalloc_calls_leave_device_memory_unchanged(td):
     assert free_after == free_before
     for count, _, d_out, _ in cases:
         assert (_results(d_out)["status"] >= 0).all()
+
+
+def test_noalloc_setup_keeps_eight_warp_blocks_launchable(td):
+    """The set-up of the first call sets the kernels' shared-memory limit; a
+    launch of 8-warp blocks (the tuned shape) must still fit afterwards."""
+    import torch
+    perms, n = td.synth_perms(46, 512, 8, 10, 50, 1, 2)
+    inst = td.prepare_perms(perms, n, 9)
+    d_in = torch.from_numpy(inst.view(np.uint8).copy()).cuda()
+    d_out = torch.zeros(len(inst) * 32, dtype=torch.uint8, device="cuda")
+    rc, msg = _call(_noalloc(td), len(inst), d_in, d_out, 0, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0, msg
+    torch.cuda.synchronize()
+    td.init_slots(1, [0], 64 << 20)
+    try:
+        td._lib.configure(8, 1)
+        for flags in (0, td._lib.FLAG_ORDERED, td._lib.FLAG_PLAIN, td._lib.FLAG_PLAIN | td._lib.FLAG_ORDERED):
+            res, _ = td.search_batch(0, inst, flags)
+            assert (res["status"] == 1).all()
+    finally:
+        td._lib.configure(4, 1)
+        td.destroy()
