@@ -496,3 +496,84 @@ extern "C" int td_emu_pinned_cycles(uint64_t L, int off, int N) {
     uint32_t fixed;
     return td_pinned_cycles(L, off, N, &fixed);
 }
+
+// Rebuilds the endgame table (td_endgame.cuh) for glued states of up to
+// `symbols` symbols: out[td_eg_base(m) + rank] = 0 where the state's missing
+// moves suffice, else the expansions of the reference-order walk that finds
+// they do not; 0xffff where the state is not glued.  Returns the number of
+// states that one spare move does not let sort either, which the engine takes
+// to be 0.  Each state's +2 children miss one move less, so states are taken
+// by their missing moves.
+extern "C" long td_emu_endgame(int symbols, uint16_t *out, int threads) {
+    const uint32_t total = td_eg_base(symbols);  // states of up to `symbols` symbols: m < symbols
+    for (uint32_t g = 0; g < total; ++g) out[g] = 0xffff;
+    std::atomic<long> bad{0};
+    auto glued = [](uint64_t L, int N, uint32_t *kept) {
+        uint32_t k = 0;
+        for (int p = 0; p < N; ++p) {
+            const int b = p ? (int)td_nib(L, p - 1) + 1 : 0, q = p ? p - 1 : N - 1;
+            const int a = q ? (int)td_nib(L, q - 1) + 1 : 0;
+            if (b != (a + 1) % N) k |= 1u << b;
+        }
+        *kept = k;
+        return td_popc(k);
+    };
+    auto state = [](uint32_t g, int *N) {
+        int m = 2;
+        while (g >= td_eg_base(m + 1)) ++m;
+        uint32_t r = g - td_eg_base(m), d[16], U = (1u << m) - 1u;
+        for (int q = 1; q <= m; ++q) { d[q] = r % q; r /= q; }
+        uint64_t L = 0;
+        for (int q = m, at = 0; q >= 1; --q, ++at) {
+            uint32_t v = U;
+            while (d[q]--) v &= v - 1;
+            const int x = __builtin_ctz(v);
+            U &= ~(1u << x);
+            L |= (uint64_t)x << (4 * at);
+        }
+        for (int at = m; at < 16; ++at) L |= (uint64_t)at << (4 * at);
+        *N = m + 1;
+        return L;
+    };
+    // sweep 0: entries of the states missing `M` moves; sweep 1: where no +2
+    // child exists, a 0 child must be sorted by its missing moves
+    auto pass = [&](int M, int sweep, int t) {
+        static thread_local Emu e;
+        for (uint32_t g = (uint32_t)t; g < total; g += (uint32_t)threads) {
+            if (sweep == 1 && (out[g] == 0 || out[g] == 0xffff)) continue;
+            int N;
+            const uint64_t L = state(g, &N);
+            uint32_t kept;
+            if (glued(L, N, &kept) != N) continue;
+            e.N = N;
+            const int odd = prepare_rows(e, L, 0);
+            if ((N - odd) / 2 != M) continue;
+            uint32_t sum = 1;
+            bool sorted = false, two = false, zero_sorted = false;
+            for (int i = 0; i < N; ++i)
+                for (int j = i + 1; j < N; ++j) {
+                    uint32_t plus, zero;
+                    td_row_classes(e.S[i], e.G[i], e.P[i], e.S[j], e.G[j], e.P[j], e.O, e.F, i, j, &plus, &zero);
+                    for (int k = j + 1; k < N; ++k) {
+                        if (!(((sweep ? plus | zero : plus) >> k) & 1u)) continue;
+                        uint64_t nL;
+                        int noff;
+                        td_apply_move(L, 0, N, i, j, k, &nL, &noff);
+                        const int n = glued(nL, N, &kept);
+                        const uint32_t v = n ? out[td_eg_base(n - 1) + td_eg_rank(nL, kept)] : 0u;
+                        if ((plus >> k) & 1u) { two = true; sum += v; sorted |= v == 0; }
+                        else zero_sorted |= v == 0;
+                    }
+                }
+            if (sweep == 0) out[g] = (uint16_t)(sorted ? 0 : sum);
+            else if (!two && !zero_sorted) ++bad;
+        }
+    };
+    for (int M = 1; M <= symbols / 2; ++M)
+        for (int sweep = 0; sweep < 2; ++sweep) {
+            std::vector<std::thread> pool;
+            for (int t = 0; t < threads; ++t) pool.emplace_back(pass, M, sweep, t);
+            for (auto &t : pool) t.join();
+        }
+    return bad.load();
+}

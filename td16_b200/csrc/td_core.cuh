@@ -253,6 +253,69 @@ TD_HD uint64_t td_tt_key(uint64_t L) {
     return (L & 0x00ffffffffffffffull) | (order << 56);
 }
 
+// ---- endgame table ------------------------------------------------------------
+//
+// Index of a state whose fixed symbols are glued to their predecessors, for
+// the table of td_endgame.cuh.
+
+#define TD_EG_SYMBOLS 11        // largest glued state in the table
+#define TD_EG_STATES 4037912    // sum over m = 2..10 of m!
+
+TD_HD int td_popc(uint32_t v) {
+#if defined(__CUDA_ARCH__)
+    return __popc(v);
+#else
+    return __builtin_popcount(v);
+#endif
+}
+
+TD_HD int td_clz(uint32_t v) {  // v != 0
+#if defined(__CUDA_ARCH__)
+    return __clz((int)v);
+#else
+    return __builtin_clz(v);
+#endif
+}
+
+// Where the states of m + 1 symbols start: the sum of q! over 2 <= q < m.
+TD_HD uint32_t td_eg_base(int m) {
+    uint32_t b = 0, f = 1;
+    for (int q = 2; q < m; ++q) {
+        f *= (uint32_t)q;
+        b += f;
+    }
+    return b;
+}
+// Index of the glued form of the pinned state L, whose symbols `fixed` are
+// glued to their predecessors and `kept` are not.  Reads the glued array from
+// symbol 0 on: where 0 is itself glued, it stands for its block, whose first
+// symbol is then the largest one kept (the block runs from it to N-1 and on
+// to 0), so that one is passed over.  Each kept symbol's digit is the number
+// of smaller ones to its right.
+TD_HD uint32_t td_eg_rank(uint64_t L, uint32_t kept) {
+    uint32_t U = kept;
+    if (kept & 1u) {
+        U &= ~1u;
+    } else {
+        U &= ~(0x80000000u >> td_clz(kept));
+    }
+    U >>= 1;  // L holds symbol - 1
+    int rem = td_popc(U);
+    uint32_t rank = 0;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int m = 0; m < 16; ++m) {  // nibbles past the state hold values outside U
+        const uint32_t bit = 1u << td_nib(L, m);
+        if (U & bit) {
+            rank = rank * (uint32_t)rem + (uint32_t)td_popc(U & (bit - 1u));
+            U &= ~bit;
+            --rem;
+        }
+    }
+    return rank;
+}
+
 // ---- restarts of the free order ----------------------------------------------
 //
 // The free-order search has a heavy tail: on near-reverse S_16 the median

@@ -60,6 +60,7 @@ __device__ __forceinline__ td_search_limits td_make_limits(uint64_t max_exp, uin
                                                            const int *abort_flag) {
     td_search_limits lim;
     lim.max_expansions = max_exp ? max_exp : ~0ull;
+    lim.max_work = ~0u;
     lim.deadline_ns = time_limit_ns ? td_globaltimer() + time_limit_ns : 0;
     lim.abort_flag = abort_flag;
     lim.tt = nullptr;
@@ -87,8 +88,9 @@ __global__ void __launch_bounds__(256) td_plain_kernel(const td_instance *__rest
     td_warp_search<ORDERED>(x, &out[idx], ws[warp], code, codeN, lim);
 }
 
-// hard_count / hard_list (or null): instances that end with TD_ERR_BUDGET are
-// listed there, for the split pass of the reference order (td_split_*).
+// hard_count / hard_list (or null): the first pass of a split batch of the
+// reference order; instances not finished within max_exp nodes expanded here
+// are listed, for the split pass (td_split_*).
 template <bool ORDERED>
 __global__ void __launch_bounds__(256, 4) td_persistent_kernel(const td_instance *__restrict__ in,
                                                            td_result *__restrict__ out, int count,
@@ -100,7 +102,8 @@ __global__ void __launch_bounds__(256, 4) td_persistent_kernel(const td_instance
     td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
     td_codes code;
     int codeN = -1;
-    const td_search_limits lim = td_make_limits(max_exp, time_limit_ns, nullptr);
+    td_search_limits lim = td_make_limits(hard_list ? 0 : max_exp, time_limit_ns, nullptr);
+    if (hard_list) lim.max_work = (uint32_t)max_exp;
     for (;;) {
         int first = 0;
         if (lane == 0) first = atomicAdd(ticket, grain);
@@ -888,6 +891,41 @@ int launch_cfg(int device, LaunchCfg *c, char *err, size_t errlen) {
     return TD_OK;
 }
 
+// Fills the endgame table (td_endgame.cuh) of the current device, once per
+// device and process: five launches, on a stream of their own so that they
+// wait for nothing else.
+constexpr int kEndgameDevices = 64;
+std::mutex g_eg_mu;
+bool g_eg_ready[kEndgameDevices];
+
+cudaError_t endgame_setup(int device, int sms) {
+    if (device < 0 || device >= kEndgameDevices) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> g(g_eg_mu);
+    if (g_eg_ready[device]) return cudaSuccess;
+    uint32_t bases[TD_EG_SYMBOLS], factorial[TD_EG_SYMBOLS];
+    for (int m = 0; m < TD_EG_SYMBOLS; ++m) {
+        bases[m] = td_eg_base(m);
+        factorial[m] = m ? (uint32_t)m * factorial[m - 1] : 1u;
+    }
+    cudaStream_t st;
+    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return e;
+    const size_t smem = smem_bytes(8);
+    e = cudaFuncSetAttribute(td_eg_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(td_eg_bases, bases, sizeof bases, 0, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyToSymbolAsync(td_eg_factorial, factorial, sizeof factorial, 0, cudaMemcpyHostToDevice, st);
+    for (int missing = 1; e == cudaSuccess && missing <= TD_EG_SYMBOLS / 2; ++missing) {
+        td_eg_build_kernel<<<4 * sms, 256, smem, st>>>(missing);
+        e = cudaGetLastError();
+    }
+    const cudaError_t done = cudaStreamSynchronize(st);
+    cudaStreamDestroy(st);
+    if (e == cudaSuccess) e = done;
+    g_eg_ready[device] = e == cudaSuccess;
+    return e;
+}
+
 int ensure_device(int device, char *err, size_t errlen) {
     if ((int)g_dev.size() <= device) g_dev.resize(device + 1);
     DeviceInfo &d = g_dev[device];
@@ -913,6 +951,7 @@ int ensure_device(int device, char *err, size_t errlen) {
     TD_CHECK(cudaFuncSetAttribute(td_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
     const int rc = preload_kernels(err, errlen);
     if (rc != TD_OK) return rc;
+    TD_CHECK(endgame_setup(device, d.sms));
     d.ready = true;
     return TD_OK;
 }
@@ -1844,6 +1883,7 @@ int noalloc_setup(int device, char *err, size_t errlen) {
                                                               smem_bytes(4)));
     TD_CHECK_NA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.persistent_blocks, td_persistent_kernel<true>,
                                                               128, smem));
+    TD_CHECK_NA(endgame_setup(device, d.sms));
     d.scratch = static_cast<uint8_t *>(ptr);
     d.ready = true;
     return TD_OK;
@@ -2029,6 +2069,7 @@ int preload_kernels(char *err, size_t errlen) {
     TD_CHECK(cudaFuncGetAttributes(&a, td_split_kernel));
     TD_CHECK(cudaFuncGetAttributes(&a, td_split_join_kernel));
     TD_CHECK(cudaFuncGetAttributes(&a, td_epoch_kernel));
+    TD_CHECK(cudaFuncGetAttributes(&a, td_eg_build_kernel));
     TD_CHECK(cudaFuncGetAttributes(&a, td_finalize_kernel));
     TD_CHECK(cudaFuncGetAttributes(&a, td_count_kernel));
     TD_CHECK(cudaFuncGetAttributes(&a, td_validate_kernel));

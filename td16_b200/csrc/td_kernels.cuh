@@ -36,6 +36,7 @@ struct td_warp_smem {
             // per level: bit u % 32 of word u / 32 is child u still to visit
             uint32_t cw[TD_MAX_DEPTH][TD_MAX_STEPS];
             uint32_t root_found[TD_MAX_STEPS];  // the root's children accepted when visited
+            uint32_t cp[TD_MAX_DEPTH][TD_MAX_STEPS];  // the +2 ones, at nodes that also have 0 children
         };
         struct {  // free move order
             // per level and lane: the expandable children of the lane's four
@@ -53,6 +54,11 @@ struct td_warp_smem {
     uint8_t off[TD_MAX_DEPTH + 1];
     uint8_t A[TD_MAX_DEPTH + 1][32];           // per level: the caller's array, one pinned label per position
     uint8_t inv[32];                           // caller position of each label
+    // per level: the moves its node can spare, where the endgame table may
+    // decide its children; else 255
+    uint8_t spare[TD_MAX_DEPTH];
+    uint16_t list[32];                         // children looked up in the endgame table
+    int eg_moves;                              // the bound where the endgame table applies, else 0
 };
 
 // Lexicographic position triples i|j<<5|k<<10 for every N, at offset C(N,4).
@@ -88,12 +94,17 @@ __device__ __forceinline__ void td_rate_masks(td_warp_smem &s, const td_instance
         }
         s.acc[D] = a;
         s.reach[D] = r;
+        // the endgame table knows full sorting; it needs every depth up to the
+        // bound accepted (the rate falls with the depth)
+        if (D == maxd) s.eg_moves = full && a ? maxd : 0;
     }
     __syncwarp();
 }
 
 struct td_search_limits {
     uint64_t max_expansions;   // per search; TD_ERR_BUDGET when exceeded
+    uint32_t max_work;         // the same for nodes expanded here (the reference order's count also
+                               // holds those the endgame table accounts for)
     uint64_t deadline_ns;      // %globaltimer value; 0 = none
     const int *abort_flag;     // optional host/device abort request
     uint64_t *tt;              // this warp's table of explored states (free order); null = none
@@ -304,7 +315,7 @@ __device__ __forceinline__ int td_evaluate_rows(td_warp_smem &s, const td_codes 
 // the plain order (ord = 0), the highest pair slot (the lexicographically
 // smallest pair) and its smallest k.  `ord` (td_order_variant) rotates the
 // lane priority, reverses the round order and takes the largest k first.
-// Returns the move or -1.
+// Returns the move, with bit 15 set for a 0 child, or -1.
 __device__ __forceinline__ int td_next_child_rows(td_warp_smem &s, const td_codes &code,
                                                   int level, uint32_t ord) {
     const int lane = threadIdx.x & 31;
@@ -345,7 +356,7 @@ __device__ __forceinline__ int td_next_child_rows(td_warp_smem &s, const td_code
     }
     __syncwarp();
     const int k = c2 ? b + 1 : b - 15;
-    return (int)((pc & 1023u) | ((uint32_t)k << 10));
+    return (int)((pc & 1023u) | ((uint32_t)k << 10) | (c2 ? 0u : 0x8000u));
 }
 
 // Reference order: classifies every child of the node at `level`; fills the
@@ -369,11 +380,12 @@ __device__ __forceinline__ int td_evaluate(td_warp_smem &s, const td_codes &code
     const int R = (int)(code[TD_MAX_ROUNDS] & 255u);
     if (lane < TD_MAX_STEPS) {
         s.cw[level][lane] = 0;
+        s.cp[level][lane] = 0;
         if (level == 0) s.root_found[lane] = 0;
     }
     __syncwarp();
     // the lane's children and found children, in order of u from u0
-    uint64_t ch = 0, fd = 0;
+    uint64_t ch = 0, fd = 0, pl = 0;
     int at = 0;
 #pragma unroll
     for (int r = 0; r < TD_MAX_ROUNDS; ++r) {
@@ -389,26 +401,24 @@ __device__ __forceinline__ int td_evaluate(td_warp_smem &s, const td_codes &code
         // k = N-1 comes first: reverse the bits
         ch |= (uint64_t)(__brev(km & ((x2 & plus) | (x0 & zero))) >> (32 - N)) << at;
         if (accepting) fd |= (uint64_t)(__brev(km & ((f2 & plus) | (f0 & zero))) >> (32 - N)) << at;
+        if (x0) pl |= (uint64_t)(__brev(km & plus) >> (32 - N)) << at;
         at += N - 1 - j;
     }
     const int u0 = (int)(code[TD_MAX_ROUNDS] >> 8), w = u0 >> 5, sh = u0 & 31;
     if (level == 0) ch |= fd;
-    if (ch) {
-        const uint64_t lo = ch << sh;
-        const uint32_t hi = sh ? (uint32_t)(ch >> (64 - sh)) : 0u;
-        if ((uint32_t)lo) atomicOr(&s.cw[level][w], (uint32_t)lo);
-        if (lo >> 32) atomicOr(&s.cw[level][w + 1], (uint32_t)(lo >> 32));
-        if (hi) atomicOr(&s.cw[level][w + 2], hi);
-    }
+    // ORs the lane's run into the 22 words of an array
+    auto put = [&](uint32_t *words, uint64_t run) {
+        const uint64_t lo = run << sh;
+        const uint32_t hi = sh ? (uint32_t)(run >> (64 - sh)) : 0u;
+        if ((uint32_t)lo) atomicOr(&words[w], (uint32_t)lo);
+        if (lo >> 32) atomicOr(&words[w + 1], (uint32_t)(lo >> 32));
+        if (hi) atomicOr(&words[w + 2], hi);
+    };
+    if (ch) put(s.cw[level], ch);
+    if (x0 && pl) put(s.cp[level], pl);
     if (accepting) {
         if (level == 0) {
-            if (fd) {
-                const uint64_t lo = fd << sh;
-                const uint32_t hi = sh ? (uint32_t)(fd >> (64 - sh)) : 0u;
-                if ((uint32_t)lo) atomicOr(&s.root_found[w], (uint32_t)lo);
-                if (lo >> 32) atomicOr(&s.root_found[w + 1], (uint32_t)(lo >> 32));
-                if (hi) atomicOr(&s.root_found[w + 2], hi);
-            }
+            if (fd) put(s.root_found, fd);
         } else {
             const uint32_t key = __reduce_min_sync(TD_FULL, fd ? (uint32_t)(u0 + __ffsll((long long)fd) - 1) : ~0u);
             if (key != ~0u) {
@@ -440,6 +450,8 @@ __device__ __forceinline__ int td_next_child(td_warp_smem &s, int level, int *ac
     __syncwarp();
     return 32 * st + b;
 }
+
+#include "td_endgame.cuh"
 
 // ---- work items (subtree roots handed between warps) ----------------------
 
@@ -912,18 +924,37 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
     int level = d0;
     uint32_t O = 0, F = 0;
     int found;
-    // prepares and evaluates the node at `level`
+    const int eg_moves = s.eg_moves;  // the endgame table decides children (0: it does not apply)
+    bool solved = false;  // free order: the table has shown the way to a witness
+    // prepares and evaluates the node at `level`, and lets the table decide its
+    // children.  A move joins at most three pairs of neighbours, so only a node
+    // of at most TD_EG_SYMBOLS + 3 symbols that omega moves has one in the table.
     auto expand = [&]() {
         const int odd = td_prepare_rows(s, level, N, O, F);
+        const int spare = eg_moves - level - ((N - odd) >> 1);
+        const int moved = N - __popc(F);  // symbols left
+        const bool endgame =
+            eg_moves > level + 1 && spare >= 0 && moved <= TD_EG_SYMBOLS + 3;  // warp-uniform
         if constexpr (ORDERED) {
             found = td_evaluate(s, code, N, level, odd, O, F);
             if (found >= 0) found = td_tri_table[last_tri - found];
+            // with two spare moves no child that the table holds is dropped
+            else if (lane == 0) s.spare[level] = (uint8_t)(endgame && spare < 2 ? spare : 255);
+            __syncwarp();
         } else {
+            if (lane == 0) s.spare[level] = (uint8_t)(endgame ? spare : 255);
             found = td_evaluate_rows(s, code, N, level, odd, O, F);
+            if (endgame && found < 0 && spare == 0) {
+                const uint4 w = s.pw[level][lane];
+                if (__reduce_add_sync(TD_FULL, (unsigned)(__popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w))) >=
+                    TD_EG_MANY)
+                    solved |= td_eg_filter(s, code, level, N);
+            }
         }
     };
     td_unpack_state(s, d0, s.L[d0], s.off[d0], N);
     expand();
+    uint32_t work = 1;  // nodes expanded here
     r.expansions = 1;
     int since_check = 0;
     bool tt_on = false;  // the table is in use (free order, after TD_TT_AFTER expansions)
@@ -942,12 +973,12 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
             r.status = TD_DFS_FOUND;
             break;
         }
-        if (r.expansions >= lim.max_expansions) {
+        if (r.expansions >= lim.max_expansions || work >= lim.max_work) {
             r.status = TD_DFS_BUDGET;
             break;
         }
         if constexpr (!ORDERED) {
-            if (attempt_exp >= attempt_budget) {
+            if (attempt_exp >= attempt_budget && !solved) {
                 // restart the subtree at d0 with the next child order; the table
                 // held nodes of the abandoned attempt that were not explored to
                 // the end, so it is cleared before its next use
@@ -962,6 +993,7 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
                 if (tt_on) tt_gen = td_tt_next_gen(lim);  // the abandoned attempt's entries no longer match
                 level = d0;
                 expand();
+                ++work;
                 ++r.expansions;
                 continue;
             }
@@ -993,12 +1025,12 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
                 // a search that has handed out subtrees no longer restarts: the
                 // subtrees of an abandoned attempt would go on being searched,
                 // and searching in parallel already varies the order
-                if (hungry > 0 && td_donate(s, *dc, code, d0, level, N, min(hungry, dc->grain)) > 0)
+                if (hungry > 0 && !solved && td_donate(s, *dc, code, d0, level, N, min(hungry, dc->grain)) > 0)
                     attempt_budget = ~0u;
             }
         }
         if constexpr (!ORDERED) {
-            if (raced && (r.expansions & 15u) == 0) {
+            if (raced && (work & 15u) == 0) {
                 int stop = 0;
                 if (lane == 0) stop = *(volatile int *)&dc->state->found;
                 if (__shfl_sync(TD_FULL, stop, 0)) {
@@ -1007,7 +1039,7 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
                 }
             }
         }
-        if ((r.expansions & 255u) == 0) {
+        if ((work & 255u) == 0) {
             int stop = 0;
             if (lane == 0) {
                 if (lim.deadline_ns && td_globaltimer() > lim.deadline_ns) stop = 1;
@@ -1025,9 +1057,21 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
         // children skipped through the table, change no expansion count, so
         // the checks above run once per expansion
         uint32_t t = 0;
-        int walk = 0;  // 1: the subtree is exhausted, 2: a root accepted on visit (ordered)
+        int walk = 0;  // 1: the subtree is exhausted, 2: a root accepted on visit (ordered), 3: out of budget
         for (;;) {
             if constexpr (ORDERED) {
+                const int spare = s.spare[level];
+                if (spare != 255) {
+                    // the walk of the children dropped here ends without a
+                    // witness; a budget that it would exhaust ends it there
+                    const uint32_t skipped = td_eg_skip(s, level, N, spare);
+                    r.expansions = r.expansions + skipped < r.expansions ? ~0u : r.expansions + skipped;
+                    if (skipped && r.expansions >= lim.max_expansions) {
+                        r.expansions = (uint32_t)lim.max_expansions;
+                        walk = 3;
+                        break;
+                    }
+                }
                 int accepted;
                 const int u = td_next_child(s, level, &accepted);
                 if (u < 0) {
@@ -1050,10 +1094,20 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
                     --level;
                     continue;
                 }
-                t = (uint32_t)m;
+                t = (uint32_t)m & 0x7fffu;
                 if (lane == 0) s.path[level] = (uint16_t)t;
                 td_apply_bytes(s, level, t, N);
-                if (lim.tt) {
+                const int spare = s.spare[level];
+                if (spare != 255) {
+                    // a 0 child has a spare move less than its parent
+                    const uint32_t e = td_eg_look(s, level + 1, N, spare == (m >> 15));
+                    if (e == 0) {
+                        solved = true;
+                        break;
+                    }
+                    if (e != TD_EG_UNKNOWN) continue;
+                }
+                if (lim.tt && !solved) {
                     if (!tt_on && r.expansions >= TD_TT_AFTER) {
                         tt_gen = td_tt_next_gen(lim);
                         tt_on = true;
@@ -1064,6 +1118,10 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
             }
         }
         if (walk == 1) break;
+        if (walk == 3) {
+            r.status = TD_DFS_BUDGET;
+            break;
+        }
         if (walk == 2) {
             r.found_move = (uint16_t)t;
             r.depth = level + 1;
@@ -1073,6 +1131,7 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
         ++level;
         expand();
         if constexpr (!ORDERED) ++attempt_exp;
+        ++work;
         ++r.expansions;
     }
     __syncwarp();

@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
     int codeN = -1;
     td_search_limits lim;
     lim.max_expansions = max_exp ? max_exp : ~0ull;
+    lim.max_work = ~0u;
     lim.deadline_ns = deadline;
     lim.abort_flag = nullptr;
     lim.tt = (!ALL_ORDERED && tt) ? tt + ((size_t)(blockIdx.x * warps + warp) << tt_bits) : nullptr;
