@@ -53,7 +53,14 @@ static_assert(sizeof(td_result) == 32, "td_result layout");
 // kernels
 // ============================================================================
 
-#define TD_TT_BITS 12  // default: 4096 explored-state entries (32 KiB) per warp of a free-order launch
+#define TD_TT_BITS 12  // default of td_configure_table
+// 16-byte entries of the table of explored states per resident warp: 2^(bits -
+// TD_TT_DOWN), rounded down to a power of two in all.  64 MiB at the default
+// for a whole B200: the L2 keeps it.
+#ifndef TD_TT_DOWN
+#define TD_TT_DOWN 2
+#endif
+#define TD_TT_INST_BITS 26  // instances per epoch in the table's search numbers
 #define TD_RESTART_BASE 16  // default base of the free order's restart budgets (expansions)
 
 __device__ __forceinline__ td_search_limits td_make_limits(uint64_t max_exp, uint64_t time_limit_ns,
@@ -64,8 +71,8 @@ __device__ __forceinline__ td_search_limits td_make_limits(uint64_t max_exp, uin
     lim.deadline_ns = time_limit_ns ? td_globaltimer() + time_limit_ns : 0;
     lim.abort_flag = abort_flag;
     lim.tt = nullptr;
-    lim.tt_gen = nullptr;
-    lim.tt_bits = 0;
+    lim.tt_id = 0;
+    lim.tt_shift = 0;
     lim.restart_base = 0;
     lim.cutoff = nullptr;
     lim.rank = 0;
@@ -392,11 +399,11 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                                                       td_item *items, uint32_t *ready, const uint32_t *epoch_ptr,
                                                       int capacity, td_inst_state *state, int grain,
                                                       int max_level, int check_every, uint64_t time_limit_ns,
-                                                      uint64_t *tt, uint32_t *tt_gen, int tt_bits,
+                                                      ulonglong2 *tt, int tt_shift, unsigned epochs,
                                                       uint32_t restart_base, uint64_t max_exp,
                                                       unsigned max_backoff_ns, int race, int spawn_base) {
     extern __shared__ __align__(16) uint8_t td_smem[];
-    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
     td_warp_smem &s = ws[warp];
     td_codes code;
@@ -406,22 +413,22 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
     // TD_ERR_BUDGET
     td_search_limits lim = td_make_limits(max_exp, time_limit_ns, nullptr);
     lim.restart_base = restart_base;
-    if (tt) {
-        lim.tt = tt + ((size_t)(blockIdx.x * warps + warp) << tt_bits);
-        lim.tt_gen = tt_gen + blockIdx.x * warps + warp;
-        lim.tt_bits = tt_bits;
-    }
     td_donate_ctx dc;
     dc.pool = pool;
     dc.items = items;
     dc.ready = ready;
     const uint32_t epoch = *epoch_ptr;  // bumped by td_epoch_kernel before this launch
     dc.epoch = epoch;
+    // this launch's numbers in the table: its `epochs` epochs, 2^26 searches each
+    lim.tt = tt;
+    lim.tt_shift = tt_shift;
+    lim.tt_id = (uint64_t)(epoch - epochs + 1u) << TD_TT_INST_BITS;
     // race: donated items use slots [0, spawn_base), queued inverse roots the rest
     dc.capacity = race ? spawn_base : capacity;
     dc.spawn_base = spawn_base;
     dc.spawn_capacity = race ? capacity - spawn_base : 0;
     dc.side = 0;
+    dc.attempt = 0;
     dc.race = 0;
     dc.grain = grain;
     dc.max_level = max_level;
@@ -553,8 +560,9 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                     dst[1] = __ldcg(src + 1);
                 }
                 const uint32_t idx = it.inst;
-                const int d0 = it.depth & 0x7f;
+                const int d0 = it.depth & 15;
                 const int side = it.depth >> 7;
+                const int attempt = ((it.depth >> 4) & 7) | ((it.off >> 5) << 3);
                 // an item names an instance of this launch and a level of the
                 // frame; one that does not is a launch error, never followed
                 if (idx >= (uint32_t)count || d0 >= TD_MAX_DEPTH || (kind == 3) != (side && d0 == 0)) {
@@ -569,13 +577,17 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                 td_setup_root(s, x, code, codeN);
                 if (lane == 0) {
                     s.L[d0] = it.L;
-                    s.off[d0] = it.off;
+                    s.off[d0] = it.off & 31;
                     for (int d = 0; d < d0; ++d) s.path[d] = it.path[d];
                 }
                 __syncwarp();
                 int stop = 0;
                 if (lane == 0) stop = *(volatile int *)&st->found;
                 stop = __shfl_sync(TD_FULL, stop, 0);
+                td_unpack_state(s, d0, it.L, it.off & 31, x.n_symbols);
+                // a donated state that another unit took up needs no second search
+                if (!stop && d0 > 0 && lim.tt && !max_exp)
+                    stop = td_tt_visit(s, lim, d0, x.n_symbols, idx, (uint32_t)(side << 6 | attempt));
                 td_dfs_out r;
                 if (stop) {
                     r.status = TD_DFS_ABORTED;
@@ -588,11 +600,16 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                     // an inverse instance restarts like any root search
                     td_search_limits ilim = lim;
                     if (d0 > 0) ilim.restart_base = 0;
+                    // a unit that may run out of its expansion budget leaves
+                    // recorded states unsearched: then only roots use the table
+                    if (d0 > 0 && max_exp) ilim.tt = nullptr;
                     dc.inst = idx;
                     dc.state = st;
                     dc.side = side;
+                    dc.attempt = attempt;
                     r = td_dfs<false>(s, code, x.n_symbols, d0, ilim, &dc);
                     dc.side = 0;
+                    dc.attempt = 0;
                     // a witness of the inverse becomes one of the instance; one that
                     // does not convert is reported as a failed replay, and one that
                     // leaves the reference's move filter on the instance's side is
@@ -615,10 +632,11 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
 
 // Advances the launch epoch that tags donated items as written; a launch
 // replayed from a CUDA graph therefore never mistakes an item of an earlier
-// launch for one of its own.
-__global__ void td_epoch_kernel(uint32_t *epoch) {
-    uint32_t e = *epoch + 1;
-    *epoch = e ? e : 1;
+// launch for one of its own.  A launch of more than 2^26 instances takes as
+// many epochs as it needs numbers in the table of explored states.
+__global__ void td_epoch_kernel(uint32_t *epoch, unsigned epochs) {
+    const uint32_t e = *epoch + epochs;
+    *epoch = e >= epochs ? e : epochs;
 }
 
 // Runs after td_steal_kernel on the same stream.  When a bounded wait of the
@@ -745,10 +763,8 @@ struct Slot {
     td_item *d_items = nullptr;
     uint32_t *d_ready = nullptr;
     int item_capacity = 0;
-    uint64_t *d_tt = nullptr;  // tables of explored states, one per resident warp
-    uint32_t *d_tt_gen = nullptr;  // their generation counters
-    size_t tt_warps = 0;
-    int tt_bits = 0;
+    ulonglong2 *d_tt = nullptr;  // table of explored states
+    int tt_log2 = 0, tt_bits = 0;  // log2 of its entries; the setting it was sized for
     td_inst_state *d_state = nullptr;
     size_t state_count = 0;
     uint32_t *d_epoch = nullptr;
@@ -820,6 +836,13 @@ std::string cuda_msg(cudaError_t e, const char *file, int line) {
             return TD_CUDA_ERROR;                                        \
         }                                                                \
     } while (0)
+
+// log2 of the entries of a table of explored states for `warps` resident warps.
+int tt_entries_log2(size_t warps, int bits) {
+    int b = 0;
+    while (b < 40 && ((size_t)1 << (b + 1)) <= ((warps << bits) >> TD_TT_DOWN)) ++b;
+    return std::max(b, 6);
+}
 
 size_t smem_bytes(int warps) { return (size_t)warps * sizeof(td_warp_smem); }
 
@@ -967,7 +990,6 @@ void release_slot(Slot &s) {
     if (s.d_items) cudaFree(s.d_items);
     if (s.d_ready) cudaFree(s.d_ready);
     if (s.d_tt) cudaFree(s.d_tt);
-    if (s.d_tt_gen) cudaFree(s.d_tt_gen);
     if (s.d_epoch) cudaFree(s.d_epoch);
     if (s.d_state) cudaFree(s.d_state);
     if (s.d_hard) cudaFree(s.d_hard);
@@ -1043,27 +1065,22 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
         const int resident = cfg.sms * cfg.steal_blocks_per_sm;
         const int share = std::max(1, resident / std::max(1, s.slots_on_device));
         const int grid = std::max(1, std::min(resident, std::max(share, (count + warps - 1) / warps)));
-        if (cfg.tt_bits > 0 && ((size_t)resident * warps > s.tt_warps || cfg.tt_bits != s.tt_bits)) {
-            // one table (8 bytes x 2^tt_bits) per resident warp, sized for
-            // the whole resident grid so that it never moves under a captured
-            // graph; replaced in stream order after the previous launch
+        const int tt_log2 = tt_entries_log2((size_t)resident * warps, cfg.tt_bits);
+        if (cfg.tt_bits > 0 && (tt_log2 > s.tt_log2 || cfg.tt_bits != s.tt_bits)) {
+            // sized for the whole resident grid so that it never moves under a
+            // captured graph; replaced in stream order after the previous launch
             if (s.d_tt) TD_CHECK(cudaFreeAsync(s.d_tt, stream));
-            if (s.d_tt_gen) TD_CHECK(cudaFreeAsync(s.d_tt_gen, stream));
             s.d_tt = nullptr;
-            s.d_tt_gen = nullptr;
-            s.tt_warps = 0;
-            const size_t tt_words = (size_t)resident * warps << cfg.tt_bits;
-            TD_CHECK(cudaMallocAsync(&s.d_tt, tt_words * sizeof(uint64_t), stream));
-            TD_CHECK(cudaMallocAsync(&s.d_tt_gen, (size_t)resident * warps * sizeof(uint32_t), stream));
-            // zero words are empty, and generations start at 1
-            TD_CHECK(cudaMemsetAsync(s.d_tt, 0, tt_words * sizeof(uint64_t), stream));
-            TD_CHECK(cudaMemsetAsync(s.d_tt_gen, 0, (size_t)resident * warps * sizeof(uint32_t), stream));
-            s.tt_warps = (size_t)resident * warps;
+            s.tt_log2 = 0;
+            TD_CHECK(cudaMallocAsync(&s.d_tt, sizeof(ulonglong2) << tt_log2, stream));
+            TD_CHECK(cudaMemsetAsync(s.d_tt, 0, sizeof(ulonglong2) << tt_log2, stream));  // zero words are empty
+            s.tt_log2 = tt_log2;
             s.tt_bits = cfg.tt_bits;
         }
+        const unsigned epochs = ((unsigned)(count - 1) >> TD_TT_INST_BITS) + 1u;
         TD_CHECK(cudaMemsetAsync(s.d_pool, 0, sizeof(td_pool), stream));
         TD_CHECK(cudaMemsetAsync(s.d_state, 0, (size_t)count * sizeof(td_inst_state), stream));
-        td_epoch_kernel<<<1, 1, 0, stream>>>(s.d_epoch);
+        td_epoch_kernel<<<1, 1, 0, stream>>>(s.d_epoch, epochs);
         // the race needs restarts, and an expansion budget per unit would make
         // one side's budget decide the other's; its queue of inverse roots
         // holds one slot per instance (each queues its inverse at most once),
@@ -1073,7 +1090,7 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
         td_steal_kernel<<<grid, threads, smem_bytes(warps), stream>>>(
             d_in, d_out, count, s.d_pool, s.d_items, s.d_ready, s.d_epoch, s.item_capacity, s.d_state,
             cfg.steal_grain, cfg.split_level, cfg.check_every, time_limit_ns(), cfg.tt_bits > 0 ? s.d_tt : nullptr,
-            s.d_tt_gen, cfg.tt_bits, cfg.restart_base, max_exp, count == 1 ? 4096u : 32768u, race, spawn_base);
+            64 - s.tt_log2, epochs, cfg.restart_base, max_exp, count == 1 ? 4096u : 32768u, race, spawn_base);
         TD_CHECK(cudaGetLastError());
         td_finalize_kernel<<<std::max(1, std::min((count + 255) / 256, 2 * cfg.sms)), 256, 0, stream>>>(
             s.d_pool, s.d_state, d_out, count);
@@ -1406,9 +1423,9 @@ TD_API int td_configure_steal(int grain, int split_level, int check_every) {
     return TD_OK;
 }
 
-// Size of the per-warp tables of explored states of later free-order launches:
-// 2^bits entries of 8 bytes per resident warp (6 <= bits <= 16), or 0 to
-// search without them.
+// Size of the table of explored states of later free-order launches:
+// 2^(bits - 2) entries of 16 bytes per resident warp (6 <= bits <= 16), rounded
+// down to a power of two in all, or 0 to search without it.
 TD_API int td_configure_table(int bits) {
     if (bits != 0 && (bits < 6 || bits > 16)) return TD_INVALID_ARG;
     std::lock_guard<std::mutex> g(g_mu);
@@ -1954,7 +1971,7 @@ TD_API int td_search_batch_noalloc(int count, const td_instance *d_instances, td
         // are tagged with a fresh epoch so an earlier call's items never count
         TD_CHECK_NA(cudaMemsetAsync(pool, 0, sizeof(td_pool), st));
         TD_CHECK_NA(cudaMemsetAsync(state, 0, (size_t)count * sizeof(td_inst_state), st));
-        td_epoch_kernel<<<1, 1, 0, st>>>(epoch);
+        td_epoch_kernel<<<1, 1, 0, st>>>(epoch, 1u);
         // the whole resident grid (the scratch does not depend on its size):
         // warps without an instance of their own take donated subtrees, so a
         // small batch is spread over the GPU; a single search wakes its
@@ -1962,7 +1979,7 @@ TD_API int td_search_batch_noalloc(int count, const td_instance *d_instances, td
         const int grid = d.sms * std::max(1, d.steal_blocks);
         td_steal_kernel<<<grid, threads, smem_bytes(warps), st>>>(
             d_instances, d_results, count, pool, items, ready, epoch, TD_NOALLOC_ITEMS, state, grain, split_level,
-            check_every, limit, nullptr, nullptr, 0, restart_base, max_exp, count == 1 ? 4096u : 32768u,
+            check_every, limit, nullptr, 64, 1u, restart_base, max_exp, count == 1 ? 4096u : 32768u,
             /*race=*/0, /*spawn_base=*/TD_NOALLOC_ITEMS);
         TD_CHECK_NA(cudaGetLastError());
         td_finalize_kernel<<<std::max(1, std::min((count + 255) / 256, 2 * d.sms)), 256, 0, st>>>(pool, state,

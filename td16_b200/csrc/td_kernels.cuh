@@ -107,9 +107,9 @@ struct td_search_limits {
                                // holds those the endgame table accounts for)
     uint64_t deadline_ns;      // %globaltimer value; 0 = none
     const int *abort_flag;     // optional host/device abort request
-    uint64_t *tt;              // this warp's table of explored states (free order); null = none
-    uint32_t *tt_gen;          // this warp's generation counter of that table (kept across launches)
-    int tt_bits;               // log2 of its entries
+    ulonglong2 *tt;            // the launch's table of explored states (free order); null = none
+    uint64_t tt_id;            // number of the launch's first search in it
+    int tt_shift;              // 64 - log2 of its entries
     uint32_t restart_base;     // free order: base of the restart budgets (td_attempt_budget); 0 = none
     const int *cutoff;         // a split ordered search: lowest rank with a witness so far; null = none
     int rank;                  // that search's own rank (it stops once *cutoff < rank)
@@ -459,9 +459,10 @@ __device__ __forceinline__ int td_next_child(td_warp_smem &s, int level, int *ac
 struct __align__(16) td_item {  // 32 bytes
     uint64_t L;
     uint32_t inst;          // instance index
-    uint8_t depth;          // bits 0-6: DFS depth of the node (0 only for the root of an inverse
-                            // instance); bit 7: the node belongs to the inverse instance's search
-    uint8_t off;
+    uint8_t depth;          // bits 0-3: DFS depth of the node (0 only for the root of an inverse
+                            // instance); bit 7: the node belongs to the inverse instance's search;
+                            // bits 4-6: low bits of the restart attempt that donated it
+    uint8_t off;            // bits 0-4; bits 5-7: high bits of that attempt
     uint16_t path[TD_MAX_DEPTH];
 };
 
@@ -512,6 +513,7 @@ struct td_donate_ctx {
     uint32_t inst;
     td_inst_state *state;
     int side;               // 1: the unit searches the instance's inverse (items carry it on)
+    int attempt;            // the restart attempt that donated the unit (0 for a root)
     int race;               // > 0: the unit queues its inverse when it starts restart attempt
                             // `race` (root units of full-sorting instances in td_steal_kernel)
     int spawn_base;         // the race's queue: item slots [spawn_base, spawn_base + spawn_capacity)
@@ -536,7 +538,7 @@ struct td_dfs_out {
 // across the warp).
 __device__ __forceinline__ int td_donate(td_warp_smem &s, const td_donate_ctx &dc,
                                          const td_codes &code, int d0, int level, int N,
-                                         int want) {
+                                         int want, int attempt) {
     const int lane = threadIdx.x & 31;
     int lv = -1;
     for (int l = d0; l <= level && l <= dc.max_level; ++l) {
@@ -606,8 +608,8 @@ __device__ __forceinline__ int td_donate(td_warp_smem &s, const td_donate_ctx &d
         td_item it;
         it.L = nL;
         it.inst = dc.inst;
-        it.depth = (uint8_t)((lv + 1) | (dc.side << 7));
-        it.off = (uint8_t)noff;
+        it.depth = (uint8_t)((lv + 1) | ((attempt & 7) << 4) | (dc.side << 7));
+        it.off = (uint8_t)(noff | ((attempt >> 3) << 5));
 #pragma unroll
         for (int d = 0; d < TD_MAX_DEPTH; ++d) it.path[d] = d < lv ? s.path[d] : (d == lv ? (uint16_t)t : 0);
         int phys = slot;
@@ -825,62 +827,61 @@ __device__ __forceinline__ bool td_filtered_witness(td_warp_smem &s, const td_in
 // or a smaller depth.  Whether a node's subtree holds a witness depends only
 // on its pinned state L (not on where the caller's array starts: a move is the
 // same cycle rotation from any start, so the reachable states do not depend
-// on it) and on its depth.  Each warp keeps a direct-mapped table of
-// (L, depth) for the states it expanded in its current unit, and skips a
-// child whose state is in the table at a depth <= the child's.  This is sound:
-// the earlier node was explored with at least as much budget, unless it is an
-// ancestor still being explored (which has more budget) or its children were
-// donated (then their takers explore them).  The search stops at the first
-// witness, so every completed entry is a state without one.
+// on it) and on its depth.  The warps of a launch share one direct-mapped
+// table of the states they took up, and a child whose state is in the table
+// for the same search at a depth <= the child's is skipped.  This is sound
+// also where the entry is another warp's, whose subtree is still being
+// searched: whoever records a state takes up each of its children, finds it
+// recorded for the same search with at least as much budget, leaves it to the
+// endgame table or donates it (the taker then records it or finds it
+// recorded).  So, by induction on the length of a state's shortest witness,
+// some warp meets the witness of every recorded state; and a search only ends
+// without one when every unit of it has ended.
 //
-// An entry is one word.  The state's 57-bit key (td_tt_key) is multiplied by
-// an odd constant modulo 2^57, a bijection; the top tt_bits bits of the
-// product pick the slot and the other 57 - tt_bits bits are stored as the
-// tag, so (slot, tag) still identifies the state.  That leaves tt_bits + 3
-// bits for a generation (15 at the default 4096 entries) under the depth in
-// the top nibble.  Entries of other generations never match.  Each unit that
-// uses the table, and each restart (which abandons the entries of the
-// attempt: their subtrees were not all searched), takes the warp's next
-// generation from a counter kept in global memory across units and launches,
-// so the table is cleared only when that counter wraps (every 32767 units at
-// 4096 entries) instead of once per unit.  Zero words are empty (generation 0
-// is never used).
+// An entry is one 16-byte word, read and written whole (128-bit relaxed
+// accesses), so it always names one state exactly:
+//   word 0: the state's key (td_tt_key, 57 bits), low 7 bits of the search's
+//           number on top
+//   word 1: the search's number (the other 51 bits), the side (1 bit: the
+//           instance or its inverse), the restart attempt (6 bits: the
+//           subtrees of an abandoned attempt were not all searched) and the
+//           depth (4 bits)
+// A search's number is its launch's epoch and its index there (58 bits), so
+// the entries of other launches never match and the table is never cleared.
+// Zero words are empty (a recorded state has depth >= 1).
+//
+// Each warp had a table of its own before (4,096 entries of 8 bytes, 155 MB in
+// all): the warps that shared a long search explored the same states again.
+// The hardest of 2,048 S_16 instances at their lower bound took 171,000 to
+// 258,000 expansions then, against about 14,000 with one table.
 
-// A unit starts using its table after this many expansions: most searches of
-// uniform permutations end sooner, and they then never touch the table.
+// A search starts using the table after this many expansions of a unit: most
+// searches of uniform permutations end sooner, and they then never touch it.
 // States expanded before are simply not recorded.
+#ifndef TD_TT_AFTER
 #define TD_TT_AFTER 32
-#define TD_TT_KEY 0x01ffffffffffffffull  // the 57 bits of a state key
-#define TD_TT_MULT 0x9E3779B97F4A7C15ull  // odd: multiplying by it permutes keys modulo 2^57
+#endif
 
-__device__ __forceinline__ void td_tt_clear(const td_search_limits &lim) {
-    const int lane = threadIdx.x & 31;
-    uint4 *t = reinterpret_cast<uint4 *>(lim.tt);
-    const int n4 = 1 << (lim.tt_bits - 1);
-    for (int q = lane; q < n4; q += 32) t[q] = make_uint4(0u, 0u, 0u, 0u);
-    __syncwarp();
+__device__ __forceinline__ void td_tt_load(const ulonglong2 *p, uint64_t &a, uint64_t &b) {
+    asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+                 : "=l"(a), "=l"(b)
+                 : "l"(p)
+                 : "memory");
 }
 
-// The warp's next table generation (uniform across the warp); clears the
-// table when the counter wraps.
-__device__ __forceinline__ uint32_t td_tt_next_gen(const td_search_limits &lim) {
-    const uint32_t gmax = (1u << (lim.tt_bits + 3)) - 1u;
-    uint32_t g = *(volatile uint32_t *)lim.tt_gen + 1u;
-    __syncwarp();
-    if (g > gmax) {
-        td_tt_clear(lim);
-        g = 1u;
-    }
-    if ((threadIdx.x & 31) == 0) *lim.tt_gen = g;
-    __syncwarp();
-    return g;
+__device__ __forceinline__ void td_tt_store(ulonglong2 *p, uint64_t a, uint64_t b) {
+    asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }"
+                 :
+                 : "l"(p), "l"(a), "l"(b)
+                 : "memory");
 }
 
-// Looks up the state of level `lv` (depth lv) in generation `gen` of the table
-// and records it there; returns whether it was already explored in this
-// generation at a depth <= lv (uniform across the warp).
+// Looks up the state of level `lv` (depth lv) in the table and records it
+// there; returns whether it was already taken up at a depth <= lv by the
+// search `sub` (side << 6 | attempt) of instance `inst` of this launch
+// (uniform across the warp).
 __device__ __forceinline__ bool td_tt_visit(const td_warp_smem &s, const td_search_limits &lim, int lv, int N,
-                                            uint32_t gen) {
+                                            uint32_t inst, uint32_t sub) {
     const int m = threadIdx.x & 31;
     const int a = m < N ? s.A[lv][m] : 0xff;
     const int c0 = __ffs(__ballot_sync(TD_FULL, a == 0)) - 1;  // caller position of label 0
@@ -897,13 +898,14 @@ __device__ __forceinline__ bool td_tt_visit(const td_warp_smem &s, const td_sear
     hi = __reduce_or_sync(TD_FULL, hi);
     int hit = 0;
     if (m == 0) {
-        const uint64_t h = (td_tt_key((((uint64_t)hi) << 32) | lo) * TD_TT_MULT) & TD_TT_KEY;
-        const int tag_bits = 57 - lim.tt_bits;
-        const uint32_t slot = (uint32_t)(h >> tag_bits);
-        const uint64_t want = (h & ((1ull << tag_bits) - 1ull)) | ((uint64_t)gen << tag_bits);
-        const uint64_t old = lim.tt[slot];
-        hit = (old & ((1ull << 60) - 1ull)) == want && (int)(old >> 60) <= lv;
-        if (!hit) lim.tt[slot] = want | ((uint64_t)lv << 60);
+        const uint64_t id = lim.tt_id + inst;
+        const uint64_t w0 = td_tt_key((((uint64_t)hi) << 32) | lo) | (id << 57);
+        const uint64_t w1 = ((id >> 7) << 7) | sub;
+        ulonglong2 *e = lim.tt + (((w0 + w1 * 0xD6E8FEB86659FD93ull) * 0x9E3779B97F4A7C15ull) >> lim.tt_shift);
+        uint64_t e0, e1;
+        td_tt_load(e, e0, e1);
+        hit = e0 == w0 && (e1 >> 4) == w1 && (int)(e1 & 15u) <= lv;
+        if (!hit) td_tt_store(e, w0, (w1 << 4) | (uint64_t)lv);
     }
     return __shfl_sync(TD_FULL, hit, 0) != 0;
 }
@@ -957,8 +959,6 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
     uint32_t work = 1;  // nodes expanded here
     r.expansions = 1;
     int since_check = 0;
-    bool tt_on = false;  // the table is in use (free order, after TD_TT_AFTER expansions)
-    uint32_t tt_gen = 0;  // its current generation
     int attempt = 0;     // free order: restarts with another child order (td_attempt_budget)
     uint32_t ord = 0, attempt_exp = 1;
     uint32_t attempt_budget = ORDERED ? ~0u : td_attempt_budget(lim.restart_base, 0);
@@ -966,6 +966,8 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
     // once it queued the inverse) looks for the other side's verdict every 16
     // expansions, so that the loser stops soon after the winner
     bool raced = !ORDERED && dc && dc->side;
+    // the search that the unit's states are recorded for (td_tt_visit)
+    const uint32_t tt_sub = dc ? (uint32_t)(dc->side << 6 | dc->attempt) : 0u;
     for (;;) {
         if (found >= 0) {
             r.found_move = (uint16_t)found;
@@ -979,9 +981,9 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
         }
         if constexpr (!ORDERED) {
             if (attempt_exp >= attempt_budget && !solved) {
-                // restart the subtree at d0 with the next child order; the table
-                // held nodes of the abandoned attempt that were not explored to
-                // the end, so it is cleared before its next use
+                // restart the subtree at d0 with the next child order; the
+                // abandoned attempt's states were not explored to the end, so
+                // the next attempt's entries have another number
                 ++attempt;
                 // a root search that may race queues its inverse when it starts
                 // attempt dc->race; another warp then searches it alongside
@@ -990,7 +992,6 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
                 ord = td_order_variant(attempt);
                 attempt_budget = td_attempt_budget(lim.restart_base, attempt);
                 attempt_exp = 1;
-                if (tt_on) tt_gen = td_tt_next_gen(lim);  // the abandoned attempt's entries no longer match
                 level = d0;
                 expand();
                 ++work;
@@ -1025,7 +1026,7 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
                 // a search that has handed out subtrees no longer restarts: the
                 // subtrees of an abandoned attempt would go on being searched,
                 // and searching in parallel already varies the order
-                if (hungry > 0 && !solved && td_donate(s, *dc, code, d0, level, N, min(hungry, dc->grain)) > 0)
+                if (hungry > 0 && !solved && td_donate(s, *dc, code, d0, level, N, min(hungry, dc->grain), dc->attempt + attempt) > 0)
                     attempt_budget = ~0u;
             }
         }
@@ -1107,13 +1108,10 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
                     }
                     if (e != TD_EG_UNKNOWN) continue;
                 }
-                if (lim.tt && !solved) {
-                    if (!tt_on && r.expansions >= TD_TT_AFTER) {
-                        tt_gen = td_tt_next_gen(lim);
-                        tt_on = true;
-                    }
-                    if (tt_on && td_tt_visit(s, lim, level + 1, N, tt_gen)) continue;  // explored with at least this budget
-                }
+                // taken up already with at least this budget?
+                if (lim.tt && !solved && (work >= TD_TT_AFTER || d0 > 0) &&
+                    td_tt_visit(s, lim, level + 1, N, dc ? dc->inst : 0u, tt_sub + (uint32_t)attempt))
+                    continue;
                 break;
             }
         }

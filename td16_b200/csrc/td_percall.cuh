@@ -46,10 +46,8 @@ struct PercallServer {
     td_pool *d_pool = nullptr;
     td_item *d_items = nullptr;
     uint32_t *d_ready = nullptr;
-    uint64_t *d_tt = nullptr;
-    uint32_t *d_tt_gen = nullptr;
-    size_t tt_warps = 0;
-    int tt_bits = 0;
+    ulonglong2 *d_tt = nullptr;
+    int tt_log2 = 0;
     // tickets are numbered across the launches of this server, so a stamp of
     // one launch never matches a request of another
     unsigned long long published = 0;
@@ -90,7 +88,6 @@ void percall_free(PercallServer &ps) {
     if (ps.d_items) cudaFree(ps.d_items);
     if (ps.d_ready) cudaFree(ps.d_ready);
     if (ps.d_tt) cudaFree(ps.d_tt);
-    if (ps.d_tt_gen) cudaFree(ps.d_tt_gen);
     if (ps.stream) cudaStreamDestroy(ps.stream);
     delete[] ps.taken;
     ps.allocated = ps.running = ps.retiring = false;
@@ -107,9 +104,7 @@ void percall_free(PercallServer &ps) {
     ps.d_items = nullptr;
     ps.d_ready = nullptr;
     ps.d_tt = nullptr;
-    ps.d_tt_gen = nullptr;
-    ps.tt_warps = 0;
-    ps.tt_bits = 0;
+    ps.tt_log2 = 0;
     ps.published = 0;
     ps.taken = nullptr;
     ps.inflight = 0;
@@ -176,21 +171,16 @@ int percall_start(PercallServer &ps, int device, char *err, size_t errlen) {
                                                            warps * 32, smem));
     // half of each SM's block slots: batch launches keep the other half
     const int grid = cfg.sms * std::max(1, per_sm / 2);
-    if (cfg.tt_bits > 0 && ((size_t)grid * warps > ps.tt_warps || cfg.tt_bits != ps.tt_bits)) {
+    const int tt_log2 = tt_entries_log2((size_t)grid * warps, cfg.tt_bits);
+    if (cfg.tt_bits > 0 && tt_log2 != ps.tt_log2) {
         // in stream order: a cudaFree would wait for the device's other
         // server launch, which may be draining
         if (ps.d_tt) TD_CHECK(cudaFreeAsync(ps.d_tt, ps.stream));
-        if (ps.d_tt_gen) TD_CHECK(cudaFreeAsync(ps.d_tt_gen, ps.stream));
         ps.d_tt = nullptr;
-        ps.d_tt_gen = nullptr;
-        ps.tt_warps = 0;
-        const size_t words = (size_t)grid * warps << cfg.tt_bits;
-        TD_CHECK(cudaMallocAsync(&ps.d_tt, words * sizeof(uint64_t), ps.stream));
-        TD_CHECK(cudaMallocAsync(&ps.d_tt_gen, (size_t)grid * warps * sizeof(uint32_t), ps.stream));
-        TD_CHECK(cudaMemsetAsync(ps.d_tt, 0, words * sizeof(uint64_t), ps.stream));
-        TD_CHECK(cudaMemsetAsync(ps.d_tt_gen, 0, (size_t)grid * warps * sizeof(uint32_t), ps.stream));
-        ps.tt_warps = (size_t)grid * warps;
-        ps.tt_bits = cfg.tt_bits;
+        ps.tt_log2 = 0;
+        TD_CHECK(cudaMallocAsync(&ps.d_tt, sizeof(ulonglong2) << tt_log2, ps.stream));
+        TD_CHECK(cudaMemsetAsync(ps.d_tt, 0, sizeof(ulonglong2) << tt_log2, ps.stream));
+        ps.tt_log2 = tt_log2;
     }
     // the launch starts at the next ticket: its dispatcher and workers begin
     // there, and the item tags of the previous launch are cleared
@@ -209,7 +199,7 @@ int percall_start(PercallServer &ps, int device, char *err, size_t errlen) {
     td_serve_kernel<TD_SERVE_PER_REQUEST><<<grid, warps * 32, smem, ps.stream>>>(
         ps.d_ring, ps.d_res, ps.d_done, kPercallRing, ps.d_hctl, ps.d_ctl, ps.d_queue, ps.d_state, ps.d_pool,
         ps.d_items, ps.d_ready, kPercallItems, cfg.serve_grain, cfg.serve_split_level, cfg.serve_check_every, 0,
-        life_ns, cfg.tt_bits > 0 ? ps.d_tt : nullptr, ps.d_tt_gen, cfg.tt_bits, cfg.restart_base, request_ns,
+        life_ns, cfg.tt_bits > 0 ? ps.d_tt : nullptr, 64 - tt_log2, cfg.restart_base, request_ns,
         (uint64_t)g_percall_idle_ns.load(), cfg.race ? 1 : 0);  // mostly idle warps: race from the first restart
     TD_CHECK(cudaGetLastError());
     ps.grid = grid;

@@ -80,12 +80,12 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                                                       td_instance *queue, td_inst_state *state, td_pool *pool,
                                                       td_item *items, uint32_t *ready, int item_capacity,
                                                       int grain, int max_level, int check_every, uint64_t max_exp,
-                                                      uint64_t time_limit_ns, uint64_t *tt, uint32_t *tt_gen,
-                                                      int tt_bits, uint32_t restart_base,
+                                                      uint64_t time_limit_ns, ulonglong2 *tt, int tt_shift,
+                                                      uint32_t restart_base,
                                                       uint64_t request_limit_ns, uint64_t idle_exit_ns, int race) {
     constexpr bool ALL_ORDERED = MODE == TD_SERVE_ORDERED;
     extern __shared__ __align__(16) uint8_t td_smem[];
-    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
     const uint64_t deadline = td_globaltimer() + time_limit_ns;
     if (blockIdx.x == 0 && warp == 0) {
@@ -152,9 +152,9 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
     lim.max_work = ~0u;
     lim.deadline_ns = deadline;
     lim.abort_flag = nullptr;
-    lim.tt = (!ALL_ORDERED && tt) ? tt + ((size_t)(blockIdx.x * warps + warp) << tt_bits) : nullptr;
-    lim.tt_gen = lim.tt ? tt_gen + blockIdx.x * warps + warp : nullptr;
-    lim.tt_bits = tt_bits;
+    lim.tt = ALL_ORDERED ? nullptr : tt;
+    lim.tt_id = 0;  // requests are numbered across the launches that share a table
+    lim.tt_shift = tt_shift;
     lim.restart_base = 0;  // serving searches are not restarted
     lim.cutoff = nullptr;
     lim.rank = 0;
@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
     dc.ring = 1;
     dc.tickets = 0;
     dc.side = 0;
+    dc.attempt = 0;
     dc.race = 0;  // set per fresh request (the per-call server's race)
     dc.spawn_base = 0;
     dc.spawn_capacity = 0;
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
         bool ord = ALL_ORDERED;  // this unit's move order (donated subtrees: free)
         int d0 = 0;
         int side = 0;  // 1: a unit of the request's inverse (the per-call server's race)
+        int attempt = 0;  // the restart attempt that donated it
         if (kind == 1) {
             const unsigned slot = (unsigned)(req % ring_size);
             const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(&queue[slot]));
@@ -296,18 +298,23 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(&queue[slot]));
                 const td_instance x = *reinterpret_cast<const td_instance *>(&v);
                 td_setup_root(s, x, code, codeN);
-                d0 = it.depth & 0x7f;
+                d0 = it.depth & 15;
                 side = it.depth >> 7;
+                attempt = ((it.depth >> 4) & 7) | ((it.off >> 5) << 3);
                 if (lane == 0) {
                     s.L[d0] = it.L;
-                    s.off[d0] = it.off;
+                    s.off[d0] = it.off & 31;
                     for (int d = 0; d < d0; ++d) s.path[d] = it.path[d];
                 }
                 __syncwarp();
                 int stop = 0;
                 if (lane == 0) stop = *(volatile int *)&state[slot].found;
                 run = !__shfl_sync(TD_FULL, stop, 0);
-                if (!run) {  // the request already has its witness
+                td_unpack_state(s, d0, it.L, it.off & 31, x.n_symbols);
+                if (run && d0 > 0 && lim.tt &&
+                    td_tt_visit(s, lim, d0, x.n_symbols, (uint32_t)req, (uint32_t)(side << 6 | attempt)))
+                    run = false;
+                if (!run) {  // the request has its witness, or another unit took the state up
                     if (td_finish_unit<true>(r, &state[slot], &results[slot], s.path, side) && lane == 0) {
                         done[slot] = (unsigned long long)req + 1ull;
                         atomicAdd(&dctl->served, 1ull);
@@ -329,10 +336,12 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
             // inverse from restart attempt `race` (td_steal_kernel's race).
             ulim.restart_base = kind == 1 || d0 == 0 ? restart_base : 0;
             dc.side = side;
+            dc.attempt = attempt;
             dc.race = MODE == TD_SERVE_PER_REQUEST && kind == 1 && !ord && restart_base && td_inst_full(x) ? race : 0;
             if (ord) r = td_dfs<true>(s, code, x.n_symbols, d0, ulim, nullptr);
             else r = td_dfs<false>(s, code, x.n_symbols, d0, ulim, &dc);
             dc.side = 0;
+            dc.attempt = 0;
             dc.race = 0;
             // a witness of the inverse becomes one of the request; one that does
             // not convert is reported as a failed replay, and one that leaves the
@@ -377,8 +386,7 @@ struct Server {
     td_item *d_items = nullptr;
     uint32_t *d_ready = nullptr;
     int item_capacity = 0;
-    uint64_t *d_tt = nullptr;  // tables of explored states, one per worker warp (free order)
-    uint32_t *d_tt_gen = nullptr;  // their generation counters
+    ulonglong2 *d_tt = nullptr;  // table of explored states (free order)
     unsigned long long published = 0;
     int workers = 0;
     // per slot: ticket + 1 of the last request whose result the client took
@@ -402,7 +410,6 @@ void server_free(Server *sv) {
     if (sv->d_items) cudaFree(sv->d_items);
     if (sv->d_ready) cudaFree(sv->d_ready);
     if (sv->d_tt) cudaFree(sv->d_tt);
-    if (sv->d_tt_gen) cudaFree(sv->d_tt_gen);
     if (sv->stream) cudaStreamDestroy(sv->stream);
     delete sv;
 }
@@ -481,15 +488,10 @@ TD_API int td_serve_open(int device, unsigned ring_size, unsigned flags, double 
     }
     const int grid = g_dev[device].sms * std::max(1, per_sm);
     sv->workers = grid * warps - 1;
-    const int tt_bits = ordered ? 0 : cfg.tt_bits;
-    if (tt_bits > 0) {
-        const size_t tt_bytes = ((size_t)grid * warps << tt_bits) * sizeof(uint64_t);
-        if ((e = cudaMalloc(&sv->d_tt, tt_bytes)) != cudaSuccess) return fail(e, __LINE__);
-        if ((e = cudaMalloc(&sv->d_tt_gen, (size_t)grid * warps * sizeof(uint32_t))) != cudaSuccess)
-            return fail(e, __LINE__);
-        if ((e = cudaMemsetAsync(sv->d_tt, 0, tt_bytes, sv->stream)) != cudaSuccess) return fail(e, __LINE__);
-        if ((e = cudaMemsetAsync(sv->d_tt_gen, 0, (size_t)grid * warps * sizeof(uint32_t), sv->stream)) !=
-            cudaSuccess)
+    const int tt_log2 = tt_entries_log2((size_t)grid * warps, cfg.tt_bits);
+    if (!ordered && cfg.tt_bits > 0) {
+        if ((e = cudaMalloc(&sv->d_tt, sizeof(ulonglong2) << tt_log2)) != cudaSuccess) return fail(e, __LINE__);
+        if ((e = cudaMemsetAsync(sv->d_tt, 0, sizeof(ulonglong2) << tt_log2, sv->stream)) != cudaSuccess)
             return fail(e, __LINE__);
     }
     const uint64_t limit_ns = (uint64_t)((time_limit_s > 0 ? time_limit_s : 60.0) * 1e9);
@@ -497,12 +499,12 @@ TD_API int td_serve_open(int device, unsigned ring_size, unsigned flags, double 
         td_serve_kernel<TD_SERVE_ORDERED><<<grid, warps * 32, smem, sv->stream>>>(
             sv->d_ring, sv->d_res, sv->d_done, ring_size, sv->d_hctl, sv->d_ctl, sv->d_queue, sv->d_state,
             sv->d_pool, sv->d_items, sv->d_ready, sv->item_capacity, cfg.serve_grain, cfg.serve_split_level,
-            cfg.serve_check_every, 0, limit_ns, nullptr, nullptr, 0, 0u, 0ull, 0ull, 0);
+            cfg.serve_check_every, 0, limit_ns, nullptr, 64, 0u, 0ull, 0ull, 0);
     else
         td_serve_kernel<TD_SERVE_FREE><<<grid, warps * 32, smem, sv->stream>>>(
             sv->d_ring, sv->d_res, sv->d_done, ring_size, sv->d_hctl, sv->d_ctl, sv->d_queue, sv->d_state,
             sv->d_pool, sv->d_items, sv->d_ready, sv->item_capacity, cfg.serve_grain, cfg.serve_split_level,
-            cfg.serve_check_every, 0, limit_ns, sv->d_tt, sv->d_tt_gen, tt_bits, 0u, 0ull, 0ull, 0);
+            cfg.serve_check_every, 0, limit_ns, sv->d_tt, 64 - tt_log2, 0u, 0ull, 0ull, 0);
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, __LINE__);
     *handle = sv;
     return TD_OK;
