@@ -137,16 +137,21 @@ int td_configure(int warps_per_block, int grain);
 int td_set_time_limit(double seconds);
 /* Work donation of the free-order engine: items per donation, deepest level
  * whose children may be donated, expansions between idle checks (default
- * 4, 2, 64: the best setting for one blocking search per call; the
- * autotuner's tuned.json holds the batch settings). */
+ * 4, 2, 64; the autotuner's tuned.json holds the settings of its buckets).
+ * They hold while fresh instances are left; a warp that has met idle warps
+ * checks 16 times as often and gives 8 times as many items (at most 32), from
+ * up to 4 levels deeper. */
 int td_configure_steal(int grain, int split_level, int check_every);
 /* The same for later serving launches (td_serve_open), kept apart because a
- * serving launch trades throughput for latency (default 1, 2, 32). */
+ * serving launch trades throughput for latency (default 1, 2, 32; a serving
+ * launch mostly has idle warps, so it gives 4 times as many items, from up to
+ * 2 levels deeper, and checks 4 times as often). */
 int td_configure_serve(int grain, int split_level, int check_every);
-/* Free order only: each warp keeps a table of the states it explored in its
- * current search and skips a child already explored with at least its depth
- * budget.  2^bits entries of 8 bytes per resident warp (6..16; default 12),
- * or 0 for none.  Verdicts do not depend on it. */
+/* Free order only: the warps of a launch share a table of the states they took
+ * up, and skip a child already taken up by the same search with at least its
+ * depth budget.  2^(bits - 2) entries of 16 bytes per resident warp, rounded
+ * down to a power of two in all (6..16; default 12: 64 MiB per slot), or 0 for
+ * none.  Verdicts do not depend on it. */
 int td_configure_table(int bits);
 /* Free-order batch searches restart with another child order after
  * base x 1, 1, 2, 1, 1, 2, 4, ... expansions (the Luby sequence; after 32

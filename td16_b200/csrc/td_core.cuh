@@ -216,6 +216,17 @@ TD_HD void td_row_classes_x(uint32_t Si, uint32_t Gi, uint32_t Pi, uint32_t Sj, 
     *zero = (all & ~split) | z_one;
 }
 
+// The +2 children of pair (i, j) where every cycle is odd: then two symbols of
+// one cycle and a third apart never gain (their merged cycle would be even),
+// and all three on one cycle (S = the common row) split it in three odd cycles
+// when the cases above hold, with P3 = ~Pi.  g1 and p1 are full masks.
+TD_HD uint32_t td_row_plus2_odd(uint32_t S, uint32_t Gi, uint32_t Pi, uint32_t Gj, uint32_t Pj, uint32_t g1,
+                                uint32_t p1) {
+    const uint32_t two = (g1 & ~(Gi ^ Gj)) | (~g1 & Gj & ~Gi);
+    const uint32_t maj = (p1 & (Pj | ~Pi)) | (~p1 & Pj & ~Pi);
+    return S & two & maj;
+}
+
 TD_HD void td_row_classes(uint32_t Si, uint32_t Gi, uint32_t Pi, uint32_t Sj, uint32_t Gj, uint32_t Pj,
                           uint32_t O, uint32_t F, int i, int j, uint32_t *plus2, uint32_t *zero) {
     td_row_classes_x(Si, Gi, Pi, Sj, Gj, Pj, O, F, 0u - ((O >> i) & 1u), 0u - ((O >> j) & 1u),

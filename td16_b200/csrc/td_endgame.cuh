@@ -129,7 +129,7 @@ __device__ __forceinline__ uint32_t td_eg_skip(td_warp_smem &s, int level, int N
 // decides the children of `level` by the table.  Where one can be sorted it
 // becomes the level's only child (returns true); otherwise only the children
 // that the table does not hold stay.
-__device__ __forceinline__ bool td_eg_filter(td_warp_smem &s, const td_codes &code, int level, int N) {
+__device__ __noinline__ bool td_eg_filter(td_warp_smem &s, int level, int N) {
     const int lane = threadIdx.x & 31;
     const uint32_t fixed = td_eg_fixed(s, level, N);
     uint64_t L;
@@ -139,6 +139,7 @@ __device__ __forceinline__ bool td_eg_filter(td_warp_smem &s, const td_codes &co
     uint32_t W0 = Wv.x, W1 = Wv.y, W2 = Wv.z, W3 = Wv.w;
     __syncwarp();
     s.pw[level][lane] = make_uint4(0u, 0u, 0u, 0u);
+    const ushort4 pq = s.pair[lane];
     bool solved = false;
     for (;;) {
         const int mine = __popc(W0) + __popc(W1) + __popc(W2) + __popc(W3);
@@ -153,11 +154,11 @@ __device__ __forceinline__ bool td_eg_filter(td_warp_smem &s, const td_codes &co
         at -= mine;
         for (int q = 0; q < mine && at < 32; ++q, ++at) {
             uint32_t pc, b;
-            if (W3) { pc = code[3]; b = __ffs(W3) - 1; W3 &= ~(1u << b); }
-            else if (W2) { pc = code[2]; b = __ffs(W2) - 1; W2 &= ~(1u << b); }
-            else if (W1) { pc = code[1]; b = __ffs(W1) - 1; W1 &= ~(1u << b); }
-            else { pc = code[0]; b = __ffs(W0) - 1; W0 &= ~(1u << b); }
-            s.list[at] = (uint16_t)((pc & 1023u) | ((b + 1) << 10));
+            if (W3) { pc = pq.w; b = __ffs(W3) - 1; W3 &= ~(1u << b); }
+            else if (W2) { pc = pq.z; b = __ffs(W2) - 1; W2 &= ~(1u << b); }
+            else if (W1) { pc = pq.y; b = __ffs(W1) - 1; W1 &= ~(1u << b); }
+            else { pc = pq.x; b = __ffs(W0) - 1; W0 &= ~(1u << b); }
+            s.list[at] = (uint16_t)(pc | ((b + 1) << 10));
         }
         __syncwarp();
         uint32_t e = 1, t = 0;
@@ -176,7 +177,7 @@ __device__ __forceinline__ bool td_eg_filter(td_warp_smem &s, const td_codes &co
             // back to its pair's slot (td_pair_code)
             const int i = t & 31, j = (t >> 5) & 31, k = (t >> 10) & 31;
             const int q = (N - 1) * (N - 2) / 2 - 1 - (i * (N - 2) - i * (i - 1) / 2 + (j - i - 1));
-            const int R = (int)(code[TD_MAX_ROUNDS] & 255u);
+            const int R = td_pair_rounds(N);
             atomicOr(reinterpret_cast<uint32_t *>(&s.pw[level][q / R]) + q % R, 1u << (k - 1));
         }
         __syncwarp();
@@ -238,8 +239,7 @@ __global__ void __launch_bounds__(256, 4) td_eg_build_kernel(int missing) {
     extern __shared__ __align__(16) uint8_t td_smem[];
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     td_warp_smem &s = reinterpret_cast<td_warp_smem *>(td_smem)[warp];
-    td_codes code;
-    int codeN = -1;
+    int pairs_n = -1;
     // a cycle of two or more symbols misses at least a third of them
     const uint32_t end = 3 * missing >= TD_EG_SYMBOLS ? TD_EG_STATES : td_eg_base(3 * missing);
     int m = 2;
@@ -272,16 +272,16 @@ __global__ void __launch_bounds__(256, 4) td_eg_build_kernel(int missing) {
         uint32_t O, F;
         const int odd = td_prepare_rows(s, 0, N, O, F);
         if ((N - odd) / 2 != missing) continue;
-        if (codeN != N) {
-            td_load_pairs(N, code);
-            codeN = N;
+        if (pairs_n != N) {
+            td_load_pairs(s, N);
+            pairs_n = N;
         }
         if (lane == 0) {  // every +2 child, and nothing else, is one to visit
             s.acc[1] = 0;
             s.reach[1] = 1u << (odd + 2);
         }
         __syncwarp();
-        td_evaluate(s, code, N, 0, odd, O, F);
+        td_evaluate(s, N, 0, odd, O, F);
         const uint32_t e = 1u + td_eg_skip(s, 0, N, 0);
         const uint32_t left = __ballot_sync(TD_FULL, lane < TD_MAX_STEPS && s.cw[0][lane] != 0);
         if (lane == 0) td_eg_table[g] = left ? 0 : (uint16_t)e;

@@ -63,20 +63,23 @@ static_assert(sizeof(td_result) == 32, "td_result layout");
 #define TD_TT_INST_BITS 26  // instances per epoch in the table's search numbers
 #define TD_RESTART_BASE 16  // default base of the free order's restart budgets (expansions)
 
-__device__ __forceinline__ td_search_limits td_make_limits(uint64_t max_exp, uint64_t time_limit_ns,
-                                                           const int *abort_flag) {
-    td_search_limits lim;
-    lim.max_expansions = max_exp ? max_exp : ~0ull;
-    lim.max_work = ~0u;
-    lim.deadline_ns = time_limit_ns ? td_globaltimer() + time_limit_ns : 0;
-    lim.abort_flag = abort_flag;
-    lim.tt = nullptr;
-    lim.tt_id = 0;
-    lim.tt_shift = 0;
-    lim.restart_base = 0;
-    lim.cutoff = nullptr;
-    lim.rank = 0;
-    return lim;
+// Sets the warp's limits: no tables, no restarts.
+__device__ __forceinline__ void td_set_limits(td_warp_smem &s, uint64_t max_exp, uint64_t time_limit_ns) {
+    if ((threadIdx.x & 31) == 0) {
+        td_search_limits lim;
+        lim.max_expansions = max_exp && max_exp < ~0u ? (uint32_t)max_exp : ~0u;
+        lim.max_work = ~0u;
+        lim.deadline_ns = time_limit_ns ? td_globaltimer() + time_limit_ns : 0;
+        lim.tt = nullptr;
+        lim.tt_id = 0;
+        lim.tt_shift = 64;
+        lim.restart_base = 0;
+        lim.cutoff = nullptr;
+        lim.rank = 0;
+        s.lim = lim;
+        s.pairs_n = -1;
+    }
+    __syncwarp();
 }
 
 template <bool ORDERED>
@@ -88,11 +91,9 @@ __global__ void __launch_bounds__(256) td_plain_kernel(const td_instance *__rest
     td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
     const int idx = blockIdx.x * warps + warp;
     if (idx >= count) return;
-    const td_search_limits lim = td_make_limits(max_exp, time_limit_ns, nullptr);
-    td_codes code;
-    int codeN = -1;
+    td_set_limits(ws[warp], max_exp, time_limit_ns);
     const td_instance x = in[idx];
-    td_warp_search<ORDERED>(x, &out[idx], ws[warp], code, codeN, lim);
+    td_warp_search<ORDERED>(x, &out[idx], ws[warp]);
 }
 
 // hard_count / hard_list (or null): the first pass of a split batch of the
@@ -107,10 +108,9 @@ __global__ void __launch_bounds__(256, 4) td_persistent_kernel(const td_instance
     extern __shared__ __align__(16) uint8_t td_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
-    td_codes code;
-    int codeN = -1;
-    td_search_limits lim = td_make_limits(hard_list ? 0 : max_exp, time_limit_ns, nullptr);
-    if (hard_list) lim.max_work = (uint32_t)max_exp;
+    td_set_limits(ws[warp], hard_list ? 0 : max_exp, time_limit_ns);
+    if (hard_list && lane == 0) ws[warp].lim.max_work = (uint32_t)max_exp;
+    __syncwarp();
     for (;;) {
         int first = 0;
         if (lane == 0) first = atomicAdd(ticket, grain);
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256, 4) td_persistent_kernel(const td_instance
         const int last = min(count, first + grain);
         for (int idx = first; idx < last; ++idx) {
             const td_instance x = in[idx];
-            const int st = td_warp_search<ORDERED>(x, &out[idx], ws[warp], code, codeN, lim);
+            const int st = td_warp_search<ORDERED>(x, &out[idx], ws[warp]);
             if (hard_list && st == TD_ERR_BUDGET && lane == 0) hard_list[atomicAdd(hard_count, 1)] = idx;
         }
     }
@@ -171,17 +171,17 @@ __global__ void __launch_bounds__(256) td_split_roots_kernel(const td_instance *
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
     td_warp_smem &s = ws[warp];
+    if (lane == 0) s.pairs_n = -1;
+    __syncwarp();
     const int H = *(volatile int *)&ctl->hard;
-    td_codes code;
-    int codeN = -1;
     for (int h = blockIdx.x * warps + warp; h < H; h += gridDim.x * warps) {
         const td_instance x = in[hard_list[h]];
-        td_setup_root(s, x, code, codeN);
+        td_setup_root(s, x);
         const int N = x.n_symbols, last_tri = td_tri_base(N) + td_triple_count(N) - 1;
         td_unpack_state(s, 0, x.perm, x.offset, N);
         uint32_t O, F;
         const int odd = td_prepare_rows(s, 0, N, O, F);
-        td_evaluate(s, code, N, 0, odd, O, F);
+        td_evaluate(s, N, 0, odd, O, F);
         // count the children, reserve their records, then list them from the
         // last one (the root's visiting order is descending u)
         const uint32_t w = lane < TD_MAX_STEPS ? s.cw[0][lane] : 0u;
@@ -234,9 +234,7 @@ __global__ void __launch_bounds__(256, 4) td_split_kernel(const td_instance *__r
     const int H = *(volatile int *)&ctl->hard;
     const int R = max(1, *(volatile int *)&ctl->max_rank);
     const unsigned long long units = (unsigned long long)H * (unsigned long long)R;
-    td_search_limits lim = td_make_limits(0, time_limit_ns, nullptr);
-    td_codes code;
-    int codeN = -1;
+    td_set_limits(s, 0, time_limit_ns);
     for (;;) {
         unsigned long long u = 0;
         if (lane == 0) u = atomicAdd(&ctl->ticket, 1ull);
@@ -247,8 +245,10 @@ __global__ void __launch_bounds__(256, 4) td_split_kernel(const td_instance *__r
         if (nk < 0) {
             if (r == 0) {
                 const int idx = hard_list[h];
-                lim.cutoff = nullptr;
-                td_warp_search<true>(in[idx], &out[idx], s, code, codeN, lim);
+                __syncwarp();
+                if (lane == 0) s.lim.cutoff = nullptr;
+                __syncwarp();
+                td_warp_search<true>(in[idx], &out[idx], s);
             }
             continue;
         }
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(256, 4) td_split_kernel(const td_instance *__r
         const uint32_t kid = kids[base[h] + r];
         const uint32_t t = kid & 0x7fffu;
         const td_instance x = in[hard_list[h]];
-        td_setup_root(s, x, code, codeN);
+        td_setup_root(s, x);
         const int N = x.n_symbols;
         if (lane == 0) s.path[0] = (uint16_t)t;
         __syncwarp();
@@ -276,11 +276,11 @@ __global__ void __launch_bounds__(256, 4) td_split_kernel(const td_instance *__r
         if (lane == 0) {
             s.L[1] = nL;
             s.off[1] = (uint8_t)noff;
+            s.lim.cutoff = &cutoff[h];
+            s.lim.rank = r;
         }
         __syncwarp();
-        lim.cutoff = &cutoff[h];
-        lim.rank = r;
-        const td_dfs_out d = td_dfs<true>(s, code, N, 1, lim, nullptr);
+        const td_dfs_out d = td_dfs<true>(s, N, 1, false);
         int status = TD_NOT_FOUND;
         if (d.status == TD_DFS_FOUND) status = TD_FOUND;
         else if (d.status == TD_DFS_ABORTED) status = TD_SPLIT_SKIPPED;
@@ -341,7 +341,7 @@ __global__ void td_split_join_kernel(const int *__restrict__ hard_list, const td
 template <bool HOST_OUT>
 __device__ __forceinline__ void td_unit_fence() {
     if (HOST_OUT) __threadfence_system();
-    else __threadfence();
+    else td_fence();
 }
 
 template <bool HOST_OUT>
@@ -401,232 +401,219 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                                                       int max_level, int check_every, uint64_t time_limit_ns,
                                                       ulonglong2 *tt, int tt_shift, unsigned epochs,
                                                       uint32_t restart_base, uint64_t max_exp,
-                                                      unsigned max_backoff_ns, int race, int spawn_base) {
+                                                      int race) {
     extern __shared__ __align__(16) uint8_t td_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
     td_warp_smem &s = ws[warp];
-    td_codes code;
-    int codeN = -1;
     // the expansion budget bounds each unit (the root search and each donated
     // subtree); an instance without a witness whose unit ran out reports
     // TD_ERR_BUDGET
-    td_search_limits lim = td_make_limits(max_exp, time_limit_ns, nullptr);
-    lim.restart_base = restart_base;
-    td_donate_ctx dc;
-    dc.pool = pool;
-    dc.items = items;
-    dc.ready = ready;
+    td_set_limits(s, max_exp, time_limit_ns);
     const uint32_t epoch = *epoch_ptr;  // bumped by td_epoch_kernel before this launch
-    dc.epoch = epoch;
-    // this launch's numbers in the table: its `epochs` epochs, 2^26 searches each
-    lim.tt = tt;
-    lim.tt_shift = tt_shift;
-    lim.tt_id = (uint64_t)(epoch - epochs + 1u) << TD_TT_INST_BITS;
-    // race: donated items use slots [0, spawn_base), queued inverse roots the rest
-    dc.capacity = race ? spawn_base : capacity;
-    dc.spawn_base = spawn_base;
-    dc.spawn_capacity = race ? capacity - spawn_base : 0;
-    dc.side = 0;
-    dc.attempt = 0;
-    dc.race = 0;
-    dc.grain = grain;
-    dc.max_level = max_level;
-    dc.check_every = check_every > 0 ? check_every : 1;
-    dc.ring = 0;
-    dc.tickets = 1;
-    dc.deadline_ns = lim.deadline_ns;
-    unsigned backoff = 64;
+    if (lane == 0) {
+        // this launch's numbers in the table: its `epochs` epochs, 2^26 searches each
+        s.lim.tt_id = (uint64_t)(epoch - epochs + 1u) << TD_TT_INST_BITS;
+        s.lim.tt_shift = tt_shift;
+        td_donate_ctx dc;
+        dc.pool = pool;
+        dc.items = items;
+        dc.ready = ready;
+        dc.epoch = epoch;
+        dc.capacity = capacity;
+        dc.grain = grain;
+        dc.max_level = max_level;
+        dc.check_every = check_every > 0 ? check_every : 1;
+        dc.ring = 0;
+        dc.tickets = 1;
+        dc.deadline_ns = s.lim.deadline_ns;
+        dc.inst = 0;
+        dc.state = nullptr;
+        dc.side = 0;
+        dc.attempt = 0;
+        dc.race = 0;
+        dc.idle_seen = 0;
+        s.dc = dc;
+        // a launch with fewer instances than warps has idle warps from the start
+        if (count < (int)(gridDim.x * (blockDim.x >> 5))) td_serve_idle_warps(s.dc);
+    }
+    __syncwarp();
     // Claims.  A warp takes fresh instances by ticket while any are left, then
-    // one item ticket (fetch-and-add: it never fails) and waits until item
-    // `ticket` has been produced; items go to the waiting warps in ticket
-    // order.  (One compare-and-swap per claim attempt instead made thousands
-    // of idle warps fail on one counter, so the long searches at the end of a
-    // launch, split into thousands of items, were served a few hundred
-    // thousand items per second.)  `outstanding` counts the root units in
-    // progress plus the items not yet finished: it is raised before an
-    // instance ticket is taken and by a donor before its items can be
-    // claimed, and lowered when a unit ends.  With no instance ticket left
-    // and nothing outstanding no unit can start again, so a waiting warp may
-    // leave: its ticket is past every item there will be.
+    // one item ticket (fetch-and-add: it never fails) and waits for its item:
+    // item i belongs to ticket i.  A waiting warp polls only the ready flag of
+    // its own item, so thousands of them load thousands of different words and
+    // none that a busy warp needs, and they can poll often.  `outstanding`
+    // counts the root units in progress plus the items not yet finished: it is
+    // raised before an instance ticket is taken and by a donor before its items
+    // can be claimed, and lowered when a unit ends.  With no instance ticket
+    // left and nothing outstanding no unit can start again: the warp that
+    // brings the count there sets `done` and then ~epoch in the flag of every
+    // ticket taken.  A warp that took its ticket too late for that reads `done`
+    // at its first poll and at every 16th.
+    //
+    // Polling the shared counters instead (five of them, at up to 32 us
+    // intervals, since shorter ones slowed the busy warps) left the warps idle
+    // for most of a launch's tail.
     //
     // Race (`race` = a, 0: off): a root search of a full-sorting instance
     // that starts its restart attempt a queues the instance's inverse
-    // (td_spawn_inverse).  Queued inverses are claimed once no fresh instance
-    // is left, before donated items, by their own tickets (fetch-and-add,
-    // taken only while some are queued).  While fresh instances remain every
-    // warp is busy, and a second search of an instance would only displace
-    // other work; at the end of the launch, where warps idle, it shortens the
+    // (td_spawn_inverse) as an item.  While fresh instances remain every warp
+    // is busy, and a second search of an instance would only displace other
+    // work; at the end of the launch, where warps idle, it shortens the
     // longest searches.  Most queued inverses belong to instances decided by
-    // then and end at once.  A ticket taken past the last inverse queued is
-    // kept until one is queued for it.
+    // then and end at once.
     int my_ticket = -1;  // lane 0: this warp's item ticket, -1 = none
-    int my_spawn = -1;   // lane 0: this warp's ticket of the queue of inverses, -1 = none
+    unsigned polls = 0;
+    bool fresh = true;   // lane 0: instance tickets may be left
+    // lane 0 lowers the outstanding count; whether the launch has no work left
+    auto release = [&]() -> bool {
+        if (atomicSub(&pool->outstanding, 1) != 1 || *(volatile int *)&pool->inst_ticket < count) return false;
+        atomicExch(&pool->done, 1);
+        __threadfence();
+        return true;
+    };
+    // wakes the waiting warps of a launch without work
+    auto wake = [&]() {
+        int from = 0, taken = 0;
+        if (lane == 0) {
+            from = *(volatile int *)&pool->produced;
+            taken = min(*(volatile int *)&pool->consumed, capacity);
+        }
+        from = __shfl_sync(TD_FULL, from, 0);
+        taken = __shfl_sync(TD_FULL, taken, 0);
+        for (int i = from + lane; i < taken; i += 32) *(volatile uint32_t *)&ready[i] = ~epoch;
+    };
+    unsigned backoff = 64;
     for (;;) {
         int kind = 0, unit = -1;
         if (lane == 0) {
-            if (*(volatile int *)&pool->inst_ticket < count) {
-                atomicAdd(&pool->outstanding, 1);
-                const int t = atomicAdd(&pool->inst_ticket, 1);
-                if (t < count) { kind = 1; unit = t; }
-                else atomicSub(&pool->outstanding, 1);
-            }
-            if (!kind && race) {
-                // slots past the queue's capacity are never claimed
-                const int queued = min(*(volatile int *)&pool->spawn_produced, dc.spawn_capacity);
-                if (my_spawn < 0 && *(volatile int *)&pool->spawn_consumed < queued)
-                    my_spawn = atomicAdd(&pool->spawn_consumed, 1);
-                if (my_spawn >= 0 && my_spawn < min(*(volatile int *)&pool->spawn_produced, dc.spawn_capacity)) {
-                    kind = 3;
-                    unit = my_spawn;
-                    my_spawn = -1;
+            if (fresh) {
+                if (*(volatile int *)&pool->inst_ticket < count) {
+                    atomicAdd(&pool->outstanding, 1);
+                    unit = atomicAdd(&pool->inst_ticket, 1);
+                    if (unit < count) kind = 1;
+                    else if (release()) kind = 4;
                 }
+                fresh = kind == 1;
             }
             if (!kind) {
-                if (my_ticket < 0) my_ticket = atomicAdd(&pool->consumed, 1);
-                if (my_ticket < *(volatile int *)&pool->produced) {
+                if (my_ticket < 0) {
+                    my_ticket = atomicAdd(&pool->consumed, 1);
+                    polls = 0;
+                    td_serve_idle_warps(s.dc);
+                }
+                const uint32_t flag = my_ticket < capacity ? *(volatile uint32_t *)&ready[my_ticket] : 0u;
+                if (flag == epoch) {
                     kind = 2;
                     unit = my_ticket;
                     my_ticket = -1;
+                } else if (flag == ~epoch) {
+                    kind = 3;
+                } else if ((polls++ & 15u) == 0) {
+                    // tickets taken after the launch ended, or past the item
+                    // space, are not woken
+                    if (*(volatile int *)&pool->done) {
+                        kind = 3;
+                    } else if (s.lim.deadline_ns && td_globaltimer() > s.lim.deadline_ns) {
+                        atomicCAS(&pool->error, 0, TD_ERR_TIMEOUT);
+                        kind = 3;
+                    }
                 }
             }
         }
         kind = __shfl_sync(TD_FULL, kind, 0);
-        unit = __shfl_sync(TD_FULL, unit, 0);
+        if (kind == 4) wake();
+        if (kind >= 3) break;
         if (!kind) {
-            int done = 0;
-            unsigned cap = max_backoff_ns;
-            if (lane == 0) {
-                // the instance tickets first: once they are gone, an
-                // outstanding count of zero stays zero
-                const int tk = *(volatile int *)&pool->inst_ticket;
-                done = tk >= count && *(volatile int *)&pool->outstanding == 0;
-                if (!done && lim.deadline_ns && td_globaltimer() > lim.deadline_ns) {
-                    atomicCAS(&pool->error, 0, TD_ERR_TIMEOUT);
-                    done = 1;
-                }
-                // the next few tickets in line are served first: they poll often
-                if (my_ticket >= 0 && my_ticket - *(volatile int *)&pool->produced < 64) cap = min(cap, 512u);
-            }
-            if (__shfl_sync(TD_FULL, done, 0)) break;
-            // waiting warps back off (to 32 us in a batch) so that their
-            // counter reads do not crowd the L2 slices the busy warps'
-            // atomics go to; a single search (one per call) caps it lower,
-            // since there the launch ends only when every waiting warp has
-            // woken up and seen that the work is done
-            cap = __shfl_sync(TD_FULL, cap, 0);
-            __nanosleep(min(backoff, cap));
-            backoff = min(backoff * 2u, cap);
+            __nanosleep(backoff);
+            backoff = min(backoff * 2u, 1024u);
             continue;
         }
+        unit = __shfl_sync(TD_FULL, unit, 0);
         backoff = 64;
-        if (kind == 1) {
-            const td_instance x = in[unit];
-            td_inst_state *st = &state[unit];
-            if (!td_instance_ok(x) || td_triple_count(x.n_symbols) == 0) {
-                td_write_result(&out[unit], td_instance_ok(x) ? TD_NOT_FOUND : TD_ERR_ARG, 0, 0, s.path, 0, 0, 8);
-            } else {
-                if (lane == 0) atomicAdd(&st->pending, 1);
-                td_setup_root(s, x, code, codeN);
-                dc.inst = (uint32_t)unit;
-                dc.state = st;
-                dc.side = 0;
-                dc.race = td_inst_full(x) ? race : 0;
-                const td_dfs_out r = td_dfs<false>(s, code, x.n_symbols, 0, lim, &dc);
-                dc.race = 0;
-                td_finish_unit<false>(r, st, &out[unit], s.path);
-            }
+        // the unit: a fresh instance, a donated subtree or a queued inverse root
+        uint32_t idx = (uint32_t)unit;
+        int d0 = 0, side = 0, attempt = 0;
+        td_item it;
+        if (kind == 2) {
+            td_fence();
+            const uint4 *src = reinterpret_cast<const uint4 *>(&items[unit]);
+            uint4 *dst = reinterpret_cast<uint4 *>(&it);
+            dst[0] = __ldcg(src);  // read through L2: the donor wrote it from another SM
+            dst[1] = __ldcg(src + 1);
+            idx = it.inst;
+            d0 = it.depth & 15;
+            side = it.depth >> 7;
+            attempt = ((it.depth >> 4) & 7) | ((it.off >> 5) << 3);
+        }
+        // an item names an instance of this launch and a level of the frame;
+        // one that does not is a launch error, never followed
+        if (kind == 2 && (idx >= (uint32_t)count || d0 >= TD_MAX_DEPTH || (d0 == 0 && !side))) {
+            if (lane == 0) atomicCAS(&pool->error, 0, TD_ERR_VERIFY);
         } else {
-            // a donated item (kind 2) or a queued inverse root (kind 3); wait
-            // until its producer has written it (bounded)
-            const int phys = kind == 3 ? spawn_base + unit : unit;
-            int ok = 0;
-            if (lane == 0) {
-                for (unsigned spin = 0; spin < (1u << 30); ++spin) {
-                    if (*(volatile uint32_t *)&ready[phys] == epoch) { ok = 1; break; }
-                    if ((spin & 1023u) == 0 && lim.deadline_ns && td_globaltimer() > lim.deadline_ns) break;
-                    __nanosleep(32);
-                }
-                if (!ok) atomicCAS(&pool->error, 0, TD_ERR_TIMEOUT);
-                __threadfence();
-            }
-            ok = __shfl_sync(TD_FULL, ok, 0);
-            if (ok) {
-                td_item it;  // read through L2: the donor wrote it from another SM
-                {
-                    const uint4 *src = reinterpret_cast<const uint4 *>(&items[phys]);
-                    uint4 *dst = reinterpret_cast<uint4 *>(&it);
-                    dst[0] = __ldcg(src);
-                    dst[1] = __ldcg(src + 1);
-                }
-                const uint32_t idx = it.inst;
-                const int d0 = it.depth & 15;
-                const int side = it.depth >> 7;
-                const int attempt = ((it.depth >> 4) & 7) | ((it.off >> 5) << 3);
-                // an item names an instance of this launch and a level of the
-                // frame; one that does not is a launch error, never followed
-                if (idx >= (uint32_t)count || d0 >= TD_MAX_DEPTH || (kind == 3) != (side && d0 == 0)) {
-                    if (lane == 0) {
-                        atomicCAS(&pool->error, 0, TD_ERR_VERIFY);
-                        atomicSub(&pool->outstanding, 1);
-                    }
-                    continue;
-                }
-                const td_instance x = in[idx];
-                td_inst_state *st = &state[idx];
-                td_setup_root(s, x, code, codeN);
-                if (lane == 0) {
-                    s.L[d0] = it.L;
-                    s.off[d0] = it.off & 31;
-                    for (int d = 0; d < d0; ++d) s.path[d] = it.path[d];
-                }
-                __syncwarp();
+            const td_instance x = in[idx];
+            td_inst_state *st = &state[idx];
+            if (kind == 1 && (!td_instance_ok(x) || td_triple_count(x.n_symbols) == 0)) {
+                td_write_result(&out[idx], td_instance_ok(x) ? TD_NOT_FOUND : TD_ERR_ARG, 0, 0, s.path, 0, 0, 8);
+            } else {
                 int stop = 0;
-                if (lane == 0) stop = *(volatile int *)&st->found;
-                stop = __shfl_sync(TD_FULL, stop, 0);
-                td_unpack_state(s, d0, it.L, it.off & 31, x.n_symbols);
-                // a donated state that another unit took up needs no second search
-                if (!stop && d0 > 0 && lim.tt && !max_exp)
-                    stop = td_tt_visit(s, lim, d0, x.n_symbols, idx, (uint32_t)(side << 6 | attempt));
-                td_dfs_out r;
-                if (stop) {
-                    r.status = TD_DFS_ABORTED;
-                    r.depth = 0;
-                    r.found_move = 0;
-                    r.expansions = 0;
-                } else {
-                    // a donated subtree is searched once, to the end: restarting it
-                    // would only repeat work when it holds no witness; the root of
-                    // an inverse instance restarts like any root search
-                    td_search_limits ilim = lim;
-                    if (d0 > 0) ilim.restart_base = 0;
+                if (lane == 0) {
+                    if (kind == 1) atomicAdd(&st->pending, 1);
+                    else stop = *(volatile int *)&st->found;
+                    // a donated subtree is searched once, to the end: restarting
+                    // it would only repeat work when it holds no witness; the
+                    // root of an inverse instance restarts like any root search
+                    s.lim.restart_base = d0 > 0 ? 0u : restart_base;
                     // a unit that may run out of its expansion budget leaves
                     // recorded states unsearched: then only roots use the table
-                    if (d0 > 0 && max_exp) ilim.tt = nullptr;
-                    dc.inst = idx;
-                    dc.state = st;
-                    dc.side = side;
-                    dc.attempt = attempt;
-                    r = td_dfs<false>(s, code, x.n_symbols, d0, ilim, &dc);
-                    dc.side = 0;
-                    dc.attempt = 0;
-                    // a witness of the inverse becomes one of the instance; one that
-                    // does not convert is reported as a failed replay, and one that
-                    // leaves the reference's move filter on the instance's side is
-                    // dropped (this side then stops; the instance's own search decides)
-                    if (side && r.status == TD_DFS_FOUND) {
-                        if (!td_inverse_result(s, x, r)) {
-                            r.status = TD_DFS_EXHAUSTED;
-                            if (lane == 0) atomicCAS(&st->error, 0, TD_ERR_VERIFY);
-                        } else if (!td_filtered_witness(s, x, r)) {
-                            r.status = TD_DFS_EXHAUSTED;
-                        }
-                    }
+                    s.lim.tt = d0 > 0 && max_exp ? nullptr : tt;
+                    s.dc.inst = idx;
+                    s.dc.state = st;
+                    s.dc.side = side;
+                    s.dc.attempt = attempt;
+                    s.dc.race = kind == 1 && td_inst_full(x) ? race : 0;
                 }
-                td_finish_unit<false>(r, st, &out[idx], s.path, side);
+                td_setup_root(s, x);
+                if (kind == 2) {
+                    if (lane == 0) {
+                        s.L[d0] = it.L;
+                        s.off[d0] = it.off & 31;
+                        for (int d = 0; d < d0; ++d) s.path[d] = it.path[d];
+                    }
+                    __syncwarp();
+                    stop = __shfl_sync(TD_FULL, stop, 0);
+                    // a donated state that another unit took up needs no second search
+                    if (!stop && d0 > 0 && s.lim.tt) {
+                        td_unpack_state(s, d0, it.L, it.off & 31, x.n_symbols);
+                        stop = td_tt_visit(s, d0, x.n_symbols, idx, (uint32_t)(side << 6 | attempt));
+                    }
+                } else {
+                    stop = 0;
+                }
+                td_dfs_out r;
+                r.status = TD_DFS_ABORTED;
+                r.depth = 0;
+                r.found_move = 0;
+                r.expansions = 0;
+                if (!stop) r = td_dfs<false>(s, x.n_symbols, d0, true);
+                // the unit's names come from shared memory again: registers
+                // are what the search is short of
+                td_inst_state *us = s.dc.state;
+                if (s.dc.side && r.status == TD_DFS_FOUND) {
+                    const int t = td_inverse_witness(s, in[s.dc.inst], r.depth, r.found_move);
+                    if (t < 0) r.status = TD_DFS_EXHAUSTED;
+                    else r.found_move = (uint16_t)t;
+                    if (t == -1 && lane == 0) atomicCAS(&us->error, 0, TD_ERR_VERIFY);
+                }
+                td_finish_unit<false>(r, us, &out[s.dc.inst], s.path, s.dc.side);
             }
         }
-        if (lane == 0) atomicSub(&pool->outstanding, 1);
+        int last = 0;
+        if (lane == 0) last = release();
+        if (__shfl_sync(TD_FULL, last, 0)) {
+            wake();
+            break;
+        }
     }
 }
 
@@ -802,8 +789,8 @@ std::vector<DeviceInfo> g_dev;
 
 int g_warps_per_block = 4;
 int g_grain = 1;            // instances per ticket (ordered persistent kernel)
-// defaults: the best per-call setting (one blocking search per slot call,
-// 16 slots, S_16) measured from native threads; batch callers use tuned ones
+// the settings while fresh instances are left; td_serve_idle_warps says what
+// they become after that
 int g_steal_grain = 4;      // items per donation
 int g_split_level = 2;      // donate children of levels <= this
 int g_check_every = 64;     // expansions between idle checks
@@ -949,6 +936,14 @@ cudaError_t endgame_setup(int device, int sms) {
     return e;
 }
 
+// Uploads the kernels' pair-slot table to the current device.
+cudaError_t upload_pairs() {
+    td_pair_row rows[TD_MAX_N + 1][32];
+    for (int N = 0; N <= TD_MAX_N; ++N)
+        for (int lane = 0; lane < 32; ++lane) rows[N][lane] = td_make_pair_row(N, lane);
+    return cudaMemcpyToSymbol(td_pair_table, rows, sizeof rows);
+}
+
 int ensure_device(int device, char *err, size_t errlen) {
     if ((int)g_dev.size() <= device) g_dev.resize(device + 1);
     DeviceInfo &d = g_dev[device];
@@ -962,6 +957,7 @@ int ensure_device(int device, char *err, size_t errlen) {
                 for (int k = j + 1; k < N; ++k) tri[base + t++] = td_pack_move(i, j, k);
     }
     TD_CHECK(cudaMemcpyToSymbol(td_tri_table, tri.data(), tri.size() * sizeof(uint16_t)));
+    TD_CHECK(upload_pairs());
     TD_CHECK(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device));
     const int max_warps = 8;
     const size_t max_smem = smem_bytes(max_warps);
@@ -1082,15 +1078,14 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
         TD_CHECK(cudaMemsetAsync(s.d_state, 0, (size_t)count * sizeof(td_inst_state), stream));
         td_epoch_kernel<<<1, 1, 0, stream>>>(s.d_epoch, epochs);
         // the race needs restarts, and an expansion budget per unit would make
-        // one side's budget decide the other's; its queue of inverse roots
-        // holds one slot per instance (each queues its inverse at most once),
-        // at the top of the item space, which keeps at least half for donation
+        // one side's budget decide the other's; each instance queues its
+        // inverse at most once, and at least half the item space is left for
+        // donation
         const int race = cfg.restart_base > 0 && max_exp == 0 && count <= s.item_capacity / 2 ? cfg.race : 0;
-        const int spawn_base = race ? s.item_capacity - count : s.item_capacity;
         td_steal_kernel<<<grid, threads, smem_bytes(warps), stream>>>(
             d_in, d_out, count, s.d_pool, s.d_items, s.d_ready, s.d_epoch, s.item_capacity, s.d_state,
             cfg.steal_grain, cfg.split_level, cfg.check_every, time_limit_ns(), cfg.tt_bits > 0 ? s.d_tt : nullptr,
-            64 - s.tt_log2, epochs, cfg.restart_base, max_exp, count == 1 ? 4096u : 32768u, race, spawn_base);
+            64 - s.tt_log2, epochs, cfg.restart_base, max_exp, race);
         TD_CHECK(cudaGetLastError());
         td_finalize_kernel<<<std::max(1, std::min((count + 255) / 256, 2 * cfg.sms)), 256, 0, stream>>>(
             s.d_pool, s.d_state, d_out, count);
@@ -1633,7 +1628,7 @@ TD_API int td_search_batch(int slot, int count, const td_instance *in, td_result
             const td_pool &pool = s->h_stats->pool;
             stats->donations = pool.donations;
             stats->donated_items = pool.donated_items;
-            stats->races = (uint64_t)pool.spawn_produced;
+            stats->races = pool.races;
             if (pool.error) {
                 set_err(err, errlen, "engine launch deadline reached");
                 return TD_TIMEOUT;
@@ -1885,6 +1880,7 @@ int noalloc_setup(int device, char *err, size_t errlen) {
                 for (int k = j + 1; k < N; ++k) g_noalloc_tri[base + t++] = td_pack_move(i, j, k);
     }
     TD_CHECK_NA(cudaMemcpyToSymbol(td_tri_table, g_noalloc_tri, sizeof g_noalloc_tri));
+    TD_CHECK_NA(upload_pairs());
     void *ptr = nullptr;
     TD_CHECK_NA(cudaGetSymbolAddress(&ptr, td_noalloc_scratch));
     TD_CHECK_NA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device));
@@ -1974,13 +1970,11 @@ TD_API int td_search_batch_noalloc(int count, const td_instance *d_instances, td
         td_epoch_kernel<<<1, 1, 0, st>>>(epoch, 1u);
         // the whole resident grid (the scratch does not depend on its size):
         // warps without an instance of their own take donated subtrees, so a
-        // small batch is spread over the GPU; a single search wakes its
-        // waiting warps sooner (backoff cap 4 us instead of 32 us)
+        // small batch is spread over the GPU
         const int grid = d.sms * std::max(1, d.steal_blocks);
         td_steal_kernel<<<grid, threads, smem_bytes(warps), st>>>(
             d_instances, d_results, count, pool, items, ready, epoch, TD_NOALLOC_ITEMS, state, grain, split_level,
-            check_every, limit, nullptr, 64, 1u, restart_base, max_exp, count == 1 ? 4096u : 32768u,
-            /*race=*/0, /*spawn_base=*/TD_NOALLOC_ITEMS);
+            check_every, limit, nullptr, 64, 1u, restart_base, max_exp, /*race=*/0);
         TD_CHECK_NA(cudaGetLastError());
         td_finalize_kernel<<<std::max(1, std::min((count + 255) / 256, 2 * d.sms)), 256, 0, st>>>(pool, state,
                                                                                                 d_results, count);

@@ -25,12 +25,99 @@
 #define TD_FULL 0xffffffffu
 #define TD_TRI_TABLE 3060      // sum over N <= 17 of C(N,3) = C(18,4)
 
+// Limits and tables of the search a warp runs.
+struct td_search_limits {
+    uint32_t max_expansions;   // per search; TD_ERR_BUDGET when exceeded (~0: none)
+    uint32_t max_work;         // the same for nodes expanded here (the reference order's count also
+                               // holds those the endgame table accounts for)
+    uint64_t deadline_ns;      // %globaltimer value; 0 = none
+    ulonglong2 *tt;            // the launch's table of explored states (free order); null = none
+    uint64_t tt_id;            // number of the launch's first search in it
+    int tt_shift;              // 64 - log2 of its entries
+    uint32_t restart_base;     // free order: base of the restart budgets (td_attempt_budget); 0 = none
+    const int *cutoff;         // a split ordered search: lowest rank with a witness so far; null = none
+    int rank;                  // that search's own rank (it stops once *cutoff < rank)
+};
+
+// ---- work items (subtree roots handed between warps) ----------------------
+
+// A node that is known to be expandable, with the moves that lead to it.
+struct __align__(16) td_item {  // 32 bytes
+    uint64_t L;
+    uint32_t inst;          // instance index
+    uint8_t depth;          // bits 0-3: DFS depth of the node (0 only for the root of an inverse
+                            // instance); bit 7: the node belongs to the inverse instance's search;
+                            // bits 4-6: low bits of the restart attempt that donated it
+    uint8_t off;            // bits 0-4; bits 5-7: high bits of that attempt
+    uint16_t path[TD_MAX_DEPTH];
+};
+
+// Per-instance bookkeeping when several warps share one search.
+struct td_inst_state {
+    int found;              // 1: a warp recorded the witness; 2: one side of a race was searched
+                            // to the end without one (the verdict is known, the other side stops)
+    int pending;            // units (the root search + items) not yet finished: the low 16 bits
+                            // count the search of the instance, the high 16 bits that of its
+                            // inverse (td_steal_kernel's race; elsewhere only the low half is used)
+    unsigned expansions;    // summed over units
+    int error;              // first error status seen (timeout)
+};
+
+// Scheduler counters of one launch.
+struct td_pool {
+    // items reserved by donors, and item tickets taken (the batch engine) or
+    // items claimed (the serving loop); read together
+    alignas(8) int produced;
+    int consumed;
+    int inst_ticket;        // next fresh instance
+    int outstanding;        // the batch engine: units in progress plus items not yet finished
+    int active;             // the serving loop: warps inside a unit or claiming one
+    int idle;               // the serving loop: warps waiting for donated work
+    int error;              // launch-level error (bounded wait expired)
+    int done;               // the batch engine: nothing outstanding, and no instance left
+    unsigned long long donations;
+    unsigned long long donated_items;
+    unsigned long long races;  // inverse roots queued
+};
+
+// Donated items live either in a per-launch array (batch launches: index i
+// at slot i, ready[i] == epoch once written, ~epoch once the launch has no work
+// left for the warp that waits for it) or in a ring (the serving launch:
+// index i at slot i % capacity, ready == td_ring_tag(i) once written and
+// td_ring_tag(i) | 0x80000000 once its taker has read it, which frees the slot).
+__device__ __forceinline__ uint32_t td_ring_tag(long long i) { return (uint32_t)((i + 1) & 0x7fffffff); }
+
+struct td_donate_ctx {
+    int ring;
+    int tickets;            // takers hold item tickets (the batch engine), see td_steal_kernel
+    uint64_t deadline_ns;   // bounds the wait for a ring slot to be freed
+    td_pool *pool;
+    td_item *items;
+    uint32_t *ready;
+    uint32_t epoch;
+    int capacity;
+    int idle_seen;          // the three settings are those for a launch with idle warps
+    int grain;              // at most this many items per donation
+    int max_level;          // donate only children of levels <= max_level
+    int check_every;        // expansions between idle checks
+    uint32_t inst;
+    td_inst_state *state;
+    int side;               // 1: the unit searches the instance's inverse (items carry it on)
+    int attempt;            // the restart attempt that donated the unit (0 for a root)
+    int race;               // > 0: the unit queues its inverse when it starts restart attempt
+                            // `race` (root units of full-sorting instances in td_steal_kernel)
+};
+
 // Per-warp shared state.
 struct td_warp_smem {
     // per caller position c: the row masks S, G, P and H (positions after c),
     // and the odd-cycle / fixed-point flags as full masks
     uint4 rows[TD_MAX_N];
     uint2 flg[TD_MAX_N];
+    // per lane: its four pair slots (td_load_pairs), i | j << 5 each, and the
+    // first child number of their run
+    ushort4 pair[32];
+    uint16_t u0[32];
     union {
         struct {  // reference move order
             // per level: bit u % 32 of word u / 32 is child u still to visit
@@ -58,8 +145,29 @@ struct td_warp_smem {
     // decide its children; else 255
     uint8_t spare[TD_MAX_DEPTH];
     uint16_t list[32];                         // children looked up in the endgame table
+    int pairs_n;                               // the N the pair slots are loaded for
     int eg_moves;                              // the bound where the endgame table applies, else 0
+    // shared memory holds what a warp's search reads rarely, so that registers
+    // are left for the evaluation
+    td_search_limits lim;
+    td_donate_ctx dc;
 };
+
+// What a warp's donation settings become once it has met idle warps: it looks
+// for them 16 times as often, gives them 8 times as many items at once and
+// from 4 levels deeper.  An item per lane and counters read behind an expansion
+// make a donation cheap, and the end of a launch is all latency: with the
+// settings that suit the time before (4 items, level 2, every 64 expansions)
+// 2,048 S_16 at their lower bound took 20 ms, with these 2.8 ms; the n = 11..13
+// mix 10.3 and 1.6 ms, 250 requests of n = 8..16 2.8 and 0.23 ms.  Called by
+// one lane.
+__device__ __forceinline__ void td_serve_idle_warps(td_donate_ctx &dc) {
+    if (dc.idle_seen) return;
+    dc.idle_seen = 1;
+    dc.grain = min(32, 8 * dc.grain);
+    dc.max_level = min(TD_MAX_DEPTH - 1, dc.max_level + 4);
+    dc.check_every = max(1, dc.check_every / 16);
+}
 
 // Lexicographic position triples i|j<<5|k<<10 for every N, at offset C(N,4).
 __device__ uint16_t td_tri_table[TD_TRI_TABLE];
@@ -101,19 +209,10 @@ __device__ __forceinline__ void td_rate_masks(td_warp_smem &s, const td_instance
     __syncwarp();
 }
 
-struct td_search_limits {
-    uint64_t max_expansions;   // per search; TD_ERR_BUDGET when exceeded
-    uint32_t max_work;         // the same for nodes expanded here (the reference order's count also
-                               // holds those the endgame table accounts for)
-    uint64_t deadline_ns;      // %globaltimer value; 0 = none
-    const int *abort_flag;     // optional host/device abort request
-    ulonglong2 *tt;            // the launch's table of explored states (free order); null = none
-    uint64_t tt_id;            // number of the launch's first search in it
-    int tt_shift;              // 64 - log2 of its entries
-    uint32_t restart_base;     // free order: base of the restart budgets (td_attempt_budget); 0 = none
-    const int *cutoff;         // a split ordered search: lowest rank with a witness so far; null = none
-    int rank;                  // that search's own rank (it stops once *cutoff < rank)
-};
+// Orders this thread's earlier accesses before its later ones for the device
+// (release and acquire; cheaper than __threadfence, which is sequentially
+// consistent).
+__device__ __forceinline__ void td_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
 __device__ __forceinline__ uint64_t td_globaltimer() {
     uint64_t t;
@@ -132,25 +231,38 @@ __device__ __forceinline__ uint64_t td_globaltimer() {
 // from the node's row masks (td_row_classes).
 
 // Rounds of the bit-sliced evaluation for N: ceil(C(N-1,2) / 32).
-__device__ __forceinline__ int td_pair_rounds(int N) {
+TD_HD int td_pair_rounds(int N) {
     const int NP = N < 3 ? 0 : (N - 1) * (N - 2) / 2;
     return (NP + 31) >> 5;
 }
 
-// A lane's pair slots and, in the last word, R | u0 << 8 (see td_load_pairs).
-typedef uint32_t td_codes[TD_MAX_ROUNDS + 1];
+// Every lane's pair slots for every N, i | j << 5 each, and the first child
+// number of their run (td_pair_row).
+struct td_pair_row {
+    uint16_t pair[TD_MAX_ROUNDS];
+    uint16_t u0;
+};
+__device__ td_pair_row td_pair_table[TD_MAX_N + 1][32];
 
-// Lane l owns slots R l + r, r < R = td_pair_rounds(N).  Child (i, j, k) is
-// number u = C(N-1-i, 3) + C(N-1-j, 2) + (N-1-k) in the reference's reversed
-// triple order (T-1-t, sorting_search.cu:588-590), so the children of a lane's
-// slots r = 0, 1, ... are one run of consecutive u, from u0.
-__device__ __forceinline__ void td_load_pairs(int N, td_codes &code) {
-    const int lane = threadIdx.x & 31;
+// Lane l owns slots R l + r, r < R = td_pair_rounds(N) (the others are empty:
+// j = N-1).  Child (i, j, k) is number u = C(N-1-i, 3) + C(N-1-j, 2) + (N-1-k)
+// in the reference's reversed triple order (T-1-t, sorting_search.cu:588-590),
+// so the children of a lane's slots r = 0, 1, ... are one run of consecutive u.
+inline td_pair_row td_make_pair_row(int N, int lane) {
+    td_pair_row w;
     const int R = td_pair_rounds(N);
-#pragma unroll
-    for (int r = 0; r < TD_MAX_ROUNDS; ++r) code[r] = td_pair_code(N, r < R ? R * lane + r : -1);
-    const int a = N - 1 - (int)(code[0] & 31u), b = N - 1 - (int)((code[0] >> 5) & 31u);
-    code[TD_MAX_ROUNDS] = (uint32_t)R | (uint32_t)(a * (a - 1) * (a - 2) / 6 + b * (b - 1) / 2) << 8;
+    for (int r = 0; r < TD_MAX_ROUNDS; ++r) w.pair[r] = (uint16_t)(td_pair_code(N, r < R ? R * lane + r : -1) & 1023u);
+    const int a = N - 1 - (w.pair[0] & 31), b = N - 1 - (w.pair[0] >> 5);
+    w.u0 = (uint16_t)(a * (a - 1) * (a - 2) / 6 + b * (b - 1) / 2);
+    return w;
+}
+
+__device__ __forceinline__ void td_load_pairs(td_warp_smem &s, int N) {
+    const int lane = threadIdx.x & 31;
+    const td_pair_row &w = td_pair_table[N][lane];
+    s.pair[lane] = make_ushort4(w.pair[0], w.pair[1], w.pair[2], w.pair[3]);
+    s.u0[lane] = w.u0;
+    __syncwarp();
 }
 
 // Pinned state (L, off) -> the caller's array of `level`.
@@ -259,7 +371,7 @@ __device__ __forceinline__ int td_prepare_rows(td_warp_smem &s, int level, int N
 
 // Classifies every child of the node at `level`; fills the level's outcome
 // words and lane summaries and returns a found move (i | j<<5 | k<<10) or -1.
-__device__ __forceinline__ int td_evaluate_rows(td_warp_smem &s, const td_codes &code, int N,
+__device__ __forceinline__ int td_evaluate_rows(td_warp_smem &s, int N,
                                                 int level, int odd, uint32_t O, uint32_t F) {
     const int lane = threadIdx.x & 31;
     const int D = level + 1;
@@ -268,28 +380,51 @@ __device__ __forceinline__ int td_evaluate_rows(td_warp_smem &s, const td_codes 
     const uint32_t x0 = (0u - ((reachD >> odd) & 1u)) & ~f0;
     const uint32_t x2 = (0u - ((reachD >> (odd + 2)) & 1u)) & ~f2;
     const bool accepting = (f0 | f2) != 0;  // warp-uniform
-    const int R = (int)(code[TD_MAX_ROUNDS] & 255u);  // warp-uniform
+    const int R = td_pair_rounds(N);  // warp-uniform
+    const ushort4 pq = s.pair[lane];
+    const uint32_t code[TD_MAX_ROUNDS] = {pq.x, pq.y, pq.z, pq.w};
     uint32_t key = 0xffffffffu;
     uint32_t W[TD_MAX_ROUNDS] = {0u, 0u, 0u, 0u};
+    // A node without a spare move only has +2 children, and nearly always odd
+    // cycles only (99% of such nodes on near-reverse S_16, and 80% to 100% of
+    // all nodes have no spare move): a third of the work, see td_row_plus2_odd.
+    // 2^19 near-reverse S_16 at bound 9: 26.8 -> 23.7 ms.
+    if (!(x0 | f0) && O == (1u << N) - 1u) {
 #pragma unroll
-    for (int r = 0; r < TD_MAX_ROUNDS; ++r) {
-        if (r >= R) break;
-        const uint32_t pc = code[r];
-        const int i = pc & 31, j = (pc >> 5) & 31;
-        const uint4 ri = s.rows[i], rj = s.rows[j];
-        const uint2 fi = s.flg[i], fj = s.flg[j];
-        uint32_t plus, zero;
-        td_row_classes_x(ri.x, ri.y, ri.z, rj.x, rj.y, rj.z, O, F, fi.x, fj.x, fi.y, fj.y, (int)(pc >> 15), &plus,
-                         &zero);
-        const uint32_t km = rj.w;  // k > j (empty slots: j's row with an empty mask is never read)
-        // +2 children at bits k-1, 0 children at bits k+15; the fields do not
-        // overlap, so the high-half multiply and the add keep this off the ALU pipe
-        W[r] = __umulhi(km & x2 & plus, 0x80000000u) + (km & x0 & zero) * 32768u;
-        if (accepting) {
-            const uint32_t fnd = km & ((f0 & zero) | (f2 & plus));
-            if (fnd && key == 0xffffffffu)
-                key = ((uint32_t)lane << 17) | ((uint32_t)r << 15) | (pc & 1023u) |
-                      ((uint32_t)(31 - __clz(fnd)) << 10);
+        for (int r = 0; r < TD_MAX_ROUNDS; ++r) {
+            if (r >= R) break;
+            const uint32_t pc = code[r];
+            const int sh = 31 - (int)(pc >> 5);  // brings bit j to the sign bit
+            const uint4 ri = s.rows[pc & 31], rj = s.rows[pc >> 5];
+            const uint32_t plus =
+                rj.w & (uint32_t)((int32_t)(ri.x << sh) >> 31) &
+                td_row_plus2_odd(ri.x, ri.y, ri.z, rj.y, rj.z, (uint32_t)((int32_t)(ri.y << sh) >> 31),
+                                 (uint32_t)((int32_t)(ri.z << sh) >> 31));
+            W[r] = (plus & x2) >> 1;
+            if (accepting && plus && key == 0xffffffffu)  // then every +2 child is accepted
+                key = ((uint32_t)lane << 17) | ((uint32_t)r << 15) | pc | ((uint32_t)(31 - __clz(plus)) << 10);
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < TD_MAX_ROUNDS; ++r) {
+            if (r >= R) break;
+            const uint32_t pc = code[r];
+            const int i = pc & 31, j = pc >> 5;
+            const uint4 ri = s.rows[i], rj = s.rows[j];
+            const uint2 fi = s.flg[i], fj = s.flg[j];
+            uint32_t plus, zero;
+            td_row_classes_x(ri.x, ri.y, ri.z, rj.x, rj.y, rj.z, O, F, fi.x, fj.x, fi.y, fj.y, 31 - j, &plus,
+                             &zero);
+            const uint32_t km = rj.w;  // k > j (empty slots: j's row with an empty mask is never read)
+            // +2 children at bits k-1, 0 children at bits k+15; the fields do not
+            // overlap, so the high-half multiply and the add keep this off the ALU pipe
+            W[r] = __umulhi(km & x2 & plus, 0x80000000u) + (km & x0 & zero) * 32768u;
+            if (accepting) {
+                const uint32_t fnd = km & ((f0 & zero) | (f2 & plus));
+                if (fnd && key == 0xffffffffu)
+                    key = ((uint32_t)lane << 17) | ((uint32_t)r << 15) | pc |
+                          ((uint32_t)(31 - __clz(fnd)) << 10);
+            }
         }
     }
     s.pw[level][lane] = make_uint4(W[0], W[1], W[2], W[3]);
@@ -316,8 +451,7 @@ __device__ __forceinline__ int td_evaluate_rows(td_warp_smem &s, const td_codes 
 // smallest pair) and its smallest k.  `ord` (td_order_variant) rotates the
 // lane priority, reverses the round order and takes the largest k first.
 // Returns the move, with bit 15 set for a 0 child, or -1.
-__device__ __forceinline__ int td_next_child_rows(td_warp_smem &s, const td_codes &code,
-                                                  int level, uint32_t ord) {
+__device__ __forceinline__ int td_next_child_rows(td_warp_smem &s, int level, uint32_t ord) {
     const int lane = threadIdx.x & 31;
     const uint32_t m2 = s.m2[level], m0 = s.m0[level];
     if ((m2 | m0) == 0) return -1;
@@ -343,8 +477,7 @@ __device__ __forceinline__ int td_next_child_rows(td_warp_smem &s, const td_code
     }
     const int b = (ord & 64u) ? 31 - __clz(w & cm) : __ffs(w & cm) - 1;
     const uint32_t nw = w & ~(1u << b);
-    const uint32_t mine = r == 3 ? code[3] : (r == 2 ? code[2] : (r == 1 ? code[1] : code[0]));
-    const uint32_t pc = __shfl_sync(TD_FULL, mine, win);
+    const uint32_t pc = reinterpret_cast<const uint16_t *>(&s.pair[win])[r];
     // does the winning lane keep children of this class?
     const uint32_t rest = (r == 0 ? nw : Wv.x) | (r == 1 ? nw : Wv.y) | (r == 2 ? nw : Wv.z) | (r == 3 ? nw : Wv.w);
     if (lane == 0) {
@@ -356,7 +489,7 @@ __device__ __forceinline__ int td_next_child_rows(td_warp_smem &s, const td_code
     }
     __syncwarp();
     const int k = c2 ? b + 1 : b - 15;
-    return (int)((pc & 1023u) | ((uint32_t)k << 10) | (c2 ? 0u : 0x8000u));
+    return (int)(pc | ((uint32_t)k << 10) | (c2 ? 0u : 0x8000u));
 }
 
 // Reference order: classifies every child of the node at `level`; fills the
@@ -368,7 +501,7 @@ __device__ __forceinline__ int td_next_child_rows(td_warp_smem &s, const td_code
 // earlier form read three pair-table entries and a class-table byte per triple
 // (22 steps per lane): 16,384 S_12 instances at bound 6 took 12.2 ms, and take
 // 7.6 ms with this one.
-__device__ __forceinline__ int td_evaluate(td_warp_smem &s, const td_codes &code, int N, int level, int odd,
+__device__ __forceinline__ int td_evaluate(td_warp_smem &s, int N, int level, int odd,
                                            uint32_t O, uint32_t F) {
     const int lane = threadIdx.x & 31;
     const int D = level + 1;
@@ -377,7 +510,9 @@ __device__ __forceinline__ int td_evaluate(td_warp_smem &s, const td_codes &code
     const uint32_t x0 = (0u - ((reachD >> odd) & 1u)) & ~f0;
     const uint32_t x2 = (0u - ((reachD >> (odd + 2)) & 1u)) & ~f2;
     const bool accepting = (f0 | f2) != 0;  // warp-uniform
-    const int R = (int)(code[TD_MAX_ROUNDS] & 255u);
+    const int R = td_pair_rounds(N);  // warp-uniform
+    const ushort4 pq = s.pair[lane];
+    const uint32_t code[TD_MAX_ROUNDS] = {pq.x, pq.y, pq.z, pq.w};
     if (lane < TD_MAX_STEPS) {
         s.cw[level][lane] = 0;
         s.cp[level][lane] = 0;
@@ -391,11 +526,11 @@ __device__ __forceinline__ int td_evaluate(td_warp_smem &s, const td_codes &code
     for (int r = 0; r < TD_MAX_ROUNDS; ++r) {
         if (r >= R) break;
         const uint32_t pc = code[r];
-        const int i = pc & 31, j = (pc >> 5) & 31;
+        const int i = pc & 31, j = pc >> 5;
         const uint4 ri = s.rows[i], rj = s.rows[j];
         const uint2 fi = s.flg[i], fj = s.flg[j];
         uint32_t plus, zero;
-        td_row_classes_x(ri.x, ri.y, ri.z, rj.x, rj.y, rj.z, O, F, fi.x, fj.x, fi.y, fj.y, (int)(pc >> 15), &plus,
+        td_row_classes_x(ri.x, ri.y, ri.z, rj.x, rj.y, rj.z, O, F, fi.x, fj.x, fi.y, fj.y, 31 - j, &plus,
                          &zero);
         const uint32_t km = rj.w;  // k > j
         // k = N-1 comes first: reverse the bits
@@ -404,7 +539,7 @@ __device__ __forceinline__ int td_evaluate(td_warp_smem &s, const td_codes &code
         if (x0) pl |= (uint64_t)(__brev(km & plus) >> (32 - N)) << at;
         at += N - 1 - j;
     }
-    const int u0 = (int)(code[TD_MAX_ROUNDS] >> 8), w = u0 >> 5, sh = u0 & 31;
+    const int u0 = s.u0[lane], w = u0 >> 5, sh = u0 & 31;
     if (level == 0) ch |= fd;
     // ORs the lane's run into the 22 words of an array
     auto put = [&](uint32_t *words, uint64_t run) {
@@ -453,73 +588,6 @@ __device__ __forceinline__ int td_next_child(td_warp_smem &s, int level, int *ac
 
 #include "td_endgame.cuh"
 
-// ---- work items (subtree roots handed between warps) ----------------------
-
-// A node that is known to be expandable, with the moves that lead to it.
-struct __align__(16) td_item {  // 32 bytes
-    uint64_t L;
-    uint32_t inst;          // instance index
-    uint8_t depth;          // bits 0-3: DFS depth of the node (0 only for the root of an inverse
-                            // instance); bit 7: the node belongs to the inverse instance's search;
-                            // bits 4-6: low bits of the restart attempt that donated it
-    uint8_t off;            // bits 0-4; bits 5-7: high bits of that attempt
-    uint16_t path[TD_MAX_DEPTH];
-};
-
-// Per-instance bookkeeping when several warps share one search.
-struct td_inst_state {
-    int found;              // 1: a warp recorded the witness; 2: one side of a race was searched
-                            // to the end without one (the verdict is known, the other side stops)
-    int pending;            // units (the root search + items) not yet finished: the low 16 bits
-                            // count the search of the instance, the high 16 bits that of its
-                            // inverse (td_steal_kernel's race; elsewhere only the low half is used)
-    unsigned expansions;    // summed over units
-    int error;              // first error status seen (timeout)
-};
-
-// Scheduler counters of one launch.
-struct td_pool {
-    int inst_ticket;        // next fresh instance
-    int produced;           // items reserved by donors
-    int consumed;           // items claimed by takers (the batch engine: item tickets taken)
-    int active;             // warps inside a unit or claiming one (the serving loop)
-    int idle;               // warps waiting for donated work (the serving loop)
-    int error;              // launch-level error (bounded wait expired)
-    int outstanding;        // the batch engine: units in progress plus items not yet finished
-    int spawn_produced;     // the batch engine's race: inverse roots queued
-    int spawn_consumed;     // and claimed
-    unsigned long long donations;
-    unsigned long long donated_items;
-};
-
-// Donated items live either in a per-launch array (batch launches: index i
-// at slot i, ready[i] == epoch once written) or in a ring (the serving launch:
-// index i at slot i % capacity, ready == td_ring_tag(i) once written and
-// td_ring_tag(i) | 0x80000000 once its taker has read it, which frees the slot).
-__device__ __forceinline__ uint32_t td_ring_tag(long long i) { return (uint32_t)((i + 1) & 0x7fffffff); }
-
-struct td_donate_ctx {
-    int ring;
-    int tickets;            // takers hold item tickets (the batch engine), see td_steal_kernel
-    uint64_t deadline_ns;   // bounds the wait for a ring slot to be freed
-    td_pool *pool;
-    td_item *items;
-    uint32_t *ready;
-    uint32_t epoch;
-    int capacity;
-    int grain;              // at most this many items per donation
-    int max_level;          // donate only children of levels <= max_level
-    int check_every;        // expansions between idle checks
-    uint32_t inst;
-    td_inst_state *state;
-    int side;               // 1: the unit searches the instance's inverse (items carry it on)
-    int attempt;            // the restart attempt that donated the unit (0 for a root)
-    int race;               // > 0: the unit queues its inverse when it starts restart attempt
-                            // `race` (root units of full-sorting instances in td_steal_kernel)
-    int spawn_base;         // the race's queue: item slots [spawn_base, spawn_base + spawn_capacity)
-    int spawn_capacity;
-};
-
 #define TD_DFS_FOUND 1
 #define TD_DFS_EXHAUSTED 0
 #define TD_DFS_BUDGET (-2)
@@ -533,12 +601,71 @@ struct td_dfs_out {
     uint32_t expansions;
 };
 
-// Hands some remaining children of the shallowest level in [d0, level] to the
-// pool as items (free move order).  Returns the number donated (uniform
-// across the warp).
-__device__ __forceinline__ int td_donate(td_warp_smem &s, const td_donate_ctx &dc,
-                                         const td_codes &code, int d0, int level, int N,
-                                         int want, int attempt) {
+// Reserves `want` item slots; returns the first (or -1) and, in `got`, how many
+// there are.  Called by one lane.  In the array (the batch engine) a
+// fetch-and-add reserves them: slots past the capacity are never written, and
+// their tickets wait for the launch to end.  In the ring at most `capacity`
+// items are unclaimed, so the count must be checked before it is raised.  The
+// pending count covers the items before any taker can finish one (takers wait
+// for the ready flag, written later), and so does the batch engine's
+// outstanding count.
+__device__ __forceinline__ int td_reserve(const td_donate_ctx &dc, int want, int unit, int *got) {
+    int base = -1, n = want;
+    if (dc.tickets) {
+        if (*(volatile int *)&dc.pool->produced < dc.capacity) {
+            base = atomicAdd(&dc.pool->produced, want);
+            n = min(want, dc.capacity - base);
+            if (n <= 0) base = -1;
+        }
+        if (base >= 0) atomicAdd(&dc.pool->outstanding, n);
+    } else {
+        int cur = *(volatile int *)&dc.pool->produced;
+        for (;;) {
+            if (cur - *(volatile int *)&dc.pool->consumed + want > dc.capacity) break;
+            const int prev = atomicCAS(&dc.pool->produced, cur, cur + want);
+            if (prev == cur) { base = cur; break; }
+            cur = prev;
+        }
+    }
+    if (base >= 0) atomicAdd(&dc.state->pending, n * unit);
+    td_fence();
+    *got = base >= 0 ? n : 0;
+    return base;
+}
+
+// Writes an item into its slot and sets the slot's ready flag.  Called by each
+// lane that holds an item.
+__device__ __forceinline__ void td_publish(const td_donate_ctx &dc, const td_item &it, int slot) {
+    int phys = slot;
+    uint32_t tag = dc.epoch;
+    if (dc.ring) {
+        phys = slot % dc.capacity;
+        tag = td_ring_tag(slot);
+        if (slot >= dc.capacity) {
+            // the slot's previous item (index slot - capacity) is claimed; wait
+            // until its taker has read it (bounded).  After an expired wait the
+            // slot still belongs to an unread item: it is left alone, and this
+            // item's taker gives up at the deadline
+            const uint32_t freed = td_ring_tag(slot - dc.capacity) | 0x80000000u;
+            for (unsigned spin = 0; *(volatile uint32_t *)&dc.ready[phys] != freed; ++spin) {
+                if ((spin & 255u) == 0 && dc.deadline_ns && td_globaltimer() > dc.deadline_ns) {
+                    atomicCAS(&dc.pool->error, 0, TD_ERR_TIMEOUT);
+                    return;
+                }
+                __nanosleep(64);
+            }
+        }
+    }
+    dc.items[phys] = it;
+    td_fence();
+    *(volatile uint32_t *)&dc.ready[phys] = tag;
+}
+
+// Hands up to `want` (at most 32) remaining children of the shallowest level
+// in [d0, level] to the pool as items, one per lane (free move order).  Returns
+// the number donated (uniform across the warp).
+__device__ __noinline__ int td_donate(td_warp_smem &s, int d0, int level, int N, int want, int attempt) {
+    const td_donate_ctx &dc = s.dc;
     const int lane = threadIdx.x & 31;
     int lv = -1;
     for (int l = d0; l <= level && l <= dc.max_level; ++l) {
@@ -548,41 +675,21 @@ __device__ __forceinline__ int td_donate(td_warp_smem &s, const td_donate_ctx &d
     const uint4 Wv = s.pw[lv][lane];
     uint32_t W0 = Wv.x, W1 = Wv.y, W2 = Wv.z, W3 = Wv.w;
     const int cnt = __popc(W0) + __popc(W1) + __popc(W2) + __popc(W3);
-    const int have = __reduce_add_sync(TD_FULL, (unsigned)cnt);
-    // leave at least one child to this warp when the level is the current one
-    const int give = min(want, have - (lv == level ? 1 : 0));
-    if (give <= 0) return 0;
     int before = cnt;  // lanes give in lane order
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(TD_FULL, before, o);
         if (lane >= o) before += v;
     }
+    const int have = __shfl_sync(TD_FULL, before, 31);
     before -= cnt;
-    const int mine = max(0, min(cnt, give - before));
-    // reserve `give` item slots; the count never passes the capacity and never
-    // goes back, so a taker only ever claims slots that a donor will write
+    // leave at least one child to this warp when the level is the current one
+    int give = min(min(want, 32), have - (lv == level ? 1 : 0));
+    if (give <= 0) return 0;
     int base = -1;
-    if (lane == 0) {
-        int cur = *(volatile int *)&dc.pool->produced;
-        for (;;) {
-            // a ring holds at most `capacity` items that are not yet claimed
-            const int used = dc.ring ? cur - *(volatile int *)&dc.pool->consumed : cur;
-            if (used + give > dc.capacity) break;
-            const int prev = atomicCAS(&dc.pool->produced, cur, cur + give);
-            if (prev == cur) { base = cur; break; }
-            cur = prev;
-        }
-        // the pending count must cover the items before any taker can finish
-        // one (takers wait for the ready flag, written below); with item
-        // tickets, so must the launch's outstanding count
-        if (base >= 0) {
-            atomicAdd(&dc.state->pending, dc.side ? give << 16 : give);
-            if (dc.tickets) atomicAdd(&dc.pool->outstanding, give);
-        }
-        __threadfence();
-    }
+    if (lane == 0) base = td_reserve(dc, give, dc.side ? 1 << 16 : 1, &give);
     base = __shfl_sync(TD_FULL, base, 0);
+    give = __shfl_sync(TD_FULL, give, 0);
     if (base < 0) return 0;  // out of item space: keep the work
     if (lane == 0) {
         atomicAdd(&dc.pool->donations, 1ull);
@@ -591,55 +698,17 @@ __device__ __forceinline__ int td_donate(td_warp_smem &s, const td_donate_ctx &d
     uint64_t Lp;
     int offp;
     td_pack_state(s, lv, N, &Lp, &offp);  // the parent in pinned form
-    int slot = base + before;
+    const ushort4 pq = s.pair[lane];
     // a lane gives its lowest slots first (the ones this warp visits last),
     // and 0-class children (high bits) before +2 children
-    for (int taken = 0; taken < mine; ++taken) {
+    const int last = min(give, before + cnt);
+    for (; before < last; ++before) {
         uint32_t pc, b;
-        if (W0) { pc = code[0]; b = 31 - __clz(W0); W0 &= ~(1u << b); }
-        else if (W1) { pc = code[1]; b = 31 - __clz(W1); W1 &= ~(1u << b); }
-        else if (W2) { pc = code[2]; b = 31 - __clz(W2); W2 &= ~(1u << b); }
-        else { pc = code[3]; b = 31 - __clz(W3); W3 &= ~(1u << b); }
-        const uint32_t k = b < 16 ? b + 1 : b - 15;
-        const uint32_t t = (pc & 1023u) | (k << 10);
-        uint64_t nL;
-        int noff;
-        td_apply_move(Lp, offp, N, t & 31, (t >> 5) & 31, (t >> 10) & 31, &nL, &noff);
-        td_item it;
-        it.L = nL;
-        it.inst = dc.inst;
-        it.depth = (uint8_t)((lv + 1) | ((attempt & 7) << 4) | (dc.side << 7));
-        it.off = (uint8_t)(noff | ((attempt >> 3) << 5));
-#pragma unroll
-        for (int d = 0; d < TD_MAX_DEPTH; ++d) it.path[d] = d < lv ? s.path[d] : (d == lv ? (uint16_t)t : 0);
-        int phys = slot;
-        uint32_t tag = dc.epoch;
-        bool freed_ok = true;
-        if (dc.ring) {
-            phys = slot % dc.capacity;
-            tag = td_ring_tag(slot);
-            if (slot >= dc.capacity) {
-                // the slot's previous item (index slot - capacity) is claimed;
-                // wait until its taker has read it (bounded)
-                const uint32_t freed = td_ring_tag(slot - dc.capacity) | 0x80000000u;
-                for (unsigned spin = 0; *(volatile uint32_t *)&dc.ready[phys] != freed; ++spin) {
-                    if ((spin & 255u) == 0 && dc.deadline_ns && td_globaltimer() > dc.deadline_ns) {
-                        atomicCAS(&dc.pool->error, 0, TD_ERR_TIMEOUT);
-                        freed_ok = false;
-                        break;
-                    }
-                    __nanosleep(64);
-                }
-            }
-        }
-        // after an expired wait the slot still belongs to an unread item: it
-        // is left alone, and this item's taker gives up at the deadline
-        if (freed_ok) {
-            dc.items[phys] = it;
-            __threadfence();
-            atomicExch(&dc.ready[phys], tag);
-        }
-        ++slot;
+        if (W0) { pc = pq.x; b = 31 - __clz(W0); W0 &= ~(1u << b); }
+        else if (W1) { pc = pq.y; b = 31 - __clz(W1); W1 &= ~(1u << b); }
+        else if (W2) { pc = pq.z; b = 31 - __clz(W2); W2 &= ~(1u << b); }
+        else { pc = pq.w; b = 31 - __clz(W3); W3 &= ~(1u << b); }
+        s.list[before] = (uint16_t)(pc | ((b < 16 ? b + 1 : b - 15) << 10));
     }
     s.pw[lv][lane] = make_uint4(W0, W1, W2, W3);
     const uint32_t any = W0 | W1 | W2 | W3;
@@ -650,64 +719,38 @@ __device__ __forceinline__ int td_donate(td_warp_smem &s, const td_donate_ctx &d
         s.m0[lv] = m0;
     }
     __syncwarp();
+    if (lane < give) {
+        const uint32_t t = s.list[lane];
+        uint64_t nL;
+        int noff;
+        td_apply_move(Lp, offp, N, t & 31, (t >> 5) & 31, (t >> 10) & 31, &nL, &noff);
+        td_item it;
+        it.L = nL;
+        it.inst = dc.inst;
+        it.depth = (uint8_t)((lv + 1) | ((attempt & 7) << 4) | (dc.side << 7));
+        it.off = (uint8_t)(noff | ((attempt >> 3) << 5));
+#pragma unroll
+        for (int d = 0; d < TD_MAX_DEPTH; ++d) it.path[d] = d < lv ? s.path[d] : (d == lv ? (uint16_t)t : 0);
+        td_publish(dc, it, base + lane);
+    }
+    __syncwarp();
     return give;
 }
 
-// Queues the inverse of the unit's instance (td_inverse_pinned) as a root item
-// of the race's queue, so that another warp searches it while this one goes
-// on; the first witness on either side ends both, and so does either side
-// searched to the end without one (found = 2).  The pending and outstanding
-// counts cover the item before it can be claimed.  In the batch engine only an
-// instance's root search queues its inverse, once, and the queue holds a slot
-// per instance of the launch, so one fetch-and-add reserves a slot: busy
-// searches queue their inverses at up to several per microsecond, and a
-// compare-and-swap loop on the counter kept them waiting.  In the serving
-// loop (dc.ring) the inverse is one more item of its ring.  Returns whether it
-// was queued (uniform across the warp).
-__device__ __forceinline__ int td_spawn_inverse(const td_warp_smem &s, const td_donate_ctx &dc, int N) {
+// Queues the inverse of the unit's instance (td_inverse_pinned) as one more
+// item, a root of the inverse's side, so that another warp searches it while
+// this one goes on; the first witness on either side ends both, and so does the
+// instance's side searched to the end without one (found = 2).  Only an
+// instance's root search queues its inverse, once.  In the batch engine items
+// are taken once no fresh instance is left, and the inverses queued until then
+// come first.  Returns whether it was queued (uniform across the warp).
+__device__ __noinline__ int td_spawn_inverse(const td_warp_smem &s, int N) {
+    const td_donate_ctx &dc = s.dc;
     int ok = 0;
     if ((threadIdx.x & 31) == 0) {
-        int slot = -1, phys = -1;
-        uint32_t tag = dc.epoch;
-        if (dc.ring) {
-            // the serving loop's ring of items: reserved like a donation (one
-            // item), and a reused slot is written once its last item was read
-            int cur = *(volatile int *)&dc.pool->produced;
-            for (;;) {
-                if (cur - *(volatile int *)&dc.pool->consumed + 1 > dc.capacity) break;
-                const int prev = atomicCAS(&dc.pool->produced, cur, cur + 1);
-                if (prev == cur) { slot = cur; break; }
-                cur = prev;
-            }
-            if (slot >= 0) {
-                phys = slot % dc.capacity;
-                tag = td_ring_tag(slot);
-                atomicAdd(&dc.state->pending, 1 << 16);
-                if (slot >= dc.capacity) {
-                    const uint32_t freed = td_ring_tag(slot - dc.capacity) | 0x80000000u;
-                    for (unsigned spin = 0; *(volatile uint32_t *)&dc.ready[phys] != freed; ++spin) {
-                        if ((spin & 255u) == 0 && dc.deadline_ns && td_globaltimer() > dc.deadline_ns) {
-                            // the slot still holds an unread item: left alone, and
-                            // this item's taker gives up at the deadline
-                            atomicCAS(&dc.pool->error, 0, TD_ERR_TIMEOUT);
-                            phys = -1;
-                            break;
-                        }
-                        __nanosleep(64);
-                    }
-                }
-            }
-        } else {
-            slot = atomicAdd(&dc.pool->spawn_produced, 1);
-            if (slot < dc.spawn_capacity) {
-                phys = dc.spawn_base + slot;
-                atomicAdd(&dc.state->pending, 1 << 16);
-                atomicAdd(&dc.pool->outstanding, 1);
-            } else {
-                slot = -1;
-            }
-        }
-        if (phys >= 0) {
+        int got;
+        const int slot = td_reserve(dc, 1, 1 << 16, &got);
+        if (slot >= 0) {
             td_item it;
             it.L = td_inverse_pinned(s.L[0], N);
             it.inst = dc.inst;
@@ -715,11 +758,10 @@ __device__ __forceinline__ int td_spawn_inverse(const td_warp_smem &s, const td_
             it.off = 0;
 #pragma unroll
             for (int d = 0; d < TD_MAX_DEPTH; ++d) it.path[d] = 0;
-            dc.items[phys] = it;
-            __threadfence();
-            atomicExch(&dc.ready[phys], tag);
+            td_publish(dc, it, slot);
+            atomicAdd(&dc.pool->races, 1ull);
+            ok = 1;
         }
-        ok = slot >= 0;
     }
     return __shfl_sync(TD_FULL, ok, 0);
 }
@@ -730,9 +772,9 @@ __device__ __forceinline__ int td_spawn_inverse(const td_warp_smem &s, const td_
 // position (arrays in registers, block swaps by shuffle, cut points by
 // ballot).  Returns 0 if it does not convert (then no witness may be
 // recorded).  Uniform across the warp.
-__device__ __forceinline__ int td_inverse_result(td_warp_smem &s, const td_instance &x, td_dfs_out &r) {
+__device__ __forceinline__ int td_inverse_result(td_warp_smem &s, const td_instance &x, int k, uint32_t *found_move) {
     const int c = threadIdx.x & 31;
-    const int N = x.n_symbols, k = r.depth;
+    const int N = x.n_symbols;
     if (k < 1 || k > TD_MAX_DEPTH) return 0;
     // the swap of blocks [i, j) and [j, kk) moves the value at src(c) to c
     auto swap = [&](uint32_t v, uint32_t mv) {
@@ -742,7 +784,7 @@ __device__ __forceinline__ int td_inverse_result(td_warp_smem &s, const td_insta
         return __shfl_sync(TD_FULL, v, src);
     };
     // lane q holds the inverse's move q, and then the converted move q
-    const uint32_t inv = c < k - 1 ? (uint32_t)s.path[c] : (c == k - 1 ? (uint32_t)r.found_move : 0u);
+    const uint32_t inv = c < k - 1 ? (uint32_t)s.path[c] : (c == k - 1 ? *found_move : 0u);
     __syncwarp();
     // X: the caller's array; S: the identity array after all the inverse's moves
     int p = c + x.offset;
@@ -784,7 +826,7 @@ __device__ __forceinline__ int td_inverse_result(td_warp_smem &s, const td_insta
     // each lane stores its own move into the path, which it alone read above;
     // the record's writers read it after the barrier
     if (c < k - 1) s.path[c] = (uint16_t)mine;
-    r.found_move = (uint16_t)__shfl_sync(TD_FULL, mine, k - 1);
+    *found_move = __shfl_sync(TD_FULL, mine, k - 1);
     __syncwarp();
     return 1;
 }
@@ -799,25 +841,37 @@ __device__ __forceinline__ int td_inverse_result(td_warp_smem &s, const td_insta
 // through other states.  Recording only witnesses that pass keeps the verdict
 // that of the instance's own filtered search.  Uses the warp's frame (levels
 // 0..depth) as scratch; uniform across the warp.
-__device__ __forceinline__ bool td_filtered_witness(td_warp_smem &s, const td_instance &x, const td_dfs_out &r) {
-    const int N = x.n_symbols, k = r.depth;
+__device__ __forceinline__ bool td_filtered_witness(td_warp_smem &s, const td_instance &x, int k, uint32_t found_move) {
+    const int N = x.n_symbols;
     if (k < 1 || k > TD_MAX_DEPTH) return false;
     td_unpack_state(s, 0, x.perm, x.offset, N);
-    uint32_t O, F;
-    int odd = td_prepare_rows(s, 0, N, O, F);
-    for (int d = 0; d < k; ++d) {
-        const uint32_t t = d == k - 1 ? (uint32_t)r.found_move : (uint32_t)s.path[d];
+    int odd = 0;
+    for (int d = 0;; ++d) {
+        uint32_t O, F;
+        const int now = td_prepare_rows(s, d, N, O, F);
+        if (d > 0) {
+            if (now != odd && now != odd + 2) return false;
+            const bool accepted = (s.acc[d] >> now) & 1u;
+            if (accepted != (d == k)) return false;
+            if (d == k) return true;
+        }
+        odd = now;
+        const uint32_t t = d == k - 1 ? found_move : (uint32_t)s.path[d];
         const int i = t & 31, j = (t >> 5) & 31, kk = (t >> 10) & 31;
         if (!(i < j && j < kk && kk < N)) return false;
         if (((F >> i) | (F >> j) | (F >> kk)) & 1u) return false;
         td_apply_bytes(s, d, t, N);
-        const int next = td_prepare_rows(s, d + 1, N, O, F);
-        if (next != odd && next != odd + 2) return false;
-        odd = next;
-        const bool accepted = (s.acc[d + 1] >> odd) & 1u;
-        if (accepted != (d == k - 1)) return false;
     }
-    return true;
+}
+
+// A unit of the inverse's side found a witness of k moves: turns it into one of
+// the instance.  Returns its last move; -1 where it does not convert (a failed
+// replay), -2 where it leaves the reference's move filter on the instance's
+// side (it is dropped: this side then stops, the instance's own search
+// decides).
+__device__ __noinline__ int td_inverse_witness(td_warp_smem &s, td_instance x, int k, uint32_t found_move) {
+    if (!td_inverse_result(s, x, k, &found_move)) return -1;
+    return td_filtered_witness(s, x, k, found_move) ? (int)found_move : -2;
 }
 
 // ---- table of explored states (free order) --------------------------------
@@ -880,7 +934,7 @@ __device__ __forceinline__ void td_tt_store(ulonglong2 *p, uint64_t a, uint64_t 
 // there; returns whether it was already taken up at a depth <= lv by the
 // search `sub` (side << 6 | attempt) of instance `inst` of this launch
 // (uniform across the warp).
-__device__ __forceinline__ bool td_tt_visit(const td_warp_smem &s, const td_search_limits &lim, int lv, int N,
+__device__ __forceinline__ bool td_tt_visit(const td_warp_smem &s, int lv, int N,
                                             uint32_t inst, uint32_t sub) {
     const int m = threadIdx.x & 31;
     const int a = m < N ? s.A[lv][m] : 0xff;
@@ -898,10 +952,10 @@ __device__ __forceinline__ bool td_tt_visit(const td_warp_smem &s, const td_sear
     hi = __reduce_or_sync(TD_FULL, hi);
     int hit = 0;
     if (m == 0) {
-        const uint64_t id = lim.tt_id + inst;
+        const uint64_t id = s.lim.tt_id + inst;
         const uint64_t w0 = td_tt_key((((uint64_t)hi) << 32) | lo) | (id << 57);
         const uint64_t w1 = ((id >> 7) << 7) | sub;
-        ulonglong2 *e = lim.tt + (((w0 + w1 * 0xD6E8FEB86659FD93ull) * 0x9E3779B97F4A7C15ull) >> lim.tt_shift);
+        ulonglong2 *e = s.lim.tt + (((w0 + w1 * 0xD6E8FEB86659FD93ull) * 0x9E3779B97F4A7C15ull) >> s.lim.tt_shift);
         uint64_t e0, e1;
         td_tt_load(e, e0, e1);
         hit = e0 == w0 && (e1 >> 4) == w1 && (int)(e1 & 15u) <= lv;
@@ -910,12 +964,18 @@ __device__ __forceinline__ bool td_tt_visit(const td_warp_smem &s, const td_sear
     return __shfl_sync(TD_FULL, hit, 0) != 0;
 }
 
-// Depth-first search from the node held at level d0 of `s` (state, path and
-// rate masks already set; `code` holds the lane's pair slots).  Leaves the
-// frames intact on TD_DFS_BUDGET.  The free order may donate subtrees through
-// `dc`.
+// Depth-first search from the node held at level d0 of `s` (state, path, rate
+// masks, pair slots and limits already set).  Leaves
+// the frames intact on TD_DFS_BUDGET.  `shared`: a unit of a search that other
+// warps may take part in (free order; s.dc says how).
+//
+// The node is expanded at one place of the loop, and what runs rarely is not
+// inlined: the loop has to fit the instruction caches.  With three copies of
+// the evaluation, two calls of this function per kernel and the rest inlined,
+// a warp of the batch engine waited 3.4 to 10.6 cycles per issued instruction
+// for its next one, more than for anything else.
 template <bool ORDERED>
-__device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d0, const td_search_limits &lim, const td_donate_ctx *dc) {
+__device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, bool shared) {
     const int lane = threadIdx.x & 31;
     const int last_tri = td_tri_base(N) + td_triple_count(N) - 1;  // child u is triple last_tri - u
     td_dfs_out r;
@@ -924,58 +984,60 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
     r.found_move = 0;
     r.expansions = 0;
     int level = d0;
-    uint32_t O = 0, F = 0;
-    int found;
-    const int eg_moves = s.eg_moves;  // the endgame table decides children (0: it does not apply)
-    bool solved = false;  // free order: the table has shown the way to a witness
-    // prepares and evaluates the node at `level`, and lets the table decide its
-    // children.  A move joins at most three pairs of neighbours, so only a node
-    // of at most TD_EG_SYMBOLS + 3 symbols that omega moves has one in the table.
-    auto expand = [&]() {
-        const int odd = td_prepare_rows(s, level, N, O, F);
-        const int spare = eg_moves - level - ((N - odd) >> 1);
-        const int moved = N - __popc(F);  // symbols left
-        const bool endgame =
-            eg_moves > level + 1 && spare >= 0 && moved <= TD_EG_SYMBOLS + 3;  // warp-uniform
-        if constexpr (ORDERED) {
-            found = td_evaluate(s, code, N, level, odd, O, F);
-            if (found >= 0) found = td_tri_table[last_tri - found];
-            // with two spare moves no child that the table holds is dropped
-            else if (lane == 0) s.spare[level] = (uint8_t)(endgame && spare < 2 ? spare : 255);
-            __syncwarp();
-        } else {
-            if (lane == 0) s.spare[level] = (uint8_t)(endgame ? spare : 255);
-            found = td_evaluate_rows(s, code, N, level, odd, O, F);
-            if (endgame && found < 0 && spare == 0) {
-                const uint4 w = s.pw[level][lane];
-                if (__reduce_add_sync(TD_FULL, (unsigned)(__popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w))) >=
-                    TD_EG_MANY)
-                    solved |= td_eg_filter(s, code, level, N);
+    bool solved = false;  // free order: the endgame table has shown the way to a witness
+    td_unpack_state(s, d0, s.L[d0], s.off[d0], N);
+    uint32_t work = 0;  // nodes expanded here
+    int since_check = 0;
+    bool due = false;            // free order: the scheduler's counters were read (lane 0)
+    int waiting = 0, ended = 0;  // idle warps not yet served by an item; the instance is decided
+    int attempt = 0;     // free order: restarts with another child order (td_attempt_budget)
+    uint32_t ord = 0, attempt_exp = 0;
+    uint32_t attempt_budget = ORDERED ? ~0u : td_attempt_budget(s.lim.restart_base, 0);
+    // a unit of a raced instance: the inverse's side, or the instance's side
+    // once it queued the inverse
+    bool raced = !ORDERED && shared && s.dc.side;
+    for (;;) {
+        // expand the node at `level`, and let the endgame table decide its
+        // children.  A move joins at most three pairs of neighbours, so only a
+        // node of at most TD_EG_SYMBOLS + 3 symbols that omega moves has one in
+        // the table.
+        {
+            uint32_t O, F;
+            const int odd = td_prepare_rows(s, level, N, O, F);
+            const int eg_moves = s.eg_moves;  // 0: the table does not apply
+            const int spare = eg_moves - level - ((N - odd) >> 1);
+            const bool endgame =
+                eg_moves > level + 1 && spare >= 0 && N - __popc(F) <= TD_EG_SYMBOLS + 3;  // warp-uniform
+            int found;
+            if constexpr (ORDERED) {
+                // with two spare moves no child that the table holds is dropped
+                if (lane == 0) s.spare[level] = (uint8_t)(endgame && spare < 2 ? spare : 255);
+                found = td_evaluate(s, N, level, odd, O, F);
+                if (found >= 0) found = td_tri_table[last_tri - found];
+            } else {
+                if (lane == 0) s.spare[level] = (uint8_t)(endgame ? spare : 255);
+                found = td_evaluate_rows(s, N, level, odd, O, F);
+            }
+            ++work;
+            if constexpr (ORDERED) ++r.expansions;
+            else r.expansions = work;
+            if (found >= 0) {
+                r.found_move = (uint16_t)found;
+                r.depth = level + 1;
+                r.status = TD_DFS_FOUND;
+                break;
+            }
+            if constexpr (!ORDERED) {
+                ++attempt_exp;
+                if (endgame && spare == 0) {
+                    const uint4 w = s.pw[level][lane];
+                    const unsigned n = __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w);
+                    if (__reduce_add_sync(TD_FULL, n) >= TD_EG_MANY)
+                        solved |= td_eg_filter(s, level, N);
+                }
             }
         }
-    };
-    td_unpack_state(s, d0, s.L[d0], s.off[d0], N);
-    expand();
-    uint32_t work = 1;  // nodes expanded here
-    r.expansions = 1;
-    int since_check = 0;
-    int attempt = 0;     // free order: restarts with another child order (td_attempt_budget)
-    uint32_t ord = 0, attempt_exp = 1;
-    uint32_t attempt_budget = ORDERED ? ~0u : td_attempt_budget(lim.restart_base, 0);
-    // a unit of a raced instance (the inverse's side, or the instance's side
-    // once it queued the inverse) looks for the other side's verdict every 16
-    // expansions, so that the loser stops soon after the winner
-    bool raced = !ORDERED && dc && dc->side;
-    // the search that the unit's states are recorded for (td_tt_visit)
-    const uint32_t tt_sub = dc ? (uint32_t)(dc->side << 6 | dc->attempt) : 0u;
-    for (;;) {
-        if (found >= 0) {
-            r.found_move = (uint16_t)found;
-            r.depth = level + 1;
-            r.status = TD_DFS_FOUND;
-            break;
-        }
-        if (r.expansions >= lim.max_expansions || work >= lim.max_work) {
+        if (r.expansions >= s.lim.max_expansions || work >= s.lim.max_work) {
             r.status = TD_DFS_BUDGET;
             break;
         }
@@ -986,67 +1048,40 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
                 // the next attempt's entries have another number
                 ++attempt;
                 // a root search that may race queues its inverse when it starts
-                // attempt dc->race; another warp then searches it alongside
-                if (dc && attempt == dc->race && !dc->side && d0 == 0 && td_spawn_inverse(s, *dc, N))
-                    raced = true;
+                // attempt dc.race; another warp then searches it alongside
+                if (shared && attempt == s.dc.race && !s.dc.side && d0 == 0 && td_spawn_inverse(s, N)) raced = true;
                 ord = td_order_variant(attempt);
-                attempt_budget = td_attempt_budget(lim.restart_base, attempt);
-                attempt_exp = 1;
+                attempt_budget = td_attempt_budget(s.lim.restart_base, attempt);
+                attempt_exp = 0;
                 level = d0;
-                expand();
-                ++work;
-                ++r.expansions;
                 continue;
             }
-        }
-        if constexpr (!ORDERED) {
-            if (dc && ++since_check >= dc->check_every) {
-                since_check = 0;
-                int hungry = 0, stop = 0;
-                if (lane == 0) {
-                    // idle warps not yet served by an unclaimed item: without
-                    // this, every busy warp would donate to the same few idle ones
-                    if (dc->tickets) {
-                        // takers holding a ticket past the last item produced
-                        hungry = *(volatile int *)&dc->pool->consumed - *(volatile int *)&dc->pool->produced;
-                    } else {
-                        const int idle = *(volatile int *)&dc->pool->idle;
-                        const int unclaimed =
-                            *(volatile int *)&dc->pool->produced - *(volatile int *)&dc->pool->consumed;
-                        hungry = idle - unclaimed;
-                    }
-                    stop = *(volatile int *)&dc->state->found;
-                }
-                stop = __shfl_sync(TD_FULL, stop, 0);
-                if (stop) {
+            if (due) {  // the counters were read before the expansion
+                due = false;
+                const int hungry = __shfl_sync(TD_FULL, waiting, 0);
+                if (__shfl_sync(TD_FULL, ended, 0)) {
                     r.status = TD_DFS_ABORTED;
                     break;
                 }
-                hungry = __shfl_sync(TD_FULL, hungry, 0);
+                if (hungry > 0 && !s.dc.idle_seen) {
+                    __syncwarp();
+                    if (lane == 0) td_serve_idle_warps(s.dc);
+                    __syncwarp();
+                }
                 // a search that has handed out subtrees no longer restarts: the
                 // subtrees of an abandoned attempt would go on being searched,
                 // and searching in parallel already varies the order
-                if (hungry > 0 && !solved && td_donate(s, *dc, code, d0, level, N, min(hungry, dc->grain), dc->attempt + attempt) > 0)
+                if (hungry > 0 && !solved &&
+                    td_donate(s, d0, level, N, min(hungry, s.dc.grain), s.dc.attempt + attempt) > 0)
                     attempt_budget = ~0u;
-            }
-        }
-        if constexpr (!ORDERED) {
-            if (raced && (work & 15u) == 0) {
-                int stop = 0;
-                if (lane == 0) stop = *(volatile int *)&dc->state->found;
-                if (__shfl_sync(TD_FULL, stop, 0)) {
-                    r.status = TD_DFS_ABORTED;
-                    break;
-                }
             }
         }
         if ((work & 255u) == 0) {
             int stop = 0;
             if (lane == 0) {
-                if (lim.deadline_ns && td_globaltimer() > lim.deadline_ns) stop = 1;
-                if (lim.abort_flag && *(volatile const int *)lim.abort_flag) stop = 1;
+                if (s.lim.deadline_ns && td_globaltimer() > s.lim.deadline_ns) stop = 1;
                 // a subtree of a split ordered search: one of lower rank has a witness
-                if (lim.cutoff && *(volatile const int *)lim.cutoff < lim.rank) stop = 2;
+                if (s.lim.cutoff && *(volatile const int *)s.lim.cutoff < s.lim.rank) stop = 2;
             }
             stop = __shfl_sync(TD_FULL, stop, 0);
             if (stop) {
@@ -1055,11 +1090,11 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
             }
         }
         // walk to the next node to expand: backtracks, and in free order the
-        // children skipped through the table, change no expansion count, so
+        // children skipped through the tables, change no expansion count, so
         // the checks above run once per expansion
-        uint32_t t = 0;
         int walk = 0;  // 1: the subtree is exhausted, 2: a root accepted on visit (ordered), 3: out of budget
         for (;;) {
+            int t;
             if constexpr (ORDERED) {
                 const int spare = s.spare[level];
                 if (spare != 255) {
@@ -1067,41 +1102,37 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
                     // witness; a budget that it would exhaust ends it there
                     const uint32_t skipped = td_eg_skip(s, level, N, spare);
                     r.expansions = r.expansions + skipped < r.expansions ? ~0u : r.expansions + skipped;
-                    if (skipped && r.expansions >= lim.max_expansions) {
-                        r.expansions = (uint32_t)lim.max_expansions;
+                    if (skipped && r.expansions >= s.lim.max_expansions) {
+                        r.expansions = s.lim.max_expansions;
                         walk = 3;
                         break;
                     }
                 }
                 int accepted;
-                const int u = td_next_child(s, level, &accepted);
-                if (u < 0) {
-                    if (level == d0) { walk = 1; break; }
-                    --level;
-                    continue;
+                t = td_next_child(s, level, &accepted);
+                if (t >= 0) {
+                    t = td_tri_table[last_tri - t];
+                    if (accepted) {
+                        r.found_move = (uint16_t)t;
+                        walk = 2;
+                        break;
+                    }
                 }
-                t = td_tri_table[last_tri - u];
-                if (accepted) {
-                    walk = 2;
-                    break;
-                }
-                if (lane == 0) s.path[level] = (uint16_t)t;
-                td_apply_bytes(s, level, t, N);
-                break;
             } else {
-                const int m = td_next_child_rows(s, code, level, td_level_order(ord, attempt, level));
-                if (m < 0) {
-                    if (level == d0) { walk = 1; break; }
-                    --level;
-                    continue;
-                }
-                t = (uint32_t)m & 0x7fffu;
-                if (lane == 0) s.path[level] = (uint16_t)t;
-                td_apply_bytes(s, level, t, N);
+                t = td_next_child_rows(s, level, td_level_order(ord, attempt, level));
+            }
+            if (t < 0) {
+                if (level == d0) { walk = 1; break; }
+                --level;
+                continue;
+            }
+            if (lane == 0) s.path[level] = (uint16_t)(t & 0x7fff);
+            td_apply_bytes(s, level, (uint32_t)t, N);
+            if constexpr (!ORDERED) {
                 const int spare = s.spare[level];
                 if (spare != 255) {
                     // a 0 child has a spare move less than its parent
-                    const uint32_t e = td_eg_look(s, level + 1, N, spare == (m >> 15));
+                    const uint32_t e = td_eg_look(s, level + 1, N, spare == (t >> 15));
                     if (e == 0) {
                         solved = true;
                         break;
@@ -1109,28 +1140,39 @@ __device__ td_dfs_out td_dfs(td_warp_smem &s, const td_codes &code, int N, int d
                     if (e != TD_EG_UNKNOWN) continue;
                 }
                 // taken up already with at least this budget?
-                if (lim.tt && !solved && (work >= TD_TT_AFTER || d0 > 0) &&
-                    td_tt_visit(s, lim, level + 1, N, dc ? dc->inst : 0u, tt_sub + (uint32_t)attempt))
+                if (!solved && (work >= TD_TT_AFTER || d0 > 0) && s.lim.tt &&
+                    td_tt_visit(s, level + 1, N, s.dc.inst, (uint32_t)(s.dc.side << 6) + (uint32_t)(s.dc.attempt + attempt)))
                     continue;
-                break;
+            }
+            break;
+        }
+        if (walk) {
+            if (walk == 2) {
+                r.depth = level + 1;
+                r.status = TD_DFS_FOUND;
+            } else if (walk == 3) {
+                r.status = TD_DFS_BUDGET;
+            }
+            break;
+        }
+        if constexpr (!ORDERED) {
+            // a raced unit looks for the other side's verdict at least every
+            // 16 expansions
+            if (shared && ++since_check >= (raced ? min(s.dc.check_every, 16) : s.dc.check_every)) {
+                // read now and used after the expansion, which hides the latency
+                since_check = 0;
+                due = true;
+                if (lane == 0) {
+                    const unsigned long long pc = *(volatile unsigned long long *)&s.dc.pool->produced;
+                    waiting = (int)(pc >> 32) - (int)(uint32_t)pc;
+                    // takers holding a ticket past the last item produced; in
+                    // the serving loop, idle warps beyond the unclaimed items
+                    if (!s.dc.tickets) waiting += *(volatile int *)&s.dc.pool->idle;
+                    ended = *(volatile int *)&s.dc.state->found;
+                }
             }
         }
-        if (walk == 1) break;
-        if (walk == 3) {
-            r.status = TD_DFS_BUDGET;
-            break;
-        }
-        if (walk == 2) {
-            r.found_move = (uint16_t)t;
-            r.depth = level + 1;
-            r.status = TD_DFS_FOUND;
-            break;
-        }
         ++level;
-        expand();
-        if constexpr (!ORDERED) ++attempt_exp;
-        ++work;
-        ++r.expansions;
     }
     __syncwarp();
     return r;
@@ -1141,13 +1183,13 @@ __device__ __forceinline__ bool td_instance_ok(const td_instance &x) {
            td_inst_init(x) <= TD_MAX_N;
 }
 
-// Loads the lane's pair slots for N (`codeN` caches the N they were loaded
-// for) and the instance's rate masks; places its root at level 0.
-__device__ __forceinline__ void td_setup_root(td_warp_smem &s, const td_instance &x, td_codes &code, int &codeN) {
+// Loads the warp's pair slots for N, unless they are, and the instance's rate
+// masks; places its root at level 0.
+__device__ __forceinline__ void td_setup_root(td_warp_smem &s, const td_instance &x) {
     const int lane = threadIdx.x & 31;
-    if (codeN != x.n_symbols) {
-        td_load_pairs(x.n_symbols, code);
-        codeN = x.n_symbols;
+    if (s.pairs_n != x.n_symbols) {
+        td_load_pairs(s, x.n_symbols);
+        if (lane == 0) s.pairs_n = x.n_symbols;
     }
     td_rate_masks(s, x);
     if (lane == 0) {
@@ -1181,16 +1223,15 @@ __device__ __forceinline__ void td_write_result(td_result *out, int status, int 
 // One complete search of instance x by the calling warp (no sharing); returns
 // the status it wrote (uniform across the warp).
 template <bool ORDERED>
-__device__ int td_warp_search(const td_instance &x, td_result *out, td_warp_smem &s,
-                               td_codes &code, int &codeN, const td_search_limits &lim) {
+__device__ int td_warp_search(const td_instance &x, td_result *out, td_warp_smem &s) {
     int status = TD_NOT_FOUND, depth = 0;
     uint32_t expansions = 0;
     uint16_t found_move = 0;
     if (!td_instance_ok(x)) {
         status = TD_ERR_ARG;
     } else if (td_triple_count(x.n_symbols) > 0) {
-        td_setup_root(s, x, code, codeN);
-        const td_dfs_out r = td_dfs<ORDERED>(s, code, x.n_symbols, 0, lim, nullptr);
+        td_setup_root(s, x);
+        const td_dfs_out r = td_dfs<ORDERED>(s, x.n_symbols, 0, false);
         expansions = r.expansions;
         if (r.status == TD_DFS_FOUND) {
             status = TD_FOUND;

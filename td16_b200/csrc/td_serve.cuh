@@ -145,36 +145,45 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
         return;
     }
     td_warp_smem &s = ws[warp];
-    td_codes code;
-    int codeN = -1;
-    td_search_limits lim;
-    lim.max_expansions = max_exp ? max_exp : ~0ull;
-    lim.max_work = ~0u;
-    lim.deadline_ns = deadline;
-    lim.abort_flag = nullptr;
-    lim.tt = ALL_ORDERED ? nullptr : tt;
-    lim.tt_id = 0;  // requests are numbered across the launches that share a table
-    lim.tt_shift = tt_shift;
-    lim.restart_base = 0;  // serving searches are not restarted
-    lim.cutoff = nullptr;
-    lim.rank = 0;
-    td_donate_ctx dc;
-    dc.ring = 1;
-    dc.tickets = 0;
-    dc.side = 0;
-    dc.attempt = 0;
-    dc.race = 0;  // set per fresh request (the per-call server's race)
-    dc.spawn_base = 0;
-    dc.spawn_capacity = 0;
-    dc.deadline_ns = deadline;
-    dc.pool = pool;
-    dc.items = items;
-    dc.ready = ready;
-    dc.epoch = 0;
-    dc.capacity = item_capacity;
-    dc.grain = grain;
-    dc.max_level = max_level;
-    dc.check_every = check_every > 0 ? check_every : 1;
+    if (lane == 0) {
+        td_search_limits lim;
+        lim.max_expansions = max_exp && max_exp < ~0u ? (uint32_t)max_exp : ~0u;
+        lim.max_work = ~0u;
+        lim.deadline_ns = deadline;
+        lim.tt = ALL_ORDERED ? nullptr : tt;
+        lim.tt_id = 0;  // requests are numbered across the launches that share a table
+        lim.tt_shift = tt_shift;
+        lim.restart_base = 0;
+        lim.cutoff = nullptr;
+        lim.rank = 0;
+        s.lim = lim;
+        s.pairs_n = -1;
+        td_donate_ctx dc;
+        dc.ring = 1;
+        dc.tickets = 0;
+        dc.deadline_ns = deadline;
+        dc.pool = pool;
+        dc.items = items;
+        dc.ready = ready;
+        dc.epoch = 0;
+        dc.capacity = item_capacity;
+        // a serving launch mostly has idle warps, but they claim items and
+        // requests by compare-and-swap, so it does not go as far as the batch
+        // engine's td_serve_idle_warps.  2,048 calls of n = 8..14 at the lower
+        // bound from 16 threads, with the default (1, 2, 32): as configured
+        // 11.2 ms, 4 x / + 2 / 1/4 7.8 ms, 8 x / + 4 / 1/16 24.8 ms
+        dc.grain = min(32, 4 * grain);
+        dc.max_level = min(TD_MAX_DEPTH - 1, max_level + 2);
+        dc.check_every = max(1, check_every / 4);
+        dc.inst = 0;
+        dc.state = nullptr;
+        dc.side = 0;
+        dc.attempt = 0;
+        dc.race = 0;  // set per fresh request (the per-call server's race)
+        dc.idle_seen = 1;
+        s.dc = dc;
+    }
+    __syncwarp();
     bool idle = false;
     unsigned backoff = 128;
     for (;;) {
@@ -261,8 +270,8 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 }
             } else {
                 if (MODE == TD_SERVE_PER_REQUEST) ord = (x.packed & TD_PACKED_ORDERED) != 0;
-                if (ord) td_setup_root(s, x, code, codeN);
-                else td_setup_root(s, x, code, codeN);
+                if (ord) td_setup_root(s, x);
+                else td_setup_root(s, x);
                 run = true;
             }
         } else {
@@ -297,7 +306,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 const unsigned slot = (unsigned)(req % ring_size);
                 const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(&queue[slot]));
                 const td_instance x = *reinterpret_cast<const td_instance *>(&v);
-                td_setup_root(s, x, code, codeN);
+                td_setup_root(s, x);
                 d0 = it.depth & 15;
                 side = it.depth >> 7;
                 attempt = ((it.depth >> 4) & 7) | ((it.off >> 5) << 3);
@@ -311,8 +320,8 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 if (lane == 0) stop = *(volatile int *)&state[slot].found;
                 run = !__shfl_sync(TD_FULL, stop, 0);
                 td_unpack_state(s, d0, it.L, it.off & 31, x.n_symbols);
-                if (run && d0 > 0 && lim.tt &&
-                    td_tt_visit(s, lim, d0, x.n_symbols, (uint32_t)req, (uint32_t)(side << 6 | attempt)))
+                if (run && d0 > 0 && !ALL_ORDERED && tt &&
+                    td_tt_visit(s, d0, x.n_symbols, (uint32_t)req, (uint32_t)(side << 6 | attempt)))
                     run = false;
                 if (!run) {  // the request has its witness, or another unit took the state up
                     if (td_finish_unit<true>(r, &state[slot], &results[slot], s.path, side) && lane == 0) {
@@ -326,33 +335,27 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
             const unsigned slot = (unsigned)(req % ring_size);
             const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(&queue[slot]));
             const td_instance x = *reinterpret_cast<const td_instance *>(&v);
-            dc.inst = (uint32_t)req;
-            dc.state = &state[slot];
-            td_search_limits ulim = lim;
-            if (request_limit_ns) ulim.deadline_ns = min(deadline, td_globaltimer() + request_limit_ns);
-            // a fresh request may restart, and so may the root of its inverse; a
-            // donated subtree is searched once.  A fresh free-order request of
-            // the per-call server with full sorting races the search of its
-            // inverse from restart attempt `race` (td_steal_kernel's race).
-            ulim.restart_base = kind == 1 || d0 == 0 ? restart_base : 0;
-            dc.side = side;
-            dc.attempt = attempt;
-            dc.race = MODE == TD_SERVE_PER_REQUEST && kind == 1 && !ord && restart_base && td_inst_full(x) ? race : 0;
-            if (ord) r = td_dfs<true>(s, code, x.n_symbols, d0, ulim, nullptr);
-            else r = td_dfs<false>(s, code, x.n_symbols, d0, ulim, &dc);
-            dc.side = 0;
-            dc.attempt = 0;
-            dc.race = 0;
-            // a witness of the inverse becomes one of the request; one that does
-            // not convert is reported as a failed replay, and one that leaves the
-            // reference's move filter on the request's side is dropped
+            if (lane == 0) {
+                s.lim.deadline_ns = request_limit_ns ? min(deadline, td_globaltimer() + request_limit_ns) : deadline;
+                // a fresh request may restart, and so may the root of its inverse;
+                // a donated subtree is searched once.  A fresh free-order request
+                // of the per-call server with full sorting races the search of its
+                // inverse from restart attempt `race` (td_steal_kernel's race).
+                s.lim.restart_base = kind == 1 || d0 == 0 ? restart_base : 0;
+                s.dc.inst = (uint32_t)req;
+                s.dc.state = &state[slot];
+                s.dc.side = side;
+                s.dc.attempt = attempt;
+                s.dc.race = MODE == TD_SERVE_PER_REQUEST && kind == 1 && !ord && restart_base && td_inst_full(x) ? race : 0;
+            }
+            __syncwarp();
+            if (ord) r = td_dfs<true>(s, x.n_symbols, d0, false);
+            else r = td_dfs<false>(s, x.n_symbols, d0, true);
             if (side && r.status == TD_DFS_FOUND) {
-                if (!td_inverse_result(s, x, r)) {
-                    r.status = TD_DFS_EXHAUSTED;
-                    if (lane == 0) atomicCAS(&state[slot].error, 0, TD_ERR_VERIFY);
-                } else if (!td_filtered_witness(s, x, r)) {
-                    r.status = TD_DFS_EXHAUSTED;
-                }
+                const int t = td_inverse_witness(s, x, r.depth, r.found_move);
+                if (t < 0) r.status = TD_DFS_EXHAUSTED;
+                else r.found_move = (uint16_t)t;
+                if (t == -1 && lane == 0) atomicCAS(&state[slot].error, 0, TD_ERR_VERIFY);
             }
             if (td_finish_unit<true>(r, &state[slot], &results[slot], s.path, side) && lane == 0) {
                 done[slot] = (unsigned long long)req + 1ull;
