@@ -106,10 +106,10 @@ TD_HD void td_apply_move(uint64_t L, int off, int N, int i, int j, int k,
     if (p1 == 0) { x = p2 - 1; y = p3 - 1; z = n; }
     else { x = p1 - 1; y = p2 - 1; z = p3 - 1; }
     const int a = y - x, b = z - y;  // lengths of the swapped blocks
-    const uint64_t keep = (L & td_low_nibbles(x)) | (L & ~td_low_nibbles(z));
-    const uint64_t blockA = (L >> (4 * x)) & td_low_nibbles(a);
-    const uint64_t blockB = (L >> (4 * y)) & td_low_nibbles(b);
-    *outL = keep | (blockB << (4 * x)) | (blockA << (4 * (x + b)));
+    // the two blocks as one segment, rotated by a: what changes is put back
+    const uint64_t seg = L >> (4 * x);
+    const uint64_t turned = ((seg >> (4 * a)) & (~0ull >> (64 - 4 * b))) | (seg << (4 * b));
+    *outL = L ^ (((seg ^ turned) & (~0ull >> (64 - 4 * (a + b)))) << (4 * x));
     // new start of the caller's array, followed through the swap
     int S = (i == 0) ? Q : off;
     if (S != 0) {
