@@ -133,7 +133,9 @@ int td_destroy(void);                   /* releases every slot */
  * instances per ticket of the ordered persistent kernel. */
 int td_configure(int warps_per_block, int grain);
 /* Deadline of every later launch in seconds (default TD16_TIME_LIMIT_S or
- * 300): searches and device waits that pass it end with a timeout status. */
+ * 300), from the launch's first operation on its stream (the growth of its
+ * buffers counts): searches and device waits that pass it end with a timeout
+ * status. */
 int td_set_time_limit(double seconds);
 /* Work donation of the free-order engine: items per donation, deepest level
  * whose children may be donated, expansions between idle checks (default
@@ -172,13 +174,13 @@ int td_configure_restart(int base);
  * the race is on.  No counterpart in the reference, whose search runs one
  * order to the end. */
 int td_configure_race(int attempt);
-/* Reference-order batches (TD_FLAG_ORDERED, no expansion budget) run every
- * walk on one warp for first_pass_expansions (default 64), then split each
- * walk left over into the subtrees of its root's children, searched at once
- * and joined in the walk's order: witness and expansion count are the
- * one-warp walk's.  records (default 2^20, at most 2^24; 34 bytes each per
- * slot) bounds the subtrees of one launch; a root whose children find no
- * room runs whole.  first_pass_expansions = 0: no split. */
+/* Reference-order batches (TD_FLAG_ORDERED, no expansion budget) walk every
+ * instance on one warp; while other warps wait, a walk that has run for
+ * first_pass_expansions (default 64) gives away the subtrees it has not come
+ * to, which are searched at once and joined in the walk's order: witness and
+ * expansion count are the one-warp walk's.  records (default 2^20, at most
+ * 2^24; 68 bytes each per slot) bounds the subtrees of one launch; a walk that
+ * finds no room goes on whole.  first_pass_expansions = 0: no split. */
 int td_configure_split(int first_pass_expansions, int records);
 
 /* ---- instance preparation (host, no GPU needed) -------------------------- */

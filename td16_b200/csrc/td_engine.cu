@@ -68,14 +68,14 @@ __device__ __forceinline__ void td_set_limits(td_warp_smem &s, uint64_t max_exp,
     if ((threadIdx.x & 31) == 0) {
         td_search_limits lim;
         lim.max_expansions = max_exp && max_exp < ~0u ? (uint32_t)max_exp : ~0u;
-        lim.max_work = ~0u;
+        lim.split_after = ~0u;
         lim.deadline_ns = time_limit_ns ? td_globaltimer() + time_limit_ns : 0;
         lim.tt = nullptr;
         lim.tt_id = 0;
         lim.tt_shift = 64;
         lim.restart_base = 0;
-        lim.cutoff = nullptr;
-        lim.rank = 0;
+        lim.cutoff = lim.cutoff2 = nullptr;
+        lim.rank = lim.rank2 = 0;
         s.lim = lim;
         s.pairs_n = -1;
     }
@@ -96,21 +96,14 @@ __global__ void __launch_bounds__(256) td_plain_kernel(const td_instance *__rest
     td_warp_search<ORDERED>(x, &out[idx], ws[warp]);
 }
 
-// hard_count / hard_list (or null): the first pass of a split batch of the
-// reference order; instances not finished within max_exp nodes expanded here
-// are listed, for the split pass (td_split_*).
-template <bool ORDERED>
 __global__ void __launch_bounds__(256, 4) td_persistent_kernel(const td_instance *__restrict__ in,
                                                            td_result *__restrict__ out, int count,
                                                            int *ticket, int grain, uint64_t max_exp,
-                                                           uint64_t time_limit_ns, int *hard_count = nullptr,
-                                                           int *hard_list = nullptr) {
+                                                           uint64_t time_limit_ns) {
     extern __shared__ __align__(16) uint8_t td_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
-    td_set_limits(ws[warp], hard_list ? 0 : max_exp, time_limit_ns);
-    if (hard_list && lane == 0) ws[warp].lim.max_work = (uint32_t)max_exp;
-    __syncwarp();
+    td_set_limits(ws[warp], max_exp, time_limit_ns);
     for (;;) {
         int first = 0;
         if (lane == 0) first = atomicAdd(ticket, grain);
@@ -119,204 +112,257 @@ __global__ void __launch_bounds__(256, 4) td_persistent_kernel(const td_instance
         const int last = min(count, first + grain);
         for (int idx = first; idx < last; ++idx) {
             const td_instance x = in[idx];
-            const int st = td_warp_search<ORDERED>(x, &out[idx], ws[warp]);
-            if (hard_list && st == TD_ERR_BUDGET && lane == 0) hard_list[atomicAdd(hard_count, 1)] = idx;
+            td_warp_search<true>(x, &out[idx], ws[warp]);
         }
     }
 }
 
-// ---- the reference order, split below the root ------------------------------
-//
-// The reference's single-queue order is one depth-first walk, so a search
-// that runs long is a long serial chain on one warp while the rest of the GPU
-// idles: the tail of an ordered batch.  The walk visits the root's children
-// c_0, c_1, ... in a fixed order and exhausts each subtree before the next, so
-// its witness is the one it meets in the first subtree that holds any, and it
-// meets it there exactly as that subtree's own walk does.  The subtrees can
-// therefore be searched at once, one warp each, and joined in rank order: the
-// witness is the found one of lowest rank r, and the walk's expansion count
-// is 1 (the root) plus the expansions of subtrees 0..r, the earlier ones run
-// to exhaustion.  Both equal the one-warp walk's, bit for bit.  A subtree
-// that ranks after a found one stops early; its result is never read.
-//
-// Only instances that a first one-warp pass did not finish within
-// TD_SPLIT_BUDGET expansions take this path (td_persistent_kernel lists
-// them); the rest keep the first pass's results.  Passes: td_split_roots_kernel
-// lists each such root's children in visiting order, td_split_kernel searches
-// the subtrees rank-major (the first subtree of every instance, then the
-// second, ...), td_split_join_kernel writes the joined results.
-
-#define TD_SPLIT_BUDGET 64        // default expansions of the one-warp first pass (td_configure_split)
-#define TD_SPLIT_RECORDS (1 << 20)  // default subtree records per launch (32 MiB)
-#define TD_SPLIT_SKIPPED 2        // a subtree result that is never read
-
-struct td_split_ctl {
-    int hard;                   // instances the first pass did not finish
-    int max_rank;               // most children of a split root
-    int items_used;             // subtree records reserved
-    unsigned long long ticket;  // units of td_split_kernel claimed
+// A launch's epoch (td_epoch_kernel) and when it began.
+struct td_epoch {
+    uint32_t epoch, pad;
+    uint64_t start_ns;
 };
 
-// Per listed instance h (grid-stride over warps): its root's children in the
-// walk's visiting order, as position triples with bit 15 set for a child
-// accepted on visit, at kids[base[h] ..], nkids[h] of them; nkids[h] = -1
-// when the record space is full (that instance then runs whole).  Also
-// clears the instance's cutoff.
-__global__ void __launch_bounds__(256) td_split_roots_kernel(const td_instance *__restrict__ in,
-                                                            const int *__restrict__ hard_list, td_split_ctl *ctl,
-                                                            uint16_t *__restrict__ kids, int *__restrict__ base,
-                                                            int *__restrict__ nkids, int *__restrict__ cutoff,
-                                                            int records) {
-    extern __shared__ __align__(16) uint8_t td_smem[];
-    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
-    td_warp_smem &s = ws[warp];
-    if (lane == 0) s.pairs_n = -1;
-    __syncwarp();
-    const int H = *(volatile int *)&ctl->hard;
-    for (int h = blockIdx.x * warps + warp; h < H; h += gridDim.x * warps) {
-        const td_instance x = in[hard_list[h]];
-        td_setup_root(s, x);
-        const int N = x.n_symbols, last_tri = td_tri_base(N) + td_triple_count(N) - 1;
-        td_unpack_state(s, 0, x.perm, x.offset, N);
-        uint32_t O, F;
-        const int odd = td_prepare_rows(s, 0, N, O, F);
-        td_evaluate(s, N, 0, odd, O, F);
-        // count the children, reserve their records, then list them from the
-        // last one (the root's visiting order is descending u)
-        const uint32_t w = lane < TD_MAX_STEPS ? s.cw[0][lane] : 0u;
-        const uint32_t fw = lane < TD_MAX_STEPS ? s.root_found[lane] : 0u;
-        int from = __popc(w);  // children in this lane's word and those after it
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_down_sync(TD_FULL, from, o);
-            if (lane + o < 32) from += v;
-        }
-        const int c = __shfl_sync(TD_FULL, from, 0);
-        int at = -1;
-        if (lane == 0) {
-            at = atomicAdd(&ctl->items_used, c);
-            if (at > records - c) at = -1;
-        }
-        at = __shfl_sync(TD_FULL, at, 0);
-        if (at >= 0) {
-            int k = at + from - __popc(w);
-            for (uint32_t rest = w; rest; ++k) {
-                const int bit = 31 - __clz(rest);
-                rest &= ~(1u << bit);
-                kids[k] = (uint16_t)(td_tri_table[last_tri - 32 * lane - bit] | (((fw >> bit) & 1u) << 15));
-            }
-        }
-        if (lane == 0) {
-            base[h] = at;
-            nkids[h] = at < 0 ? -1 : c;
-            cutoff[h] = 0x7fffffff;  // no witness yet
-            if (at >= 0) atomicMax(&ctl->max_rank, c);
-        }
-        __syncwarp();
-    }
-}
+// ---- claiming work --------------------------------------------------------------
+//
+// How the warps of a launch share instances and items (td_steal_kernel,
+// td_ordered_kernel).  A warp takes fresh instances by ticket while any are
+// left, then one item ticket (fetch-and-add: it never fails) and waits for its
+// item: item i belongs to ticket i.  A waiting warp polls only the ready flag
+// of its own item, so thousands of them load thousands of different words and
+// none that a busy warp needs, and they can poll often.  `outstanding` counts
+// the instances in progress plus the items not yet finished: it is raised
+// before an instance ticket is taken and before items can be claimed, and
+// lowered when a unit ends.  With no instance ticket left and nothing
+// outstanding no unit can start again: the warp that brings the count there
+// sets `done` and then ~epoch in the flag of every ticket taken.  A warp that
+// took its ticket too late for that reads `done` at its first poll and at every
+// 16th.  Every wait ends at the launch deadline.
+//
+// Polling the shared counters instead (five of them, at up to 32 us
+// intervals, since shorter ones slowed the busy warps) left the warps idle for
+// most of a launch's tail.
+struct td_claims {
+    td_pool *pool;
+    uint32_t *ready;
+    uint32_t epoch;
+    int count, capacity;
+    int my_ticket;  // lane 0: this warp's item ticket, -1 = none
+    bool fresh;     // lane 0: instance tickets may be left
 
-// Resident grid over the units of the split, rank-major: unit u is rank
-// r = u / H of listed instance h = u % H, i.e. subtree r of its root, or for
-// an instance without records (nkids[h] < 0) the whole search at r = 0 (so
-// the longest units start first).
-__global__ void __launch_bounds__(256, 4) td_split_kernel(const td_instance *__restrict__ in,
-                                                      td_result *__restrict__ out, const int *__restrict__ hard_list,
-                                                      td_split_ctl *ctl, const uint16_t *__restrict__ kids,
-                                                      const int *__restrict__ base, const int *__restrict__ nkids,
-                                                      int *cutoff, td_result *__restrict__ items,
-                                                      uint64_t time_limit_ns) {
+    // Lowers the outstanding count (lane 0); whether the launch has no work left.
+    __device__ __forceinline__ bool release() {
+        if (atomicSub(&pool->outstanding, 1) != 1 || *(volatile int *)&pool->inst_ticket < count) return false;
+        atomicExch(&pool->done, 1);
+        __threadfence();
+        return true;
+    }
+
+    // Wakes the waiting warps of a launch without work.
+    __device__ __forceinline__ void wake() {
+        const int lane = threadIdx.x & 31;
+        int from = 0, taken = 0;
+        if (lane == 0) {
+            from = *(volatile int *)&pool->produced;
+            taken = min(*(volatile int *)&pool->consumed, capacity);
+        }
+        from = __shfl_sync(TD_FULL, from, 0);
+        taken = __shfl_sync(TD_FULL, taken, 0);
+        for (int i = from + lane; i < taken; i += 32) *(volatile uint32_t *)&ready[i] = ~epoch;
+    }
+
+    // Ends a unit; whether the launch has no work left (uniform across the warp).
+    __device__ __forceinline__ bool finish() {
+        int last = 0;
+        if ((threadIdx.x & 31) == 0) last = release();
+        last = __shfl_sync(TD_FULL, last, 0);
+        if (last) wake();
+        return last != 0;
+    }
+
+    // The next unit: 1 an instance, 2 an item, 0 no work left (uniform across
+    // the warp).
+    __device__ __forceinline__ int next(td_warp_smem &s, int *unit_out) {
+        const int lane = threadIdx.x & 31;
+        unsigned backoff = 64, polls = 0;
+        for (;;) {
+            int kind = 0, unit = -1;
+            if (lane == 0) {
+                if (fresh) {
+                    if (*(volatile int *)&pool->inst_ticket < count) {
+                        atomicAdd(&pool->outstanding, 1);
+                        unit = atomicAdd(&pool->inst_ticket, 1);
+                        if (unit < count) kind = 1;
+                        else if (release()) kind = 4;
+                    }
+                    fresh = kind == 1;
+                }
+                if (!kind) {
+                    if (my_ticket < 0) {
+                        my_ticket = atomicAdd(&pool->consumed, 1);
+                        td_serve_idle_warps(s.dc);
+                    }
+                    const uint32_t flag = my_ticket < capacity ? *(volatile uint32_t *)&ready[my_ticket] : 0u;
+                    if (flag == epoch) {
+                        kind = 2;
+                        unit = my_ticket;
+                        my_ticket = -1;
+                    } else if (flag == ~epoch) {
+                        kind = 3;
+                    } else if ((polls++ & 15u) == 0) {
+                        if (*(volatile int *)&pool->done) {
+                            kind = 3;
+                        } else if (s.lim.deadline_ns && td_globaltimer() > s.lim.deadline_ns) {
+                            atomicCAS(&pool->error, 0, TD_ERR_TIMEOUT);
+                            kind = 3;
+                        }
+                    }
+                }
+            }
+            kind = __shfl_sync(TD_FULL, kind, 0);
+            if (kind == 4) wake();
+            if (kind >= 3) return 0;
+            if (kind) {
+                *unit_out = __shfl_sync(TD_FULL, unit, 0);
+                if (kind == 2) td_fence();
+                return kind;
+            }
+            __nanosleep(backoff);
+            backoff = min(backoff * 2u, 1024u);
+        }
+    }
+};
+
+#define TD_SPLIT_BUDGET 64          // default expansions of a walk before it may be split (td_configure_split)
+#define TD_SPLIT_RECORDS (1 << 20)  // default subtree records per launch
+
+// Resident grid of the reference order: instances by ticket, then the subtrees
+// that long walks give away (td_ordered.cuh).
+__global__ void __launch_bounds__(256, 4) td_ordered_kernel(const td_instance *__restrict__ in,
+                                                        td_result *__restrict__ out, int count, td_pool *pool,
+                                                        td_split_space sp, uint32_t *ready, const td_epoch *ep,
+                                                        int capacity, int split_after, uint64_t time_limit_ns) {
     extern __shared__ __align__(16) uint8_t td_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    td_warp_smem *ws = reinterpret_cast<td_warp_smem *>(td_smem);
-    td_warp_smem &s = ws[warp];
-    const int H = *(volatile int *)&ctl->hard;
-    const int R = max(1, *(volatile int *)&ctl->max_rank);
-    const unsigned long long units = (unsigned long long)H * (unsigned long long)R;
+    td_warp_smem &s = reinterpret_cast<td_warp_smem *>(td_smem)[warp];
     td_set_limits(s, 0, time_limit_ns);
-    for (;;) {
-        unsigned long long u = 0;
-        if (lane == 0) u = atomicAdd(&ctl->ticket, 1ull);
-        u = __shfl_sync(TD_FULL, u, 0);
-        if (u >= units) break;
-        const int r = (int)(u / (unsigned long long)H), h = (int)(u % (unsigned long long)H);
-        const int nk = nkids[h];
-        if (nk < 0) {
-            if (r == 0) {
-                const int idx = hard_list[h];
-                __syncwarp();
-                if (lane == 0) s.lim.cutoff = nullptr;
-                __syncwarp();
-                td_warp_search<true>(in[idx], &out[idx], s);
-            }
-            continue;
-        }
-        if (r >= nk) continue;  // that root has fewer children; the join reads only nkids[h]
-        td_result *it = &items[base[h] + r];
-        if (*(volatile int *)&cutoff[h] < r) {
-            td_write_result(it, TD_SPLIT_SKIPPED, 0, 0, s.path, 0, 0, 8);
-            continue;
-        }
-        const uint32_t kid = kids[base[h] + r];
-        const uint32_t t = kid & 0x7fffu;
-        const td_instance x = in[hard_list[h]];
-        td_setup_root(s, x);
-        const int N = x.n_symbols;
-        if (lane == 0) s.path[0] = (uint16_t)t;
-        __syncwarp();
-        if (kid & 0x8000u) {  // accepted on visit: the one-move witness
-            td_write_result(it, TD_FOUND, 1, (uint16_t)t, s.path, 0, 0, 8);
-            if (lane == 0) atomicMin(&cutoff[h], r);
-            continue;
-        }
-        uint64_t nL;
-        int noff;
-        td_apply_move(s.L[0], s.off[0], N, t & 31, (t >> 5) & 31, (t >> 10) & 31, &nL, &noff);
-        if (lane == 0) {
-            s.L[1] = nL;
-            s.off[1] = (uint8_t)noff;
-            s.lim.cutoff = &cutoff[h];
-            s.lim.rank = r;
-        }
-        __syncwarp();
-        const td_dfs_out d = td_dfs<true>(s, N, 1, false);
-        int status = TD_NOT_FOUND;
-        if (d.status == TD_DFS_FOUND) status = TD_FOUND;
-        else if (d.status == TD_DFS_ABORTED) status = TD_SPLIT_SKIPPED;
-        else if (d.status == TD_DFS_TIMEOUT) status = TD_ERR_TIMEOUT;
-        td_write_result(it, status, status == TD_FOUND ? d.depth : 0, d.found_move, s.path, d.expansions, 0, 8);
-        if (status == TD_FOUND && lane == 0) atomicMin(&cutoff[h], r);
+    if (lane == 0) {
+        s.dc.pool = pool;
+        s.dc.ready = ready;
+        s.dc.epoch = ep->epoch;
+        if (time_limit_ns) s.lim.deadline_ns = ep->start_ns + time_limit_ns;
+        s.dc.capacity = capacity;
+        s.dc.idle_seen = 1;
+        s.dc.check_every = 8;
+        s.sp = sp;
     }
-}
-
-// The joined result of each split instance, as the one-warp walk would give it.
-__global__ void td_split_join_kernel(const int *__restrict__ hard_list, const td_split_ctl *ctl,
-                                     const int *__restrict__ base, const int *__restrict__ nkids,
-                                     const td_result *__restrict__ items, td_result *__restrict__ out) {
-    const int H = *(volatile const int *)&ctl->hard;
-    for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < H; h += gridDim.x * blockDim.x) {
-        const int nk = nkids[h];
-        if (nk < 0) continue;  // searched whole
-        td_result res;
-        memset(&res, 0, sizeof res);
-        res.status = TD_NOT_FOUND;
-        uint64_t exp = 1;  // the root
-        for (int r = 0; r < nk; ++r) {
-            const td_result it = items[base[h] + r];
-            if (it.status == TD_FOUND) {
-                res = it;
-                exp += it.expansions;
-                break;
-            }
-            if (it.status != TD_NOT_FOUND) {  // a subtree before any witness timed out
-                res.status = TD_ERR_TIMEOUT;
-                break;
-            }
-            exp += it.expansions;
+    __syncwarp();
+    td_claims cl;
+    cl.pool = pool;
+    cl.ready = ready;
+    cl.epoch = s.dc.epoch;
+    cl.count = count;
+    cl.capacity = capacity;
+    cl.my_ticket = -1;
+    cl.fresh = true;
+    for (;;) {
+        int unit;
+        const int kind = cl.next(s, &unit);
+        if (!kind) return;
+        int inst = unit, node = -1, rank = 0, d0 = 0, stop = 0;
+        uint32_t kid = 0;
+        const td_split_node *nd = nullptr;
+        if (kind == 2) {
+            const uint2 w = __ldcg(reinterpret_cast<const uint2 *>(&sp.items[unit]));
+            node = (int)w.x;
+            rank = (int)(w.y & 0xffffu);
+            kid = w.y >> 16;
+            nd = &sp.nodes[node];
+            inst = __ldcg(&nd->inst);
+            d0 = (int)__ldcg(&nd->depth) + 1;
         }
-        res.expansions = exp > 0xffffffffull ? 0xffffffffu : (uint32_t)exp;
-        out[hard_list[h]] = res;
+        const td_instance x = in[inst];
+        const int N = x.n_symbols;
+        td_dfs_out r;
+        r.status = TD_DFS_EXHAUSTED;
+        r.depth = 0;
+        r.found_move = 0;
+        r.expansions = 0;
+        if (lane == 0) {
+            s.sp_inst = inst;
+            s.sp_node = node;
+            s.sp_rank = rank;
+            // a first walk is split after split_after nodes, one that was given
+            // away sooner
+            s.lim.split_after = (uint32_t)(kind == 2 ? split_after / 8 : split_after);
+            s.lim.cutoff = s.lim.cutoff2 = nullptr;
+        }
+        __syncwarp();
+        if (td_instance_ok(x) && td_triple_count(N) > 0) {
+            td_setup_root(s, x);
+            if (kind == 2) {
+                // the moves to the subtree
+                uint64_t L = x.perm;
+                int off = x.offset;
+                for (int d = 0; d < d0; ++d) {
+                    const uint32_t t = d == d0 - 1 ? kid & 0x7fffu : (uint32_t)__ldcg(&nd->path[d]);
+                    td_apply_move(L, off, N, t & 31, (t >> 5) & 31, (t >> 10) & 31, &L, &off);
+                    if (lane == 0) s.path[d] = (uint16_t)t;
+                }
+                if (lane == 0) {
+                    s.L[d0] = L;
+                    s.off[d0] = (uint8_t)off;
+                    // skipped where a lower rank of its node, or of a node further
+                    // up, has a witness; the search goes on looking at two of them
+                    int k = node, rk = rank;
+                    for (int up = 0; k >= 0 && up < 16; ++up) {
+                        const td_split_node *q = &sp.nodes[k];
+                        if (rk > 0) {
+                            if (*(volatile const int *)&q->cutoff < rk) stop = 1;
+                            if (!s.lim.cutoff) {
+                                s.lim.cutoff = &q->cutoff;
+                                s.lim.rank = rk;
+                            } else if (!s.lim.cutoff2) {
+                                s.lim.cutoff2 = &q->cutoff;
+                                s.lim.rank2 = rk;
+                            }
+                        }
+                        rk = __ldcg(&q->rank);
+                        k = __ldcg(&q->parent);
+                    }
+                    // a walk looks at the deadline every 256 nodes, more than
+                    // most subtrees have
+                    if (!stop && s.lim.deadline_ns && td_globaltimer() > s.lim.deadline_ns) stop = 2;
+                }
+                stop = __shfl_sync(TD_FULL, stop, 0);
+                __syncwarp();
+            }
+            if (stop) {
+                r.status = stop == 2 ? TD_DFS_TIMEOUT : TD_DFS_ABORTED;
+            } else if (kid & 0x8000u) {  // accepted when visited: the one-move witness
+                r.status = TD_DFS_FOUND;
+                r.depth = 1;
+                r.found_move = (uint16_t)(kid & 0x7fffu);
+            } else {
+                r = td_dfs<true>(s, N, d0, true);
+            }
+        }
+        int status = r.status == TD_DFS_FOUND ? TD_FOUND
+                     : r.status == TD_DFS_TIMEOUT ? TD_ERR_TIMEOUT
+                     : r.status == TD_DFS_ABORTED ? TD_SPLIT_SKIPPED : TD_NOT_FOUND;
+        if (kind == 1 && !td_instance_ok(x)) status = TD_ERR_ARG;
+        __syncwarp();
+        node = s.sp_node;  // the walk may have been split
+        rank = s.sp_rank;
+        td_result *to = node < 0 ? &out[inst] : &sp.records[__ldcg(&sp.nodes[node].base) + rank];
+        td_write_result(to, status, r.depth, r.found_move, s.path, r.expansions, 0, 8);
+        if (node >= 0) {
+            if (lane == 0 && status == TD_FOUND) atomicMin(&sp.nodes[node].cutoff, rank);
+            td_fence();
+            __syncwarp();
+            td_split_complete(s.sp, node);
+        }
+        if (cl.finish()) return;
     }
 }
 
@@ -396,7 +442,7 @@ __device__ __forceinline__ int td_finish_unit(const td_dfs_out &r, td_inst_state
 #endif
 __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(const td_instance *__restrict__ in,
                                                       td_result *__restrict__ out, int count, td_pool *pool,
-                                                      td_item *items, uint32_t *ready, const uint32_t *epoch_ptr,
+                                                      td_item *items, uint32_t *ready, const td_epoch *ep,
                                                       int capacity, td_inst_state *state, int grain,
                                                       int max_level, int check_every, uint64_t time_limit_ns,
                                                       ulonglong2 *tt, int tt_shift, unsigned epochs,
@@ -410,8 +456,9 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
     // subtree); an instance without a witness whose unit ran out reports
     // TD_ERR_BUDGET
     td_set_limits(s, max_exp, time_limit_ns);
-    const uint32_t epoch = *epoch_ptr;  // bumped by td_epoch_kernel before this launch
+    const uint32_t epoch = ep->epoch;  // bumped by td_epoch_kernel before this launch
     if (lane == 0) {
+        if (time_limit_ns) s.lim.deadline_ns = ep->start_ns + time_limit_ns;
         // this launch's numbers in the table: its `epochs` epochs, 2^26 searches each
         s.lim.tt_id = (uint64_t)(epoch - epochs + 1u) << TD_TT_INST_BITS;
         s.lim.tt_shift = tt_shift;
@@ -438,23 +485,6 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
         if (count < (int)(gridDim.x * (blockDim.x >> 5))) td_serve_idle_warps(s.dc);
     }
     __syncwarp();
-    // Claims.  A warp takes fresh instances by ticket while any are left, then
-    // one item ticket (fetch-and-add: it never fails) and waits for its item:
-    // item i belongs to ticket i.  A waiting warp polls only the ready flag of
-    // its own item, so thousands of them load thousands of different words and
-    // none that a busy warp needs, and they can poll often.  `outstanding`
-    // counts the root units in progress plus the items not yet finished: it is
-    // raised before an instance ticket is taken and by a donor before its items
-    // can be claimed, and lowered when a unit ends.  With no instance ticket
-    // left and nothing outstanding no unit can start again: the warp that
-    // brings the count there sets `done` and then ~epoch in the flag of every
-    // ticket taken.  A warp that took its ticket too late for that reads `done`
-    // at its first poll and at every 16th.
-    //
-    // Polling the shared counters instead (five of them, at up to 32 us
-    // intervals, since shorter ones slowed the busy warps) left the warps idle
-    // for most of a launch's tail.
-    //
     // Race (`race` = a, 0: off): a root search of a full-sorting instance
     // that starts its restart attempt a queues the instance's inverse
     // (td_spawn_inverse) as an item.  While fresh instances remain every warp
@@ -462,81 +492,23 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
     // work; at the end of the launch, where warps idle, it shortens the
     // longest searches.  Most queued inverses belong to instances decided by
     // then and end at once.
-    int my_ticket = -1;  // lane 0: this warp's item ticket, -1 = none
-    unsigned polls = 0;
-    bool fresh = true;   // lane 0: instance tickets may be left
-    // lane 0 lowers the outstanding count; whether the launch has no work left
-    auto release = [&]() -> bool {
-        if (atomicSub(&pool->outstanding, 1) != 1 || *(volatile int *)&pool->inst_ticket < count) return false;
-        atomicExch(&pool->done, 1);
-        __threadfence();
-        return true;
-    };
-    // wakes the waiting warps of a launch without work
-    auto wake = [&]() {
-        int from = 0, taken = 0;
-        if (lane == 0) {
-            from = *(volatile int *)&pool->produced;
-            taken = min(*(volatile int *)&pool->consumed, capacity);
-        }
-        from = __shfl_sync(TD_FULL, from, 0);
-        taken = __shfl_sync(TD_FULL, taken, 0);
-        for (int i = from + lane; i < taken; i += 32) *(volatile uint32_t *)&ready[i] = ~epoch;
-    };
-    unsigned backoff = 64;
+    td_claims cl;
+    cl.pool = pool;
+    cl.ready = ready;
+    cl.epoch = epoch;
+    cl.count = count;
+    cl.capacity = capacity;
+    cl.my_ticket = -1;
+    cl.fresh = true;
     for (;;) {
-        int kind = 0, unit = -1;
-        if (lane == 0) {
-            if (fresh) {
-                if (*(volatile int *)&pool->inst_ticket < count) {
-                    atomicAdd(&pool->outstanding, 1);
-                    unit = atomicAdd(&pool->inst_ticket, 1);
-                    if (unit < count) kind = 1;
-                    else if (release()) kind = 4;
-                }
-                fresh = kind == 1;
-            }
-            if (!kind) {
-                if (my_ticket < 0) {
-                    my_ticket = atomicAdd(&pool->consumed, 1);
-                    polls = 0;
-                    td_serve_idle_warps(s.dc);
-                }
-                const uint32_t flag = my_ticket < capacity ? *(volatile uint32_t *)&ready[my_ticket] : 0u;
-                if (flag == epoch) {
-                    kind = 2;
-                    unit = my_ticket;
-                    my_ticket = -1;
-                } else if (flag == ~epoch) {
-                    kind = 3;
-                } else if ((polls++ & 15u) == 0) {
-                    // tickets taken after the launch ended, or past the item
-                    // space, are not woken
-                    if (*(volatile int *)&pool->done) {
-                        kind = 3;
-                    } else if (s.lim.deadline_ns && td_globaltimer() > s.lim.deadline_ns) {
-                        atomicCAS(&pool->error, 0, TD_ERR_TIMEOUT);
-                        kind = 3;
-                    }
-                }
-            }
-        }
-        kind = __shfl_sync(TD_FULL, kind, 0);
-        if (kind == 4) wake();
-        if (kind >= 3) break;
-        if (!kind) {
-            __nanosleep(backoff);
-            backoff = min(backoff * 2u, 1024u);
-            continue;
-        }
-        unit = __shfl_sync(TD_FULL, unit, 0);
-        backoff = 64;
+        int unit;
+        const int kind = cl.next(s, &unit);
+        if (!kind) return;
         // the unit: a fresh instance, a donated subtree or a queued inverse root
         uint32_t idx = (uint32_t)unit;
         int d0 = 0, side = 0, attempt = 0;
         td_item it;
         if (kind == 2) {
-            td_fence();
             const uint4 *src = reinterpret_cast<const uint4 *>(&items[unit]);
             uint4 *dst = reinterpret_cast<uint4 *>(&it);
             dst[0] = __ldcg(src);  // read through L2: the donor wrote it from another SM
@@ -559,7 +531,12 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                 int stop = 0;
                 if (lane == 0) {
                     if (kind == 1) atomicAdd(&st->pending, 1);
-                    else stop = *(volatile int *)&st->found;
+                    else {
+                        // a search looks at the deadline every 256 expansions,
+                        // more than most donated subtrees have
+                        stop = *(volatile int *)&st->found;
+                        if (!stop && s.lim.deadline_ns && td_globaltimer() > s.lim.deadline_ns) stop = 2;
+                    }
                     // a donated subtree is searched once, to the end: restarting
                     // it would only repeat work when it holds no witness; the
                     // root of an inverse instance restarts like any root search
@@ -591,7 +568,7 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                     stop = 0;
                 }
                 td_dfs_out r;
-                r.status = TD_DFS_ABORTED;
+                r.status = stop == 2 ? TD_DFS_TIMEOUT : TD_DFS_ABORTED;
                 r.depth = 0;
                 r.found_move = 0;
                 r.expansions = 0;
@@ -608,22 +585,20 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                 td_finish_unit<false>(r, us, &out[s.dc.inst], s.path, s.dc.side);
             }
         }
-        int last = 0;
-        if (lane == 0) last = release();
-        if (__shfl_sync(TD_FULL, last, 0)) {
-            wake();
-            break;
-        }
+        if (cl.finish()) return;
     }
 }
 
+// The first operation of a launch: its deadline counts from here, so that it
+// holds for the growth of the launch's buffers too.
 // Advances the launch epoch that tags donated items as written; a launch
 // replayed from a CUDA graph therefore never mistakes an item of an earlier
 // launch for one of its own.  A launch of more than 2^26 instances takes as
 // many epochs as it needs numbers in the table of explored states.
-__global__ void td_epoch_kernel(uint32_t *epoch, unsigned epochs) {
-    const uint32_t e = *epoch + epochs;
-    *epoch = e >= epochs ? e : epochs;
+__global__ void td_epoch_kernel(td_epoch *ep, unsigned epochs) {
+    const uint32_t e = ep->epoch + epochs;
+    ep->epoch = e >= epochs ? e : epochs;
+    ep->start_ns = td_globaltimer();
 }
 
 // Runs after td_steal_kernel on the same stream.  When a bounded wait of the
@@ -820,17 +795,14 @@ struct Slot {
     int tt_log2 = 0, tt_bits = 0;  // log2 of its entries; the setting it was sized for
     td_inst_state *d_state = nullptr;
     size_t state_count = 0;
-    uint32_t *d_epoch = nullptr;
-    // split pass of the reference order: the listed instances, the pass's
-    // counters, each root's children, the subtree results and the cutoffs
-    int *d_hard = nullptr;
-    size_t hard_cap = 0;
-    td_split_ctl *d_split = nullptr;
-    uint16_t *d_kids = nullptr;
-    int *d_base = nullptr;
-    int *d_nkids = nullptr;
-    int *d_cutoff = nullptr;
-    td_result *d_split_items = nullptr;
+    td_epoch *d_epoch = nullptr;
+    // reference order: the queue's counters, items and flags, the nodes of split
+    // walks and the results of their subtrees
+    td_pool *d_split_pool = nullptr;  // followed by the node and record counts and the launch epoch
+    uint32_t *d_split_ready = nullptr;
+    td_split_node *d_nodes = nullptr;
+    td_split_item *d_split_items = nullptr;
+    td_result *d_split_records = nullptr;
     int split_records = 0;
     // td_batch_stats of host-buffer batches: device totals and their pinned copy
     td_counts *d_counts = nullptr;
@@ -889,6 +861,13 @@ std::string cuda_msg(cudaError_t e, const char *file, int line) {
             return TD_CUDA_ERROR;                                        \
         }                                                                \
     } while (0)
+
+constexpr size_t TD_SPLIT_HEAD = 256;  // a td_pool, the node and record counts and the epoch
+static_assert(sizeof(td_pool) % 8 == 0 && sizeof(td_pool) + 2 * sizeof(int) + sizeof(td_epoch) <= TD_SPLIT_HEAD, "split head");
+
+// Nodes of split walks for `records` subtrees (a split node has more than one
+// child nearly always; a walk that finds no node runs whole).
+size_t split_nodes(int records) { return (size_t)std::max(1, records / 2); }
 
 // log2 of the entries of a table of explored states for `warps` resident warps.
 int tt_entries_log2(size_t warps, int bits) {
@@ -957,7 +936,7 @@ int launch_cfg(int device, LaunchCfg *c, char *err, size_t errlen) {
     }
     if (d.blocks_per_sm == 0) {
         int b = 0;
-        TD_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, td_persistent_kernel<false>, threads,
+        TD_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, td_ordered_kernel, threads,
                                                                smem_bytes(c->warps)));
         d.blocks_per_sm = std::max(1, b);
     }
@@ -1029,11 +1008,9 @@ int ensure_device(int device, char *err, size_t errlen) {
     const size_t max_smem = smem_bytes(max_warps);
     TD_CHECK(cudaFuncSetAttribute(td_plain_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
     TD_CHECK(cudaFuncSetAttribute(td_plain_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
-    TD_CHECK(cudaFuncSetAttribute(td_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
-    TD_CHECK(cudaFuncSetAttribute(td_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
+    TD_CHECK(cudaFuncSetAttribute(td_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
     TD_CHECK(cudaFuncSetAttribute(td_steal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
-    TD_CHECK(cudaFuncSetAttribute(td_split_roots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
-    TD_CHECK(cudaFuncSetAttribute(td_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
+    TD_CHECK(cudaFuncSetAttribute(td_ordered_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
     const int rc = preload_kernels(err, errlen);
     if (rc != TD_OK) return rc;
     TD_CHECK(endgame_setup(device, d.sms));
@@ -1054,12 +1031,10 @@ void release_slot(Slot &s) {
     if (s.d_tt) cudaFree(s.d_tt);
     if (s.d_epoch) cudaFree(s.d_epoch);
     if (s.d_state) cudaFree(s.d_state);
-    if (s.d_hard) cudaFree(s.d_hard);
-    if (s.d_split) cudaFree(s.d_split);
-    if (s.d_kids) cudaFree(s.d_kids);
-    if (s.d_base) cudaFree(s.d_base);
-    if (s.d_nkids) cudaFree(s.d_nkids);
-    if (s.d_cutoff) cudaFree(s.d_cutoff);
+    if (s.d_split_pool) cudaFree(s.d_split_pool);
+    if (s.d_split_ready) cudaFree(s.d_split_ready);
+    if (s.d_nodes) cudaFree(s.d_nodes);
+    if (s.d_split_records) cudaFree(s.d_split_records);
     if (s.d_split_items) cudaFree(s.d_split_items);
     if (s.d_counts) cudaFree(s.d_counts);
     if (s.h_stats) cudaFreeHost(s.h_stats);
@@ -1101,6 +1076,12 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
         if (ordered) td_plain_kernel<true><<<blocks, threads, smem, stream>>>(d_in, d_out, count, max_exp, time_limit_ns());
         else td_plain_kernel<false><<<blocks, threads, smem, stream>>>(d_in, d_out, count, max_exp, time_limit_ns());
     } else if (!ordered) {
+        const unsigned epochs = ((unsigned)(count - 1) >> TD_TT_INST_BITS) + 1u;
+        if (s.d_epoch == nullptr) {
+            TD_CHECK(cudaMalloc(&s.d_epoch, sizeof(td_epoch)));
+            TD_CHECK(cudaMemsetAsync(s.d_epoch, 0, sizeof(td_epoch), stream));
+        }
+        td_epoch_kernel<<<1, 1, 0, stream>>>(s.d_epoch, epochs);
         // item space: the slot budget (the reference's queue budget) less the
         // per-instance state, at 36 bytes per item (record + ready flag)
         if (s.d_pool == nullptr) {
@@ -1109,8 +1090,6 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
             TD_CHECK(cudaMalloc(&s.d_items, cap * sizeof(td_item)));
             TD_CHECK(cudaMalloc(&s.d_ready, cap * sizeof(uint32_t)));
             TD_CHECK(cudaMemsetAsync(s.d_ready, 0, cap * sizeof(uint32_t), stream));
-            TD_CHECK(cudaMalloc(&s.d_epoch, sizeof(uint32_t)));
-            TD_CHECK(cudaMemsetAsync(s.d_epoch, 0, sizeof(uint32_t), stream));
             s.item_capacity = (int)cap;
         }
         // buffers grow in stream order: a cudaFree would wait for all work on
@@ -1139,10 +1118,8 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
             s.tt_log2 = tt_log2;
             s.tt_bits = cfg.tt_bits;
         }
-        const unsigned epochs = ((unsigned)(count - 1) >> TD_TT_INST_BITS) + 1u;
         TD_CHECK(cudaMemsetAsync(s.d_pool, 0, sizeof(td_pool), stream));
         TD_CHECK(cudaMemsetAsync(s.d_state, 0, (size_t)count * sizeof(td_inst_state), stream));
-        td_epoch_kernel<<<1, 1, 0, stream>>>(s.d_epoch, epochs);
         // the race needs restarts, and an expansion budget per unit would make
         // one side's budget decide the other's; each instance queues its
         // inverse at most once, and at least half the item space is left for
@@ -1158,49 +1135,51 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
     } else {
         const int grid_max = cfg.sms * cfg.blocks_per_sm;
         const int grid = std::max(1, std::min(grid_max, (count + warps - 1) / warps));
-        TD_CHECK(cudaMemsetAsync(s.d_ticket, 0, sizeof(int), stream));
         if (ordered && max_exp == 0 && cfg.split_budget > 0) {
-            // one warp per instance within split_budget expansions, then the
-            // split pass for the instances left (stream-ordered buffers)
-            if (s.d_split == nullptr) TD_CHECK(cudaMallocAsync(&s.d_split, sizeof(td_split_ctl), stream));
+            // stream-ordered buffers; the flags start at zero, epochs at 1
+            if (s.d_split_pool == nullptr) {
+                TD_CHECK(cudaMallocAsync(&s.d_split_pool, TD_SPLIT_HEAD, stream));
+                TD_CHECK(cudaMemsetAsync(s.d_split_pool, 0, TD_SPLIT_HEAD, stream));
+            }
+            int *node_count = reinterpret_cast<int *>(s.d_split_pool + 1);
+            td_epoch *epoch = reinterpret_cast<td_epoch *>(node_count + 2);
+            td_epoch_kernel<<<1, 1, 0, stream>>>(epoch, 1u);
             if (cfg.split_records > s.split_records) {
-                if (s.d_kids) TD_CHECK(cudaFreeAsync(s.d_kids, stream));
+                if (s.d_split_ready) TD_CHECK(cudaFreeAsync(s.d_split_ready, stream));
+                if (s.d_nodes) TD_CHECK(cudaFreeAsync(s.d_nodes, stream));
                 if (s.d_split_items) TD_CHECK(cudaFreeAsync(s.d_split_items, stream));
-                s.d_kids = nullptr;
+                if (s.d_split_records) TD_CHECK(cudaFreeAsync(s.d_split_records, stream));
+                s.d_split_ready = nullptr;
+                s.d_nodes = nullptr;
                 s.d_split_items = nullptr;
+                s.d_split_records = nullptr;
                 s.split_records = 0;
-                TD_CHECK(cudaMallocAsync(&s.d_kids, sizeof(uint16_t) * (size_t)cfg.split_records, stream));
-                TD_CHECK(cudaMallocAsync(&s.d_split_items, sizeof(td_result) * (size_t)cfg.split_records, stream));
+                const size_t n = (size_t)cfg.split_records;
+                TD_CHECK(cudaMallocAsync(&s.d_split_ready, sizeof(uint32_t) * n, stream));
+                TD_CHECK(cudaMallocAsync(&s.d_nodes, sizeof(td_split_node) * split_nodes(cfg.split_records), stream));
+                TD_CHECK(cudaMallocAsync(&s.d_split_items, sizeof(td_split_item) * n, stream));
+                TD_CHECK(cudaMallocAsync(&s.d_split_records, sizeof(td_result) * n, stream));
+                TD_CHECK(cudaMemsetAsync(s.d_split_ready, 0, sizeof(uint32_t) * n, stream));
                 s.split_records = cfg.split_records;
             }
-            if ((size_t)count > s.hard_cap) {
-                for (int *p : {s.d_hard, s.d_base, s.d_nkids, s.d_cutoff})
-                    if (p) TD_CHECK(cudaFreeAsync(p, stream));
-                s.d_hard = s.d_base = s.d_nkids = s.d_cutoff = nullptr;
-                s.hard_cap = 0;
-                TD_CHECK(cudaMallocAsync(&s.d_hard, sizeof(int) * (size_t)count, stream));
-                TD_CHECK(cudaMallocAsync(&s.d_base, sizeof(int) * (size_t)count, stream));
-                TD_CHECK(cudaMallocAsync(&s.d_nkids, sizeof(int) * (size_t)count, stream));
-                TD_CHECK(cudaMallocAsync(&s.d_cutoff, sizeof(int) * (size_t)count, stream));
-                s.hard_cap = (size_t)count;
-            }
-            TD_CHECK(cudaMemsetAsync(s.d_split, 0, sizeof(td_split_ctl), stream));
-            td_persistent_kernel<true><<<grid, threads, smem, stream>>>(d_in, d_out, count, s.d_ticket, cfg.grain,
-                                                                        (uint64_t)cfg.split_budget, time_limit_ns(),
-                                                                        &s.d_split->hard, s.d_hard);
-            td_split_roots_kernel<<<grid_max, threads, smem, stream>>>(d_in, s.d_hard, s.d_split, s.d_kids, s.d_base,
-                                                                       s.d_nkids, s.d_cutoff, cfg.split_records);
-            td_split_kernel<<<grid_max, threads, smem, stream>>>(d_in, d_out, s.d_hard, s.d_split, s.d_kids, s.d_base,
-                                                                 s.d_nkids, s.d_cutoff, s.d_split_items,
-                                                                 time_limit_ns());
-            td_split_join_kernel<<<std::max(1, std::min((count + 255) / 256, 2 * cfg.sms)), 256, 0, stream>>>(
-                s.d_hard, s.d_split, s.d_base, s.d_nkids, s.d_split_items, d_out);
-        } else if (ordered)
-            td_persistent_kernel<true><<<grid, threads, smem, stream>>>(d_in, d_out, count, s.d_ticket, cfg.grain,
+            // the counters start at zero in every launch
+            TD_CHECK(cudaMemsetAsync(s.d_split_pool, 0, sizeof(td_pool) + 2 * sizeof(int), stream));
+            td_split_space sp;
+            sp.nodes = s.d_nodes;
+            sp.node_count = node_count;
+            sp.record_count = node_count + 1;
+            sp.max_nodes = (int)split_nodes(cfg.split_records);
+            sp.items = s.d_split_items;
+            sp.records = s.d_split_records;
+            sp.out = d_out;
+            td_ordered_kernel<<<grid_max, threads, smem, stream>>>(d_in, d_out, count, s.d_split_pool, sp,
+                                                                  s.d_split_ready, epoch, cfg.split_records,
+                                                                  cfg.split_budget, time_limit_ns());
+        } else {
+            TD_CHECK(cudaMemsetAsync(s.d_ticket, 0, sizeof(int), stream));
+            td_persistent_kernel<<<grid, threads, smem, stream>>>(d_in, d_out, count, s.d_ticket, cfg.grain,
                                                                         max_exp, time_limit_ns());
-        else
-            td_persistent_kernel<false><<<grid, threads, smem, stream>>>(d_in, d_out, count, s.d_ticket, cfg.grain,
-                                                                         max_exp, time_limit_ns());
+        }
     }
     TD_CHECK(cudaGetLastError());
     if (flags & TD_FLAG_VERIFY) {
@@ -1894,7 +1873,7 @@ TD_API int td_int_issue_peak(int device, float target_ms, double *issue_per_s, d
 #define TD_NOALLOC_READY_OFF (TD_NOALLOC_ITEMS_OFF + TD_NOALLOC_ITEMS * 32)
 #define TD_NOALLOC_BYTES (TD_NOALLOC_READY_OFF + TD_NOALLOC_ITEMS * 4)   // 3.25 MiB + 256 B
 
-static_assert(sizeof(td_pool) + 2 * sizeof(uint32_t) <= TD_NOALLOC_HEAD, "scratch head");
+static_assert(sizeof(td_pool) + sizeof(td_epoch) + sizeof(int) <= TD_NOALLOC_HEAD, "scratch head");
 static_assert(sizeof(td_inst_state) == 16 && sizeof(td_item) == 32, "scratch records");
 
 static __device__ __align__(256) uint8_t td_noalloc_scratch[TD_NOALLOC_BYTES];
@@ -1956,11 +1935,11 @@ int noalloc_setup(int device, char *err, size_t errlen) {
     const int limit = (int)smem_bytes(8);
     TD_CHECK_NA(cudaFuncSetAttribute(td_plain_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
     TD_CHECK_NA(cudaFuncSetAttribute(td_plain_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
-    TD_CHECK_NA(cudaFuncSetAttribute(td_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+    TD_CHECK_NA(cudaFuncSetAttribute(td_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
     TD_CHECK_NA(cudaFuncSetAttribute(td_steal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
     TD_CHECK_NA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.steal_blocks, td_steal_kernel, 128,
                                                               smem_bytes(4)));
-    TD_CHECK_NA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.persistent_blocks, td_persistent_kernel<true>,
+    TD_CHECK_NA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.persistent_blocks, td_persistent_kernel,
                                                               128, smem));
     TD_CHECK_NA(endgame_setup(device, d.sms));
     d.scratch = static_cast<uint8_t *>(ptr);
@@ -2001,8 +1980,8 @@ TD_API int td_search_batch_noalloc(int count, const td_instance *d_instances, td
     const bool ordered = flags & TD_FLAG_ORDERED;
     const uint64_t limit = time_limit_ns();
     td_pool *pool = reinterpret_cast<td_pool *>(d.scratch);
-    uint32_t *epoch = reinterpret_cast<uint32_t *>(d.scratch + sizeof(td_pool));
-    int *ticket = reinterpret_cast<int *>(d.scratch + sizeof(td_pool) + sizeof(uint32_t));
+    td_epoch *epoch = reinterpret_cast<td_epoch *>(d.scratch + sizeof(td_pool));
+    int *ticket = reinterpret_cast<int *>(d.scratch + sizeof(td_pool) + sizeof(td_epoch));
     td_inst_state *state = reinterpret_cast<td_inst_state *>(d.scratch + TD_NOALLOC_STATE_OFF);
     td_item *items = reinterpret_cast<td_item *>(d.scratch + TD_NOALLOC_ITEMS_OFF);
     uint32_t *ready = reinterpret_cast<uint32_t *>(d.scratch + TD_NOALLOC_READY_OFF);
@@ -2015,7 +1994,7 @@ TD_API int td_search_batch_noalloc(int count, const td_instance *d_instances, td
     } else if (ordered) {
         TD_CHECK_NA(cudaMemsetAsync(ticket, 0, sizeof(int), st));
         const int grid = std::max(1, std::min(d.sms * std::max(1, d.persistent_blocks), blocks_needed));
-        td_persistent_kernel<true><<<grid, threads, smem, st>>>(d_instances, d_results, count, ticket, 1, max_exp,
+        td_persistent_kernel<<<grid, threads, smem, st>>>(d_instances, d_results, count, ticket, 1, max_exp,
                                                                 limit);
     } else {
         // the donation settings, read together (a concurrent td_configure_steal
@@ -2139,12 +2118,9 @@ int preload_kernels(char *err, size_t errlen) {
     cudaFuncAttributes a;
     TD_CHECK(cudaFuncGetAttributes(&a, td_plain_kernel<true>));
     TD_CHECK(cudaFuncGetAttributes(&a, td_plain_kernel<false>));
-    TD_CHECK(cudaFuncGetAttributes(&a, td_persistent_kernel<true>));
-    TD_CHECK(cudaFuncGetAttributes(&a, td_persistent_kernel<false>));
+    TD_CHECK(cudaFuncGetAttributes(&a, td_persistent_kernel));
     TD_CHECK(cudaFuncGetAttributes(&a, td_steal_kernel));
-    TD_CHECK(cudaFuncGetAttributes(&a, td_split_roots_kernel));
-    TD_CHECK(cudaFuncGetAttributes(&a, td_split_kernel));
-    TD_CHECK(cudaFuncGetAttributes(&a, td_split_join_kernel));
+    TD_CHECK(cudaFuncGetAttributes(&a, td_ordered_kernel));
     TD_CHECK(cudaFuncGetAttributes(&a, td_epoch_kernel));
     TD_CHECK(cudaFuncGetAttributes(&a, td_eg_build_kernel));
     TD_CHECK(cudaFuncGetAttributes(&a, td_finalize_kernel));

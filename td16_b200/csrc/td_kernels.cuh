@@ -28,15 +28,17 @@
 // Limits and tables of the search a warp runs.
 struct td_search_limits {
     uint32_t max_expansions;   // per search; TD_ERR_BUDGET when exceeded (~0: none)
-    uint32_t max_work;         // the same for nodes expanded here (the reference order's count also
-                               // holds those the endgame table accounts for)
+    uint32_t split_after;      // a walk of the reference order may be split after this many nodes
     uint64_t deadline_ns;      // %globaltimer value; 0 = none
     ulonglong2 *tt;            // the launch's table of explored states (free order); null = none
     uint64_t tt_id;            // number of the launch's first search in it
     int tt_shift;              // 64 - log2 of its entries
     uint32_t restart_base;     // free order: base of the restart budgets (td_attempt_budget); 0 = none
-    const int *cutoff;         // a split ordered search: lowest rank with a witness so far; null = none
-    int rank;                  // that search's own rank (it stops once *cutoff < rank)
+    // a subtree of a split ordered search: it stops once *cutoff < rank, or
+    // *cutoff2 < rank2 (the lowest rank with a witness so far, at its node and at
+    // that node's); null = none
+    const int *cutoff, *cutoff2;
+    int rank, rank2;
 };
 
 // ---- work items (subtree roots handed between warps) ----------------------
@@ -108,6 +110,19 @@ struct td_donate_ctx {
                             // `race` (root units of full-sorting instances in td_steal_kernel)
 };
 
+// The buffers of a launch of the reference order whose walks may be split
+// (td_ordered.cuh).
+struct td_split_node;
+struct td_split_item;
+struct td_split_space {
+    td_split_node *nodes;
+    int *node_count, *record_count;
+    int max_nodes;
+    td_split_item *items;  // by item ticket
+    td_result *records;    // by node base + rank
+    td_result *out;        // by instance
+};
+
 // Per-warp shared state.
 struct td_warp_smem {
     // per caller position c: the row masks S, G, P and H (positions after c),
@@ -124,6 +139,11 @@ struct td_warp_smem {
             uint32_t cw[TD_MAX_DEPTH][TD_MAX_STEPS];
             uint32_t root_found[TD_MAX_STEPS];  // the root's children accepted when visited
             uint32_t cp[TD_MAX_DEPTH][TD_MAX_STEPS];  // the +2 ones, at nodes that also have 0 children
+            // a node being split: its children in visiting order (bit 15:
+            // accepted when visited), and what the endgame table says of each
+            uint16_t kid[TD_MAX_TRIPLES], kid_e[TD_MAX_TRIPLES];
+            td_split_space sp;
+            int sp_inst, sp_node, sp_rank;  // where the walk's result goes (node -1: to the instance's)
         };
         struct {  // free move order
             // per level and lane: the expandable children of the lane's four
@@ -964,10 +984,12 @@ __device__ __forceinline__ bool td_tt_visit(const td_warp_smem &s, int lv, int N
     return __shfl_sync(TD_FULL, hit, 0) != 0;
 }
 
+#include "td_ordered.cuh"
+
 // Depth-first search from the node held at level d0 of `s` (state, path, rate
 // masks, pair slots and limits already set).  Leaves
 // the frames intact on TD_DFS_BUDGET.  `shared`: a unit of a search that other
-// warps may take part in (free order; s.dc says how).
+// warps may take part in (s.dc says how; in the reference order also s.sp).
 //
 // The node is expanded at one place of the loop, and what runs rarely is not
 // inlined: the loop has to fit the instruction caches.  With three copies of
@@ -988,7 +1010,7 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
     td_unpack_state(s, d0, s.L[d0], s.off[d0], N);
     uint32_t work = 0;  // nodes expanded here
     int since_check = 0;
-    bool due = false;            // free order: the scheduler's counters were read (lane 0)
+    bool due = false;            // the scheduler's counters were read (lane 0)
     int waiting = 0, ended = 0;  // idle warps not yet served by an item; the instance is decided
     int attempt = 0;     // free order: restarts with another child order (td_attempt_budget)
     uint32_t ord = 0, attempt_exp = 0;
@@ -1037,7 +1059,7 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
                 }
             }
         }
-        if (r.expansions >= s.lim.max_expansions || work >= s.lim.max_work) {
+        if (r.expansions >= s.lim.max_expansions) {
             r.status = TD_DFS_BUDGET;
             break;
         }
@@ -1076,12 +1098,19 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
                     attempt_budget = ~0u;
             }
         }
+        if constexpr (ORDERED) {
+            if (due) {
+                due = false;
+                if (__shfl_sync(TD_FULL, waiting, 0) > 0) r.expansions += td_split(s, d0, level, N);
+            }
+        }
         if ((work & 255u) == 0) {
             int stop = 0;
             if (lane == 0) {
                 if (s.lim.deadline_ns && td_globaltimer() > s.lim.deadline_ns) stop = 1;
                 // a subtree of a split ordered search: one of lower rank has a witness
                 if (s.lim.cutoff && *(volatile const int *)s.lim.cutoff < s.lim.rank) stop = 2;
+                if (s.lim.cutoff2 && *(volatile const int *)s.lim.cutoff2 < s.lim.rank2) stop = 2;
             }
             stop = __shfl_sync(TD_FULL, stop, 0);
             if (stop) {
@@ -1155,7 +1184,16 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
             }
             break;
         }
-        if constexpr (!ORDERED) {
+        if constexpr (ORDERED) {
+            if (shared && work >= s.lim.split_after && ++since_check >= s.dc.check_every) {
+                since_check = 0;
+                due = true;
+                if (lane == 0) {
+                    const unsigned long long pc = *(volatile unsigned long long *)&s.dc.pool->produced;
+                    waiting = (int)(pc >> 32) - (int)(uint32_t)pc;
+                }
+            }
+        } else {
             // a raced unit looks for the other side's verdict at least every
             // 16 expansions
             if (shared && ++since_check >= (raced ? min(s.dc.check_every, 16) : s.dc.check_every)) {

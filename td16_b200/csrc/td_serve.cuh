@@ -148,14 +148,14 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
     if (lane == 0) {
         td_search_limits lim;
         lim.max_expansions = max_exp && max_exp < ~0u ? (uint32_t)max_exp : ~0u;
-        lim.max_work = ~0u;
+        lim.split_after = ~0u;
         lim.deadline_ns = deadline;
         lim.tt = ALL_ORDERED ? nullptr : tt;
         lim.tt_id = 0;  // requests are numbered across the launches that share a table
         lim.tt_shift = tt_shift;
         lim.restart_base = 0;
-        lim.cutoff = nullptr;
-        lim.rank = 0;
+        lim.cutoff = lim.cutoff2 = nullptr;
+        lim.rank = lim.rank2 = 0;
         s.lim = lim;
         s.pairs_n = -1;
         td_donate_ctx dc;
