@@ -145,8 +145,8 @@ int td_set_time_limit(double seconds);
  * up to 4 levels deeper. */
 int td_configure_steal(int grain, int split_level, int check_every);
 /* The same for later serving launches (td_serve_open), kept apart because a
- * serving launch trades throughput for latency (default 1, 2, 32; a serving
- * launch mostly has idle warps, so it gives 4 times as many items, from up to
+ * serving launch trades throughput for latency (default 1, 2, 32; a request
+ * whose bound is its cycle-graph lower bound gives 4 times as many items, from
  * 2 levels deeper, and checks 4 times as often). */
 int td_configure_serve(int grain, int split_level, int check_every);
 /* Free order only: the warps of a launch share a table of the states they took

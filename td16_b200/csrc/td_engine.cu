@@ -479,6 +479,8 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
         dc.side = 0;
         dc.attempt = 0;
         dc.race = 0;
+        dc.step = 3;
+        dc.idle_after = 0;
         dc.idle_seen = 0;
         s.dc = dc;
         // a launch with fewer instances than warps has idle warps from the start

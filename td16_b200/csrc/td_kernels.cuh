@@ -98,7 +98,9 @@ struct td_donate_ctx {
     uint32_t *ready;
     uint32_t epoch;
     int capacity;
-    int idle_seen;          // the three settings are those for a launch with idle warps
+    int step;               // td_serve_idle_warps: 3 in the batch engine, 2 in the serving loop
+    int idle_after;         // a unit calls it at the first idle warps after this many expansions
+    int idle_seen;          // it was called for the three settings below
     int grain;              // at most this many items per donation
     int max_level;          // donate only children of levels <= max_level
     int check_every;        // expansions between idle checks
@@ -173,20 +175,22 @@ struct td_warp_smem {
     td_donate_ctx dc;
 };
 
-// What a warp's donation settings become once it has met idle warps: it looks
-// for them 16 times as often, gives them 8 times as many items at once and
-// from 4 levels deeper.  An item per lane and counters read behind an expansion
-// make a donation cheap, and the end of a launch is all latency: with the
-// settings that suit the time before (4 items, level 2, every 64 expansions)
-// 2,048 S_16 at their lower bound took 20 ms, with these 2.8 ms; the n = 11..13
-// mix 10.3 and 1.6 ms, 250 requests of n = 8..16 2.8 and 0.23 ms.  Called by
-// one lane.
+// What a warp's donation settings become once it has met idle warps, in the
+// batch engine (step 3): it looks for them 16 times as often, gives them 8
+// times as many items at once and from 4 levels deeper.  An item per lane and
+// counters read behind an expansion make a donation cheap, and the end of a
+// launch is all latency: with the settings that suit the time before (4 items,
+// level 2, every 64 expansions) 2,048 S_16 at their lower bound took 20 ms,
+// with these 2.8 ms; the n = 11..13 mix 10.3 and 1.6 ms, 250 requests of n =
+// 8..16 2.8 and 0.23 ms.  The serving loop's warps claim by compare-and-swap,
+// so there it is 4 times as often and as many, from 2 levels deeper (step 2).
+// Called by one lane.
 __device__ __forceinline__ void td_serve_idle_warps(td_donate_ctx &dc) {
     if (dc.idle_seen) return;
     dc.idle_seen = 1;
-    dc.grain = min(32, 8 * dc.grain);
-    dc.max_level = min(TD_MAX_DEPTH - 1, dc.max_level + 4);
-    dc.check_every = max(1, dc.check_every / 16);
+    dc.grain = min(32, dc.grain << dc.step);
+    dc.max_level = min(TD_MAX_DEPTH - 1, dc.max_level + 2 * (dc.step - 1));
+    dc.check_every = max(1, dc.check_every >> (2 * (dc.step - 1)));
 }
 
 // Lexicographic position triples i|j<<5|k<<10 for every N, at offset C(N,4).
@@ -1085,7 +1089,7 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
                     r.status = TD_DFS_ABORTED;
                     break;
                 }
-                if (hungry > 0 && !s.dc.idle_seen) {
+                if (hungry > 0 && !s.dc.idle_seen && work >= s.dc.idle_after) {
                     __syncwarp();
                     if (lane == 0) td_serve_idle_warps(s.dc);
                     __syncwarp();

@@ -57,6 +57,14 @@ __device__ __forceinline__ void td_serve_record(td_serve_dev_ctl *dctl, const td
 #define TD_SERVE_BACKOFF_CAP 2048u
 #endif
 
+// The dispatcher and the warps of the first blocks poll more often: a lone
+// request then waits less for its warp (33.6 -> 31.2 us per td_search_ordered
+// call of n = 5..9 from Python), and all warps polling so often would crowd the
+// counters.
+#define TD_SERVE_FIRST_CAP 256u
+#define TD_SERVE_FIRST_BLOCKS 8
+#define TD_SERVE_IDLE_AFTER 128  // expansions of a unit before it serves idle warps so in any case
+
 // Move order of a serving launch: every request in the free order, every
 // request in the reference order, or per request (TD_PACKED_ORDERED in the
 // request's packed byte; the per-call server of td_search and
@@ -140,7 +148,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 break;
             }
             __nanosleep(backoff);
-            backoff = min(backoff * 2u, (unsigned)TD_SERVE_BACKOFF_CAP);
+            backoff = min(backoff * 2u, TD_SERVE_FIRST_CAP);
         }
         return;
     }
@@ -167,23 +175,21 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
         dc.ready = ready;
         dc.epoch = 0;
         dc.capacity = item_capacity;
-        // a serving launch mostly has idle warps, but they claim items and
-        // requests by compare-and-swap, so it does not go as far as the batch
-        // engine's td_serve_idle_warps.  2,048 calls of n = 8..14 at the lower
-        // bound from 16 threads, with the default (1, 2, 32): as configured
-        // 11.2 ms, 4 x / + 2 / 1/4 7.8 ms, 8 x / + 4 / 1/16 24.8 ms
-        dc.grain = min(32, 4 * grain);
-        dc.max_level = min(TD_MAX_DEPTH - 1, max_level + 2);
-        dc.check_every = max(1, check_every / 4);
+        dc.step = 2;
+        dc.idle_after = TD_SERVE_IDLE_AFTER;
         dc.inst = 0;
         dc.state = nullptr;
         dc.side = 0;
         dc.attempt = 0;
         dc.race = 0;  // set per fresh request (the per-call server's race)
-        dc.idle_seen = 1;
+        dc.idle_seen = 0;  // with the settings, per unit
+        dc.grain = grain;
+        dc.max_level = max_level;
+        dc.check_every = check_every;
         s.dc = dc;
     }
     __syncwarp();
+    const unsigned cap = blockIdx.x < TD_SERVE_FIRST_BLOCKS ? TD_SERVE_FIRST_CAP : (unsigned)TD_SERVE_BACKOFF_CAP;
     bool idle = false;
     unsigned backoff = 128;
     for (;;) {
@@ -230,7 +236,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
             }
             if (__shfl_sync(TD_FULL, stop, 0)) break;
             __nanosleep(backoff);
-            backoff = min(backoff * 2u, (unsigned)TD_SERVE_BACKOFF_CAP);
+            backoff = min(backoff * 2u, cap);
             continue;
         }
         if (lane == 0 && idle) { atomicSub(&pool->idle, 1); idle = false; }
@@ -342,6 +348,17 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 // of the per-call server with full sorting races the search of its
                 // inverse from restart attempt `race` (td_steal_kernel's race).
                 s.lim.restart_base = kind == 1 || d0 == 0 ? restart_base : 0;
+                // A request with a spare move mostly ends with a witness soon, and
+                // restarts find it best: it gives subtrees away as configured.
+                // One without must search a narrow tree to its end: the idle
+                // warps take part at once (2,048 such calls of n = 8..14 from 16
+                // threads: 11.1 -> 7.8 ms; S_16 at bound 9 the same way would
+                // fall from 252,000 to 81,000 calls/s).
+                s.dc.idle_seen = 0;
+                s.dc.grain = grain;
+                s.dc.max_level = max_level;
+                s.dc.check_every = check_every > 0 ? check_every : 1;
+                if (td_inst_full(x) && 2 * x.max_moves <= x.n_symbols - td_inst_init(x)) td_serve_idle_warps(s.dc);
                 s.dc.inst = (uint32_t)req;
                 s.dc.state = &state[slot];
                 s.dc.side = side;
