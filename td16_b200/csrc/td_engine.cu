@@ -150,14 +150,6 @@ struct td_claims {
     int my_ticket;  // lane 0: this warp's item ticket, -1 = none
     bool fresh;     // lane 0: instance tickets may be left
 
-    // Lowers the outstanding count (lane 0); whether the launch has no work left.
-    __device__ __forceinline__ bool release() {
-        if (atomicSub(&pool->outstanding, 1) != 1 || *(volatile int *)&pool->inst_ticket < count) return false;
-        atomicExch(&pool->done, 1);
-        __threadfence();
-        return true;
-    }
-
     // Wakes the waiting warps of a launch without work.
     __device__ __forceinline__ void wake() {
         const int lane = threadIdx.x & 31;
@@ -171,31 +163,26 @@ struct td_claims {
         for (int i = from + lane; i < taken; i += 32) *(volatile uint32_t *)&ready[i] = ~epoch;
     }
 
-    // Ends a unit; whether the launch has no work left (uniform across the warp).
-    __device__ __forceinline__ bool finish() {
-        int last = 0;
-        if ((threadIdx.x & 31) == 0) last = release();
-        last = __shfl_sync(TD_FULL, last, 0);
-        if (last) wake();
-        return last != 0;
-    }
-
-    // The next unit: 1 an instance, 2 an item, 0 no work left (uniform across
-    // the warp).
-    __device__ __forceinline__ int next(td_warp_smem &s, int *unit_out) {
+    // Ends the unit before, if any, and claims the next one: 1 an instance, 2 an
+    // item, 0 no work left (uniform across the warp).
+    __device__ __forceinline__ int next(td_warp_smem &s, bool first, int *unit_out) {
         const int lane = threadIdx.x & 31;
         unsigned backoff = 64, polls = 0;
         for (;;) {
             int kind = 0, unit = -1;
             if (lane == 0) {
+                // both atomics are under way before either result is used
+                const int before = first ? 0 : atomicSub(&pool->outstanding, 1);
+                first = true;
                 if (fresh) {
-                    if (*(volatile int *)&pool->inst_ticket < count) {
-                        atomicAdd(&pool->outstanding, 1);
-                        unit = atomicAdd(&pool->inst_ticket, 1);
-                        if (unit < count) kind = 1;
-                        else if (release()) kind = 4;
-                    }
-                    fresh = kind == 1;
+                    unit = atomicAdd(&pool->inst_ticket, 1);
+                    if (unit < count) kind = 1;
+                    else fresh = false;
+                }
+                if (before == 1) {
+                    atomicExch(&pool->done, 1);
+                    __threadfence();
+                    kind = 4;
                 }
                 if (!kind) {
                     if (my_ticket < 0) {
@@ -265,9 +252,9 @@ __global__ void __launch_bounds__(256, 4) td_ordered_kernel(const td_instance *_
     cl.capacity = capacity;
     cl.my_ticket = -1;
     cl.fresh = true;
-    for (;;) {
+    for (bool first = true;; first = false) {
         int unit;
-        const int kind = cl.next(s, &unit);
+        const int kind = cl.next(s, first, &unit);
         if (!kind) return;
         int inst = unit, node = -1, rank = 0, d0 = 0, stop = 0;
         uint32_t kid = 0;
@@ -362,7 +349,6 @@ __global__ void __launch_bounds__(256, 4) td_ordered_kernel(const td_instance *_
             __syncwarp();
             td_split_complete(s.sp, node);
         }
-        if (cl.finish()) return;
     }
 }
 
@@ -384,6 +370,11 @@ __global__ void __launch_bounds__(256, 4) td_ordered_kernel(const td_instance *_
 // HOST_OUT: `out` is host memory mapped into the device (the serving loop), so
 // the fences are system-scope; the batch engine's results are device memory,
 // where device-scope fences order the same writes at a fraction of the cost.
+// Records the first error of a search.
+__device__ __forceinline__ void td_note_error(td_inst_state *st, int err) {
+    atomicCAS(reinterpret_cast<unsigned short *>(&st->error), (unsigned short)0, (unsigned short)err);
+}
+
 template <bool HOST_OUT>
 __device__ __forceinline__ void td_unit_fence() {
     if (HOST_OUT) __threadfence_system();
@@ -392,35 +383,45 @@ __device__ __forceinline__ void td_unit_fence() {
 
 template <bool HOST_OUT>
 __device__ __forceinline__ int td_finish_unit(const td_dfs_out &r, td_inst_state *st, td_result *out,
-                                              const uint16_t *path, int side = 0) {
+                                              const uint16_t *path, int side, int gave) {
     const int lane = threadIdx.x & 31;
+    if (!gave) {  // a root search by itself: its outcome is the instance's
+        const int status = r.status == TD_DFS_FOUND     ? TD_FOUND
+                           : r.status == TD_DFS_TIMEOUT ? TD_ERR_TIMEOUT
+                           : r.status == TD_DFS_BUDGET  ? TD_ERR_BUDGET
+                                                        : TD_NOT_FOUND;
+        td_write_result(out, status, status == TD_FOUND ? r.depth : 0, r.found_move, path, r.expansions, 0, 8);
+        __syncwarp();
+        if (HOST_OUT && lane == 0) __threadfence_system();
+        return 1;
+    }
     int win = 0, last = 0;
     if (lane == 0) {
         atomicAdd(&st->expansions, r.expansions);
-        if (r.status == TD_DFS_FOUND) win = atomicCAS(&st->found, 0, 1) == 0;
-        if (r.status == TD_DFS_TIMEOUT) atomicCAS(&st->error, 0, TD_ERR_TIMEOUT);
-        if (r.status == TD_DFS_BUDGET) atomicCAS(&st->error, 0, TD_ERR_BUDGET);
+        if (r.status == TD_DFS_FOUND) win = atomicCAS(&st->found, (unsigned short)0, (unsigned short)1) == 0;
+        const int err = r.status == TD_DFS_TIMEOUT ? TD_ERR_TIMEOUT : r.status == TD_DFS_BUDGET ? TD_ERR_BUDGET : 0;
+        if (err) td_note_error(st, err);
     }
     win = __shfl_sync(TD_FULL, win, 0);
     if (win) td_write_result(out, TD_FOUND, r.depth, r.found_move, path, 0, 0, 7);
     __syncwarp();
     if (lane == 0) {
         td_unit_fence<HOST_OUT>();
-        const int unit = side ? 1 << 16 : 1;
-        const int before = atomicSub(&st->pending, unit);
+        const unsigned long long unit = side ? TD_UNIT_INVERSE : 1ull;
+        const unsigned long long before = atomicAdd(&st->pending, 0ull - unit);
         last = before == unit;
         if (last) td_unit_fence<HOST_OUT>();
-        else if (!side && ((before - unit) & 0x0000ffff) == 0 && *(volatile int *)&st->found == 0 &&
-                 *(volatile int *)&st->error == 0)
-            atomicCAS(&st->found, 0, 2);
+        else if (!side && (uint32_t)before == 1u && *(volatile unsigned short *)&st->found == 0 &&
+                 *(volatile short *)&st->error == 0)
+            atomicCAS(&st->found, (unsigned short)0, (unsigned short)2);
     }
     last = __shfl_sync(TD_FULL, last, 0);
     if (last) {
         int found = 0, err = 0;
         unsigned exp = 0;
         if (lane == 0) {
-            found = *(volatile int *)&st->found;
-            err = *(volatile int *)&st->error;
+            found = *(volatile unsigned short *)&st->found;
+            err = *(volatile short *)&st->error;
             exp = *(volatile unsigned *)&st->expansions;
         }
         found = __shfl_sync(TD_FULL, found, 0);
@@ -478,6 +479,7 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
         dc.state = nullptr;
         dc.side = 0;
         dc.attempt = 0;
+        dc.gave = 0;
         dc.race = 0;
         dc.step = 3;
         dc.idle_after = 0;
@@ -502,9 +504,9 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
     cl.capacity = capacity;
     cl.my_ticket = -1;
     cl.fresh = true;
-    for (;;) {
+    for (bool first = true;; first = false) {
         int unit;
-        const int kind = cl.next(s, &unit);
+        const int kind = cl.next(s, first, &unit);
         if (!kind) return;
         // the unit: a fresh instance, a donated subtree or a queued inverse root
         uint32_t idx = (uint32_t)unit;
@@ -527,16 +529,17 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
         } else {
             const td_instance x = in[idx];
             td_inst_state *st = &state[idx];
+            // other warps see it only through items, published after a fence
+            if (kind == 1 && lane == 0) *reinterpret_cast<uint4 *>(st) = make_uint4(0u, 0u, 0u, 0u);
             if (kind == 1 && (!td_instance_ok(x) || td_triple_count(x.n_symbols) == 0)) {
                 td_write_result(&out[idx], td_instance_ok(x) ? TD_NOT_FOUND : TD_ERR_ARG, 0, 0, s.path, 0, 0, 8);
             } else {
                 int stop = 0;
                 if (lane == 0) {
-                    if (kind == 1) atomicAdd(&st->pending, 1);
-                    else {
+                    if (kind == 2) {
                         // a search looks at the deadline every 256 expansions,
                         // more than most donated subtrees have
-                        stop = *(volatile int *)&st->found;
+                        stop = *(volatile unsigned short *)&st->found != 0;
                         if (!stop && s.lim.deadline_ns && td_globaltimer() > s.lim.deadline_ns) stop = 2;
                     }
                     // a donated subtree is searched once, to the end: restarting
@@ -550,6 +553,7 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                     s.dc.state = st;
                     s.dc.side = side;
                     s.dc.attempt = attempt;
+                    s.dc.gave = kind == 2;
                     s.dc.race = kind == 1 && td_inst_full(x) ? race : 0;
                 }
                 td_setup_root(s, x);
@@ -582,25 +586,29 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
                     const int t = td_inverse_witness(s, in[s.dc.inst], r.depth, r.found_move);
                     if (t < 0) r.status = TD_DFS_EXHAUSTED;
                     else r.found_move = (uint16_t)t;
-                    if (t == -1 && lane == 0) atomicCAS(&us->error, 0, TD_ERR_VERIFY);
+                    if (t == -1 && lane == 0) td_note_error(us, TD_ERR_VERIFY);
                 }
-                td_finish_unit<false>(r, us, &out[s.dc.inst], s.path, s.dc.side);
+                td_finish_unit<false>(r, us, &out[s.dc.inst], s.path, s.dc.side, s.dc.gave);
             }
         }
-        if (cl.finish()) return;
     }
 }
 
-// The first operation of a launch: its deadline counts from here, so that it
-// holds for the growth of the launch's buffers too.
+// The first operation of a launch: sets its counters, and its deadline counts
+// from here, so that it holds for the growth of the launch's buffers too.
 // Advances the launch epoch that tags donated items as written; a launch
 // replayed from a CUDA graph therefore never mistakes an item of an earlier
 // launch for one of its own.  A launch of more than 2^26 instances takes as
 // many epochs as it needs numbers in the table of explored states.
-__global__ void td_epoch_kernel(td_epoch *ep, unsigned epochs) {
+__global__ void td_epoch_kernel(td_epoch *ep, unsigned epochs, td_pool *pool, int count, int *zeros, int n_zeros) {
     const uint32_t e = ep->epoch + epochs;
     ep->epoch = e >= epochs ? e : epochs;
     ep->start_ns = td_globaltimer();
+    td_pool p;
+    memset(&p, 0, sizeof p);
+    p.outstanding = count;
+    *pool = p;
+    for (int i = 0; i < n_zeros; ++i) zeros[i] = 0;
 }
 
 // Runs after td_steal_kernel on the same stream.  When a bounded wait of the
@@ -1080,14 +1088,14 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
     } else if (!ordered) {
         const unsigned epochs = ((unsigned)(count - 1) >> TD_TT_INST_BITS) + 1u;
         if (s.d_epoch == nullptr) {
+            TD_CHECK(cudaMalloc(&s.d_pool, sizeof(td_pool)));
             TD_CHECK(cudaMalloc(&s.d_epoch, sizeof(td_epoch)));
             TD_CHECK(cudaMemsetAsync(s.d_epoch, 0, sizeof(td_epoch), stream));
         }
-        td_epoch_kernel<<<1, 1, 0, stream>>>(s.d_epoch, epochs);
+        td_epoch_kernel<<<1, 1, 0, stream>>>(s.d_epoch, epochs, s.d_pool, count, nullptr, 0);
         // item space: the slot budget (the reference's queue budget) less the
         // per-instance state, at 36 bytes per item (record + ready flag)
-        if (s.d_pool == nullptr) {
-            TD_CHECK(cudaMalloc(&s.d_pool, sizeof(td_pool)));
+        if (s.d_items == nullptr) {
             const size_t cap = std::max<size_t>(1024, std::min<size_t>(s.budget / 36, 1u << 26));
             TD_CHECK(cudaMalloc(&s.d_items, cap * sizeof(td_item)));
             TD_CHECK(cudaMalloc(&s.d_ready, cap * sizeof(uint32_t)));
@@ -1120,8 +1128,6 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
             s.tt_log2 = tt_log2;
             s.tt_bits = cfg.tt_bits;
         }
-        TD_CHECK(cudaMemsetAsync(s.d_pool, 0, sizeof(td_pool), stream));
-        TD_CHECK(cudaMemsetAsync(s.d_state, 0, (size_t)count * sizeof(td_inst_state), stream));
         // the race needs restarts, and an expansion budget per unit would make
         // one side's budget decide the other's; each instance queues its
         // inverse at most once, and at least half the item space is left for
@@ -1145,7 +1151,8 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
             }
             int *node_count = reinterpret_cast<int *>(s.d_split_pool + 1);
             td_epoch *epoch = reinterpret_cast<td_epoch *>(node_count + 2);
-            td_epoch_kernel<<<1, 1, 0, stream>>>(epoch, 1u);
+            // the node and record counts start at zero in every launch
+            td_epoch_kernel<<<1, 1, 0, stream>>>(epoch, 1u, s.d_split_pool, count, node_count, 2);
             if (cfg.split_records > s.split_records) {
                 if (s.d_split_ready) TD_CHECK(cudaFreeAsync(s.d_split_ready, stream));
                 if (s.d_nodes) TD_CHECK(cudaFreeAsync(s.d_nodes, stream));
@@ -1164,8 +1171,6 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
                 TD_CHECK(cudaMemsetAsync(s.d_split_ready, 0, sizeof(uint32_t) * n, stream));
                 s.split_records = cfg.split_records;
             }
-            // the counters start at zero in every launch
-            TD_CHECK(cudaMemsetAsync(s.d_split_pool, 0, sizeof(td_pool) + 2 * sizeof(int), stream));
             td_split_space sp;
             sp.nodes = s.d_nodes;
             sp.node_count = node_count;
@@ -2010,11 +2015,9 @@ TD_API int td_search_batch_noalloc(int count, const td_instance *d_instances, td
             check_every = g_check_every;
             restart_base = g_restart_base;
         }
-        // counters and per-instance state start at zero on every call; items
+        // the counters start afresh on every call; items
         // are tagged with a fresh epoch so an earlier call's items never count
-        TD_CHECK_NA(cudaMemsetAsync(pool, 0, sizeof(td_pool), st));
-        TD_CHECK_NA(cudaMemsetAsync(state, 0, (size_t)count * sizeof(td_inst_state), st));
-        td_epoch_kernel<<<1, 1, 0, st>>>(epoch, 1u);
+        td_epoch_kernel<<<1, 1, 0, st>>>(epoch, 1u, pool, count, nullptr, 0);
         // the whole resident grid (the scratch does not depend on its size):
         // warps without an instance of their own take donated subtrees, so a
         // small batch is spread over the GPU

@@ -54,16 +54,18 @@ struct __align__(16) td_item {  // 32 bytes
     uint16_t path[TD_MAX_DEPTH];
 };
 
-// Per-instance bookkeeping when several warps share one search.
-struct td_inst_state {
-    int found;              // 1: a warp recorded the witness; 2: one side of a race was searched
+// Per-instance bookkeeping when several warps share one search.  A search that
+// never gives anything away does not use it.
+struct __align__(16) td_inst_state {
+    // units (the root search + items) not yet finished: the low 32 bits count
+    // the search of the instance, the high 32 bits that of its inverse
+    unsigned long long pending;
+    unsigned short found;   // 1: a warp recorded the witness; 2: one side of a race was searched
                             // to the end without one (the verdict is known, the other side stops)
-    int pending;            // units (the root search + items) not yet finished: the low 16 bits
-                            // count the search of the instance, the high 16 bits that of its
-                            // inverse (td_steal_kernel's race; elsewhere only the low half is used)
+    short error;            // first error status seen (timeout)
     unsigned expansions;    // summed over units
-    int error;              // first error status seen (timeout)
 };
+#define TD_UNIT_INVERSE (1ull << 32)
 
 // Scheduler counters of one launch.
 struct td_pool {
@@ -108,6 +110,7 @@ struct td_donate_ctx {
     td_inst_state *state;
     int side;               // 1: the unit searches the instance's inverse (items carry it on)
     int attempt;            // the restart attempt that donated the unit (0 for a root)
+    int gave;               // 0: a root search that has given nothing away (no other warp knows of it)
     int race;               // > 0: the unit queues its inverse when it starts restart attempt
                             // `race` (root units of full-sorting instances in td_steal_kernel)
 };
@@ -633,7 +636,7 @@ struct td_dfs_out {
 // pending count covers the items before any taker can finish one (takers wait
 // for the ready flag, written later), and so does the batch engine's
 // outstanding count.
-__device__ __forceinline__ int td_reserve(const td_donate_ctx &dc, int want, int unit, int *got) {
+__device__ __forceinline__ int td_reserve(td_donate_ctx &dc, int want, unsigned long long unit, int *got) {
     int base = -1, n = want;
     if (dc.tickets) {
         if (*(volatile int *)&dc.pool->produced < dc.capacity) {
@@ -651,7 +654,11 @@ __device__ __forceinline__ int td_reserve(const td_donate_ctx &dc, int want, int
             cur = prev;
         }
     }
-    if (base >= 0) atomicAdd(&dc.state->pending, n * unit);
+    if (base >= 0) {
+        // the first time, a root search counts itself too
+        atomicAdd(&dc.state->pending, (unsigned long long)n * unit + (dc.gave ? 0ull : 1ull));
+        dc.gave = 1;
+    }
     td_fence();
     *got = base >= 0 ? n : 0;
     return base;
@@ -711,7 +718,7 @@ __device__ __noinline__ int td_donate(td_warp_smem &s, int d0, int level, int N,
     int give = min(min(want, 32), have - (lv == level ? 1 : 0));
     if (give <= 0) return 0;
     int base = -1;
-    if (lane == 0) base = td_reserve(dc, give, dc.side ? 1 << 16 : 1, &give);
+    if (lane == 0) base = td_reserve(s.dc, give, dc.side ? TD_UNIT_INVERSE : 1ull, &give);
     base = __shfl_sync(TD_FULL, base, 0);
     give = __shfl_sync(TD_FULL, give, 0);
     if (base < 0) return 0;  // out of item space: keep the work
@@ -768,12 +775,12 @@ __device__ __noinline__ int td_donate(td_warp_smem &s, int d0, int level, int N,
 // instance's root search queues its inverse, once.  In the batch engine items
 // are taken once no fresh instance is left, and the inverses queued until then
 // come first.  Returns whether it was queued (uniform across the warp).
-__device__ __noinline__ int td_spawn_inverse(const td_warp_smem &s, int N) {
+__device__ __noinline__ int td_spawn_inverse(td_warp_smem &s, int N) {
     const td_donate_ctx &dc = s.dc;
     int ok = 0;
     if ((threadIdx.x & 31) == 0) {
         int got;
-        const int slot = td_reserve(dc, 1, 1 << 16, &got);
+        const int slot = td_reserve(s.dc, 1, TD_UNIT_INVERSE, &got);
         if (slot >= 0) {
             td_item it;
             it.L = td_inverse_pinned(s.L[0], N);
@@ -1210,7 +1217,7 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
                     // takers holding a ticket past the last item produced; in
                     // the serving loop, idle warps beyond the unclaimed items
                     if (!s.dc.tickets) waiting += *(volatile int *)&s.dc.pool->idle;
-                    ended = *(volatile int *)&s.dc.state->found;
+                    ended = s.dc.gave ? *(volatile unsigned short *)&s.dc.state->found : 0;
                 }
             }
         }

@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
         dc.state = nullptr;
         dc.side = 0;
         dc.attempt = 0;
+        dc.gave = 0;
         dc.race = 0;  // set per fresh request (the per-call server's race)
         dc.idle_seen = 0;  // with the settings, per unit
         dc.grain = grain;
@@ -257,13 +258,9 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
             const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(&queue[slot]));
             const td_instance x = *reinterpret_cast<const td_instance *>(&v);
             td_inst_state *st = &state[slot];
-            if (lane == 0) {  // the slot's previous request is done: start afresh
-                st->found = 0;
-                st->expansions = 0;
-                st->error = 0;
-                st->pending = 1;
-                __threadfence();
-            }
+            // the slot's previous request is done: start afresh (other warps see it
+            // only through items, which are published after a fence)
+            if (lane == 0) *reinterpret_cast<uint4 *>(st) = make_uint4(0u, 0u, 0u, 0u);
             __syncwarp();
             if (!td_instance_ok(x) || td_triple_count(x.n_symbols) == 0) {
                 td_write_result(&results[slot], td_instance_ok(x) ? TD_NOT_FOUND : TD_ERR_ARG, 0, 0, s.path, 0,
@@ -323,14 +320,14 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 }
                 __syncwarp();
                 int stop = 0;
-                if (lane == 0) stop = *(volatile int *)&state[slot].found;
+                if (lane == 0) stop = *(volatile unsigned short *)&state[slot].found != 0;
                 run = !__shfl_sync(TD_FULL, stop, 0);
                 td_unpack_state(s, d0, it.L, it.off & 31, x.n_symbols);
                 if (run && d0 > 0 && !ALL_ORDERED && tt &&
                     td_tt_visit(s, d0, x.n_symbols, (uint32_t)req, (uint32_t)(side << 6 | attempt)))
                     run = false;
                 if (!run) {  // the request has its witness, or another unit took the state up
-                    if (td_finish_unit<true>(r, &state[slot], &results[slot], s.path, side) && lane == 0) {
+                    if (td_finish_unit<true>(r, &state[slot], &results[slot], s.path, side, 1) && lane == 0) {
                         done[slot] = (unsigned long long)req + 1ull;
                         atomicAdd(&dctl->served, 1ull);
                     }
@@ -363,6 +360,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 s.dc.state = &state[slot];
                 s.dc.side = side;
                 s.dc.attempt = attempt;
+                s.dc.gave = kind == 2;
                 s.dc.race = MODE == TD_SERVE_PER_REQUEST && kind == 1 && !ord && restart_base && td_inst_full(x) ? race : 0;
             }
             __syncwarp();
@@ -372,9 +370,10 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 const int t = td_inverse_witness(s, x, r.depth, r.found_move);
                 if (t < 0) r.status = TD_DFS_EXHAUSTED;
                 else r.found_move = (uint16_t)t;
-                if (t == -1 && lane == 0) atomicCAS(&state[slot].error, 0, TD_ERR_VERIFY);
+                if (t == -1 && lane == 0) td_note_error(&state[slot], TD_ERR_VERIFY);
             }
-            if (td_finish_unit<true>(r, &state[slot], &results[slot], s.path, side) && lane == 0) {
+            const int gave = s.dc.gave;
+            if (td_finish_unit<true>(r, &state[slot], &results[slot], s.path, side, gave) && lane == 0) {
                 done[slot] = (unsigned long long)req + 1ull;
                 atomicAdd(&dctl->served, 1ull);
             }
