@@ -603,18 +603,18 @@ TD_HD int td_prepare_pair(const uint8_t *beta, const uint8_t *omega, int N, int 
             seen_b |= 1u << beta[x];
             seen_o |= 1u << omega[x];
         }
-        const uint32_t all = (N == 32) ? ~0u : ((1u << N) - 1u);
+        const uint32_t all = (1u << N) - 1u;
         if (seen_b != all || seen_o != all) return TD_ERR_ARG;
-        uint8_t next_of[TD_MAX_N], rho[TD_MAX_N], sigma[TD_MAX_N];
-        for (int x = 0; x < N; ++x) next_of[beta[x]] = beta[(x + 1) % N];
-        for (int x = 0; x < N; ++x) rho[x] = omega[next_of[x]];
+        // rho = omega . beta is a permutation, so it is one cycle when the walk
+        // from beta[0] comes back after N steps and no sooner
+        uint8_t next_of[TD_MAX_N], sigma[TD_MAX_N];
+        for (int x = 0; x + 1 < N; ++x) next_of[beta[x]] = beta[x + 1];
+        next_of[beta[N - 1]] = beta[0];
         int r = beta[0];
-        for (int m = 0; m < N; ++m) { sigma[r] = (uint8_t)m; r = rho[r]; }
-        if (r != beta[0]) return TD_ERR_ARG;
-        for (int x = 0; x < N; ++x) {  // rho must visit every symbol once
-            int steps = 0, y = x;
-            do { y = rho[y]; ++steps; } while (y != x && steps <= N);
-            if (steps != N) return TD_ERR_ARG;
+        for (int m = 0; m < N; ++m) {
+            if (m > 0 && r == beta[0]) return TD_ERR_ARG;
+            sigma[r] = (uint8_t)m;
+            r = omega[next_of[r]];
         }
         L = 0;
         for (int m = 0; m < 16; ++m) {
