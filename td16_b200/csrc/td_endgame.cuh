@@ -128,8 +128,16 @@ __device__ __forceinline__ uint32_t td_eg_skip(td_warp_smem &s, int level, int N
 // Free order, a node without a spare move (all its children are +2 ones):
 // decides the children of `level` by the table.  Where one can be sorted it
 // becomes the level's only child (returns true); otherwise only the children
-// that the table does not hold stay.
-__device__ __noinline__ bool td_eg_filter(td_warp_smem &s, int level, int N) {
+// that the table does not hold stay.  `attempt` >= 0: the search is shared by
+// several warps, and of those the ones that the table of explored states holds
+// for this attempt are dropped too, 32 looks at once instead of one after the
+// other when they are visited (where the others are recorded, as ever).  2,048
+// S_16 instances at their lower bound took 2.41 ms without those looks and take
+// 2.18 ms, the 250 of S_8..S_16 at lower + 1 0.166 and 0.152 ms; for searches
+// that one warp ends alone, whose few repeated states it meets soon, they cost
+// as much as they give (2^16 mixed instances 1.72 ms and 1.74 ms), and on nodes
+// further from the end they made 2^19 near-reverse ones slower (21.6 and 22.1).
+__device__ __noinline__ bool td_eg_filter(td_warp_smem &s, int level, int N, int attempt) {
     const int lane = threadIdx.x & 31;
     const uint32_t fixed = td_eg_fixed(s, level, N);
     uint64_t L;
@@ -165,6 +173,14 @@ __device__ __noinline__ bool td_eg_filter(td_warp_smem &s, int level, int N) {
         if (lane < all) {
             t = s.list[lane];
             e = td_eg_probe(s, level, N, L, off, fixed, t, true);
+            if (e == TD_EG_UNKNOWN && attempt >= 0) {
+                uint64_t nL;
+                int noff;
+                td_apply_move(L, off, N, t & 31, (t >> 5) & 31, (t >> 10) & 31, &nL, &noff);
+                const uint32_t sub = (uint32_t)(s.dc.side << 6) + (uint32_t)(s.dc.attempt + attempt);
+                if (td_tt_peek(s.lim, nL & (~0ull >> (64 - 4 * (N - 1))), level + 1, s.dc.inst, sub))
+                    e = 1;  // taken up already with at least this budget
+            }
         }
         __syncwarp();
         const uint32_t yes = __ballot_sync(TD_FULL, e == 0);

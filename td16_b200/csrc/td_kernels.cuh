@@ -613,6 +613,112 @@ __device__ __forceinline__ int td_next_child(td_warp_smem &s, int level, int *ac
     return 32 * st + b;
 }
 
+// ---- table of explored states (free order) --------------------------------
+//
+// Different move orders reach the same state: on near-reverse S_16 about 80%
+// of the free-order expansions re-expand a state already expanded at the same
+// or a smaller depth.  Whether a node's subtree holds a witness depends only
+// on its pinned state L (not on where the caller's array starts: a move is the
+// same cycle rotation from any start, so the reachable states do not depend
+// on it) and on its depth.  The warps of a launch share one direct-mapped
+// table of the states they took up, and a child whose state is in the table
+// for the same search at a depth <= the child's is skipped.  This is sound
+// also where the entry is another warp's, whose subtree is still being
+// searched: whoever records a state takes up each of its children, finds it
+// recorded for the same search with at least as much budget, leaves it to the
+// endgame table or donates it (the taker then records it or finds it
+// recorded).  So, by induction on the length of a state's shortest witness,
+// some warp meets the witness of every recorded state; and a search only ends
+// without one when every unit of it has ended.
+//
+// An entry is one 16-byte word, read and written whole (128-bit relaxed
+// accesses), so it always names one state exactly:
+//   word 0: the state's key (td_tt_key, 57 bits), low 7 bits of the search's
+//           number on top
+//   word 1: the search's number (the other 51 bits), the side (1 bit: the
+//           instance or its inverse), the restart attempt (6 bits: the
+//           subtrees of an abandoned attempt were not all searched) and the
+//           depth (4 bits)
+// A search's number is its launch's epoch and its index there (58 bits), so
+// the entries of other launches never match and the table is never cleared.
+// Zero words are empty (a recorded state has depth >= 1).
+//
+// Each warp had a table of its own before (4,096 entries of 8 bytes, 155 MB in
+// all): the warps that shared a long search explored the same states again.
+// The hardest of 2,048 S_16 instances at their lower bound took 171,000 to
+// 258,000 expansions then, against about 14,000 with one table.
+
+// A search starts using the table after this many expansions of a unit: most
+// searches of uniform permutations end sooner, and they then never touch it.
+// States expanded before are simply not recorded.
+#ifndef TD_TT_AFTER
+#define TD_TT_AFTER 32
+#endif
+
+__device__ __forceinline__ void td_tt_load(const ulonglong2 *p, uint64_t &a, uint64_t &b) {
+    asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+                 : "=l"(a), "=l"(b)
+                 : "l"(p)
+                 : "memory");
+}
+
+__device__ __forceinline__ void td_tt_store(ulonglong2 *p, uint64_t a, uint64_t b) {
+    asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }"
+                 :
+                 : "l"(p), "l"(a), "l"(b)
+                 : "memory");
+}
+
+// The place of a state's entry, and its two words (word 1 without the depth).
+__device__ __forceinline__ ulonglong2 *td_tt_entry(const td_search_limits &lim, uint64_t L, uint32_t inst, uint32_t sub,
+                                                   uint64_t *w0, uint64_t *w1) {
+    const uint64_t id = lim.tt_id + inst;
+    *w0 = td_tt_key(L) | (id << 57);
+    *w1 = ((id >> 7) << 7) | sub;
+    return lim.tt + (((*w0 + *w1 * 0xD6E8FEB86659FD93ull) * 0x9E3779B97F4A7C15ull) >> lim.tt_shift);
+}
+
+// Whether the state L (nibbles from N-1 on cleared) is in the table at a depth
+// <= lv.
+__device__ __forceinline__ bool td_tt_peek(const td_search_limits &lim, uint64_t L, int lv, uint32_t inst, uint32_t sub) {
+    uint64_t w0, w1, e0, e1;
+    const ulonglong2 *e = td_tt_entry(lim, L, inst, sub, &w0, &w1);
+    td_tt_load(e, e0, e1);
+    return e0 == w0 && (e1 >> 4) == w1 && (int)(e1 & 15u) <= lv;
+}
+
+// Looks up the state of level `lv` (depth lv) in the table and records it
+// there; returns whether it was already taken up at a depth <= lv by the
+// search `sub` (side << 6 | attempt) of instance `inst` of this launch
+// (uniform across the warp).
+__device__ __forceinline__ bool td_tt_visit(const td_warp_smem &s, int lv, int N,
+                                            uint32_t inst, uint32_t sub) {
+    const int m = threadIdx.x & 31;
+    const int a = m < N ? s.A[lv][m] : 0xff;
+    const int c0 = __ffs(__ballot_sync(TD_FULL, a == 0)) - 1;  // caller position of label 0
+    // L[m] = A[(m + 1 + c0) mod N] - 1 for m < N - 1
+    int src = m + 1 + c0;
+    src -= src >= N ? N : 0;
+    const int v = __shfl_sync(TD_FULL, a, m < N - 1 ? src : m) - 1;
+    uint32_t lo = 0, hi = 0;
+    if (m < N - 1) {
+        if (m < 8) lo = (uint32_t)v << (4 * m);
+        else hi = (uint32_t)v << (4 * (m - 8));
+    }
+    lo = __reduce_or_sync(TD_FULL, lo);
+    hi = __reduce_or_sync(TD_FULL, hi);
+    int hit = 0;
+    if (m == 0) {
+        uint64_t w0, w1;
+        ulonglong2 *e = td_tt_entry(s.lim, (((uint64_t)hi) << 32) | lo, inst, sub, &w0, &w1);
+        uint64_t e0, e1;
+        td_tt_load(e, e0, e1);
+        hit = e0 == w0 && (e1 >> 4) == w1 && (int)(e1 & 15u) <= lv;
+        if (!hit) td_tt_store(e, w0, (w1 << 4) | (uint64_t)lv);
+    }
+    return __shfl_sync(TD_FULL, hit, 0) != 0;
+}
+
 #include "td_endgame.cuh"
 
 #define TD_DFS_FOUND 1
@@ -905,96 +1011,6 @@ __device__ __noinline__ int td_inverse_witness(td_warp_smem &s, td_instance x, i
     return td_filtered_witness(s, x, k, found_move) ? (int)found_move : -2;
 }
 
-// ---- table of explored states (free order) --------------------------------
-//
-// Different move orders reach the same state: on near-reverse S_16 about 80%
-// of the free-order expansions re-expand a state already expanded at the same
-// or a smaller depth.  Whether a node's subtree holds a witness depends only
-// on its pinned state L (not on where the caller's array starts: a move is the
-// same cycle rotation from any start, so the reachable states do not depend
-// on it) and on its depth.  The warps of a launch share one direct-mapped
-// table of the states they took up, and a child whose state is in the table
-// for the same search at a depth <= the child's is skipped.  This is sound
-// also where the entry is another warp's, whose subtree is still being
-// searched: whoever records a state takes up each of its children, finds it
-// recorded for the same search with at least as much budget, leaves it to the
-// endgame table or donates it (the taker then records it or finds it
-// recorded).  So, by induction on the length of a state's shortest witness,
-// some warp meets the witness of every recorded state; and a search only ends
-// without one when every unit of it has ended.
-//
-// An entry is one 16-byte word, read and written whole (128-bit relaxed
-// accesses), so it always names one state exactly:
-//   word 0: the state's key (td_tt_key, 57 bits), low 7 bits of the search's
-//           number on top
-//   word 1: the search's number (the other 51 bits), the side (1 bit: the
-//           instance or its inverse), the restart attempt (6 bits: the
-//           subtrees of an abandoned attempt were not all searched) and the
-//           depth (4 bits)
-// A search's number is its launch's epoch and its index there (58 bits), so
-// the entries of other launches never match and the table is never cleared.
-// Zero words are empty (a recorded state has depth >= 1).
-//
-// Each warp had a table of its own before (4,096 entries of 8 bytes, 155 MB in
-// all): the warps that shared a long search explored the same states again.
-// The hardest of 2,048 S_16 instances at their lower bound took 171,000 to
-// 258,000 expansions then, against about 14,000 with one table.
-
-// A search starts using the table after this many expansions of a unit: most
-// searches of uniform permutations end sooner, and they then never touch it.
-// States expanded before are simply not recorded.
-#ifndef TD_TT_AFTER
-#define TD_TT_AFTER 32
-#endif
-
-__device__ __forceinline__ void td_tt_load(const ulonglong2 *p, uint64_t &a, uint64_t &b) {
-    asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
-                 : "=l"(a), "=l"(b)
-                 : "l"(p)
-                 : "memory");
-}
-
-__device__ __forceinline__ void td_tt_store(ulonglong2 *p, uint64_t a, uint64_t b) {
-    asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }"
-                 :
-                 : "l"(p), "l"(a), "l"(b)
-                 : "memory");
-}
-
-// Looks up the state of level `lv` (depth lv) in the table and records it
-// there; returns whether it was already taken up at a depth <= lv by the
-// search `sub` (side << 6 | attempt) of instance `inst` of this launch
-// (uniform across the warp).
-__device__ __forceinline__ bool td_tt_visit(const td_warp_smem &s, int lv, int N,
-                                            uint32_t inst, uint32_t sub) {
-    const int m = threadIdx.x & 31;
-    const int a = m < N ? s.A[lv][m] : 0xff;
-    const int c0 = __ffs(__ballot_sync(TD_FULL, a == 0)) - 1;  // caller position of label 0
-    // L[m] = A[(m + 1 + c0) mod N] - 1 for m < N - 1
-    int src = m + 1 + c0;
-    src -= src >= N ? N : 0;
-    const int v = __shfl_sync(TD_FULL, a, m < N - 1 ? src : m) - 1;
-    uint32_t lo = 0, hi = 0;
-    if (m < N - 1) {
-        if (m < 8) lo = (uint32_t)v << (4 * m);
-        else hi = (uint32_t)v << (4 * (m - 8));
-    }
-    lo = __reduce_or_sync(TD_FULL, lo);
-    hi = __reduce_or_sync(TD_FULL, hi);
-    int hit = 0;
-    if (m == 0) {
-        const uint64_t id = s.lim.tt_id + inst;
-        const uint64_t w0 = td_tt_key((((uint64_t)hi) << 32) | lo) | (id << 57);
-        const uint64_t w1 = ((id >> 7) << 7) | sub;
-        ulonglong2 *e = s.lim.tt + (((w0 + w1 * 0xD6E8FEB86659FD93ull) * 0x9E3779B97F4A7C15ull) >> s.lim.tt_shift);
-        uint64_t e0, e1;
-        td_tt_load(e, e0, e1);
-        hit = e0 == w0 && (e1 >> 4) == w1 && (int)(e1 & 15u) <= lv;
-        if (!hit) td_tt_store(e, w0, (w1 << 4) | (uint64_t)lv);
-    }
-    return __shfl_sync(TD_FULL, hit, 0) != 0;
-}
-
 #include "td_ordered.cuh"
 
 // Depth-first search from the node held at level d0 of `s` (state, path, rate
@@ -1066,7 +1082,7 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
                     const uint4 w = s.pw[level][lane];
                     const unsigned n = __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w);
                     if (__reduce_add_sync(TD_FULL, n) >= TD_EG_MANY)
-                        solved |= td_eg_filter(s, level, N);
+                        solved |= td_eg_filter(s, level, N, s.dc.gave && s.lim.tt ? attempt : -1);
                 }
             }
         }
