@@ -31,7 +31,7 @@ def test_shared_searches_keep_the_verdict(slots, oracle, N, over):
     bound = ((N - init + 1) // 2 + over).astype(np.int32)
     inst = td.prepare_pairs(beta, omega, N, init, np.zeros(6, np.float32), bound, np.ones(6, np.uint8))
     ref, _ = td.search_batch(0, inst, td._lib.FLAG_ORDERED | td._lib.FLAG_VERIFY, 200000)
-    done = ref["status"] != 2
+    done = ref["status"] >= 0
     assert done.any()
     for _ in range(8):  # who gives what to whom differs from run to run
         free, _ = td.search_batch(0, inst, td._lib.FLAG_VERIFY)
