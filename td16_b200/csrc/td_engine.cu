@@ -438,6 +438,8 @@ __device__ __forceinline__ int td_finish_unit(const td_dfs_out &r, td_inst_state
     return last;
 }
 
+#define TD_EAGER_UNITS 16  // instances per warp up to which a launch shares its searches from the start
+
 #ifndef TD_STEAL_MIN_BLOCKS
 #define TD_STEAL_MIN_BLOCKS 4  // resident blocks of 8 warps per SM the register budget is sized for
 #endif
@@ -485,8 +487,15 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
         dc.idle_after = 0;
         dc.idle_seen = 0;
         s.dc = dc;
-        // a launch with fewer instances than warps has idle warps from the start
-        if (count < (int)(gridDim.x * (blockDim.x >> 5))) td_serve_idle_warps(s.dc);
+        // Few instances per warp: most of the launch is its tail, in which a few
+        // long searches are all that is left, and giving subtrees away late
+        // costs more than doing it too often.  With up to 16 instances a warp
+        // the settings for idle warps hold from the start (only with fewer
+        // instances than warps before: 20,011 S_12..S_14 2.13 -> 1.49 ms, 2^16
+        // mixed 1.69 -> 1.32, 8,000 S_13 1.16 -> 0.82).  With 21 (10^5 uniform
+        // S_16) they took 0.79 ms, and 0.75 without: there the loads of the
+        // idle checks are work that nothing waits for.
+        if (count <= TD_EAGER_UNITS * (int)(gridDim.x * (blockDim.x >> 5))) td_serve_idle_warps(s.dc);
     }
     __syncwarp();
     // Race (`race` = a, 0: off): a root search of a full-sorting instance
@@ -954,6 +963,8 @@ static_assert(sizeof(td_pool) % 8 == 0 && sizeof(td_pool) + 2 * sizeof(int) + si
 // child nearly always; a walk that finds no node runs whole).
 size_t split_nodes(int records) { return (size_t)std::max(1, records / 2); }
 
+constexpr int TD_INSTANCE_WARPS = 4;  // a free-order batch's warps per instance, where the device has them
+
 // log2 of the entries of a table of explored states for `warps` resident warps.
 int tt_entries_log2(size_t warps, int bits) {
     int b = 0;
@@ -1189,10 +1200,19 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
             s.state_count = (size_t)count;
         }
         // at least the slot's share of the resident grid, so that a small batch
-        // (one search from td_search) is spread over that many warps by donation
+        // (one search from td_search) is spread over that many warps by donation,
+        // and TD_INSTANCE_WARPS warps per instance: with one each, the warps
+        // whose instance was easy were too few for what the hard ones give away.
+        // With 16 slots, 2,048 S_16 at their lower bound took 5.1 ms with one
+        // warp each, 2.2 with two and 2.0 with four; 250 of S_8..S_16 0.30, 0.27
+        // and 0.22.  It holds for launches side by side too (they end sooner, and
+        // make room): from 16 threads 3.8 and 2.2 ms a batch of the former, 0.11
+        // and 0.10 ms of the latter.  The whole grid for every batch is no
+        // better alone, and slower there (0.25 ms).
         const int resident = cfg.sms * cfg.steal_blocks_per_sm;
         const int share = std::max(1, resident / std::max(1, s.slots_on_device));
-        const int grid = std::max(1, std::min(resident, std::max(share, (count + warps - 1) / warps)));
+        const int64_t wanted = ((int64_t)count * TD_INSTANCE_WARPS + warps - 1) / warps;
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(resident, std::max<int64_t>(share, wanted)));
         const int tt_log2 = tt_entries_log2((size_t)resident * warps, cfg.tt_bits);
         if (cfg.tt_bits > 0 && (tt_log2 > s.tt_log2 || cfg.tt_bits != s.tt_bits)) {
             // sized for the whole resident grid so that it never moves under a

@@ -36,3 +36,19 @@ def test_shared_searches_keep_the_verdict(slots, oracle, N, over):
     for _ in range(8):  # who gives what to whom differs from run to run
         free, _ = td.search_batch(0, inst, td._lib.FLAG_VERIFY)
         assert (free["status"][done] == ref["status"][done]).all()
+
+
+@pytest.mark.parametrize("count", [1, 73, 74, 75, 295, 297, 1183, 1185, 75775, 75777])
+def test_verdicts_at_the_edges_of_the_launch_shapes(td, oracle, count):
+    """Around the counts at which a launch leaves its slot's share of the
+    device, fills the device, and stops sharing its searches from the start."""
+    td.destroy()
+    td.init_slots(16, [0], 64 * MiB)
+    perms, n = oracle.synth_perms(count, count, 6, 9, 50, 1, 2)
+    inst = td.prepare_perms(perms, n, 9)
+    init = (inst["packed"] & 31).astype(np.int32)
+    inst["max_moves"] = np.clip((n.astype(np.int32) + 2 - init) // 2, 1, 9)
+    ref, _ = td.search_batch(0, inst, td._lib.FLAG_ORDERED | td._lib.FLAG_VERIFY)
+    free, _ = td.search_batch(0, inst, td._lib.FLAG_VERIFY)
+    assert (free["status"] == ref["status"]).all()
+    assert (free["status"] >= 0).all()
