@@ -519,6 +519,46 @@ __device__ __forceinline__ int td_next_child_rows(td_warp_smem &s, int level, ui
     return (int)(pc | ((uint32_t)k << 10) | (c2 ? 0u : 0x8000u));
 }
 
+// Free order, the node of `level` just expanded (s.inv is its inverse): takes
+// its move that fixes two symbols or three, a +2 child, and returns it, or -1
+// where there is none or it is not among the level's children.  Positions x, y,
+// z one step of omega apart give that move where their cyclic order is a
+// move's; of several, the one of lowest x.  Fewer symbols are left after it, so
+// the endgame table is nearer: 2^19 near-reverse S_16 take 41 expansions each
+// with it and took 47 without (21.6 -> 19.0 ms), 2^16 mixed ones 11.0 and 12.6
+// (1.32 -> 1.21 ms); uniform S_16, which are short, lose what they win (3.50 and
+// 3.53 ms).  Only a root search's first attempt uses it: later attempts live on
+// other orders (with it in every second one 19.7 ms), and a subtree given away
+// is mostly searched to its end.  Called: inlined, it made every search slower.
+__device__ __noinline__ int td_take_fixing(td_warp_smem &s, int level, int N) {
+    const int x = threadIdx.x & 31;
+    int y = x;
+    if (x < N) {
+        const int p = s.A[level][x == 0 ? N - 1 : x - 1];
+        y = s.inv[p + 1 == N ? 0 : p + 1];
+    }
+    const int z = __shfl_sync(TD_FULL, y, y);
+    const uint32_t good = __ballot_sync(TD_FULL, (x < y) + (y < z) + (z < x) == 2);
+    if (!good) return -1;
+    const int p = __ffs(good) - 1;
+    const int q = __shfl_sync(TD_FULL, y, p), u = __shfl_sync(TD_FULL, z, p);
+    const int t = p < q ? q < u ? p | q << 5 | u << 10 : u | p << 5 | q << 10 : q | u << 5 | p << 10;
+    const ushort4 pq = s.pair[x];
+    const uint32_t code = t & 1023, bit = 1u << ((t >> 10) - 1);
+    uint4 W = s.pw[level][x];
+    bool mine = false;
+    if (pq.x == code && (W.x & bit)) { W.x &= ~bit; mine = true; }
+    if (pq.y == code && (W.y & bit)) { W.y &= ~bit; mine = true; }
+    if (pq.z == code && (W.z & bit)) { W.z &= ~bit; mine = true; }
+    if (pq.w == code && (W.w & bit)) { W.w &= ~bit; mine = true; }
+    if (mine) {
+        s.pw[level][x] = W;
+        if (!((W.x | W.y | W.z | W.w) & 0xffffu)) s.m2[level] &= ~(1u << x);
+    }
+    __syncwarp();
+    return __any_sync(TD_FULL, mine) ? t : -1;
+}
+
 // Reference order: classifies every child of the node at `level`; fills the
 // level's child words and returns the found child's u, or -1.  A node's found
 // child is the one of lowest u (the lowest lane of the first 32-chunk,
@@ -1154,8 +1194,8 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
         // children skipped through the tables, change no expansion count, so
         // the checks above run once per expansion
         int walk = 0;  // 1: the subtree is exhausted, 2: a root accepted on visit (ordered), 3: out of budget
-        for (;;) {
-            int t;
+        for (bool fresh = !ORDERED && attempt + solved + d0 == 0;; fresh = false) {
+            int t = -1;
             if constexpr (ORDERED) {
                 const int spare = s.spare[level];
                 if (spare != 255) {
@@ -1180,7 +1220,8 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
                     }
                 }
             } else {
-                t = td_next_child_rows(s, level, td_level_order(ord, attempt, level));
+                if (fresh) t = td_take_fixing(s, level, N);
+                if (t < 0) t = td_next_child_rows(s, level, td_level_order(ord, attempt, level));
             }
             if (t < 0) {
                 if (level == d0) { walk = 1; break; }
