@@ -43,17 +43,17 @@ WORKLOAD = "full-size decision search: 2^20 S_16 perms, 50% uniform / 50% revers
 # pass ncu captures of td_steal_kernel on one launch of this benchmark's 2^20-
 # instance batch with the tuned launch shape and the race from attempt 8,
 # summarised with their commands in profiles/td_steal_kernel_s16_2p20_counters.md.
-# 36.870 G warp instructions and 19.901 G ALU-pipe instructions over the
-# launch's 49.02 M expansions (restarts, races, skipped children, donation and
-# scheduling included) in 85.21 M SM cycles: the ALU pipe busy 78.9 % of its 2
-# warp instructions per cycle per SM, issue 73.1 % of 4; 0.963 GB read and
-# 0.840 GB written.
+# 20.192 G warp instructions and 10.333 G ALU-pipe instructions over the
+# launch's 25.85 M expansions (restarts, races, table look-ups, skipped children,
+# donation and scheduling included) in 43.94 M SM cycles: the ALU pipe busy 79.5 %
+# of its 2 warp instructions per cycle per SM, issue 77.6 % of 4; 0.096 GB read
+# and 0.264 GB written.
 PLAIN_WARPS = 4  # block shape of the plain one-launch-per-batch leg
-INST_PER_EXPANSION = 36.870e9 / 49.02e6
-ALU_INST_PER_EXPANSION = 19.901e9 / 49.02e6
-ALU_BUSY_MEASURED = 19.901e9 / (85.21e6 * 148 * 2)
-ISSUE_MEASURED = 36.870e9 / (85.21e6 * 148 * 4)
-DRAM_BYTES_PER_LAUNCH = 0.963e9 + 0.840e9
+INST_PER_EXPANSION = 20.192e9 / 25.85e6
+ALU_INST_PER_EXPANSION = 10.333e9 / 25.85e6
+ALU_BUSY_MEASURED = 10.333e9 / (43.94e6 * 148 * 2)
+ISSUE_MEASURED = 20.192e9 / (43.94e6 * 148 * 4)
+DRAM_BYTES_PER_LAUNCH = 0.096e9 + 0.264e9
 
 
 def rank_info():
@@ -523,7 +523,7 @@ def run_engine(args):
                 "traffic": DRAM_BYTES_PER_LAUNCH * count / COUNT,
                 "traffic_note": "DRAM bytes of one 2^20 launch (ncu, one pass, the benchmark launch itself); the "
                                 "algorithmic bytes are 48 per instance (16 in, 32 out): 50 MB; the rest is the "
-                                "explored-state tables (4736 warps x 32 KiB = 155 MB > the 126 MB L2)",
+                                "per-instance state and the table of explored states (64 MiB)",
                 "alu_busy_measured": ALU_BUSY_MEASURED, "issue_measured": ISSUE_MEASURED,
                 "nodes_per_s": nodes_per_s, "triples_per_s": triples_per_s}
 

@@ -140,9 +140,10 @@ int td_set_time_limit(double seconds);
 /* Work donation of the free-order engine: items per donation, deepest level
  * whose children may be donated, expansions between idle checks (default
  * 4, 2, 64; the autotuner's tuned.json holds the settings of its buckets).
- * They hold while fresh instances are left; a warp that has met idle warps
- * checks 16 times as often and gives 8 times as many items (at most 32), from
- * up to 4 levels deeper. */
+ * They hold while fresh instances are left; a warp that has met idle warps, and
+ * every warp of a launch of up to 16 instances per warp, checks 16 times as
+ * often and gives 8 times as many items (at most 32), from up to 4 levels
+ * deeper. */
 int td_configure_steal(int grain, int split_level, int check_every);
 /* The same for later serving launches (td_serve_open), kept apart because a
  * serving launch trades throughput for latency (default 1, 2, 32; a request

@@ -316,7 +316,7 @@ def configure_steal(grain: int, split_level: int, check_every: int) -> None:
 
 
 def configure_table(bits: int) -> None:
-    """Explored-state tables of the free order: 2^bits entries per warp, 0 = none."""
+    """Table of explored states of the free order: 2^(bits - 2) entries per resident warp in all, 0 = none."""
     if lib().td_configure_table(int(bits)) != OK:
         raise TdError(INVALID_ARG, "table bits must be 0 or 6..16")
 

@@ -33,7 +33,7 @@
 #define TD_MAX_TRIPLES 680
 #define TD_MAX_STEPS 22  // ceil(680 / 32)
 #define TD_MAX_ROUNDS 4  // ceil(C(16,2) / 32): pair slots of the bit-sliced evaluation
-#define TD_PT_STRIDE 32  // pair table row stride (bytes)
+#define TD_PT_STRIDE 32  // pair table row stride (bytes; the host emulation)
 
 // ---- C-ABI records (mirrored in include/td16_b200.h) ----------------------
 
@@ -164,7 +164,7 @@ TD_HD int td_class_of_index(int idx) {
     return TD_CLASS_SKIP;
 }
 
-// ---- bit-sliced classification (free move order) ---------------------------
+// ---- bit-sliced classification (both move orders) ---------------------------
 //
 // The same classes for every third position k of a pair (i, j) at once, one
 // bit per k, from row masks of the node indexed by caller position:

@@ -2,8 +2,16 @@
 //
 // Kernels
 //   td_plain_kernel       one warp per instance, one launch per batch
-//   td_persistent_kernel  resident grid; warps claim instances with an atomic
-//                         ticket (steal granularity = instances per claim)
+//   td_steal_kernel       free order: resident grid; instances by ticket, then
+//                         the subtrees that busy warps give away
+//   td_ordered_kernel     reference order: the same, with the subtrees joined in
+//                         the walk's order (td_ordered.cuh)
+//   td_persistent_kernel  reference order, one warp per walk: batches with an
+//                         expansion budget or the split off, and the
+//                         allocation-free entry
+//   td_serve_kernel       requests as they arrive (td_serve.cuh, td_percall.cuh)
+//   td_eg_build_kernel    the endgame table, once per device (td_endgame.cuh)
+//   td_pairs_*_kernel     pairs to instances and results to triples
 //   td_validate_kernel    replays witnesses in pinned form
 // Host
 //   slots (stream + completion event + device scratch per slot) with the

@@ -7,11 +7,10 @@ Every case runs with the benchmark's launch shape (td16_b200/tuned.json).
 
   steal    td_steal_kernel: the S_16 benchmark instances (seed 2, half
            near-reverse), bound 9, free order (default 2^18 instances)
-  ordered  td_persistent_kernel<true>: 4096 x S_10 (seed 0), bound 6, the
-           reference's single-queue order (with its split below the root)
-  split    td_split_kernel: 4096 x S_13 (seed 5, half near-reverse), bound
-           6, the reference's order; most walks outlast the one-warp first
-           pass and are split below the root
+  ordered  td_ordered_kernel: 4096 x S_10 (seed 0), bound 6, the reference's
+           single-queue order
+  split    td_ordered_kernel: 4096 x S_13 (seed 5, half near-reverse), bound
+           6, the reference's order; the long walks give subtrees away
   plain    td_plain_kernel<false>: the plain one-launch-per-batch form on the
            first 8192 S_16 benchmark instances
   replay   td_replay_symbols_kernel: the certificates of 2^18 S_16 searches,
@@ -133,7 +132,7 @@ def main():
                                          "percall"])
     ap.add_argument("--count", type=int, default=None)
     ap.add_argument("--table-bits", type=int, default=None,
-                    help="entries of the explored-state tables (2^bits per warp; 0 = none; default 12)")
+                    help="size of the table of explored states (td_configure_table; 0 = none; default 12)")
     a = ap.parse_args()
     t0 = time.perf_counter()
     out = run(a.case, a.count, a.table_bits)
