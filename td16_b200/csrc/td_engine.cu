@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(256, 4) td_ordered_kernel(const td_instance *_
             s.sp_inst = inst;
             s.sp_node = node;
             s.sp_rank = rank;
-            // a first walk is split after split_after nodes, one that was given
+            // a first walk is split after split_after expansions, one that was given
             // away sooner
             s.lim.split_after = (uint32_t)(kind == 2 ? split_after / 8 : split_after);
             s.lim.cutoff = s.lim.cutoff2 = nullptr;

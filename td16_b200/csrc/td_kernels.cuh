@@ -28,7 +28,7 @@
 // Limits and tables of the search a warp runs.
 struct td_search_limits {
     uint32_t max_expansions;   // per search; TD_ERR_BUDGET when exceeded (~0: none)
-    uint32_t split_after;      // a walk of the reference order may be split after this many nodes
+    uint32_t split_after;      // a walk of the reference order may be split after this many expansions
     uint64_t deadline_ns;      // %globaltimer value; 0 = none
     ulonglong2 *tt;            // the launch's table of explored states (free order); null = none
     uint64_t tt_id;            // number of the launch's first search in it
@@ -1258,7 +1258,7 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
             break;
         }
         if constexpr (ORDERED) {
-            if (shared && work >= s.lim.split_after && ++since_check >= s.dc.check_every) {
+            if (shared && r.expansions >= s.lim.split_after && ++since_check >= s.dc.check_every) {
                 since_check = 0;
                 due = true;
                 if (lane == 0) {

@@ -19,12 +19,21 @@
 // The warp that completes the last record of a node joins them into the record
 // that the walk itself had, and so on up (td_split_complete).  Nothing is
 // walked twice, and nothing is split while every warp is busy.  A subtree that
-// ranks after a found one stops early; its result is never read.
+// ranks after a found one stops early; its result is never read.  A child of the
+// root that is accepted when visited ends the list: no walk goes past it.
+// (Without that rule three of four items of 3,001 partial-sorting pairs were
+// such subtrees, and their queue kept the walks from being split again: 1.8 to
+// 2.1 ms, now 1.2 to 1.7.)
+//
+// A walk may be split once it has counted `split_after` expansions, those that
+// the endgame table spares it included, since they say how long it will be:
+// 16,384 S_12 at bound 6 take 0.68 ms, and 0.82 counting the nodes expanded; 512
+// S_14 at their lower bound 0.51 and 0.67 ms.
 //
 // Splitting each root as soon as its walk had run for 64 expansions instead (a
 // launch each for the first pass, the listing, the subtrees and the join) took
 // 11 to 31 ms for 3,001 partial-sorting pairs, depending on their longest
-// subtree, and 33 ms for 256 S_16 at their lower bound; this takes 1.6 to 2.1
+// subtree, and 33 ms for 256 S_16 at their lower bound; this takes 1.2 to 1.7
 // and 3.4 ms.  In one queue the early split loses where most instances have a
 // witness (8,192 near-reverse S_13 at bound 7: 18.6 against 6.9 ms): subtrees
 // of high rank then run before the ones that cut them off.
@@ -138,6 +147,7 @@ __device__ __noinline__ uint32_t td_split(td_warp_smem &s, int d0, int level, in
                 const bool plus2 = spare == 0 || ((s.cp[lv][u >> 5] >> (u & 31)) & 1u);
                 e = td_eg_probe(s, lv, N, L, off, fixed, t, plus2 ? spare == 0 : spare == 1);
             }
+            if (accepted) e = 0;  // the walk goes no further than this child
             s.kid[c + lane] = (uint16_t)(t | accepted << 15);
             s.kid_e[c + lane] = (uint16_t)(e == TD_EG_UNKNOWN ? 0xffffu : e);
             if (c + lane >= own) atomicAnd(&s.cw[lv][u >> 5], ~(1u << (u & 31)));
