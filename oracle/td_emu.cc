@@ -577,3 +577,245 @@ extern "C" long td_emu_endgame(int symbols, uint16_t *out, int threads) {
         }
     return bad.load();
 }
+
+// ---- reference-order walks with the endgame table and given-away children ------
+
+namespace {
+
+// One search of td_ordered.cuh with a warp always waiting, one unit after the
+// other: the rules of td_eg_skip, td_split and td_split_complete.
+struct SplitEmu {
+    struct Child {
+        uint16_t move;
+        bool plus2, accepted;
+    };
+    struct Rec {  // one record of a split node, or an item still to be walked
+        bool item, accepted;
+        uint32_t exp;
+        uint16_t move;
+    };
+    struct Node {
+        int depth;
+        uint64_t L;  // of the node whose children were given away
+        int off;
+        uint16_t path[TD_MAX_DEPTH];
+        std::vector<Rec> recs;  // ranks 1, 2, ...
+    };
+    const uint16_t *table;
+    int split_after, check_every, eg_moves;
+    long splits = 0, kept = 0;  // nodes made, and levels that kept their children since the table decides them
+    Emu e;
+
+    // what the table says of the state: -1 unknown, 0 sorted within the moves left, else its walk's expansions
+    int probe(uint64_t L, bool tight) const {
+        const int N = e.N;
+        uint32_t kept = 0;
+        for (int p = 0; p < N; ++p) {
+            const int b = p ? (int)td_nib(L, p - 1) + 1 : 0, q = p ? p - 1 : N - 1;
+            const int a = q ? (int)td_nib(L, q - 1) + 1 : 0;
+            if (b != (a + 1) % N) kept |= 1u << b;
+        }
+        const int n = td_popc(kept);
+        if (n > TD_EG_SYMBOLS) return -1;
+        if (n == 0 || !tight) return 0;
+        return table[td_eg_base(n - 1) + td_eg_rank(L, kept)];
+    }
+    int decide(uint64_t L, int off, int spare, const Child &c) const {
+        if (spare < 0) return -1;
+        uint64_t nL;
+        int noff;
+        td_apply_move(L, off, e.N, c.move & 31, (c.move >> 5) & 31, (c.move >> 10) & 31, &nL, &noff);
+        return probe(nL, c.plus2 ? spare == 0 : spare == 1);
+    }
+
+    // A walk from (L, off) at depth d0, path[0 .. d0-1] before it; its own record
+    // (status, expansions, moves), the nodes it was split into joined.
+    td_result walk(uint64_t L0, int off0, int d0, const uint16_t *before, int after) {
+        std::vector<Child> kids[TD_MAX_DEPTH];  // still to visit, the next one last
+        int spare[TD_MAX_DEPTH];                // -1: the table drops no child
+        uint64_t L[TD_MAX_DEPTH + 1];
+        int off[TD_MAX_DEPTH + 1];
+        uint16_t path[TD_MAX_DEPTH];
+        for (int d = 0; d < d0; ++d) path[d] = before[d];
+        std::vector<Node> nodes;
+        td_result r;
+        memset(&r, 0, sizeof r);
+        uint64_t exp = 0;
+        int level = d0, since = 0;
+        bool due = false;
+        L[d0] = L0;
+        off[d0] = off0;
+        auto record = [&](uint16_t last) {
+            r.status = TD_FOUND;
+            r.depth = level + 1;
+            for (int d = 0; d < level; ++d) r.moves[d] = path[d];
+            r.moves[level] = last;
+        };
+        for (bool done = false; !done;) {
+            const int odd = prepare(e, L[level], off[level]);
+            uint32_t fixed;
+            td_pinned_cycles(L[level], off[level], e.N, &fixed);
+            const int sp = eg_moves - level - ((e.N - odd) >> 1);
+            spare[level] = eg_moves > level + 1 && sp >= 0 && sp < 2 && e.N - td_popc(fixed) <= TD_EG_SYMBOLS + 3 ? sp : -1;
+            const int found = evaluate(e, level, odd);
+            ++exp;
+            auto move_of = [&](int u) {
+                const int t = e.T - 1 - u;
+                return td_pack_move(e.tri_i[t], e.tri_j[t], e.tri_k[t]);
+            };
+            if (found >= 0) {
+                record(move_of(found));
+                break;
+            }
+            kids[level].clear();
+            for (;;) {
+                Child c;
+                int accepted;
+                const int u = next_child(e, level, &accepted);
+                if (u < 0) break;
+                c.move = move_of(u);
+                c.accepted = accepted != 0;
+                uint64_t nL;
+                int noff;
+                uint32_t f;
+                td_apply_move(L[level], off[level], e.N, c.move & 31, (c.move >> 5) & 31, (c.move >> 10) & 31, &nL, &noff);
+                c.plus2 = td_pinned_cycles(nL, noff, e.N, &f) == odd + 2;
+                kids[level].insert(kids[level].begin(), c);
+            }
+            if (due) {
+                due = false;
+                split(nodes, kids, spare, L, off, path, d0, level);
+            }
+            for (;;) {
+                while (spare[level] >= 0 && !kids[level].empty()) {
+                    const int v = decide(L[level], off[level], spare[level], kids[level].back());
+                    if (v <= 0) break;
+                    exp += (uint64_t)v;
+                    kids[level].pop_back();
+                }
+                if (kids[level].empty()) {
+                    if (level == d0) { done = true; break; }
+                    --level;
+                    continue;
+                }
+                const Child c = kids[level].back();
+                kids[level].pop_back();
+                if (c.accepted) {
+                    record(c.move);
+                    done = true;
+                    break;
+                }
+                path[level] = c.move;
+                td_apply_move(L[level], off[level], e.N, c.move & 31, (c.move >> 5) & 31, (c.move >> 10) & 31,
+                              &L[level + 1], &off[level + 1]);
+                break;
+            }
+            if (done) break;
+            if (exp >= (uint64_t)after && ++since >= check_every) {
+                since = 0;
+                due = true;
+            }
+            ++level;
+        }
+        // the walk's record is rank 0 of its last node, whose join is rank 0 of the one before
+        for (size_t k = nodes.size(); k-- > 0 && r.status != TD_FOUND;) {
+            const Node &nd = nodes[k];
+            for (const Rec &q : nd.recs) {
+                if (!q.item) {
+                    exp += q.exp;
+                    continue;
+                }
+                uint16_t p[TD_MAX_DEPTH];
+                for (int d = 0; d < nd.depth; ++d) p[d] = nd.path[d];
+                p[nd.depth] = q.move;
+                if (q.accepted) {
+                    r.status = TD_FOUND;
+                    r.depth = 1;
+                    r.moves[0] = q.move;
+                    break;
+                }
+                uint64_t nL;
+                int noff;
+                td_apply_move(nd.L, nd.off, e.N, q.move & 31, (q.move >> 5) & 31, (q.move >> 10) & 31, &nL, &noff);
+                const td_result sub = walk(nL, noff, nd.depth + 1, p, split_after / 8);
+                exp += sub.expansions;
+                if (sub.status == TD_FOUND) {
+                    r = sub;
+                    break;
+                }
+            }
+        }
+        r.expansions = (uint32_t)exp;
+        return r;
+    }
+
+    void split(std::vector<Node> &nodes, std::vector<Child> *kids, const int *spare, const uint64_t *L, const int *off,
+               const uint16_t *path, int d0, int level) {
+        int lv = d0;
+        while (lv <= level && kids[lv].empty()) ++lv;
+        if (lv > level) return;
+        const int own = lv == level ? 1 : 0;
+        Node nd;
+        int units = 0, rank = 0;
+        for (size_t q = kids[lv].size(); q-- > 0; ++rank) {
+            const Child &c = kids[lv][q];
+            const int v = c.accepted ? 0 : decide(L[lv], off[lv], spare[lv], c);
+            if (rank >= own) {
+                nd.recs.push_back(Rec{v <= 0, c.accepted, v > 0 ? (uint32_t)v : 0u, c.move});
+                units += v <= 0;
+            }
+            if (v == 0) break;  // the walk gets no further
+        }
+        if (units == 0) {  // they count where the walk gets to them
+            kept += !nd.recs.empty();
+            return;
+        }
+        nd.depth = lv;
+        nd.L = L[lv];
+        nd.off = off[lv];
+        for (int q = 0; q < lv; ++q) nd.path[q] = path[q];
+        if (own) kids[lv].erase(kids[lv].begin(), kids[lv].end() - 1);
+        else kids[lv].clear();
+        nodes.push_back(nd);
+        ++splits;
+    }
+};
+
+}  // namespace
+
+// A reference-order search whose walks are split as td_ordered_kernel splits
+// them while warps wait: from `split_after` expansions on, every `check_every`
+// of them.  `table`: td_emu_endgame's, for 11 symbols.  counts: the nodes made,
+// and how often a level kept its children since the table decides them all.
+extern "C" int td_emu_split_search(const td_instance *x, const uint16_t *table, int split_after, int check_every,
+                                   td_result *res, long *counts) {
+    static thread_local SplitEmu s;
+    Emu &e = s.e;
+    e.N = x->n_symbols;
+    e.maxd = x->max_moves;
+    e.ordered = 1;
+    e.T = td_triple_count(e.N);
+    e.steps = (e.T + 31) / 32;
+    int t = 0;
+    for (int i = 0; i < e.N - 2; ++i)
+        for (int j = i + 1; j < e.N - 1; ++j)
+            for (int k = j + 1; k < e.N; ++k) { e.tri_i[t] = i; e.tri_j[t] = j; e.tri_k[t] = k; ++t; }
+    for (int idx = 0; idx < 4096; ++idx) e.lut[idx] = (uint8_t)td_class_of_index(idx);
+    const int init = td_inst_init(*x), full = td_inst_full(*x);
+    for (int D = 0; D <= TD_MAX_DEPTH + 1; ++D) {
+        e.acc[D] = e.reach[D] = 0;
+        for (int o = 0; o < 32; ++o) {
+            if (td_accepts(e.N, init, x->min_rate, full, o, D)) e.acc[D] |= 1u << o;
+            if (td_can_reach(e.N, init, x->min_rate, e.maxd, full, o, D)) e.reach[D] |= 1u << o;
+        }
+    }
+    s.table = table;
+    s.split_after = split_after;
+    s.check_every = check_every;
+    s.eg_moves = full && td_accepts(e.N, init, x->min_rate, 1, e.N, e.maxd) ? e.maxd : 0;
+    s.splits = s.kept = 0;
+    *res = s.walk(x->perm, x->offset, 0, nullptr, split_after);
+    counts[0] = s.splits;
+    counts[1] = s.kept;
+    return res->status;
+}

@@ -1173,7 +1173,7 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
         if constexpr (ORDERED) {
             if (due) {
                 due = false;
-                if (__shfl_sync(TD_FULL, waiting, 0) > 0) r.expansions += td_split(s, d0, level, N);
+                if (__shfl_sync(TD_FULL, waiting, 0) > 0) td_split(s, d0, level, N);
             }
         }
         if ((work & 255u) == 0) {

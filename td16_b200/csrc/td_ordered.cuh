@@ -114,9 +114,13 @@ __device__ __noinline__ void td_split_complete(const td_split_space &sp, int k) 
 // level] that has any (of `level` itself, whose node was just expanded, all but
 // the first).  Children that the endgame table decides become records at once,
 // and those after one that it knows to be sorted are dropped (the walk never
-// gets there).  Returns the expansions of the dropped walks where the table
-// decides all of them: no node is needed then.
-__device__ __noinline__ uint32_t td_split(td_warp_smem &s, int d0, int level, int N) {
+// gets there).  Where the table decides all of them the level keeps them: they
+// rank after the subtree that the walk is in, so they count only if the walk gets
+// to them.  (Counted at once they made the expansions of about one in a thousand
+// solved near-reverse instances of n = 13..15 too high.)  No deeper level is
+// looked at then: of 9,000 nodes made by walks of n = 12..14, in the host
+// restatement, one would lie below such a level.
+__device__ __noinline__ void td_split(td_warp_smem &s, int d0, int level, int N) {
     const int lane = threadIdx.x & 31;
     const td_split_space &sp = s.sp;
     int lv = d0;
@@ -125,7 +129,7 @@ __device__ __noinline__ uint32_t td_split(td_warp_smem &s, int d0, int level, in
         w = lane < TD_MAX_STEPS ? s.cw[lv][lane] : 0u;
         if (__ballot_sync(TD_FULL, w != 0)) break;
     }
-    if (lv > level) return 0;
+    if (lv > level) return;
     const int last_tri = td_tri_base(N) + td_triple_count(N) - 1;
     const int spare = s.spare[lv];  // 255: the table does not apply
     const uint32_t fixed = td_eg_fixed(s, lv, N);
@@ -134,7 +138,6 @@ __device__ __noinline__ uint32_t td_split(td_warp_smem &s, int d0, int level, in
     td_pack_state(s, lv, N, &L, &off);
     const int own = lv == level ? 1 : 0;  // children that this walk keeps
     int c = 0, units = 0;
-    uint32_t sum = 0;
     for (;;) {
         const int all = td_eg_list(s, lv);
         if (all == 0) break;
@@ -156,7 +159,6 @@ __device__ __noinline__ uint32_t td_split(td_warp_smem &s, int d0, int level, in
         const int got = yes ? __ffs(yes) : min(all, 32);
         const bool mine = lane < got && c + lane >= own;
         units += __popc(__ballot_sync(TD_FULL, mine && (e == 0 || e == TD_EG_UNKNOWN)));
-        sum += __reduce_add_sync(TD_FULL, mine && e != TD_EG_UNKNOWN ? e : 0u);
         c += got;
         __syncwarp();
         if (yes) break;
@@ -208,14 +210,13 @@ __device__ __noinline__ uint32_t td_split(td_warp_smem &s, int d0, int level, in
         }
     }
     base = __shfl_sync(TD_FULL, base, 0);
-    if (units > 0 && base < 0) {  // no room: the walk keeps its children
+    if (base < 0) {  // all decided, or no room: the walk keeps its children
         if (lane < TD_MAX_STEPS) s.cw[lv][lane] = w;
         __syncwarp();
-        return 0;
+        return;
     }
     if (lane < TD_MAX_STEPS) s.cw[lv][lane] = keep;
     __syncwarp();
-    if (units == 0) return sum;
     first = __shfl_sync(TD_FULL, first, 0);
     k = __shfl_sync(TD_FULL, k, 0);
     // until the join, the instance reads as timed out
@@ -250,5 +251,4 @@ __device__ __noinline__ uint32_t td_split(td_warp_smem &s, int d0, int level, in
         s.sp_rank = 0;
     }
     __syncwarp();
-    return 0;
 }
