@@ -819,3 +819,10 @@ extern "C" int td_emu_split_search(const td_instance *x, const uint16_t *table, 
     counts[1] = s.kept;
     return res->status;
 }
+
+// The expansion counts, budgets and statuses of the kernels (td_core.cuh).
+extern "C" uint32_t td_emu_add_count(uint32_t a, uint32_t b) { return td_add_count(a, b); }
+extern "C" int td_emu_over_budget(uint32_t count, uint64_t max_expansions) {
+    return td_over_budget(count, td_budget(max_expansions));
+}
+extern "C" int td_emu_status_of_dfs(int dfs) { return td_status_of_dfs(dfs); }

@@ -66,6 +66,13 @@ struct td_result {
 
 #define TD_FLAG_ORDERED 1u  // reproduce the reference's single-queue move order
 
+// How a warp's walk of a subtree ended.
+#define TD_DFS_FOUND 1
+#define TD_DFS_EXHAUSTED 0
+#define TD_DFS_BUDGET (-2)
+#define TD_DFS_TIMEOUT (-5)
+#define TD_DFS_ABORTED (-7)
+
 // ---- small helpers ---------------------------------------------------------
 
 TD_HD int td_triple_count(int n) { return n < 3 ? 0 : n * (n - 1) * (n - 2) / 6; }
@@ -119,6 +126,29 @@ TD_HD void td_apply_move(uint64_t L, int off, int N, int i, int j, int k,
         S = e + 1;
     }
     *outOff = S;
+}
+
+// ---- expansion counts -------------------------------------------------------
+//
+// A count saturates at 2^32 - 1.  Budgets have 64 bits, so that no count reaches
+// TD_NO_BUDGET, a saturated one included: a search without a budget never ends
+// by it.
+
+#define TD_NO_BUDGET (~0ull)
+
+TD_HD uint32_t td_add_count(uint32_t a, uint32_t b) { return a + b < a ? ~0u : a + b; }
+
+TD_HD uint64_t td_budget(uint64_t max_expansions) { return max_expansions ? max_expansions : TD_NO_BUDGET; }
+
+TD_HD bool td_over_budget(uint32_t count, uint64_t budget) { return count >= budget; }
+
+// The result status of a walk that ran by itself.  "Not found" is only said of
+// one searched to its end.
+TD_HD int td_status_of_dfs(int dfs) {
+    return dfs == TD_DFS_FOUND       ? TD_FOUND
+           : dfs == TD_DFS_EXHAUSTED ? TD_NOT_FOUND
+           : dfs == TD_DFS_BUDGET    ? TD_ERR_BUDGET
+                                     : TD_ERR_TIMEOUT;
 }
 
 // ---- triple classification -------------------------------------------------

@@ -81,7 +81,7 @@ __device__ __forceinline__ void td_wait_predecessor() { asm volatile("griddepcon
 __device__ __forceinline__ void td_set_limits(td_warp_smem &s, uint64_t max_exp, uint64_t time_limit_ns) {
     if ((threadIdx.x & 31) == 0) {
         td_search_limits lim;
-        lim.max_expansions = max_exp && max_exp < ~0u ? (uint32_t)max_exp : ~0u;
+        lim.max_expansions = td_budget(max_exp);
         lim.split_after = ~0u;
         lim.deadline_ns = time_limit_ns ? td_globaltimer() + time_limit_ns : 0;
         lim.tt = nullptr;
@@ -349,9 +349,7 @@ __global__ void __launch_bounds__(256, 4) td_ordered_kernel(const td_instance *_
                 r = td_dfs<true>(s, N, d0, true);
             }
         }
-        int status = r.status == TD_DFS_FOUND ? TD_FOUND
-                     : r.status == TD_DFS_TIMEOUT ? TD_ERR_TIMEOUT
-                     : r.status == TD_DFS_ABORTED ? TD_SPLIT_SKIPPED : TD_NOT_FOUND;
+        int status = r.status == TD_DFS_ABORTED ? TD_SPLIT_SKIPPED : td_status_of_dfs(r.status);
         if (kind == 1 && !td_instance_ok(x)) status = TD_ERR_ARG;
         __syncwarp();
         node = s.sp_node;  // the walk may have been split
@@ -401,10 +399,7 @@ __device__ __forceinline__ int td_finish_unit(const td_dfs_out &r, td_inst_state
                                               const uint16_t *path, int side, int gave) {
     const int lane = threadIdx.x & 31;
     if (!gave) {  // a root search by itself: its outcome is the instance's
-        const int status = r.status == TD_DFS_FOUND     ? TD_FOUND
-                           : r.status == TD_DFS_TIMEOUT ? TD_ERR_TIMEOUT
-                           : r.status == TD_DFS_BUDGET  ? TD_ERR_BUDGET
-                                                        : TD_NOT_FOUND;
+        const int status = td_status_of_dfs(r.status);
         td_write_result(out, status, status == TD_FOUND ? r.depth : 0, r.found_move, path, r.expansions, 0, 8);
         __syncwarp();
         if (HOST_OUT && lane == 0) __threadfence_system();

@@ -27,7 +27,7 @@
 
 // Limits and tables of the search a warp runs.
 struct td_search_limits {
-    uint32_t max_expansions;   // per search; TD_ERR_BUDGET when exceeded (~0: none)
+    uint64_t max_expansions;   // per search; TD_ERR_BUDGET when reached (td_budget)
     uint32_t split_after;      // a walk of the reference order may be split after this many expansions
     uint64_t deadline_ns;      // %globaltimer value; 0 = none
     ulonglong2 *tt;            // the launch's table of explored states (free order); null = none
@@ -761,12 +761,6 @@ __device__ __forceinline__ bool td_tt_visit(const td_warp_smem &s, int lv, int N
 
 #include "td_endgame.cuh"
 
-#define TD_DFS_FOUND 1
-#define TD_DFS_EXHAUSTED 0
-#define TD_DFS_BUDGET (-2)
-#define TD_DFS_TIMEOUT (-5)
-#define TD_DFS_ABORTED (-7)
-
 struct td_dfs_out {
     int status;
     int depth;
@@ -1108,7 +1102,7 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
                 found = td_evaluate_rows(s, N, level, odd, O, F);
             }
             ++work;
-            if constexpr (ORDERED) ++r.expansions;
+            if constexpr (ORDERED) r.expansions = td_add_count(r.expansions, 1u);
             else r.expansions = work;
             if (found >= 0) {
                 r.found_move = (uint16_t)found;
@@ -1126,7 +1120,7 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
                 }
             }
         }
-        if (r.expansions >= s.lim.max_expansions) {
+        if (td_over_budget(r.expansions, s.lim.max_expansions)) {
             r.status = TD_DFS_BUDGET;
             break;
         }
@@ -1202,9 +1196,9 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
                     // the walk of the children dropped here ends without a
                     // witness; a budget that it would exhaust ends it there
                     const uint32_t skipped = td_eg_skip(s, level, N, spare);
-                    r.expansions = r.expansions + skipped < r.expansions ? ~0u : r.expansions + skipped;
-                    if (skipped && r.expansions >= s.lim.max_expansions) {
-                        r.expansions = s.lim.max_expansions;
+                    r.expansions = td_add_count(r.expansions, skipped);
+                    if (skipped && td_over_budget(r.expansions, s.lim.max_expansions)) {
+                        r.expansions = (uint32_t)s.lim.max_expansions;
                         walk = 3;
                         break;
                     }
@@ -1344,14 +1338,10 @@ __device__ int td_warp_search(const td_instance &x, td_result *out, td_warp_smem
         td_setup_root(s, x);
         const td_dfs_out r = td_dfs<ORDERED>(s, x.n_symbols, 0, false);
         expansions = r.expansions;
-        if (r.status == TD_DFS_FOUND) {
-            status = TD_FOUND;
+        status = td_status_of_dfs(r.status);
+        if (status == TD_FOUND) {
             depth = r.depth;
             found_move = r.found_move;
-        } else if (r.status == TD_DFS_BUDGET) {
-            status = TD_ERR_BUDGET;
-        } else if (r.status == TD_DFS_TIMEOUT) {
-            status = TD_ERR_TIMEOUT;
         }
     }
     __syncwarp();

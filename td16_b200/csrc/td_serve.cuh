@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
     td_warp_smem &s = ws[warp];
     if (lane == 0) {
         td_search_limits lim;
-        lim.max_expansions = max_exp && max_exp < ~0u ? (uint32_t)max_exp : ~0u;
+        lim.max_expansions = td_budget(max_exp);
         lim.split_after = ~0u;
         lim.deadline_ns = deadline;
         lim.tt = ALL_ORDERED ? nullptr : tt;
