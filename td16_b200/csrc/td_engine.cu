@@ -1057,17 +1057,28 @@ int launch_cfg(int device, LaunchCfg *c, char *err, size_t errlen) {
     return TD_OK;
 }
 
-// Fills the endgame table (td_endgame.cuh) of the current device, once per
-// device and process: five launches, on a stream of their own so that they
-// wait for nothing else.
-constexpr int kEndgameDevices = 64;
-std::mutex g_eg_mu;
-bool g_eg_ready[kEndgameDevices];
+// Fills the tables of the current device, once per device and process: the
+// triple and pair-slot tables are uploaded and the endgame table
+// (td_endgame.cuh) is built from them in five launches, all on one stream of
+// their own, so that they wait for nothing else and each finds what it reads,
+// and waited for.  No heap.
+constexpr int kTableDevices = 64;
+std::mutex g_tables_mu;
+bool g_tables_ready[kTableDevices];
+uint16_t g_tri[TD_TRI_TABLE];
+td_pair_row g_pair_rows[TD_MAX_N + 1][32];
 
-cudaError_t endgame_setup(int device, int sms) {
-    if (device < 0 || device >= kEndgameDevices) return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> g(g_eg_mu);
-    if (g_eg_ready[device]) return cudaSuccess;
+cudaError_t tables_setup(int device, int sms) {
+    if (device < 0 || device >= kTableDevices) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> g(g_tables_mu);
+    if (g_tables_ready[device]) return cudaSuccess;
+    for (int N = 0; N <= TD_MAX_N; ++N) {
+        int t = td_tri_base(N);
+        for (int i = 0; i < N - 2; ++i)
+            for (int j = i + 1; j < N - 1; ++j)
+                for (int k = j + 1; k < N; ++k) g_tri[t++] = td_pack_move(i, j, k);
+        for (int lane = 0; lane < 32; ++lane) g_pair_rows[N][lane] = td_make_pair_row(N, lane);
+    }
     uint32_t bases[TD_EG_SYMBOLS], factorial[TD_EG_SYMBOLS];
     for (int m = 0; m < TD_EG_SYMBOLS; ++m) {
         bases[m] = td_eg_base(m);
@@ -1078,6 +1089,9 @@ cudaError_t endgame_setup(int device, int sms) {
     if (e != cudaSuccess) return e;
     const size_t smem = smem_bytes(8);
     e = cudaFuncSetAttribute(td_eg_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(td_tri_table, g_tri, sizeof g_tri, 0, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyToSymbolAsync(td_pair_table, g_pair_rows, sizeof g_pair_rows, 0, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(td_eg_bases, bases, sizeof bases, 0, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
         e = cudaMemcpyToSymbolAsync(td_eg_factorial, factorial, sizeof factorial, 0, cudaMemcpyHostToDevice, st);
@@ -1088,16 +1102,8 @@ cudaError_t endgame_setup(int device, int sms) {
     const cudaError_t done = cudaStreamSynchronize(st);
     cudaStreamDestroy(st);
     if (e == cudaSuccess) e = done;
-    g_eg_ready[device] = e == cudaSuccess;
+    g_tables_ready[device] = e == cudaSuccess;
     return e;
-}
-
-// Uploads the kernels' pair-slot table to the current device.
-cudaError_t upload_pairs() {
-    td_pair_row rows[TD_MAX_N + 1][32];
-    for (int N = 0; N <= TD_MAX_N; ++N)
-        for (int lane = 0; lane < 32; ++lane) rows[N][lane] = td_make_pair_row(N, lane);
-    return cudaMemcpyToSymbol(td_pair_table, rows, sizeof rows);
 }
 
 int ensure_device(int device, char *err, size_t errlen) {
@@ -1105,15 +1111,6 @@ int ensure_device(int device, char *err, size_t errlen) {
     DeviceInfo &d = g_dev[device];
     if (d.ready) return TD_OK;
     TD_CHECK(cudaSetDevice(device));
-    std::vector<uint16_t> tri(TD_TRI_TABLE, 0);
-    for (int N = 3; N <= TD_MAX_N; ++N) {
-        int base = N < 4 ? 0 : N * (N - 1) * (N - 2) * (N - 3) / 24, t = 0;
-        for (int i = 0; i < N - 2; ++i)
-            for (int j = i + 1; j < N - 1; ++j)
-                for (int k = j + 1; k < N; ++k) tri[base + t++] = td_pack_move(i, j, k);
-    }
-    TD_CHECK(cudaMemcpyToSymbol(td_tri_table, tri.data(), tri.size() * sizeof(uint16_t)));
-    TD_CHECK(upload_pairs());
     TD_CHECK(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device));
     const int max_warps = 8;
     const size_t max_smem = smem_bytes(max_warps);
@@ -1124,7 +1121,7 @@ int ensure_device(int device, char *err, size_t errlen) {
     TD_CHECK(cudaFuncSetAttribute(td_ordered_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
     const int rc = preload_kernels(err, errlen);
     if (rc != TD_OK) return rc;
-    TD_CHECK(endgame_setup(device, d.sms));
+    TD_CHECK(tables_setup(device, d.sms));
     d.ready = true;
     return TD_OK;
 }
@@ -2070,23 +2067,13 @@ struct NoAllocDevice {
 
 std::mutex g_noalloc_mu;
 NoAllocDevice g_noalloc[kNoAllocDevices];
-uint16_t g_noalloc_tri[TD_TRI_TABLE];  // host copy of the device table, no heap
 
-// Once per device, with that device current: uploads the triple
-// table and takes the scratch array's device address.  In host code the
+// Once per device, with that device current: takes the scratch array's device
+// address and sets the device's tables up (tables_setup).  In host code the
 // name td_noalloc_scratch is only a host-side stand-in, never a device address.
 int noalloc_setup(int device, char *err, size_t errlen) {
     NoAllocDevice &d = g_noalloc[device];
     if (d.ready) return TD_OK;
-    for (int N = 3; N <= TD_MAX_N; ++N) {
-        int t = 0;
-        const int base = td_tri_base(N);
-        for (int i = 0; i < N - 2; ++i)
-            for (int j = i + 1; j < N - 1; ++j)
-                for (int k = j + 1; k < N; ++k) g_noalloc_tri[base + t++] = td_pack_move(i, j, k);
-    }
-    TD_CHECK_NA(cudaMemcpyToSymbol(td_tri_table, g_noalloc_tri, sizeof g_noalloc_tri));
-    TD_CHECK_NA(upload_pairs());
     void *ptr = nullptr;
     TD_CHECK_NA(cudaGetSymbolAddress(&ptr, td_noalloc_scratch));
     TD_CHECK_NA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device));
@@ -2102,7 +2089,7 @@ int noalloc_setup(int device, char *err, size_t errlen) {
                                                               smem_bytes(4)));
     TD_CHECK_NA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.persistent_blocks, td_persistent_kernel,
                                                               128, smem));
-    TD_CHECK_NA(endgame_setup(device, d.sms));
+    TD_CHECK_NA(tables_setup(device, d.sms));
     d.scratch = static_cast<uint8_t *>(ptr);
     d.ready = true;
     return TD_OK;

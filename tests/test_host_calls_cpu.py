@@ -1,0 +1,66 @@
+"""What the engine's host code asks of the CUDA runtime, seen by a runtime without
+a device (fake_cudart/fake_cudart.cc, preloaded into a child process)."""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+@pytest.fixture(scope="module")
+def calls(td, tmp_path_factory):
+    """Runs Python code in a child with the fake runtime; returns the log's lines."""
+    from td16_b200 import build
+    work = tmp_path_factory.mktemp("fake")
+    fake = str(work / "libfake_cudart.so")
+    include = os.path.join(os.path.dirname(os.path.dirname(shutil.which("nvcc") or build.nvcc())), "include")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I", include, "-o", fake,
+                    os.path.join(HERE, "fake_cudart", "fake_cudart.cc")], check=True)
+
+    def run(code):
+        log = str(work / "log")
+        if os.path.exists(log):
+            os.remove(log)
+        env = dict(os.environ, LD_PRELOAD=fake, FAKE_CUDART_LOG=log, PYTHONPATH=ROOT)
+        subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=120)
+        with open(log) as f:
+            return f.read().splitlines()
+
+    return run
+
+
+INIT = "import td16_b200 as td; td.init_slots(1, [0], 64 << 20)\n"
+NOALLOC = """
+import ctypes as C
+from td16_b200 import _lib
+err = C.create_string_buffer(256)
+buf = (C.c_uint8 * 64)()
+rc = _lib.lib().td_search_batch_noalloc(C.c_int(1), buf, buf, C.c_uint(0), C.c_uint64(0), None, err, C.c_size_t(256))
+assert rc == 0, err.value
+"""
+
+
+@pytest.mark.parametrize("code", [INIT, NOALLOC, INIT + NOALLOC, NOALLOC + INIT])
+def test_tables_are_on_the_device_before_a_kernel_reads_them(calls, code):
+    """The build of the endgame table reads the triple and pair tables on a stream
+    that waits for no other: they are uploaded on that stream, or their upload has
+    been waited for.  (An upload from pageable memory on the default stream may
+    return before it has arrived.)"""
+    arrived, pending, builds = set(), {}, 0
+    for line in calls(code):
+        what, *rest = line.split()
+        if what == "upload":
+            pending[rest[0]] = rest[2]
+            arrived.discard(rest[0])
+        elif what == "synchronize":
+            arrived |= {t for t, st in pending.items() if st == rest[1]}
+            pending = {t: st for t, st in pending.items() if st != rest[1]}
+        elif what == "launch" and "td_" in rest[0]:
+            builds += "td_eg_build" in rest[0]
+            for table in ("td_tri_table", "td_pair_table"):
+                assert table in arrived or pending.get(table) == rest[2], (line, table)
+    assert builds == 5  # one pass per number of missing moves, once per device
