@@ -112,7 +112,8 @@ struct td_donate_ctx {
     int attempt;            // the restart attempt that donated the unit (0 for a root)
     int gave;               // 0: a root search that has given nothing away (no other warp knows of it)
     int race;               // > 0: the unit queues its inverse when it starts restart attempt
-                            // `race` (root units of full-sorting instances in td_steal_kernel)
+                            // `race` (root units of full-sorting instances in td_steal_kernel),
+                            // and 0 once it has
 };
 
 // The buffers of a launch of the reference order whose walks may be split
@@ -912,7 +913,9 @@ __device__ __noinline__ int td_donate(td_warp_smem &s, int d0, int level, int N,
 // item, a root of the inverse's side, so that another warp searches it while
 // this one goes on; the first witness on either side ends both, and so does the
 // instance's side searched to the end without one (found = 2).  Only an
-// instance's root search queues its inverse, once.  In the batch engine items
+// instance's root search queues its inverse, and once: the race is off for it
+// from then on (a second inverse root would share the first one's entries in
+// the table of explored states).  In the batch engine items
 // are taken once no fresh instance is left, and the inverses queued until then
 // come first.  Returns whether it was queued (uniform across the warp).
 __device__ __noinline__ int td_spawn_inverse(td_warp_smem &s, int N) {
@@ -931,9 +934,11 @@ __device__ __noinline__ int td_spawn_inverse(td_warp_smem &s, int N) {
             for (int d = 0; d < TD_MAX_DEPTH; ++d) it.path[d] = 0;
             td_publish(dc, it, slot);
             atomicAdd(&dc.pool->races, 1ull);
+            s.dc.race = 0;
             ok = 1;
         }
     }
+    __syncwarp();
     return __shfl_sync(TD_FULL, ok, 0);
 }
 
