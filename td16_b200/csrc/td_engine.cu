@@ -892,7 +892,8 @@ struct Slot {
     int *d_ticket = nullptr;
     void *d_batch = nullptr;
     size_t d_batch_bytes = 0;
-    // the arrays of td_search_pairs on the device and pinned on the host
+    // the arrays of td_search_pairs on the device, and the pinned memory
+    // (kPairStage bytes) that their copies go through
     uint8_t *d_pairs = nullptr, *h_pairs = nullptr;
     size_t pairs_bytes = 0;
     // donation scratch: pool counters, item array + ready flags, instance state
@@ -1356,6 +1357,30 @@ td_pair_arrays pair_arrays(uint8_t *base, size_t c) {
     a.depth = a.status + c;
     a.ijk = (int16_t *)(a.depth + c);
     return a;
+}
+
+// Pinned memory of a slot that td_search_pairs' copies go through: allocated at
+// the slot's first such call and kept until the slot goes, so that no later call
+// pins or frees host memory, which may wait for all work on the device.  65,536
+// pairs (the pair consumer's default batch) go in one piece each way.
+constexpr size_t kPairStage = 4u << 20;
+
+// A stretch of the arrays of a call and the caller's memory for it.
+struct PairPart {
+    size_t at, bytes;
+    char *host;
+};
+
+// Copies what [from, from + bytes) holds of `parts` between the pinned memory,
+// which holds that range, and the caller's arrays.
+void stage_parts(const PairPart *parts, int count, size_t from, size_t bytes, uint8_t *stage, bool in) {
+    for (int i = 0; i < count; ++i) {
+        const size_t a = std::max(from, parts[i].at), b = std::min(from + bytes, parts[i].at + parts[i].bytes);
+        if (a >= b) continue;
+        char *host = parts[i].host + (a - parts[i].at);
+        if (in) std::memcpy(stage + (a - from), host, b - a);
+        else std::memcpy(host, stage + (a - from), b - a);
+    }
 }
 
 Slot *get_slot(int slot, char *err, size_t errlen) {
@@ -1881,44 +1906,50 @@ TD_API int td_search_pairs(int slot, int count, const uint8_t *beta, const uint8
     TD_CHECK(cudaSetDevice(s->device));
     const size_t c = (size_t)count;
     const size_t in_bytes = pairs_in_bytes(c), bytes = in_bytes + pairs_out_bytes(c);
+    if (!s->h_pairs) TD_CHECK(cudaMallocHost(&s->h_pairs, kPairStage));
     if (bytes > s->pairs_bytes) {  // grows in stream order (no device-wide wait)
         if (s->d_pairs) TD_CHECK(cudaFreeAsync(s->d_pairs, s->stream));
-        if (s->h_pairs) {
-            TD_CHECK(cudaStreamSynchronize(s->stream));
-            TD_CHECK(cudaFreeHost(s->h_pairs));
-        }
-        s->d_pairs = s->h_pairs = nullptr;
+        s->d_pairs = nullptr;
         s->pairs_bytes = 0;
         TD_CHECK(cudaMallocAsync(&s->d_pairs, bytes, s->stream));
-        TD_CHECK(cudaMallocHost(&s->h_pairs, bytes));
         s->pairs_bytes = bytes;
     }
     int rc = ensure_batch(*s, c, err, errlen);
     if (rc != TD_OK) return rc;
     td_instance *d_in = (td_instance *)s->d_batch;
     td_result *d_out = (td_result *)((char *)s->d_batch + c * sizeof(td_instance));
-    const td_pair_arrays h = pair_arrays(s->h_pairs, c), d = pair_arrays(s->d_pairs, c);
-    std::memcpy(h.beta, beta, c * TD_MAX_N);
-    std::memcpy(h.omega, omega, c * TD_MAX_N);
-    std::memcpy(h.n, n, c);
-    std::memcpy(h.full, full, c);
-    std::memcpy(h.init, init, c * sizeof *init);
-    std::memcpy(h.rate, min_rate, c * sizeof *min_rate);
-    std::memcpy(h.max_moves, max_moves, c * sizeof *max_moves);
-    TD_CHECK(cudaMemcpyAsync(s->d_pairs, s->h_pairs, in_bytes, cudaMemcpyHostToDevice, s->stream));
+    const td_pair_arrays d = pair_arrays(s->d_pairs, c);
+    auto part = [&](const void *device, const void *host, size_t n) {
+        return PairPart{(size_t)((const uint8_t *)device - s->d_pairs), n, (char *)host};
+    };
+    const PairPart ins[] = {part(d.init, init, c * sizeof *init),
+                            part(d.max_moves, max_moves, c * sizeof *max_moves),
+                            part(d.rate, min_rate, c * sizeof *min_rate),
+                            part(d.beta, beta, c * TD_MAX_N),
+                            part(d.omega, omega, c * TD_MAX_N),
+                            part(d.n, n, c),
+                            part(d.full, full, c)};
+    const PairPart outs[] = {part(d.status, status, c * sizeof *status), part(d.depth, depth, c * sizeof *depth),
+                             part(d.ijk, out_ijk, 27 * c * sizeof *out_ijk)};
+    for (size_t at = 0; at < in_bytes; at += kPairStage) {
+        const size_t m = std::min(kPairStage, in_bytes - at);
+        if (at) TD_CHECK(cudaStreamSynchronize(s->stream));  // the piece before has left the pinned memory
+        stage_parts(ins, 7, at, m, s->h_pairs, true);
+        TD_CHECK(cudaMemcpyAsync(s->d_pairs + at, s->h_pairs, m, cudaMemcpyHostToDevice, s->stream));
+    }
     td_pairs_prepare_kernel<<<(count + 127) / 128, 128, 0, s->stream>>>(d, d_in, count);
     TD_CHECK(cudaGetLastError());
     rc = launch_batch(*s, count, d_in, d_out, flags & TD_FLAG_ORDERED, 0, s->stream, err, errlen);
     if (rc != TD_OK) return rc;
     td_pairs_unpack_kernel<<<(unsigned)((27 * c + 255) / 256), 256, 0, s->stream>>>(d, d_out, count);
     TD_CHECK(cudaGetLastError());
-    TD_CHECK(cudaMemcpyAsync(s->h_pairs + in_bytes, s->d_pairs + in_bytes, bytes - in_bytes, cudaMemcpyDeviceToHost,
-                             s->stream));
-    TD_CHECK(cudaEventRecord(s->done, s->stream));
-    TD_CHECK(cudaEventSynchronize(s->done));
-    std::memcpy(status, h.status, c * sizeof *status);
-    std::memcpy(depth, h.depth, c * sizeof *depth);
-    std::memcpy(out_ijk, h.ijk, 27 * c * sizeof *out_ijk);
+    for (size_t at = in_bytes; at < bytes; at += kPairStage) {
+        const size_t m = std::min(kPairStage, bytes - at);
+        TD_CHECK(cudaMemcpyAsync(s->h_pairs, s->d_pairs + at, m, cudaMemcpyDeviceToHost, s->stream));
+        TD_CHECK(cudaEventRecord(s->done, s->stream));
+        TD_CHECK(cudaEventSynchronize(s->done));
+        stage_parts(outs, 3, at, m, s->h_pairs, false);
+    }
     return TD_OK;
 }
 

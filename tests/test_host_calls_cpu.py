@@ -64,3 +64,22 @@ def test_tables_are_on_the_device_before_a_kernel_reads_them(calls, code):
             for table in ("td_tri_table", "td_pair_table"):
                 assert table in arrived or pending.get(table) == rest[2], (line, table)
     assert builds == 5  # one pass per number of missing moves, once per device
+
+
+def test_pairs_pin_host_memory_once(calls):
+    """Groups of pairs that grow from call to call: one pinned block of bounded
+    size per slot, pinned by the first call."""
+    lines = calls(INIT + """
+import numpy as np
+for slot_calls in range(2):
+    for count in (1, 10, 11, 1000, 70000, 200003):
+        pair = np.tile(np.arange(17, dtype=np.uint8), (count, 1))
+        td._lib.search_pairs(0, pair, pair, 17, 1, 0.0, 9, 1)
+td.init_slots(2, [0], 64 << 20)
+td._lib.search_pairs(1, pair, pair, 17, 1, 0.0, 9, 1)
+""")
+    prepared = [i for i, line in enumerate(lines) if "td_pairs_prepare" in line]
+    assert len(prepared) == 13
+    pinned = [int(line.split()[1]) for line in lines[: prepared[11]] if line.startswith("hostalloc")]
+    assert sum(pinned) <= 5 << 20
+    assert not [line for line in lines[prepared[0]: prepared[11]] if line.startswith("host")]
