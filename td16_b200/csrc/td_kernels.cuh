@@ -530,7 +530,11 @@ __device__ __forceinline__ int td_next_child_rows(td_warp_smem &s, int level, ui
 // (1.32 -> 1.21 ms); uniform S_16, which are short, lose what they win (3.50 and
 // 3.53 ms).  Only a root search's first attempt uses it: later attempts live on
 // other orders (with it in every second one 19.7 ms), and a subtree given away
-// is mostly searched to its end.  Called: inlined, it made every search slower.
+// is mostly searched to its end.  Where the table does not apply (partial
+// sorting, a rate that the bound does not meet) there is nothing to win: the
+// batch engine's partial sorting takes the same time with and without it, and
+// td_plain_kernel's, whose one attempt is the whole search, 1.71 ms without and
+// 1.86 with it (3,001 of n = 8..12).  Called: inlined, it made every search slower.
 __device__ __noinline__ int td_take_fixing(td_warp_smem &s, int level, int N) {
     const int x = threadIdx.x & 31;
     int y = x;
@@ -1193,7 +1197,7 @@ __device__ __forceinline__ td_dfs_out td_dfs(td_warp_smem &s, int N, int d0, boo
         // children skipped through the tables, change no expansion count, so
         // the checks above run once per expansion
         int walk = 0;  // 1: the subtree is exhausted, 2: a root accepted on visit (ordered), 3: out of budget
-        for (bool fresh = !ORDERED && attempt + solved + d0 == 0;; fresh = false) {
+        for (bool fresh = !ORDERED && attempt + solved + d0 == 0 && s.eg_moves != 0;; fresh = false) {
             int t = -1;
             if constexpr (ORDERED) {
                 const int spare = s.spare[level];
