@@ -24,6 +24,10 @@ std::map<const void *, void *> &symbols() {
     static std::map<const void *, void *> m;
     return m;
 }
+std::map<cudaEvent_t, unsigned> &event_flags() {
+    static std::map<cudaEvent_t, unsigned> m;
+    return m;
+}
 std::mutex mu;
 struct {
     dim3 grid, block;
@@ -150,11 +154,18 @@ FAKE cudaError_t cudaStreamSynchronize(cudaStream_t s) {
 FAKE cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
 FAKE cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) { return handle(g); }
 FAKE cudaError_t cudaEventCreate(cudaEvent_t *e) { return handle(e); }
-FAKE cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return handle(e); }
+FAKE cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned flags) {
+    const cudaError_t r = handle(e);
+    event_flags()[*e] = flags;
+    return r;
+}
 FAKE cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 FAKE cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { *ms = 0; return cudaSuccess; }
 FAKE cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-FAKE cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+FAKE cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+    say("wait event %s", event_flags()[e] & cudaEventBlockingSync ? "blocking" : "spinning");
+    return cudaSuccess;
+}
 FAKE cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **, size_t, cudaStream_t s) {
     say("launch %s stream %zx", name(f), (size_t)s);
     return cudaSuccess;

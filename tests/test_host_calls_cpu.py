@@ -83,3 +83,17 @@ td._lib.search_pairs(1, pair, pair, 17, 1, 0.0, 9, 1)
     pinned = [int(line.split()[1]) for line in lines[: prepared[11]] if line.startswith("hostalloc")]
     assert sum(pinned) <= 5 << 20
     assert not [line for line in lines[prepared[0]: prepared[11]] if line.startswith("host")]
+
+
+def test_pairs_do_not_sleep_on_a_blocking_event(calls):
+    """The outputs come back through pinned memory, so their copy does not end the
+    wait by itself; a thread that sleeps until then wakes late."""
+    lines = calls(INIT + """
+import numpy as np
+pair = np.tile(np.arange(17, dtype=np.uint8), (16, 1))
+td._lib.search_pairs(0, pair, pair, 17, 1, 0.0, 9, 1)
+""")
+    lines = lines[[i for i, line in enumerate(lines) if "td_pairs_prepare" in line][0]:]
+    lines = lines[[i for i, line in enumerate(lines) if "td_pairs_unpack" in line][0]:]
+    assert "wait event blocking" not in lines
+    assert lines[1].startswith(("synchronize stream", "wait event spinning"))
