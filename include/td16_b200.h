@@ -213,7 +213,8 @@ int td_synth_perms(uint64_t seed, int count, int n_min, int n_max, int hard_pct,
  * max_expansions (all batch forms): 0 = no budget; otherwise a search that
  * expands more nodes without finding a witness ends with status -2 (budget).
  * In the free order the budget bounds each unit of work, i.e. the root search
- * and each subtree donated to another warp.  stats may be NULL; its totals are
+ * and each subtree donated to another warp; with a budget of at most the
+ * interval of td_configure_steal nothing is donated.  stats may be NULL; its totals are
  * reduced on the device. */
 int td_search_batch(int slot, int count, const td_instance *instances,
                     td_result *results, unsigned flags,

@@ -506,7 +506,13 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
         // mixed 1.69 -> 1.32, 8,000 S_13 1.16 -> 0.82).  With 21 (10^5 uniform
         // S_16) they took 0.79 ms, and 0.75 without: there the loads of the
         // idle checks are work that nothing waits for.
-        if (count <= TD_EAGER_UNITS * (int)(gridDim.x * (blockDim.x >> 5))) td_serve_idle_warps(s.dc);
+        // An expansion budget bounds each unit, so sharing multiplies it: where it
+        // ends before a search's first look at the idle warps, nothing is shared
+        // and it bounds the instance (16 expansions each, 4,096 of S_8..S_13:
+        // 0.25 ms and 23,000 expansions, shared 0.38 and 62,000).
+        if (count <= TD_EAGER_UNITS * (int)(gridDim.x * (blockDim.x >> 5)) &&
+            (max_exp == 0 || max_exp > (uint64_t)check_every))
+            td_serve_idle_warps(s.dc);
     }
     __syncwarp();
     // Race (`race` = a, 0: off): a root search of a full-sorting instance
