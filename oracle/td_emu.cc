@@ -826,3 +826,9 @@ extern "C" int td_emu_over_budget(uint32_t count, uint64_t max_expansions) {
     return td_over_budget(count, td_budget(max_expansions));
 }
 extern "C" int td_emu_status_of_dfs(int dfs) { return td_status_of_dfs(dfs); }
+
+// The numbers of launches and requests (td_core.cuh).
+extern "C" uint32_t td_emu_next_epoch(uint32_t last, uint32_t epochs, int *again) {
+    return td_next_epoch(last, epochs, again);
+}
+extern "C" uint64_t td_emu_request_number(uint64_t claimed, uint32_t low) { return td_request_number(claimed, low); }

@@ -294,6 +294,29 @@ TD_HD uint64_t td_tt_key(uint64_t L) {
     return (L & 0x00ffffffffffffffull) | (order << 56);
 }
 
+// ---- numbers of launches and searches ------------------------------------------
+//
+// Flags of items hold the epoch of the launch that wrote them, or its complement,
+// and entries of the table of explored states a number made of the epoch; neither
+// is cleared between launches.  Epochs have 31 bits, so that none is another's
+// complement, and when they start again (about 12 hours of launches of 20 us)
+// the flags and the table are cleared first.
+
+#define TD_EPOCH_MAX 0x7fffffffu
+
+// The epoch of a launch that takes `epochs` of them (its last one), after `last`;
+// *again is set where the numbers start again.
+TD_HD uint32_t td_next_epoch(uint32_t last, uint32_t epochs, int *again) {
+    *again = last > TD_EPOCH_MAX - epochs;
+    return *again ? epochs : last + epochs;
+}
+
+// A request's number from its low 32 bits, given how many requests were claimed
+// (it among them, and within the last 2^32 of them).
+TD_HD uint64_t td_request_number(uint64_t claimed, uint32_t low) {
+    return claimed - (uint32_t)((uint32_t)claimed - low);
+}
+
 // ---- endgame table ------------------------------------------------------------
 //
 // Index of a state whose fixed symbols are glued to their predecessors, for

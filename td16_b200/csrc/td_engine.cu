@@ -625,11 +625,18 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
 // Advances the launch epoch that tags donated items as written; a launch
 // replayed from a CUDA graph therefore never mistakes an item of an earlier
 // launch for one of its own.  A launch of more than 2^26 instances takes as
-// many epochs as it needs numbers in the table of explored states.
-__global__ void td_epoch_kernel(td_epoch *ep, unsigned epochs, td_pool *pool, int count, int *zeros, int n_zeros) {
+// many epochs as it needs numbers in the table of explored states.  Where the
+// epochs start again, the items' flags and the table are cleared (by this one
+// thread: it happens once in 2^31 launches).
+__global__ void td_epoch_kernel(td_epoch *ep, unsigned epochs, td_pool *pool, int count, int *zeros, int n_zeros,
+                                uint32_t *ready, int n_ready, ulonglong2 *tt, size_t n_tt) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const uint32_t e = ep->epoch + epochs;
-    ep->epoch = e >= epochs ? e : epochs;
+    int again;
+    ep->epoch = td_next_epoch(ep->epoch, epochs, &again);
+    if (again) {
+        for (int i = 0; i < n_ready; ++i) ready[i] = 0;
+        for (size_t i = 0; i < n_tt; ++i) tt[i] = make_ulonglong2(0ull, 0ull);
+    }
     ep->start_ns = td_globaltimer();
     td_pool p;
     memset(&p, 0, sizeof p);
@@ -1220,7 +1227,8 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
             TD_CHECK(cudaMalloc(&s.d_epoch, sizeof(td_epoch)));
             TD_CHECK(cudaMemsetAsync(s.d_epoch, 0, sizeof(td_epoch), stream));
         }
-        td_epoch_kernel<<<1, 1, 0, stream>>>(s.d_epoch, epochs, s.d_pool, count, nullptr, 0);
+        td_epoch_kernel<<<1, 1, 0, stream>>>(s.d_epoch, epochs, s.d_pool, count, nullptr, 0, s.d_ready, s.item_capacity,
+                                             s.d_tt, s.tt_log2 ? (size_t)1 << s.tt_log2 : 0);
         // item space: the slot budget (the reference's queue budget) less the
         // per-instance state, at 36 bytes per item (record + ready flag)
         if (s.d_items == nullptr) {
@@ -1288,7 +1296,8 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
             int *node_count = reinterpret_cast<int *>(s.d_split_pool + 1);
             td_epoch *epoch = reinterpret_cast<td_epoch *>(node_count + 2);
             // the node and record counts start at zero in every launch
-            td_epoch_kernel<<<1, 1, 0, stream>>>(epoch, 1u, s.d_split_pool, count, node_count, 2);
+            td_epoch_kernel<<<1, 1, 0, stream>>>(epoch, 1u, s.d_split_pool, count, node_count, 2, s.d_split_ready,
+                                                 s.split_records, nullptr, 0);
             if (cfg.split_records > s.split_records) {
                 if (s.d_split_ready) TD_CHECK(cudaFreeAsync(s.d_split_ready, stream));
                 if (s.d_nodes) TD_CHECK(cudaFreeAsync(s.d_nodes, stream));
@@ -2196,7 +2205,7 @@ TD_API int td_search_batch_noalloc(int count, const td_instance *d_instances, td
         }
         // the counters start afresh on every call; items
         // are tagged with a fresh epoch so an earlier call's items never count
-        td_epoch_kernel<<<1, 1, 0, st>>>(epoch, 1u, pool, count, nullptr, 0);
+        td_epoch_kernel<<<1, 1, 0, st>>>(epoch, 1u, pool, count, nullptr, 0, ready, TD_NOALLOC_ITEMS, nullptr, 0);
         // the whole resident grid (the scratch does not depend on its size):
         // warps without an instance of their own take donated subtrees, so a
         // small batch is spread over the GPU

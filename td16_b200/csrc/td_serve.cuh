@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
         lim.split_after = ~0u;
         lim.deadline_ns = deadline;
         lim.tt = ALL_ORDERED ? nullptr : tt;
-        lim.tt_id = 0;  // requests are numbered across the launches that share a table
+        lim.tt_id = 0;  // per unit: a request's number, across the launches that share a table
         lim.tt_shift = tt_shift;
         lim.restart_base = 0;
         lim.cutoff = lim.cutoff2 = nullptr;
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                     __threadfence();
                     atomicExch(&ready[phys], tag | 0x80000000u);
                 }
-                req = it.inst;
+                req = (long long)td_request_number(*(volatile unsigned long long *)&dctl->claimed, it.inst);
                 const unsigned slot = (unsigned)(req % ring_size);
                 const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(&queue[slot]));
                 const td_instance x = *reinterpret_cast<const td_instance *>(&v);
@@ -317,6 +317,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                     s.L[d0] = it.L;
                     s.off[d0] = it.off & 31;
                     for (int d = 0; d < d0; ++d) s.path[d] = it.path[d];
+                    s.lim.tt_id = (uint64_t)req & ~0xffffffffull;
                 }
                 __syncwarp();
                 int stop = 0;
@@ -345,6 +346,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 // of the per-call server with full sorting races the search of its
                 // inverse from restart attempt `race` (td_steal_kernel's race).
                 s.lim.restart_base = kind == 1 || d0 == 0 ? restart_base : 0;
+                s.lim.tt_id = (uint64_t)req & ~0xffffffffull;
                 // A request with a spare move mostly ends with a witness soon, and
                 // restarts find it best: it gives subtrees away as configured.
                 // One without must search a narrow tree to its end: the idle
