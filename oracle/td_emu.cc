@@ -10,7 +10,9 @@
 //     step bitmasks and the single-queue child order;
 //   free order: row masks and bit-sliced classes (td_row_classes), pair slots,
 //     the +2-first child order, the table of explored states and the restarts
-//     with their child orders (td_attempt_budget, td_level_order).
+//     with their child orders (td_attempt_budget, td_level_order), and, once
+//     td_emu_set_endgame has given it one, the endgame table with the moves that
+//     fix symbols first (td_eg_filter, td_eg_look, td_take_fixing).
 // It shares the kernel's helpers in td_core.cuh.  The product library does not
 // contain or call it.
 #include "../td16_b200/csrc/td_core.cuh"
@@ -32,6 +34,7 @@ struct Emu {
     uint32_t m1[TD_MAX_DEPTH + 1][32], m2[TD_MAX_DEPTH + 1][32];
     // free order (bit-sliced): rows by caller position, masks, pair slots, outcome words
     uint32_t S[32], G[32], P[32], O, F;
+    int next[32];  // next caller position along omega
     uint32_t pc[TD_MAX_ROUNDS][32];
     uint32_t pw[TD_MAX_DEPTH + 1][TD_MAX_ROUNDS][32];
     int rounds;
@@ -94,6 +97,7 @@ int prepare_rows(Emu &e, uint64_t L, int off) {
         const int y = (B[q] + 1) % N;
         nxt[c] = (pos[y] - off + N) % N;
     }
+    for (int c = 0; c < 32; ++c) e.next[c] = nxt[c];
     for (int c = 0; c < 32; ++c) {
         int m = c, x = nxt[c], l = 1;
         while (x != c) { if (x < m) m = x; x = nxt[x]; ++l; }
@@ -163,7 +167,7 @@ int evaluate_rows(Emu &e, int level, int odd) {
 // order (ord = 0) the highest pair slot R*lane + r (lexicographically smallest
 // pair) and the smallest k.  `ord` (td_order_variant) rotates the lane
 // priority, reverses the round order and takes the largest k first, as the
-// kernel does.  Returns the move or -1.
+// kernel does.  Returns the move, with bit 15 set for a 0 child, or -1.
 int next_child_rows(Emu &e, int level, uint32_t ord) {
     bool any2 = false;
     for (int lane = 0; lane < 32; ++lane)
@@ -184,7 +188,7 @@ int next_child_rows(Emu &e, int level, uint32_t ord) {
     const int b = (ord & 64u) ? 31 - __builtin_clz(w) : __builtin_ctz(w);
     e.pw[level][r][lane] &= ~(1u << b);
     const int k = any2 ? b + 1 : b - 15;
-    return (int)((e.pc[r][lane] & 1023u) | ((uint32_t)k << 10));
+    return (int)((e.pc[r][lane] & 1023u) | ((uint32_t)k << 10) | (any2 ? 0u : 0x8000u));
 }
 
 // Evaluate the children of the node at `level` (parent odd count `odd`).
@@ -298,7 +302,74 @@ uint32_t tt_next_gen(uint64_t *tt, uint32_t &counter) {
     return counter;
 }
 
-int search_rows(Emu &e, td_result *res) {
+const uint16_t *g_endgame = nullptr;  // td_emu_endgame's for TD_EG_SYMBOLS symbols, or none
+
+// What the endgame table says of the state L: -1 unknown, 0 sorted within the
+// moves left, else the expansions of its walk.  `tight`: no spare move.
+int endgame_probe(const uint16_t *table, int N, uint64_t L, bool tight) {
+    uint32_t kept = 0;
+    for (int p = 0; p < N; ++p) {
+        const int b = p ? (int)td_nib(L, p - 1) + 1 : 0, q = p ? p - 1 : N - 1;
+        const int a = q ? (int)td_nib(L, q - 1) + 1 : 0;
+        if (b != (a + 1) % N) kept |= 1u << b;
+    }
+    const int n = td_popc(kept);
+    if (n > TD_EG_SYMBOLS) return -1;
+    if (n == 0 || !tight) return 0;
+    return table[td_eg_base(n - 1) + td_eg_rank(L, kept)];
+}
+
+// The same for the child that `move` makes of the state of `level`.
+int endgame_child(const Emu &e, const uint16_t *table, int level, uint32_t move, bool tight) {
+    uint64_t nL;
+    int noff;
+    td_apply_move(e.L[level], e.off[level], e.N, move & 31, (move >> 5) & 31, (move >> 10) & 31, &nL, &noff);
+    return endgame_probe(table, e.N, nL, tight);
+}
+
+// td_eg_filter: a node without a spare move.  The first child that can be sorted
+// becomes its only one (returns true), else those that the table does not hold
+// stay.
+bool endgame_filter(Emu &e, int level) {
+    bool solved = false;
+    for (int lane = 0; lane < 32 && !solved; ++lane)
+        for (int r = e.rounds - 1; r >= 0 && !solved; --r)
+            for (uint32_t w = e.pw[level][r][lane]; w && !solved; w &= w - 1) {
+                const int b = __builtin_ctz(w);
+                const int v = endgame_child(e, g_endgame, level, (e.pc[r][lane] & 1023u) | ((uint32_t)(b + 1) << 10), true);
+                if (v == 0) {
+                    solved = true;
+                    for (int q = 0; q < e.rounds; ++q)
+                        for (int l = 0; l < 32; ++l) e.pw[level][q][l] = 0;
+                    e.pw[level][r][lane] = 1u << b;
+                } else if (v > 0) {
+                    e.pw[level][r][lane] &= ~(1u << b);
+                }
+            }
+    return solved;
+}
+
+// td_take_fixing: the move that fixes two symbols or three, of lowest position,
+// where it is among the +2 children of `level`; or -1.
+int take_fixing(Emu &e, int level) {
+    for (int x = 0; x < e.N; ++x) {
+        const int y = e.next[x], z = e.next[y];
+        if ((x < y) + (y < z) + (z < x) != 2) continue;
+        int c[3] = {x, y, z};
+        const int s = x < y && x < z ? 0 : y < z ? 1 : 2;
+        const int i = c[s], j = c[(s + 1) % 3], k = c[(s + 2) % 3];
+        for (int lane = 0; lane < 32; ++lane)
+            for (int r = 0; r < e.rounds; ++r)
+                if ((e.pc[r][lane] & 1023u) == (uint32_t)(i | j << 5) && ((e.pw[level][r][lane] >> (k - 1)) & 1u)) {
+                    e.pw[level][r][lane] &= ~(1u << (k - 1));
+                    return i | j << 5 | k << 10;
+                }
+        return -1;
+    }
+    return -1;
+}
+
+int search_rows(Emu &e, int eg_moves, td_result *res) {
     static thread_local uint64_t tt[1 << EMU_TT_BITS];  // zero-initialised: every word empty
     static thread_local uint32_t tt_counter = 0;
     bool tt_on = false;  // in use after 32 expansions, as in the kernel
@@ -309,9 +380,23 @@ int search_rows(Emu &e, td_result *res) {
     e.rounds = (NP + 31) / 32;
     for (int r = 0; r < TD_MAX_ROUNDS; ++r)
         for (int lane = 0; lane < 32; ++lane) e.pc[r][lane] = td_pair_code(e.N, r < e.rounds ? e.rounds * lane + r : -1);
-    int level = 0;
-    int odd = prepare_rows(e, e.L[0], e.off[0]);
-    int found = evaluate_rows(e, 0, odd);
+    if (!g_endgame) eg_moves = 0;
+    int level = 0, spare[TD_MAX_DEPTH];  // -1: the endgame table decides no child
+    bool solved = false;
+    int found = -1;
+    // expands the node at `level`, and lets the table decide its children
+    auto expand = [&] {
+        const int odd = prepare_rows(e, e.L[level], e.off[level]);
+        const int sp = eg_moves - level - ((e.N - odd) >> 1);
+        spare[level] = eg_moves > level + 1 && sp >= 0 && e.N - td_popc(e.F) <= TD_EG_SYMBOLS + 3 ? sp : -1;
+        found = evaluate_rows(e, level, odd);
+        if (found >= 0 || spare[level] != 0) return;
+        int children = 0;
+        for (int lane = 0; lane < 32; ++lane)
+            for (int r = 0; r < e.rounds; ++r) children += td_popc(e.pw[level][r][lane]);
+        if (children >= 8) solved |= endgame_filter(e, level);
+    };
+    expand();
     for (;;) {
         if (found >= 0) {
             for (int d = 0; d < level; ++d) res->moves[d] = e.path[d];
@@ -320,35 +405,48 @@ int search_rows(Emu &e, td_result *res) {
             res->status = TD_FOUND;
             break;
         }
-        if (attempt_exp >= attempt_budget) {
+        if (attempt_exp >= attempt_budget && !solved) {
             ++attempt;
             ord = td_order_variant(attempt);
             attempt_budget = td_attempt_budget(g_restart_base, attempt);
             attempt_exp = 1;
             if (tt_on) tt_gen = tt_next_gen(tt, tt_counter);  // the abandoned attempt's entries no longer match
             level = 0;
-            odd = prepare_rows(e, e.L[0], e.off[0]);
-            found = evaluate_rows(e, 0, odd);
+            expand();
             continue;
         }
-        const int t = next_child_rows(e, level, td_level_order(ord, attempt, level));
-        if (t < 0) {
-            if (level == 0) { res->status = TD_NOT_FOUND; break; }
-            --level;
-            continue;
+        bool done = false;
+        for (bool fresh = attempt + solved == 0 && eg_moves != 0;; fresh = false) {
+            int t = fresh ? take_fixing(e, level) : -1;
+            if (t < 0) t = next_child_rows(e, level, td_level_order(ord, attempt, level));
+            if (t < 0) {
+                if (level == 0) { done = true; break; }
+                --level;
+                continue;
+            }
+            e.path[level] = (uint16_t)(t & 0x7fff);
+            int noff;
+            td_apply_move(e.L[level], e.off[level], e.N, t & 31, (t >> 5) & 31, (t >> 10) & 31, &e.L[level + 1], &noff);
+            e.off[level + 1] = noff;
+            if (spare[level] >= 0) {
+                const int v = endgame_probe(g_endgame, e.N, e.L[level + 1], spare[level] == (t >> 15));
+                if (v == 0) {
+                    solved = true;
+                    break;
+                }
+                if (v > 0) continue;
+            }
+            if (solved) break;
+            if (!tt_on && e.expansions >= 32) {
+                tt_gen = tt_next_gen(tt, tt_counter);
+                tt_on = true;
+            }
+            if (tt_on && tt_visit(tt, e.L[level + 1], e.N, level + 1, tt_gen)) continue;  // explored with at least this budget
+            break;
         }
-        e.path[level] = (uint16_t)t;
-        int noff;
-        td_apply_move(e.L[level], e.off[level], e.N, t & 31, (t >> 5) & 31, (t >> 10) & 31, &e.L[level + 1], &noff);
-        e.off[level + 1] = noff;
-        if (!tt_on && e.expansions >= 32) {
-            tt_gen = tt_next_gen(tt, tt_counter);
-            tt_on = true;
-        }
-        if (tt_on && tt_visit(tt, e.L[level + 1], e.N, level + 1, tt_gen)) continue;  // explored with at least this budget
+        if (done) { res->status = TD_NOT_FOUND; break; }
         ++level;
-        odd = prepare_rows(e, e.L[level], e.off[level]);
-        found = evaluate_rows(e, level, odd);
+        expand();
         ++attempt_exp;
     }
     res->expansions = e.expansions;
@@ -384,6 +482,10 @@ extern "C" int td_emu_row_check(uint64_t L, int off, int N) {
     return bad;
 }
 
+// Gives later free-order searches the endgame table (td_emu_endgame's for
+// TD_EG_SYMBOLS symbols; it must outlive them), or takes it away (null).
+extern "C" void td_emu_set_endgame(const uint16_t *table) { g_endgame = table; }
+
 extern "C" int td_emu_search(const td_instance *x, unsigned flags, td_result *res) {
     static thread_local Emu e;
     memset(res, 0, sizeof *res);
@@ -410,7 +512,8 @@ extern "C" int td_emu_search(const td_instance *x, unsigned flags, td_result *re
     e.expansions = 0;
     e.L[0] = x->perm;
     e.off[0] = x->offset;
-    if (!e.ordered) return search_rows(e, res);
+    if (!e.ordered)
+        return search_rows(e, full && td_accepts(e.N, init, x->min_rate, 1, e.N, e.maxd) ? e.maxd : 0, res);
     int level = 0;
     int odd = prepare(e, e.L[0], e.off[0]);
     int found = evaluate(e, 0, odd);
@@ -606,26 +709,12 @@ struct SplitEmu {
     long splits = 0, kept = 0;  // nodes made, and levels that kept their children since the table decides them
     Emu e;
 
-    // what the table says of the state: -1 unknown, 0 sorted within the moves left, else its walk's expansions
-    int probe(uint64_t L, bool tight) const {
-        const int N = e.N;
-        uint32_t kept = 0;
-        for (int p = 0; p < N; ++p) {
-            const int b = p ? (int)td_nib(L, p - 1) + 1 : 0, q = p ? p - 1 : N - 1;
-            const int a = q ? (int)td_nib(L, q - 1) + 1 : 0;
-            if (b != (a + 1) % N) kept |= 1u << b;
-        }
-        const int n = td_popc(kept);
-        if (n > TD_EG_SYMBOLS) return -1;
-        if (n == 0 || !tight) return 0;
-        return table[td_eg_base(n - 1) + td_eg_rank(L, kept)];
-    }
     int decide(uint64_t L, int off, int spare, const Child &c) const {
         if (spare < 0) return -1;
         uint64_t nL;
         int noff;
         td_apply_move(L, off, e.N, c.move & 31, (c.move >> 5) & 31, (c.move >> 10) & 31, &nL, &noff);
-        return probe(nL, c.plus2 ? spare == 0 : spare == 1);
+        return endgame_probe(table, e.N, nL, c.plus2 ? spare == 0 : spare == 1);
     }
 
     // A walk from (L, off) at depth d0, path[0 .. d0-1] before it; its own record
