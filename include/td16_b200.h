@@ -53,7 +53,10 @@ typedef struct td_result {
     int32_t depth;        /* number of moves */
     uint16_t moves[9];
     uint16_t reserved;
-    uint32_t expansions;  /* nodes whose children were evaluated */
+    uint32_t expansions;  /* nodes whose children were evaluated; in the reference
+                             order the walk's nodes, those of subtrees that the
+                             endgame table decides unwalked included (2^32 - 1:
+                             that many or more) */
 } td_result;
 
 /* batch flags */

@@ -311,6 +311,10 @@ def set_time_limit(seconds: float) -> None:
 
 
 def configure_steal(grain: int, split_level: int, check_every: int) -> None:
+    """Work donation of free-order batches while every warp has an instance of
+    its own; from the first idle warps on (and from the start with at most 16
+    instances per warp) a warp gives 8 times as many items (at most 32), from 4
+    levels deeper, and checks 16 times as often."""
     if lib().td_configure_steal(int(grain), int(split_level), int(check_every)) != OK:
         raise TdError(INVALID_ARG, "invalid donation parameters")
 
@@ -336,9 +340,9 @@ def configure_race(attempt: int) -> None:
 
 
 def configure_split(first_pass_expansions: int = 64, records: int = 1 << 20) -> None:
-    """Reference-order batches: one-warp first pass of `first_pass_expansions`
-    (0 = no split), then walks left over split below the root into at most
-    `records` subtrees per launch.  Results do not depend on either."""
+    """Reference-order batches: a walk that has run for `first_pass_expansions`
+    (0 = never) gives subtrees away while warps wait, at most `records` of them
+    per launch.  Results do not depend on either."""
     if lib().td_configure_split(int(first_pass_expansions), int(records)) != OK:
         raise TdError(INVALID_ARG, "split settings: expansions >= 0, 1 <= records <= 2^24")
 

@@ -11,7 +11,10 @@ and then, with the winning shape, the restart budget base of the root searches
 base and the base swept once more, since restarts shorten the searches that
 the donation knobs were tuned for, and last the restart attempt from which a
 search races the search of its inverse permutation (0 = no race; the race
-needs restarts).  The fastest point by device time is kept,
+needs restarts).  The donation knobs are what a launch begins with: from the
+first idle warps on, and throughout a launch of at most 16 instances per warp
+(the mix bucket), the engine uses 8 times the grain (at most 32), 4 levels more
+(at most 8) and a sixteenth of the interval.  The fastest point by device time is kept,
 and the winners per bucket are stored in td16_b200/tuned.json.  `apply(N)`
 configures the engine for a bucket.
 

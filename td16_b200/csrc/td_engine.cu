@@ -365,11 +365,20 @@ __global__ void __launch_bounds__(256, 4) td_ordered_kernel(const td_instance *_
     }
 }
 
-// Resident grid with work donation (free move order).  Warps take fresh
-// instances by ticket; a warp that finds neither tickets nor items counts
-// itself idle, and busy warps then hand the remaining children of their
-// shallowest DFS level to the item array.  Every wait is bounded by the
-// launch deadline; the launch ends when no ticket, item or unit is left.
+// Records the first error of a search.
+__device__ __forceinline__ void td_note_error(td_inst_state *st, int err) {
+    atomicCAS(reinterpret_cast<unsigned short *>(&st->error), (unsigned short)0, (unsigned short)err);
+}
+
+// HOST_OUT: `out` is host memory mapped into the device (the serving loop), so
+// the fences are system-scope; the batch engine's results are device memory,
+// where device-scope fences order the same writes at a fraction of the cost.
+template <bool HOST_OUT>
+__device__ __forceinline__ void td_unit_fence() {
+    if (HOST_OUT) __threadfence_system();
+    else td_fence();
+}
+
 // Ends one unit of a shared search: records a found witness (first finder
 // wins), and the unit that finishes the search last writes the final status
 // and the summed expansions.  Returns 1 in the warp that finished last.
@@ -380,20 +389,6 @@ __global__ void __launch_bounds__(256, 4) td_ordered_kernel(const td_instance *_
 // was searched: the instance has no witness within the bound, and found = 2
 // stops the inverse's side.  The inverse's side never decides "no witness":
 // the filter applies to a different tree there.
-// HOST_OUT: `out` is host memory mapped into the device (the serving loop), so
-// the fences are system-scope; the batch engine's results are device memory,
-// where device-scope fences order the same writes at a fraction of the cost.
-// Records the first error of a search.
-__device__ __forceinline__ void td_note_error(td_inst_state *st, int err) {
-    atomicCAS(reinterpret_cast<unsigned short *>(&st->error), (unsigned short)0, (unsigned short)err);
-}
-
-template <bool HOST_OUT>
-__device__ __forceinline__ void td_unit_fence() {
-    if (HOST_OUT) __threadfence_system();
-    else td_fence();
-}
-
 template <bool HOST_OUT>
 __device__ __forceinline__ int td_finish_unit(const td_dfs_out &r, td_inst_state *st, td_result *out,
                                               const uint16_t *path, int side, int gave) {
@@ -453,6 +448,11 @@ __device__ __forceinline__ int td_finish_unit(const td_dfs_out &r, td_inst_state
 #ifndef TD_STEAL_MIN_BLOCKS
 #define TD_STEAL_MIN_BLOCKS 4  // resident blocks of 8 warps per SM the register budget is sized for
 #endif
+// Resident grid with work donation (free move order).  Warps take fresh
+// instances by ticket, then items (td_claims): while item tickets run ahead of
+// the items produced, busy warps hand the remaining children of their
+// shallowest DFS level to the item array.  Every wait is bounded by the launch
+// deadline; the launch ends when no ticket, item or unit is left.
 __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(const td_instance *__restrict__ in,
                                                       td_result *__restrict__ out, int count, td_pool *pool,
                                                       td_item *items, uint32_t *ready, const td_epoch *ep,
@@ -700,13 +700,12 @@ __global__ void __launch_bounds__(256) td_count_kernel(const td_result *__restri
     }
 }
 
-// Witness replay in pinned form with the search's own rules: every move is an
-// in-range position triple i<j<k whose symbols omega does not fix and whose
-// odd-cycle change is 0 or +2 (sorting_search.cu:375-380,608-610), there are
-// at most max_moves of them, and the last node passes the acceptance test of
-// the instance (satisfies_rate, sorting_search.cu:336-346: with full sorting,
-// omega = id).  With full sorting this is CertificateValidator's replay
-// (CertificateValidator.java:14-50) in pinned form.
+// Witness replay in pinned form, the rule of td_witness_ok: every move is an
+// in-range position triple i<j<k, there are at most max_moves of them, and the
+// last node passes the acceptance test of the instance (satisfies_rate,
+// sorting_search.cu:336-346: with full sorting, omega = id).  With full sorting
+// this is CertificateValidator's replay (CertificateValidator.java:14-50) in
+// pinned form plus the rate test.  The search's move filter is not part of it.
 // One thread per instance, 16-byte loads where the buffers allow them.  With full sorting
 // the witness holds when the pinned state ends sorted and the last move's depth
 // passes the rate test, and the moves are taken from registers in an unrolled
@@ -961,7 +960,7 @@ int g_serve_split_level = 2;
 int g_serve_check_every = 32;
 int g_tt_bits = TD_TT_BITS;  // log2 entries of the explored-state tables; 0 = no table
 uint32_t g_restart_base = TD_RESTART_BASE;  // free-order restart budget base; 0 = no restarts
-int g_split_budget = TD_SPLIT_BUDGET;       // reference order: first-pass expansions before a split; 0 = none
+int g_split_budget = TD_SPLIT_BUDGET;       // reference order: expansions of a walk before a split; 0 = none
 int g_split_records = TD_SPLIT_RECORDS;     // reference order: subtree records per launch
 int g_race = 8;  // free-order batches: attempt at which a search starts racing its inverse, 0 = off (td_configure_race)
 
@@ -1287,7 +1286,7 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
     } else {
         const int grid_max = cfg.sms * cfg.blocks_per_sm;
         const int grid = std::max(1, std::min(grid_max, (count + warps - 1) / warps));
-        if (ordered && max_exp == 0 && cfg.split_budget > 0) {
+        if (max_exp == 0 && cfg.split_budget > 0) {
             // stream-ordered buffers; the flags start at zero, epochs at 1
             if (s.d_split_pool == nullptr) {
                 TD_CHECK(cudaMallocAsync(&s.d_split_pool, TD_SPLIT_HEAD, stream));
@@ -1662,7 +1661,10 @@ TD_API int td_set_time_limit(double seconds) {
 }
 
 // Work-donation parameters of the free-order engine: items per donation,
-// deepest level whose children may be donated, expansions between checks.
+// deepest level whose children may be donated, expansions between checks.  They
+// hold while every warp has an instance of its own; from the first idle warps
+// on, and from the start in launches of few instances per warp,
+// td_serve_idle_warps derives sharper ones from them.
 TD_API int td_configure_steal(int grain, int split_level, int check_every) {
     if (grain < 1 || split_level < 0 || split_level >= TD_MAX_DEPTH || check_every < 1) return TD_INVALID_ARG;
     std::lock_guard<std::mutex> g(g_mu);
@@ -1682,13 +1684,9 @@ TD_API int td_configure_table(int bits) {
     return TD_OK;
 }
 
-// Restarts of later free-order batch searches: a search that has spent
-// base x luby(a) expansions in attempt a starts again with another child order
-// (td_attempt_budget, td_order_variant); 0 turns restarts off.  Verdicts do
-// not depend on it.
-// The split pass of reference-order batches: expansions of the one-warp first
-// pass (0: no split, every walk on one warp) and subtree records per launch
-// (a root whose children find no room runs whole).  Results do not depend on
+// Walks of reference-order batches: the expansions after which one may give
+// subtrees away (0: never, every walk on one warp) and the subtree records per
+// launch (a walk that finds no room goes on whole).  Results do not depend on
 // either.
 TD_API int td_configure_split(int first_pass_expansions, int records) {
     if (first_pass_expansions < 0 || records < 1 || records > (1 << 24)) return TD_INVALID_ARG;
@@ -1698,6 +1696,10 @@ TD_API int td_configure_split(int first_pass_expansions, int records) {
     return TD_OK;
 }
 
+// Restarts of later free-order batch searches: a search that has spent
+// base x luby(a) expansions in attempt a starts again with another child order
+// (td_attempt_budget, td_order_variant); 0 turns restarts off.  Verdicts do
+// not depend on it.
 TD_API int td_configure_restart(int base) {
     if (base < 0 || (base > 0 && base < 16)) return TD_INVALID_ARG;
     std::lock_guard<std::mutex> g(g_mu);
@@ -2061,9 +2063,10 @@ TD_API int td_int_issue_peak(int device, float target_ms, double *issue_per_s, d
 // their own streams, or a host process whose device memory is already held by
 // another allocator, so that a new allocation would fail although the caller's
 // buffers exist.  The caller passes device buffers for instances and results;
-// every other byte the search needs lives in td_noalloc_scratch below, a
-// fixed array that each GPU loading this library holds until the process
-// exits.  Limits: TD_NOALLOC_MAX_INSTANCES instances per call and
+// every other byte the search needs lives in td_noalloc_scratch below and in
+// the tables that every search reads (td_eg_table, 8 MiB, is the largest), fixed
+// arrays that each GPU loading this library holds until the process exits.
+// Limits: TD_NOALLOC_MAX_INSTANCES instances per call and
 // TD_NOALLOC_ITEMS donated subtrees in flight (when the item space is full the
 // donor keeps the work, so a full item space only costs balance, not results).
 // All calls share this one array and it keeps the last call's contents, so
@@ -2148,9 +2151,11 @@ int noalloc_setup(int device, char *err, size_t errlen) {
 // device memory.  d_instances / d_results: caller-owned device buffers of
 // `count` records; flags as for td_search_batch_device (TD_FLAG_ORDERED,
 // TD_FLAG_PLAIN, TD_FLAG_VERIFY).  Enqueues on `stream` and returns.  The
-// first call on a device performs the one-time set-up above (table uploads
-// and a symbol-address query, both synchronous), so make that first call
-// before any stream capture.  count > 65536 is rejected.
+// first call on a device performs the one-time set-up above unless slots were
+// made there before (a symbol-address query, and on a stream of its own the
+// table uploads and the five launches that build the endgame table, about 5 ms,
+// waited for), so make that first call before any stream capture.  count > 65536
+// is rejected.
 TD_API int td_search_batch_noalloc(int count, const td_instance *d_instances, td_result *d_results, unsigned flags,
                                    uint64_t max_exp, void *stream, char *err, size_t errlen) {
     if (count < 0 || count > TD_NOALLOC_MAX_INSTANCES)

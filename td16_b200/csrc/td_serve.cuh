@@ -273,8 +273,7 @@ __global__ void __launch_bounds__(256, 3) td_serve_kernel(const td_instance *rin
                 }
             } else {
                 if (MODE == TD_SERVE_PER_REQUEST) ord = (x.packed & TD_PACKED_ORDERED) != 0;
-                if (ord) td_setup_root(s, x);
-                else td_setup_root(s, x);
+                td_setup_root(s, x);
                 run = true;
             }
         } else {
