@@ -503,9 +503,14 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
         // costs more than doing it too often.  With up to 16 instances a warp
         // the settings for idle warps hold from the start (only with fewer
         // instances than warps before: 20,011 S_12..S_14 2.13 -> 1.49 ms, 2^16
-        // mixed 1.69 -> 1.32, 8,000 S_13 1.16 -> 0.82).  With 21 (10^5 uniform
-        // S_16) they took 0.79 ms, and 0.75 without: there the loads of the
-        // idle checks are work that nothing waits for.
+        // mixed 1.69 -> 1.32, 8,000 S_13 1.16 -> 0.82).  Without them and with
+        // them, at 8, 16, 20 and 32 instances a warp: near-reverse S_16 2.22/2.01,
+        // 3.32/3.16, 3.90/3.75 and 5.88/5.72 ms, the mix of S_11..S_13 1.28/0.93,
+        // 1.78/1.29, 2.15/1.57 and 2.92/2.35, uniform S_16 0.35/0.36, 0.56/0.59,
+        // 0.73/0.70 and 1.11/1.10.  So the line is not where the two cross: it
+        // was drawn at 10^5 uniform S_16, 21 a warp in 8-warp blocks, where the
+        // loads of the idle checks are work that nothing waits for (0.79 ms
+        // against 0.75), and uneven batches above it would still gain.
         // An expansion budget bounds each unit, so sharing multiplies it: where it
         // ends before a search's first look at the idle warps, nothing is shared
         // and it bounds the instance (16 expansions each, 4,096 of S_8..S_13:
