@@ -938,6 +938,10 @@ struct Slot {
         td_pool pool;
     } *h_stats = nullptr;
     int slots_on_device = 1;
+    // a batch was captured: buffers that a launch uses stay where they are until
+    // the slot goes, and those they outgrew wait in `kept`
+    bool captured = false;
+    std::vector<void *> kept;
     std::mutex *mu = nullptr;
 };
 
@@ -1164,6 +1168,7 @@ void release_slot(Slot &s) {
     if (s.d_nodes) cudaFree(s.d_nodes);
     if (s.d_split_records) cudaFree(s.d_split_records);
     if (s.d_split_items) cudaFree(s.d_split_items);
+    for (void *p : s.kept) cudaFree(p);
     if (s.d_counts) cudaFree(s.d_counts);
     if (s.h_stats) cudaFreeHost(s.h_stats);
     if (s.h_inst) cudaFreeHost(s.h_inst);
@@ -1209,6 +1214,22 @@ cudaError_t launch_after(void (*kernel)(P...), int grid, int threads, size_t sme
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Gives a launch buffer that is outgrown back, in stream order (a cudaFree would
+// wait for all work on the device, the per-call server's resident launch
+// included), or keeps it for the captured launches that hold its address.
+template <typename T>
+cudaError_t outgrown(Slot &s, T *&p, cudaStream_t stream) {
+    cudaError_t e = cudaSuccess;
+    if (p && s.captured) s.kept.push_back(p);
+    else if (p) e = cudaFreeAsync(p, stream);
+    p = nullptr;
+    return e;
+}
+
+// The size a launch buffer grows to: what is needed, and once old ones are kept
+// at least twice the last, so that they hold no more than it does.
+size_t grown(const Slot &s, size_t needed, size_t last) { return s.captured ? std::max(needed, 2 * last) : needed; }
+
 // Launch one batch on `stream`.  Instances and results are device pointers.
 int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, unsigned flags,
                  uint64_t max_exp, cudaStream_t stream, char *err, size_t errlen) {
@@ -1242,14 +1263,12 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
             TD_CHECK(cudaMemsetAsync(s.d_ready, 0, cap * sizeof(uint32_t), stream));
             s.item_capacity = (int)cap;
         }
-        // buffers grow in stream order: a cudaFree would wait for all work on
-        // the device, the per-call server's resident launch included
         if ((size_t)count > s.state_count) {
-            if (s.d_state) TD_CHECK(cudaFreeAsync(s.d_state, stream));
-            s.d_state = nullptr;
+            const size_t n = grown(s, (size_t)count, s.state_count);
+            TD_CHECK(outgrown(s, s.d_state, stream));
             s.state_count = 0;
-            TD_CHECK(cudaMallocAsync(&s.d_state, (size_t)count * sizeof(td_inst_state), stream));
-            s.state_count = (size_t)count;
+            TD_CHECK(cudaMallocAsync(&s.d_state, n * sizeof(td_inst_state), stream));
+            s.state_count = n;
         }
         // at least the slot's share of the resident grid, so that a small batch
         // (one search from td_search) is spread over that many warps by donation,
@@ -1266,11 +1285,11 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
         const int64_t wanted = ((int64_t)count * TD_INSTANCE_WARPS + warps - 1) / warps;
         const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(resident, std::max<int64_t>(share, wanted)));
         const int tt_log2 = tt_entries_log2((size_t)resident * warps, cfg.tt_bits);
-        if (cfg.tt_bits > 0 && (tt_log2 > s.tt_log2 || cfg.tt_bits != s.tt_bits)) {
-            // sized for the whole resident grid so that it never moves under a
-            // captured graph; replaced in stream order after the previous launch
-            if (s.d_tt) TD_CHECK(cudaFreeAsync(s.d_tt, stream));
-            s.d_tt = nullptr;
+        if (cfg.tt_bits > 0 && (tt_log2 > s.tt_log2 || (cfg.tt_bits != s.tt_bits && !s.captured))) {
+            // sized for the whole resident grid; replaced in stream order after the
+            // previous launch (a captured launch keeps it, and then a smaller
+            // setting keeps the larger table)
+            TD_CHECK(outgrown(s, s.d_tt, stream));
             s.tt_log2 = 0;
             TD_CHECK(cudaMallocAsync(&s.d_tt, sizeof(ulonglong2) << tt_log2, stream));
             TD_CHECK(cudaMemsetAsync(s.d_tt, 0, sizeof(ulonglong2) << tt_log2, stream));  // zero words are empty
@@ -1303,22 +1322,18 @@ int launch_batch(Slot &s, int count, const td_instance *d_in, td_result *d_out, 
             td_epoch_kernel<<<1, 1, 0, stream>>>(epoch, 1u, s.d_split_pool, count, node_count, 2, s.d_split_ready,
                                                  s.split_records, nullptr, 0);
             if (cfg.split_records > s.split_records) {
-                if (s.d_split_ready) TD_CHECK(cudaFreeAsync(s.d_split_ready, stream));
-                if (s.d_nodes) TD_CHECK(cudaFreeAsync(s.d_nodes, stream));
-                if (s.d_split_items) TD_CHECK(cudaFreeAsync(s.d_split_items, stream));
-                if (s.d_split_records) TD_CHECK(cudaFreeAsync(s.d_split_records, stream));
-                s.d_split_ready = nullptr;
-                s.d_nodes = nullptr;
-                s.d_split_items = nullptr;
-                s.d_split_records = nullptr;
+                const size_t n = grown(s, (size_t)cfg.split_records, (size_t)s.split_records);
+                TD_CHECK(outgrown(s, s.d_split_ready, stream));
+                TD_CHECK(outgrown(s, s.d_nodes, stream));
+                TD_CHECK(outgrown(s, s.d_split_items, stream));
+                TD_CHECK(outgrown(s, s.d_split_records, stream));
                 s.split_records = 0;
-                const size_t n = (size_t)cfg.split_records;
                 TD_CHECK(cudaMallocAsync(&s.d_split_ready, sizeof(uint32_t) * n, stream));
-                TD_CHECK(cudaMallocAsync(&s.d_nodes, sizeof(td_split_node) * split_nodes(cfg.split_records), stream));
+                TD_CHECK(cudaMallocAsync(&s.d_nodes, sizeof(td_split_node) * split_nodes((int)n), stream));
                 TD_CHECK(cudaMallocAsync(&s.d_split_items, sizeof(td_split_item) * n, stream));
                 TD_CHECK(cudaMallocAsync(&s.d_split_records, sizeof(td_result) * n, stream));
                 TD_CHECK(cudaMemsetAsync(s.d_split_ready, 0, sizeof(uint32_t) * n, stream));
-                s.split_records = cfg.split_records;
+                s.split_records = (int)n;
             }
             td_split_space sp;
             sp.nodes = s.d_nodes;
@@ -2267,6 +2282,7 @@ TD_API int td_batch_graph_create(int slot, int count, const td_instance *d_in, t
     int rc = launch_batch(*s, count, d_in, d_out, flags, max_exp, s->stream, err, errlen);
     if (rc != TD_OK) return rc;
     TD_CHECK(cudaStreamSynchronize(s->stream));
+    s->captured = true;
     auto *bg = new BatchGraph();
     bg->device = s->device;
     cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);

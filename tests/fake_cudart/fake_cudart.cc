@@ -110,9 +110,21 @@ FAKE cudaError_t cudaMalloc(void **p, size_t n) {
     *p = std::calloc(1, n);
     return cudaSuccess;
 }
-FAKE cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) { *p = std::calloc(1, n); return cudaSuccess; }
-FAKE cudaError_t cudaFree(void *p) { std::free(p); return cudaSuccess; }
-FAKE cudaError_t cudaFreeAsync(void *p, cudaStream_t) { std::free(p); return cudaSuccess; }
+FAKE cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) {
+    *p = std::calloc(1, n);
+    say("mallocasync %p %zu", *p, n);
+    return cudaSuccess;
+}
+FAKE cudaError_t cudaFree(void *p) {
+    say("free %p", p);
+    std::free(p);
+    return cudaSuccess;
+}
+FAKE cudaError_t cudaFreeAsync(void *p, cudaStream_t) {
+    say("free %p", p);
+    std::free(p);
+    return cudaSuccess;
+}
 FAKE cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
     say("hostalloc %zu", n);
     *p = std::calloc(1, n);
@@ -151,7 +163,10 @@ FAKE cudaError_t cudaStreamSynchronize(cudaStream_t s) {
     say("synchronize stream %zx", (size_t)s);
     return cudaSuccess;
 }
-FAKE cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
+FAKE cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
+    say("capture");
+    return cudaSuccess;
+}
 FAKE cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) { return handle(g); }
 FAKE cudaError_t cudaEventCreate(cudaEvent_t *e) { return handle(e); }
 FAKE cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned flags) {

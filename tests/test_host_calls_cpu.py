@@ -97,3 +97,40 @@ td._lib.search_pairs(0, pair, pair, 17, 1, 0.0, 9, 1)
     lines = lines[[i for i, line in enumerate(lines) if "td_pairs_unpack" in line][0]:]
     assert "wait event blocking" not in lines
     assert lines[1].startswith(("synchronize stream", "wait event spinning"))
+
+
+@pytest.mark.parametrize("flags", [0, 1])
+def test_captured_launches_keep_their_buffers(calls, flags):
+    """Batches that outgrow what a captured launch was given: its buffers are freed
+    with the slot and not before, and what is kept for it is bounded by what the
+    slot holds anyway."""
+    lines = calls(INIT + f"""
+import ctypes as C
+buf = (C.c_uint8 * (1 << 20))()
+at = C.addressof(buf)
+g = td._lib.BatchGraph(0, 10, at, at, {flags})
+for count in range(20, 2000, 20):
+    td._lib.search_batch_device(0, count, at, at, {flags})
+    td._lib.configure_split(64, (1 << 20) + count)
+    td._lib.configure_table(6 + count % 7)
+g.launch()
+g.close()
+import os
+open(os.environ["FAKE_CUDART_LOG"], "a").write("destroy\\n")
+td.destroy()
+""")
+    start, end = lines.index("capture"), lines.index("destroy")
+    live, freed_early = {}, []
+    for i, line in enumerate(lines):
+        what, *rest = line.split()
+        if what == "mallocasync":
+            live[rest[0]] = int(rest[1])
+        elif what == "free" and rest[0] in live:
+            if start < i < end:
+                freed_early.append(rest[0])
+            del live[rest[0]]
+        if i == end:
+            held = sum(live.values())
+    assert not freed_early
+    assert not live  # the slot gives everything back
+    assert held <= (420 << 20)
