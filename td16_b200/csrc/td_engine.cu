@@ -625,6 +625,13 @@ __global__ void __launch_bounds__(256, TD_STEAL_MIN_BLOCKS) td_steal_kernel(cons
     }
 }
 
+// Clears the items' flags and the table (td_epoch_kernel; called, so that the
+// kernel, which every launch waits for, stays as short as it is without it).
+__device__ __noinline__ void td_clear_tags(uint32_t *ready, int n_ready, ulonglong2 *tt, size_t n_tt) {
+    for (int i = 0; i < n_ready; ++i) ready[i] = 0;
+    for (size_t i = 0; i < n_tt; ++i) tt[i] = make_ulonglong2(0ull, 0ull);
+}
+
 // The first operation of a launch: sets its counters, and its deadline counts
 // from here, so that it holds for the growth of the launch's buffers too.
 // Advances the launch epoch that tags donated items as written; a launch
@@ -638,10 +645,7 @@ __global__ void td_epoch_kernel(td_epoch *ep, unsigned epochs, td_pool *pool, in
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     int again;
     ep->epoch = td_next_epoch(ep->epoch, epochs, &again);
-    if (again) {
-        for (int i = 0; i < n_ready; ++i) ready[i] = 0;
-        for (size_t i = 0; i < n_tt; ++i) tt[i] = make_ulonglong2(0ull, 0ull);
-    }
+    if (again) td_clear_tags(ready, n_ready, tt, n_tt);
     ep->start_ns = td_globaltimer();
     td_pool p;
     memset(&p, 0, sizeof p);
